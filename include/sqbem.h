@@ -139,6 +139,12 @@ int sqbem_solve_dense(int n, int nrhs, const double* A, double* B, int* pivoted)
  * Relative accuracy about 2^-16 per product. */
 int sqbem_gemm_mixed(int M, int N, int K, float alpha, const float* A, int lda, const float* B, int ldb,
                      float beta, float* C, int ldc);
+/* gemm, src/utils/linalg.hpp:42-48, in the form the SQBEM_FP64 path uses: C = alpha
+ * op(A) op(B) + beta C in FP64 for column-major host arrays (op(A): M x K, op(B): K x
+ * N; ta, tb: transposed).  route -1: the path's own choice, 0: the FP64 pipe, 1: digit
+ * products on the tensor cores (K >= 1). */
+int sqbem_gemm64(int route, int ta, int tb, int M, int N, int K, double alpha, const double* A, int lda,
+                 const double* B, int ldb, double beta, double* C, int ldc);
 /* The same with the kernel's tile variant chosen by the caller (-1: the one
  * the tuning table gives for the shape; see sqbem_gemm_variants) and 3
  * products (hi*hi + hi*lo + lo*hi) or 2 (hi*hi + hi*lo: A rounded to BF16,

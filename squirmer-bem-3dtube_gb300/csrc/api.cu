@@ -16,6 +16,7 @@
 #include "bem/utils/mesh.hpp"
 #include "common.cuh"
 #include "dense.cuh"
+#include "oz_gemm.cuh"
 #include "solver.cuh"
 
 namespace sqbem {
@@ -280,10 +281,42 @@ extern "C" int sqbem_solve_dense(int n, int nrhs, const double* A, double* B, in
         if (nrhs) dB.upload(B, (size_t)n * nrhs);
         LU64 lu;
         lu.factor_inplace(std::move(dA), n, s, "dgesv failed");
-        lu.solve(dB.get(), n, nrhs, s);
+        WaitError we;
+        lu.solve(dB.get(), n, nrhs, s, we.get(s));
+        we.check();
         if (nrhs) dB.download(B, (size_t)n * nrhs);
         CUDA_CHECK(cudaStreamSynchronize(s));
         if (pivoted) *pivoted = lu.pivoted ? 1 : 0;
+    });
+}
+
+extern "C" int sqbem_gemm64(int route, int ta, int tb, int M, int N, int K, double alpha, const double* A, int lda,
+                            const double* B, int ldb, double beta, double* C, int ldc) {
+    return guarded([&] {
+        const int ca = ta ? M : K, cb = tb ? K : N;
+        if (route < -1 || route > 1 || M < 0 || N < 0 || K <= 0 || !A || !B || !C || lda < (ta ? K : M) ||
+            ldb < (tb ? N : K) || ldc < M)
+            fail(SQBEM_ERR_ARG, "gemm64: bad arguments");
+        if (M == 0 || N == 0) return;
+        require_device();
+        Stream s;
+        DevBuf<double> dA((size_t)lda * ca, s), dB((size_t)ldb * cb, s), dC((size_t)ldc * N, s);
+        dA.upload(A, (size_t)lda * ca);
+        dB.upload(B, (size_t)ldb * cb);
+        dC.upload(C, (size_t)ldc * N);
+        WaitError we;
+        if (route == 1) {
+            OzMat a, b;
+            a.split(dA.get(), ta ? lda : 1, ta ? 1 : lda, M, K, s);
+            b.split(dB.get(), tb ? 1 : ldb, tb ? ldb : 1, N, K, s);
+            oz_gemm(a, b, alpha, beta, dC.get(), ldc, we.get(s), s);
+        } else {
+            gemm64(ta, tb, M, N, K, alpha, dA.get(), lda, dB.get(), ldb, beta, dC.get(), ldc, s,
+                   route == 0 ? nullptr : we.get(s));
+        }
+        dC.download(C, (size_t)ldc * N);
+        CUDA_CHECK(cudaStreamSynchronize(s));
+        we.check();
     });
 }
 

@@ -24,11 +24,22 @@
 
 namespace sqbem {
 
-constexpr int LU_NB = 64;  // panel width of the blocked LU (FP64)
+constexpr int LU_NB = 256;  // panel width of the blocked LU (FP64)
 
-// C(MxN) = alpha * op(A) * op(B) + beta * C   (column-major, FP64)
+// The word that a bounded wait of the tensor-core products sets when it runs out, for the
+// calls of one stream.
+struct WaitError {
+    DevBuf<int> w;
+    int* get(cudaStream_t st);  // the word, zeroed at first use
+    void check();               // waits for the stream; SQBEM_ERR_TIMEOUT if a wait ran out
+};
+
+// C(MxN) = alpha * op(A) * op(B) + beta * C   (column-major, FP64).  With err (a
+// WaitError's word, checked by the caller) large products run as digit products on the
+// tensor cores (oz_gemm.cuh); C must not overlap A or B.
 void gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const double* A, long long lda,
-            const double* B, long long ldb, double beta, double* C, long long ldc, cudaStream_t st);
+            const double* B, long long ldb, double beta, double* C, long long ldc, cudaStream_t st,
+            int* err = nullptr);
 
 // LU factorisation (dgetrf semantics) of an n x n column-major matrix, kept on
 // the device with the inverses of its diagonal blocks (used by the solves).
@@ -46,8 +57,8 @@ struct LU64 {
     void factor(const double* M, int n, long long ld, cudaStream_t st, const char* what);
     // Take ownership of a device buffer (n x n, leading dimension n) and factor it in place.
     void factor_inplace(DevBuf<double>&& M, int n, cudaStream_t st, const char* what);
-    // B <- A^{-1} B for B (n x nrhs, leading dimension ldb, device)
-    void solve(double* B, long long ldb, int nrhs, cudaStream_t st) const;
+    // B <- A^{-1} B for B (n x nrhs, leading dimension ldb, device); err as in gemm64
+    void solve(double* B, long long ldb, int nrhs, cudaStream_t st, int* err = nullptr) const;
     // B <- A^{-T} B (dgetrs 'T'): U^T then L^T solves, then the row exchanges undone
     void solve_transpose(double* B, long long ldb, int nrhs, cudaStream_t st) const;
 };

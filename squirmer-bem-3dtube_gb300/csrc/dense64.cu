@@ -2,9 +2,10 @@
 // pivoting fallback, and blocked LU solves (the SQBEM_FP64 path; replaces the
 // reference's dgemm_/dgetrf_/dgetrs_/dgesv_, src/utils/linalg.hpp:17-78).
 //
-// GB300 executes FP64 at roughly 1 TFLOP/s (CUDA-core DFMA and DMMA alike), so
-// these kernels are register-tiled DFMA loops sized to keep that pipe busy; the
-// fast path of the solver is the mixed-precision tensor-core code (tc_gemm.cu).
+// GB300 executes FP64 at roughly 1 TFLOP/s (CUDA-core DFMA and DMMA alike).  Large
+// products therefore run as digit products on the BF16 tensor cores with FP64
+// results (oz_gemm.cu); what stays on the FP64 pipe is the work around them: the
+// 128-wide panels of the LU, and products with a few columns.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -12,6 +13,7 @@
 
 #include "common.cuh"
 #include "dense.cuh"
+#include "oz_gemm.cuh"
 
 namespace sqbem {
 
@@ -81,13 +83,118 @@ __global__ void __launch_bounds__(256) dgemm_kernel(int M, int N, int K, double 
     }
 }
 
+// Products with up to 8 columns (right-hand sides).  Reading A is the work: 8 bytes
+// per 2 n FP64 operations, so above n = 2 the FP64 pipe bounds it.  The 64 x 64
+// tiles above put such a product on a handful of CTAs, each walking all of K.
+constexpr int SK_N = 8;
+
+// C = alpha A B + beta C, A column-major: 32 rows per CTA, 8 warps split K, each
+// lane one row (a column's 32 rows are one 256-byte read).
+template <int N>
+__global__ void __launch_bounds__(256) skinny_n_kernel(int M, int K, double alpha, const double* __restrict__ A,
+                                                       long long lda, const double* __restrict__ B, long long ldb,
+                                                       double beta, double* __restrict__ C, long long ldc) {
+    __shared__ double part[8][N][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int m = blockIdx.x * 32 + lane;
+    double acc[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) acc[j] = 0.0;
+    if (m < M) {
+#pragma unroll 8
+        for (int k = w; k < K; k += 8) {
+            const double a = A[m + k * lda];
+#pragma unroll
+            for (int j = 0; j < N; ++j) acc[j] = fma(a, B[k + j * ldb], acc[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) part[w][j][lane] = acc[j];
+    __syncthreads();
+    if (m >= M) return;
+    for (int j = w; j < N; j += 8) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s += part[q][j][lane];
+        double* c = C + m + j * ldc;
+        *c = beta == 0.0 ? alpha * s : fma(alpha, s, beta * *c);
+    }
+}
+
+// C = alpha A^T B + beta C: a warp per row of C, the lanes along K (contiguous in A).
+template <int N>
+__global__ void __launch_bounds__(256) skinny_t_kernel(int M, int K, double alpha, const double* __restrict__ A,
+                                                       long long lda, const double* __restrict__ B, long long ldb,
+                                                       double beta, double* __restrict__ C, long long ldc) {
+    const int lane = threadIdx.x & 31, m = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (m >= M) return;
+    double acc[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) acc[j] = 0.0;
+    const double* a = A + m * lda;
+#pragma unroll 4
+    for (int k = lane; k < K; k += 32) {
+        const double x = a[k];
+#pragma unroll
+        for (int j = 0; j < N; ++j) acc[j] = fma(x, B[k + j * ldb], acc[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+        if (lane == j) {
+            double* c = C + m + j * ldc;
+            *c = beta == 0.0 ? alpha * acc[j] : fma(alpha, acc[j], beta * *c);
+        }
+}
+
+template <int N>
+static void skinny(bool ta, int M, int K, double alpha, const double* A, long long lda, const double* B, long long ldb,
+                   double beta, double* C, long long ldc, cudaStream_t st) {
+    const double fl = 2.0 * M * N * K, by = 8.0 * ((double)M * K + (double)K * N + (beta == 0.0 ? 1.0 : 2.0) * M * N);
+    if (ta)
+        TIMED_LAUNCH("dgemm", fl, by, skinny_t_kernel<N>, ceil_div(M, 8), 256, 0, st, M, K, alpha, A, lda, B, ldb, beta,
+                     C, ldc);
+    else
+        TIMED_LAUNCH("dgemm", fl, by, skinny_n_kernel<N>, ceil_div(M, 32), 256, 0, st, M, K, alpha, A, lda, B, ldb, beta,
+                     C, ldc);
+}
+
+// The digit products need about 60 us whatever the size (two splits, a tile's 36
+// products and read-outs), in which the FP64 pipe does 6e7 operations; and a tile of
+// 128 x 128 with a K below 64 costs more to read out than to multiply.
+static bool use_tensor(int M, int N, int K, const int* err) {
+    return err && K >= 64 && M >= 64 && N >= 64 && 2.0 * M * N * K > 6e7;
+}
+
 void gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const double* A, long long lda, const double* B,
-            long long ldb, double beta, double* C, long long ldc, cudaStream_t st) {
+            long long ldb, double beta, double* C, long long ldc, cudaStream_t st, int* err) {
     if (M <= 0 || N <= 0) return;
     if (K <= 0) {
         // C = beta C
         if (beta == 1.0) return;
         K = 0;
+    }
+    if (N <= SK_N && !tb) {
+        switch (N) {
+            case 1: return skinny<1>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
+            case 2: return skinny<2>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
+            case 3: return skinny<3>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
+            case 4: return skinny<4>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
+            case 5: return skinny<5>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
+            case 6: return skinny<6>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
+            case 7: return skinny<7>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
+            default: return skinny<8>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
+        }
+    }
+    if (use_tensor(M, N, K, err)) {
+        OzMat a, b;
+        a.split(A, ta ? lda : 1, ta ? 1 : lda, M, K, st);
+        b.split(B, tb ? 1 : ldb, tb ? ldb : 1, N, K, st);
+        oz_gemm(a, b, alpha, beta, C, ldc, err, st);
+        return;
     }
     dim3 grid(ceil_div(M, GB_M), ceil_div(N, GB_N));
     const double fl = 2.0 * M * N * K;
@@ -104,6 +211,22 @@ void gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const double* A
     else
         TIMED_LAUNCH("dgemm", fl, by, (dgemm_kernel<true, true>), grid, 256, 0, st, M, N, K, alpha, A, lda, B, ldb,
                      beta, C, ldc);
+}
+
+void WaitError::check() {
+    if (!w.get()) return;
+    int h = 0;
+    w.download(&h, 1);
+    CUDA_CHECK(cudaStreamSynchronize(w.st));
+    if (h) fail(SQBEM_ERR_TIMEOUT, "a bounded wait in the FP64 tensor-core product expired");
+}
+
+int* WaitError::get(cudaStream_t st) {
+    if (!w.get()) {
+        w.alloc(1, st);
+        w.zero();
+    }
+    return w.get();
 }
 
 // ---------------------------------------------------------------- small helpers
@@ -144,84 +267,252 @@ void max_abs64(const double* A, long long lda, int rows, int cols, double* out, 
            out);
 }
 
-// copy W (rows x cols, ld rows) into A and flag |entry| > 1 (bit 0) or a
-// non-finite entry (bit 1)
-__global__ void copy_check_kernel(const double* __restrict__ W, double* __restrict__ A, long long lda, int rows,
-                                  int cols, int* flag) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)rows * cols) return;
-    const int r = (int)(t % rows), c = (int)(t / rows);
-    const double v = W[t];
-    A[r + c * lda] = v;
-    if (!(fabs(v) <= 1.0)) atomicOr(flag, isfinite(v) ? 1 : 2);
+// ---------------------------------------------------------------- panels of the LU
+// A panel of HB = 128 columns is factored in steps of PB = 32 columns:
+//   diag      the 32 x 32 diagonal block (one CTA);
+//   trsm32    below it L21 = A21 U11^{-1}, right of it U12 = L11^{-1} A12 within
+//             the panel, 32 rows or columns per CTA;
+//   update32  the rest of the panel, A22 -= L21 U12; the CTA of the next diagonal
+//             block updates only that block and factors it at once.
+// All of it is bound by the FP64 pipe of the SMs it is spread over (1.7 FMA per clock
+// and SM) and its latency, hence the small blocks and short CTAs.
+constexpr int PB = 32, HB = 128;
+
+// 1/x by Newton's iteration y <- y + y (1 - x y) from an FP32 reciprocal of the
+// significand (relative error 2^-23, 2^-46, then FP64 rounding); four dependent FMAs
+// where the full division is on the factorisation's serial chain.
+__device__ __forceinline__ double recip(double x) {
+    const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+    if (e < 64 || e > 1980) return 1.0 / x;
+    const double m = __hiloint2double((hi & 0x800fffff) | 0x3ff00000, __double2loint(x));
+    double y = (double)(1.0f / (float)m);
+    y = fma(y, fma(-m, y, 1.0), y);
+    y = fma(y, fma(-m, y, 1.0), y);
+    return __hiloint2double(__double2hiint(y) + ((1023 - e) << 20), __double2loint(y));
 }
 
-// ---------------------------------------------------------------- diagonal blocks
-// Inverses of the unit-lower and upper triangles of the kb x kb block a (shared,
-// row stride LU_NB + 1), written column-major with leading dimension LU_NB.
-__device__ void block_inverses(const double (*a)[LU_NB + 1], int kb, double* Linv, double* Uinv) {
-    const int c = threadIdx.x;
-    if (c < kb) {
-        // column c of L^{-1}: X(c,c) = 1, X(i,c) = -sum_{k=c}^{i-1} L(i,k) X(k,c)
-        for (int i = 0; i < LU_NB; ++i) Linv[i + c * LU_NB] = i == c ? 1.0 : 0.0;
-        for (int i = c + 1; i < kb; ++i) {
-            double s = 0.0;
-            for (int k = c; k < i; ++k) s = fma(a[i][k], Linv[k + c * LU_NB], s);
-            Linv[i + c * LU_NB] = -s;
-        }
-        // column c of U^{-1}: X(c,c) = 1/U(c,c), X(i,c) = -sum_{k=i+1}^{c} U(i,k) X(k,c) / U(i,i)
-        for (int i = 0; i < LU_NB; ++i) Uinv[i + c * LU_NB] = 0.0;
-        Uinv[c + c * LU_NB] = 1.0 / a[c][c];
-        for (int i = c - 1; i >= 0; --i) {
-            double s = 0.0;
-            for (int k = i + 1; k <= c; ++k) s = fma(a[i][k], Uinv[k + c * LU_NB], s);
-            Uinv[i + c * LU_NB] = -s / a[i][i];
-        }
-    } else if (c < LU_NB) {
-        for (int i = 0; i < LU_NB; ++i) {
-            Linv[i + c * LU_NB] = 0.0;
-            Uinv[i + c * LU_NB] = 0.0;
+// LU of the kb x kb block a in shared memory by 128 threads, without exchanges; flag
+// bit 0 if a multiplier exceeds 1 in magnitude, bit 1 on a zero / non-finite pivot.
+// Warp 0 keeps one column ahead: it updates and scales the next column while the
+// other warps finish the step's update.
+__device__ void lu32(double (*a)[PB + 1], int kb, int* flag) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w == 0) {
+        const double piv = a[0][0], v = lane < kb ? a[lane][0] : 0.0;
+        if (lane == 0 && !(piv != 0.0 && isfinite(piv))) atomicOr(flag, 2);
+        if (lane > 0 && lane < kb) {
+            if (!(fabs(v) <= fabs(piv))) atomicOr(flag, isfinite(v) ? 1 : 2);
+            a[lane][0] = v * recip(piv);
         }
     }
-}
-
-// Factor the kb x kb diagonal block in place without exchanges; flag bit 0 if
-// a multiplier exceeds 1 in magnitude, bit 1 on a zero / non-finite pivot.
-__global__ void __launch_bounds__(256) lu_diag_kernel(double* A, long long lda, int kb, double* Linv, double* Uinv,
-                                                      int* flag) {
-    __shared__ double a[LU_NB][LU_NB + 1];
-    const int tid = threadIdx.x;
-    for (int e = tid; e < kb * kb; e += blockDim.x) a[e % kb][e / kb] = A[(e % kb) + (e / kb) * lda];
     __syncthreads();
-    for (int j = 0; j < kb; ++j) {
-        const double piv = a[j][j];
-        if (tid == 0 && !(piv != 0.0 && isfinite(piv))) atomicOr(flag, 2);
-        for (int i = j + 1 + tid; i < kb; i += blockDim.x) {
-            const double l = a[i][j] / piv;
-            a[i][j] = l;
-            if (!(fabs(l) <= 1.0)) atomicOr(flag, isfinite(l) ? 1 : 2);
-        }
-        __syncthreads();
-        const int w = kb - j - 1;
-        for (int e = tid; e < w * w; e += blockDim.x) {
-            const int i = j + 1 + e % w, c = j + 1 + e / w;
-            a[i][c] = fma(-a[i][j], a[j][c], a[i][c]);
+    for (int j = 0; j + 1 < kb; ++j) {
+        const double l = lane > j && lane < kb ? a[lane][j] : 0.0;
+        if (w == 0) {
+            const int c = j + 1;
+            double v = lane > j && lane < kb ? fma(-l, a[j][c], a[lane][c]) : 0.0;
+            const double piv = __shfl_sync(0xffffffffu, v, c);
+            const double r = recip(piv);
+            if (lane == c && !(piv != 0.0 && isfinite(piv))) atomicOr(flag, 2);
+            if (lane > c && lane < kb) {
+                if (!(fabs(v) <= fabs(piv))) atomicOr(flag, isfinite(v) ? 1 : 2);
+                v *= r;
+            }
+            if (lane > j && lane < kb) a[lane][c] = v;
+        } else if (lane > j && lane < kb) {
+            for (int c = j + 1 + w; c < kb; c += 3) a[lane][c] = fma(-l, a[j][c], a[lane][c]);
         }
         __syncthreads();
     }
-    for (int e = tid; e < kb * kb; e += blockDim.x) A[(e % kb) + (e / kb) * lda] = a[e % kb][e / kb];
-    block_inverses(a, kb, Linv, Uinv);
 }
 
-// Inverses of all diagonal blocks of a factored matrix (after the pivoted path).
-__global__ void __launch_bounds__(LU_NB) diag_inv_kernel(const double* A, long long lda, int n, double* Linv,
-                                                         double* Uinv) {
-    __shared__ double a[LU_NB][LU_NB + 1];
-    const int k0 = blockIdx.x * LU_NB, kb = min(LU_NB, n - k0);
-    for (int e = threadIdx.x; e < kb * kb; e += blockDim.x)
-        a[e % kb][e / kb] = A[(k0 + e % kb) + (long long)(k0 + e / kb) * lda];
+__global__ void __launch_bounds__(128) lu_diag_kernel(double* A, long long lda, int kb, int* flag) {
+    __shared__ double a[PB][PB + 1];
+    for (int e = threadIdx.x; e < kb * kb; e += 128) a[e % kb][e / kb] = A[(e % kb) + (e / kb) * lda];
     __syncthreads();
-    block_inverses(a, kb, Linv + (long long)blockIdx.x * LU_NB * LU_NB, Uinv + (long long)blockIdx.x * LU_NB * LU_NB);
+    lu32(a, kb, flag);
+    for (int e = threadIdx.x; e < kb * kb; e += 128) A[(e % kb) + (e / kb) * lda] = a[e % kb][e / kb];
+}
+
+// A points at the factored kb x kb diagonal block (kb <= 32); m rows below it, w columns
+// right of it.  CTAs 0 .. ceil(m / 32) - 1 take rows, the others columns; four lanes
+// share a row (column), each holding every fourth of its 32 entries.
+__global__ void __launch_bounds__(128) lu_trsm32_kernel(double* A, long long lda, int kb, int m, int w, int* flag) {
+    __shared__ double t[PB][PB + 1];  // rows: U11 by [j][k]; columns: L11^T by [j][i]
+    __shared__ double rd[PB], ad[PB];
+    const int nrow = (m + 31) >> 5;
+    const bool rows = (int)blockIdx.x < nrow;
+    for (int e = threadIdx.x; e < PB * PB; e += 128) {
+        const int i = e & 31, j = e >> 5;
+        const double v = i < kb && j < kb ? A[i + j * lda] : (i == j ? 1.0 : 0.0);
+        if (rows) t[i][j] = v;
+        else t[j][i] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < PB) {
+        rd[threadIdx.x] = rows ? recip(t[threadIdx.x][threadIdx.x]) : 1.0;
+        ad[threadIdx.x] = fabs(t[threadIdx.x][threadIdx.x]);
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, q = lane & 3;
+    const int idx = (rows ? blockIdx.x : blockIdx.x - nrow) * 32 + (threadIdx.x >> 2);
+    const bool in = idx < (rows ? m : w);
+    // entry k of this row (column)
+    double* const p = rows ? A + kb + idx : A + (kb + idx) * lda;
+    const long long s = rows ? lda : 1;
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = in && q + 4 * u < kb ? p[(q + 4 * u) * s] : 0.0;
+    int bad = 0;
+#pragma unroll
+    for (int j = 0; j < PB; ++j) {
+        const double x0 = __shfl_sync(0xffffffffu, v[j >> 2], (lane & ~3) | (j & 3));
+        if (rows && !(fabs(x0) <= ad[j])) bad |= isfinite(x0) ? 1 : 2;
+        const double x = x0 * rd[j];
+        if (q == (j & 3)) v[j >> 2] = x;
+        else if (q > (j & 3)) v[j >> 2] = fma(-x, t[j][q + (j & ~3)], v[j >> 2]);
+#pragma unroll
+        for (int u = (j >> 2) + 1; u < 8; ++u) v[u] = fma(-x, t[j][q + 4 * u], v[u]);
+    }
+    if (in && bad) atomicOr(flag, bad);
+    if (in)
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (q + 4 * u < kb) p[(q + 4 * u) * s] = v[u];
+}
+
+// A22 -= L21 U12 for the m rows and w <= 96 columns past a full 32 x 32 diagonal block
+// at A.  CTA 0 takes the next diagonal block (nb x nb) and factors it; the others 16 rows
+// each, without that block's columns in its rows.
+__global__ void __launch_bounds__(128) lu_update32_kernel(double* A, long long lda, int m, int w, int nb, int* flag) {
+    __shared__ double L[PB][PB + 1];      // [k][row]
+    __shared__ double U[PB][3 * PB + 1];  // [k][column]
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    if (blockIdx.x == 0) {
+        double acc[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int c = wp + 4 * u;
+            L[c][lane] = lane < nb ? A[PB + lane + c * lda] : 0.0;
+            U[lane][c] = c < nb ? A[lane + (PB + c) * lda] : 0.0;
+            acc[u] = lane < nb && c < nb ? A[PB + lane + (PB + c) * lda] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int k = 0; k < PB; ++k) {
+            const double l = L[k][lane];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) acc[u] = fma(-l, U[k][wp + 4 * u], acc[u]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 8; ++u) L[lane][wp + 4 * u] = acc[u];
+        __syncthreads();
+        lu32(L, nb, flag);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (lane < nb && wp + 4 * u < nb) A[PB + lane + (PB + wp + 4 * u) * lda] = L[lane][wp + 4 * u];
+        return;
+    }
+    const int row = (blockIdx.x - 1) * 16 + (lane & 15), g = wp * 2 + (lane >> 4);
+    const int c0 = row < nb ? nb : 0;
+    for (int k = g; k < PB; k += 8) L[k][lane & 15] = row < m ? A[PB + row + k * lda] : 0.0;
+    for (int c = wp; c < w; c += 4) U[lane][c] = A[lane + (PB + c) * lda];
+    __syncthreads();
+    double acc[12];
+#pragma unroll
+    for (int u = 0; u < 12; ++u) {
+        const int c = g + 8 * u;
+        acc[u] = row < m && c < w ? A[PB + row + (PB + c) * lda] : 0.0;
+    }
+#pragma unroll 4
+    for (int k = 0; k < PB; ++k) {
+        const double l = L[k][lane & 15];
+#pragma unroll
+        for (int u = 0; u < 12; ++u)
+            if (8 * u < w) acc[u] = fma(-l, U[k][g + 8 * u], acc[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 12; ++u) {
+        const int c = g + 8 * u;
+        if (row < m && c >= c0 && c < w) A[PB + row + (PB + c) * lda] = acc[u];
+    }
+}
+
+// X <- L^{-1} X or U^{-1} X for the diagonal blocks (nbk wide) of a factored matrix, four
+// columns per CTA, a thread per row, one barrier per step.  The triangle's column for a
+// step does not depend on the steps before, so eight are loaded ahead (waiting for
+// each one's L2 round trip took 64 us for 128 steps).
+//   lu_lower_kernel    X = columns of the matrix right of block A (in place)
+//   lu_inverse_kernel  X = identity: Linv and Uinv of block blockIdx.x, column-major with
+//                      leading dimension LU_NB, zero padded; blockIdx.y < LU_NB / 4: L.
+constexpr int INV_C = 4, INV_AHEAD = 8;
+template <bool LOWER>
+__device__ void tri_solve(const double* a, long long lda, int rows, int first, int steps, double rd,
+                          double (&r)[INV_C], double (*x)[INV_C]) {
+    const int i = threadIdx.x, d = LOWER ? 1 : -1;
+    auto entry = [&](int s) {
+        const int j = first + d * s;
+        return s < steps && i < rows && (LOWER ? i > j : i < j) ? a[i + (long long)j * lda] : 0.0;
+    };
+    double t[INV_AHEAD];
+#pragma unroll
+    for (int u = 0; u < INV_AHEAD; ++u) t[u] = entry(u);
+    for (int s0 = 0; s0 < steps; s0 += INV_AHEAD) {
+        double nx[INV_AHEAD];
+#pragma unroll
+        for (int u = 0; u < INV_AHEAD; ++u) nx[u] = entry(s0 + INV_AHEAD + u);
+#pragma unroll
+        for (int u = 0; u < INV_AHEAD; ++u) {
+            if (s0 + u >= steps) break;
+            const int j = first + d * (s0 + u);
+            if (i == j)
+#pragma unroll
+                for (int c = 0; c < INV_C; ++c) {
+                    if (!LOWER) r[c] *= rd;
+                    x[j][c] = r[c];
+                }
+            __syncthreads();
+#pragma unroll
+            for (int c = 0; c < INV_C; ++c) r[c] = fma(-t[u], x[j][c], r[c]);
+        }
+#pragma unroll
+        for (int u = 0; u < INV_AHEAD; ++u) t[u] = nx[u];
+    }
+}
+
+__global__ void __launch_bounds__(HB) lu_lower_kernel(double* A, long long lda, int w) {
+    __shared__ double x[HB][INV_C];
+    const int i = threadIdx.x, c0 = blockIdx.x * INV_C;
+    double* X = A + (long long)(HB + c0) * lda + i;
+    double r[INV_C];
+#pragma unroll
+    for (int c = 0; c < INV_C; ++c) r[c] = c0 + c < w ? X[c * lda] : 0.0;
+    tri_solve<true>(A, lda, HB, 0, HB, 1.0, r, x);
+#pragma unroll
+    for (int c = 0; c < INV_C; ++c)
+        if (c0 + c < w) X[c * lda] = r[c];
+}
+
+__global__ void __launch_bounds__(LU_NB) lu_inverse_kernel(const double* __restrict__ A, long long lda, int n,
+                                                           double* __restrict__ Linv, double* __restrict__ Uinv) {
+    __shared__ double x[LU_NB][INV_C];
+    const int k0 = blockIdx.x * LU_NB, kb = min(LU_NB, n - k0), i = threadIdx.x;
+    const bool lower = blockIdx.y < LU_NB / INV_C;
+    const int c0 = (lower ? blockIdx.y : blockIdx.y - LU_NB / INV_C) * INV_C;
+    const double* a = A + k0 + (long long)k0 * lda;
+    double r[INV_C];
+#pragma unroll
+    for (int c = 0; c < INV_C; ++c) r[c] = i == c0 + c && i < kb ? 1.0 : 0.0;
+    if (c0 < kb) {
+        const int last = min(kb, c0 + INV_C) - 1;
+        // rows past the block hold zeros and read none of its entries
+        if (lower) tri_solve<true>(a, lda, kb, c0, kb - c0, 1.0, r, x);
+        else tri_solve<false>(a, lda, kb, last, last + 1, i < kb ? recip(a[i + (long long)i * lda]) : 0.0, r, x);
+    }
+    double* o = (lower ? Linv : Uinv) + (long long)blockIdx.x * LU_NB * LU_NB + i;
+#pragma unroll
+    for (int c = 0; c < INV_C; ++c) o[(c0 + c) * LU_NB] = i < kb ? r[c] : 0.0;
 }
 
 // ---------------------------------------------------------------- pivoted fallback
@@ -292,27 +583,52 @@ __global__ void laswp_kernel(double* B, long long ldb, int n, int nrhs, const in
 }
 
 // ---------------------------------------------------------------- LU64
-static void run_fast(double* A, long long ld, int n, double* Linv, double* Uinv, int* flag, cudaStream_t st) {
-    DevBuf<double> W1((size_t)LU_NB * n, st), W2((size_t)LU_NB * n, st);
+// C = alpha (op A) B + beta C where the operands' digits serve once.
+static void tensor_product(const double* A, long long lda, const double* B, long long ldb, int M, int N, int K,
+                           double alpha, double beta, double* C, long long ldc, int* err, cudaStream_t st) {
+    OzMat a, b;
+    a.split(A, 1, lda, M, K, st);
+    b.split(B, ldb, 1, N, K, st);
+    oz_gemm(a, b, alpha, beta, C, ldc, err, st);
+}
+
+// The panel of columns [k0, k0 + kb), kb <= HB, of the n x n matrix, all rows below.
+static void factor_panel(double* A, long long ld, int n, int k0, int kb, int* flag, cudaStream_t st) {
+    double* A11 = A + k0 + k0 * ld;
+    LAUNCH(lu_diag_kernel, 1, 128, 0, st, A11, ld, std::min(PB, kb), flag);
+    for (int j = 0; j < kb; j += PB) {
+        const int jb = std::min(PB, kb - j), m = n - k0 - j - jb, w = kb - j - jb;
+        double* D = A11 + j + j * ld;
+        if (m > 0) LAUNCH(lu_trsm32_kernel, ceil_div(m, 32) + ceil_div(w, 32), 128, 0, st, D, ld, jb, m, w, flag);
+        if (w > 0) LAUNCH(lu_update32_kernel, 1 + ceil_div(m, 16), 128, 0, st, D, ld, m, w, std::min(PB, w), flag);
+    }
+}
+
+// Panels of LU_NB = 256 columns, each as two of 128.  With 256 the trailing update's tiles
+// multiply for longer (18 us) than they take to read out, which 128 do not.
+static void run_fast(double* A, long long ld, int n, double* Linv, double* Uinv, int* flag, int* err, cudaStream_t st) {
     for (int k0 = 0, b = 0; k0 < n; k0 += LU_NB, ++b) {
-        const int kb = std::min(LU_NB, n - k0), n2 = n - k0 - kb;
+        const int kb = std::min(LU_NB, n - k0), n2 = n - k0 - kb, h = std::min(HB, kb), h2 = kb - h;
         double* A11 = A + k0 + k0 * ld;
-        double* Li = Linv + (long long)b * LU_NB * LU_NB;
-        double* Ui = Uinv + (long long)b * LU_NB * LU_NB;
-        LAUNCH(lu_diag_kernel, 1, 256, 0, st, A11, ld, kb, Li, Ui, flag);
+        factor_panel(A, ld, n, k0, h, flag, st);
+        if (h2 > 0) {
+            double* right = A11 + h * ld;
+            LAUNCH(lu_lower_kernel, ceil_div(h2, INV_C), HB, 0, st, A11, ld, h2);
+            tensor_product(A11 + h, ld, right, ld, n - k0 - h, h2, h, -1.0, 1.0, right + h, ld, err, st);
+            factor_panel(A, ld, n, k0 + h, h2, flag, st);
+        }
         if (n2 == 0) break;
+        double* Li = Linv + (long long)b * LU_NB * LU_NB;
         double* A12 = A + k0 + (k0 + kb) * ld;
         double* A21 = A + (k0 + kb) + k0 * ld;
         double* A22 = A + (k0 + kb) + (k0 + kb) * ld;
         // U12 = L11^{-1} A12
-        gemm64(false, false, kb, n2, kb, 1.0, Li, LU_NB, A12, ld, 0.0, W1.get(), kb, st);
-        copy_matrix64(W1.get(), kb, A12, ld, kb, n2, st);
-        // L21 = A21 U11^{-1}, certified |L21| <= 1
-        gemm64(false, false, n2, kb, kb, 1.0, A21, ld, Ui, LU_NB, 0.0, W2.get(), n2, st);
-        LAUNCH(copy_check_kernel, ceil_div((long long)n2 * kb, 256), 256, 0, st, W2.get(), A21, ld, n2, kb, flag);
+        LAUNCH(lu_inverse_kernel, dim3(1, LU_NB / INV_C), LU_NB, 0, st, A11, ld, kb, Li, (double*)nullptr);
+        tensor_product(Li, LU_NB, A12, ld, kb, n2, kb, 1.0, 0.0, A12, ld, err, st);
         // A22 -= L21 U12
-        gemm64(false, false, n2, n2, kb, -1.0, A21, ld, A12, ld, 1.0, A22, ld, st);
+        tensor_product(A21, ld, A12, ld, n2, n2, kb, -1.0, 1.0, A22, ld, err, st);
     }
+    LAUNCH(lu_inverse_kernel, dim3(ceil_div(n, LU_NB), 2 * LU_NB / INV_C), LU_NB, 0, st, A, ld, n, Linv, Uinv);
 }
 
 static void run_pivoted(double* A, long long ld, int n, int* ipiv, double* Linv, double* Uinv, int* flag,
@@ -325,15 +641,17 @@ static void run_pivoted(double* A, long long ld, int n, int* ipiv, double* Linv,
             LAUNCH(scale_col_kernel, ceil_div(n - j - 1, 256), 256, 0, st, A, ld, n, j);
         }
     }
-    LAUNCH(diag_inv_kernel, ceil_div(n, LU_NB), LU_NB, 0, st, A, ld, n, Linv, Uinv);
+    LAUNCH(lu_inverse_kernel, dim3(ceil_div(n, LU_NB), 2 * LU_NB / INV_C), LU_NB, 0, st, A, ld, n, Linv, Uinv);
 }
 
+// [0]: the certificate, [1]: a bounded wait of the tensor-core products expired
 static int read_flag(const int* flag, cudaStream_t st) {
-    int h = 0;
-    CUDA_CHECK(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    count_d2h(sizeof(int));
+    int h[2] = {0, 0};
+    CUDA_CHECK(cudaMemcpyAsync(h, flag, sizeof h, cudaMemcpyDeviceToHost, st));
+    count_d2h(sizeof h);
     CUDA_CHECK(cudaStreamSynchronize(st));
-    return h;
+    if (h[1]) fail(SQBEM_ERR_TIMEOUT, "LU: a bounded wait in the FP64 tensor-core product expired");
+    return h[0];
 }
 
 void LU64::factor_inplace(DevBuf<double>&& M, int n_, cudaStream_t st, const char* what) {
@@ -343,11 +661,11 @@ void LU64::factor_inplace(DevBuf<double>&& M, int n_, cudaStream_t st, const cha
     const int nblk = ceil_div(n, LU_NB);
     Linv.alloc((size_t)nblk * LU_NB * LU_NB, st);
     Uinv.alloc((size_t)nblk * LU_NB * LU_NB, st);
-    DevBuf<int> flag(1, st);
+    DevBuf<int> flag(2, st);
     flag.zero();
     DevBuf<double> saved((size_t)n * n, st);
     CUDA_CHECK(cudaMemcpyAsync(saved.get(), A.get(), sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToDevice, st));
-    run_fast(A.get(), ld, n, Linv.get(), Uinv.get(), flag.get(), st);
+    run_fast(A.get(), ld, n, Linv.get(), Uinv.get(), flag.get(), flag.get() + 1, st);
     int f = read_flag(flag.get(), st);
     pivoted = false;
     if (f != 0) {
@@ -368,30 +686,54 @@ void LU64::factor(const double* M, int n_, long long ldm, cudaStream_t st, const
     factor_inplace(std::move(a), n_, st, what);
 }
 
-void LU64::solve(double* B, long long ldb, int nrhs, cudaStream_t st) const {
-    if (nrhs <= 0 || n == 0) return;
+// Few right-hand sides: per block one product with the block's inverse and one update of
+// the rows past it, between B and a second buffer (no copies).
+static void solve_few(const LU64& lu, double* B, long long ldb, int nrhs, cudaStream_t st) {
+    const int n = lu.n, nblk = ceil_div(n, LU_NB);
+    const long long ld = lu.ld;
+    const double* A = lu.A.get();
     // per-call scratch (stream-ordered), so handles sharing one factor on
     // different streams never share a buffer
-    DevBuf<double> work((size_t)LU_NB * nrhs, st);
-    double* W = work.get();
+    DevBuf<double> X((size_t)n * nrhs, st);
+    double* x = X.get();
+    for (int b = 0; b < nblk; ++b) {  // forward: unit lower L, B -> X
+        const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0);
+        gemm64(false, false, kb, nrhs, kb, 1.0, lu.Linv.get() + (long long)b * LU_NB * LU_NB, LU_NB, B + k0, ldb, 0.0,
+               x + k0, n, st);
+        gemm64(false, false, n - k0 - kb, nrhs, kb, -1.0, A + (k0 + kb) + k0 * ld, ld, x + k0, n, 1.0, B + k0 + kb, ldb,
+               st);
+    }
+    for (int b = nblk - 1; b >= 0; --b) {  // backward: U, X -> B
+        const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0);
+        gemm64(false, false, kb, nrhs, kb, 1.0, lu.Uinv.get() + (long long)b * LU_NB * LU_NB, LU_NB, x + k0, n, 0.0,
+               B + k0, ldb, st);
+        gemm64(false, false, k0, nrhs, kb, -1.0, A + k0 * ld, ld, B + k0, ldb, 1.0, x, n, st);
+    }
+}
+
+void LU64::solve(double* B, long long ldb, int nrhs, cudaStream_t st, int* err) const {
+    if (nrhs <= 0 || n == 0) return;
     if (pivoted) LAUNCH(laswp_kernel, ceil_div(nrhs, 128), 128, 0, st, B, ldb, n, nrhs, ipiv.get());
+    if (nrhs < 64 || !err) {
+        for (int c = 0; c < nrhs; c += SK_N) solve_few(*this, B + c * ldb, ldb, std::min(SK_N, nrhs - c), st);
+        return;
+    }
+    // many: the block inverses and the updates as tensor-core products
     const int nblk = ceil_div(n, LU_NB);
     for (int b = 0; b < nblk; ++b) {  // forward: unit lower L
-        const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0);
-        gemm64(false, false, kb, nrhs, kb, 1.0, Linv.get() + (long long)b * LU_NB * LU_NB, LU_NB, B + k0, ldb, 0.0, W,
-               kb, st);
-        copy_matrix64(W, kb, B + k0, ldb, kb, nrhs, st);
-        if (k0 + kb < n)
-            gemm64(false, false, n - k0 - kb, nrhs, kb, -1.0, A.get() + (k0 + kb) + k0 * ld, ld, B + k0, ldb, 1.0,
-                   B + k0 + kb, ldb, st);
+        const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0), n2 = n - k0 - kb;
+        tensor_product(Linv.get() + (long long)b * LU_NB * LU_NB, LU_NB, B + k0, ldb, kb, nrhs, kb, 1.0, 0.0, B + k0, ldb,
+                       err, st);
+        if (n2 > 0)
+            tensor_product(A.get() + (k0 + kb) + k0 * ld, ld, B + k0, ldb, n2, nrhs, kb, -1.0, 1.0, B + k0 + kb, ldb, err,
+                           st);
     }
     for (int b = nblk - 1; b >= 0; --b) {  // backward: U
         const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0);
-        gemm64(false, false, kb, nrhs, kb, 1.0, Uinv.get() + (long long)b * LU_NB * LU_NB, LU_NB, B + k0, ldb, 0.0, W,
-               kb, st);
-        copy_matrix64(W, kb, B + k0, ldb, kb, nrhs, st);
+        tensor_product(Uinv.get() + (long long)b * LU_NB * LU_NB, LU_NB, B + k0, ldb, kb, nrhs, kb, 1.0, 0.0, B + k0, ldb,
+                       err, st);
         if (k0 > 0)
-            gemm64(false, false, k0, nrhs, kb, -1.0, A.get() + k0 * ld, ld, B + k0, ldb, 1.0, B, ldb, st);
+            tensor_product(A.get() + k0 * ld, ld, B + k0, ldb, k0, nrhs, kb, -1.0, 1.0, B, ldb, err, st);
     }
 }
 
@@ -418,25 +760,25 @@ __global__ void laswp_reverse_kernel(double* B, long long ldb, int n, int nrhs, 
 // (backward); the off-diagonal blocks enter as transposed GEMM operands.
 void LU64::solve_transpose(double* B, long long ldb, int nrhs, cudaStream_t st) const {
     if (nrhs <= 0 || n == 0) return;
-    DevBuf<double> work((size_t)LU_NB * nrhs, st);
-    double* W = work.get();
     const int nblk = ceil_div(n, LU_NB);
-    for (int b = 0; b < nblk; ++b) {  // forward with U^T
-        const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0);
-        if (k0 > 0)  // B_k -= (U_{0:k0, k})^T X_{0:k0}
-            gemm64(true, false, kb, nrhs, k0, -1.0, A.get() + k0 * ld, ld, B, ldb, 1.0, B + k0, ldb, st);
-        gemm64(true, false, kb, nrhs, kb, 1.0, Uinv.get() + (long long)b * LU_NB * LU_NB, LU_NB, B + k0, ldb, 0.0, W,
-               kb, st);
-        copy_matrix64(W, kb, B + k0, ldb, kb, nrhs, st);
-    }
-    for (int b = nblk - 1; b >= 0; --b) {  // backward with L^T (unit)
-        const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0);
-        if (k0 + kb < n)  // B_k -= (L_{k0+kb:n, k})^T X_{k0+kb:n}
-            gemm64(true, false, kb, nrhs, n - k0 - kb, -1.0, A.get() + (k0 + kb) + k0 * ld, ld, B + k0 + kb, ldb, 1.0,
-                   B + k0, ldb, st);
-        gemm64(true, false, kb, nrhs, kb, 1.0, Linv.get() + (long long)b * LU_NB * LU_NB, LU_NB, B + k0, ldb, 0.0, W,
-               kb, st);
-        copy_matrix64(W, kb, B + k0, ldb, kb, nrhs, st);
+    DevBuf<double> X((size_t)n * std::min(nrhs, SK_N), st);
+    double* x = X.get();
+    for (int c = 0; c < nrhs; c += SK_N) {
+        const int nr = std::min(SK_N, nrhs - c);
+        double* R = B + c * ldb;
+        for (int b = 0; b < nblk; ++b) {  // forward with U^T, R -> x: the columns past the block as rows
+            const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0);
+            gemm64(true, false, kb, nr, kb, 1.0, Uinv.get() + (long long)b * LU_NB * LU_NB, LU_NB, R + k0, ldb, 0.0,
+                   x + k0, n, st);
+            gemm64(true, false, n - k0 - kb, nr, kb, -1.0, A.get() + k0 + (k0 + kb) * ld, ld, x + k0, n, 1.0,
+                   R + k0 + kb, ldb, st);
+        }
+        for (int b = nblk - 1; b >= 0; --b) {  // backward with L^T (unit), x -> R
+            const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0);
+            gemm64(true, false, kb, nr, kb, 1.0, Linv.get() + (long long)b * LU_NB * LU_NB, LU_NB, x + k0, n, 0.0,
+                   R + k0, ldb, st);
+            gemm64(true, false, k0, nr, kb, -1.0, A.get() + k0, ld, R + k0, ldb, 1.0, x, n, st);
+        }
     }
     if (pivoted) LAUNCH(laswp_reverse_kernel, ceil_div(nrhs, 128), 128, 0, st, B, ldb, n, nrhs, ipiv.get());
 }

@@ -1,0 +1,43 @@
+// oz_gemm.cuh -- FP64 matrix products on the BF16 tensor cores (tcgen05).
+//
+// Every row of A and every column of B is scaled by its own power of two to
+// 64-bit fixed point and cut into eight signed base-256 digits, d_0 (most
+// significant) .. d_7, |d_i| <= 128: small integers, exact in BF16 (the error-free
+// splitting of Ozaki, Ogita, Oishi and Rump, "Error-free transformations of
+// matrix multiplication", Numer. Algorithms 59, 2012).  A product of two digits is
+// at most 2^14, so sums of them are exact in the FP32 accumulators up to 2^24.
+// The 36 digit products with i + j <= 7 are summed by their weight i + j, each sum
+// is read back as an integer, all of them are added in two 64-bit integers and the
+// 96-bit total is rounded to FP64 once.  What is dropped lies below 2^-60 of the
+// row's largest entry times the column's, against the FP64 loop's rounding of
+// every partial sum.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "common.cuh"
+
+namespace sqbem {
+
+// Digits of an operand: rows x k values (the rows of A, or the columns of B) as
+// blocks of 128 rows x 16 k x 8 digits (32 KB), each digit's 128 x 16 BF16 in the
+// tensor cores' no-swizzle order (two halves of 8 k, 16 bytes per row), zero
+// padded; the biased exponent of every row's largest entry beside them.
+struct OzMat {
+    DevBuf<uint4> d;
+    DevBuf<int> ex;
+    int rows = 0, k = 0, k16 = 0;
+    // the values' source, for rows that hold an infinity or a NaN
+    const double* src = nullptr;
+    long long rs = 0, ks = 0;
+    // element (r, c) of the operand is a[r * rs + c * ks]
+    void split(const double* a, long long rs, long long ks, int rows, int k, cudaStream_t st);
+};
+
+// C (M x N, column-major) = alpha A B + beta C for the digits of A (M rows) and of
+// B (N columns, given as rows) over the same k.  The sources of A and B must be
+// alive and unchanged until the launch has run, and C must not overlap them.
+// *err is set if a bounded wait expires (SQBEM_ERR_TIMEOUT to the caller).
+void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* C, long long ldc, int* err,
+             cudaStream_t st);
+
+}  // namespace sqbem

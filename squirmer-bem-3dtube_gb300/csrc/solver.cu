@@ -173,11 +173,15 @@ void sqbem_swimmer::build_fp64() {
     Gs = std::move(E);
     if (tube) {
         // Y = T^{-1} [B | Ct];  Gs = E - D Y_s;  Gc = Cs - D Y_c  (238-249)
-        tube->lu.solve(Y.get(), nt, ns + 6, st);
-        gemm64(false, false, ns, ns, nt, -1.0, D.get(), ns, Y.get(), nt, 1.0, Gs.get(), ns, st);
+        WaitError we;
+        tube->lu.solve(Y.get(), nt, ns + 6, st, we.get(st));
+        gemm64(false, false, ns, ns, nt, -1.0, D.get(), ns, Y.get(), nt, 1.0, Gs.get(), ns, st, we.get(st));
         gemm64(false, false, ns, 6, nt, -1.0, D.get(), ns, Y.get() + (size_t)nt * ns, nt, 1.0, Gc.get(), ns, st);
+        clock2.stop(st);
+        we.check();
+    } else {
+        clock2.stop(st);
     }
-    clock2.stop(st);
     t_assembly = clock.seconds();
     t_schur = clock2.seconds();
 }

@@ -88,6 +88,7 @@ SIGNATURES = {
     "sqbem_run_trajectory": (_c_i, [_VP, ctypes.c_char_p, _c_i, _c_i, ctypes.c_char_p, _c_i]),
     "sqbem_trajectory_ensemble": (_c_i, [_c_i, _D, _D, _VP, _c_i, _c_i, _c_i, _D, _D, _D, _I, _D]),
     "sqbem_ensemble_field": (_c_i, [_c_i, _D, _D, _VP, _c_i, _c_i, _c_i, _c_d, _c_i, _D, _D]),
+    "sqbem_gemm64": (_c_i, [_c_i, _c_i, _c_i, _c_i, _c_i, _c_i, _c_d, _D, _c_i, _D, _c_i, _c_d, _D, _c_i]),
     "sqbem_gemm_mixed": (_c_i, [_c_i, _c_i, _c_i, ctypes.c_float, ctypes.POINTER(ctypes.c_float), _c_i,
                                 ctypes.POINTER(ctypes.c_float), _c_i, ctypes.c_float,
                                 ctypes.POINTER(ctypes.c_float), _c_i]),
@@ -116,6 +117,20 @@ def gemm_mixed(A, B, C=None, alpha=1.0, beta=0.0, variant=-1, products=3):
     else:
         _check(lib().sqbem_gemm_mixed_ex(variant, products, M, N, K, alpha, A.ctypes.data_as(fp), M,
                                          B.ctypes.data_as(fp), K, beta, Cm.ctypes.data_as(fp), M))
+    return Cm
+
+
+def gemm64(A, B, C=None, alpha=1.0, beta=0.0, ta=False, tb=False, route=-1):
+    """linalg.hpp:42-48 gemm in FP64 as the FP64 path runs it: returns alpha op(A)
+    op(B) + beta C.  route: -1 the path's own choice, 0 the FP64 pipe, 1 digit
+    products on the tensor cores."""
+    A = np.asfortranarray(np.asarray(A, dtype=np.float64))
+    B = np.asfortranarray(np.asarray(B, dtype=np.float64))
+    M, K = A.shape[::-1] if ta else A.shape
+    N = B.shape[0] if tb else B.shape[1]
+    Cm = np.asfortranarray(np.zeros((M, N)) if C is None else np.asarray(C, dtype=np.float64).copy())
+    _check(lib().sqbem_gemm64(route, int(ta), int(tb), M, N, K, alpha, A.ctypes.data_as(_D), A.shape[0],
+                              B.ctypes.data_as(_D), B.shape[0], beta, Cm.ctypes.data_as(_D), M))
     return Cm
 
 
