@@ -271,114 +271,159 @@ void max_abs64(const double* A, long long lda, int rows, int cols, double* out, 
 // A panel of HB = 128 columns is factored in steps of PB = 32 columns:
 //   diag      the 32 x 32 diagonal block (one CTA);
 //   trsm32    below it L21 = A21 U11^{-1}, right of it U12 = L11^{-1} A12 within
-//             the panel, 32 rows or columns per CTA;
+//             the panel, 16 rows or columns per CTA;
 //   update32  the rest of the panel, A22 -= L21 U12; the CTA of the next diagonal
 //             block updates only that block and factors it at once.
-// All of it is bound by the FP64 pipe of the SMs it is spread over (1.7 FMA per clock
-// and SM) and its latency, hence the small blocks and short CTAs.
+// An FP64 warp instruction occupies its SM quarter's pipe for 64 to 76 cycles, whether its
+// lanes are needed or not and whether the next one depends on it or not.  So the kernels
+// here count warp instructions: work spread over many CTAs of four warps, no FP64 comparisons
+// (integers order like the magnitudes), no per-step divisions.
 constexpr int PB = 32, HB = 128;
 
-// 1/x by Newton's iteration y <- y + y (1 - x y) from an FP32 reciprocal of the
-// significand (relative error 2^-23, 2^-46, then FP64 rounding); four dependent FMAs
-// where the full division is on the factorisation's serial chain.
+// 1/x from an FP32 reciprocal y of the significand m (relative error e = 1 - m y about
+// 2^-23): 1/m = y / (1 - e) = y (1 + e + e^2 + ..), cut after e^2, so 2^-69 and the
+// rounding.  Three FP64 operations where the full division (430 cycles) is on the
+// factorisation's serial chain.
 __device__ __forceinline__ double recip(double x) {
     const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
     if (e < 64 || e > 1980) return 1.0 / x;
     const double m = __hiloint2double((hi & 0x800fffff) | 0x3ff00000, __double2loint(x));
-    double y = (double)(1.0f / (float)m);
-    y = fma(y, fma(-m, y, 1.0), y);
-    y = fma(y, fma(-m, y, 1.0), y);
-    return __hiloint2double(__double2hiint(y) + ((1023 - e) << 20), __double2loint(y));
+    const double y = (double)(1.0f / (float)m), d = fma(-m, y, 1.0);
+    const double r = fma(y, fma(d, d, d), y);
+    return __hiloint2double(__double2hiint(r) + ((1023 - e) << 20), __double2loint(r));
 }
 
-// LU of the kb x kb block a in shared memory by 128 threads, without exchanges; flag
-// bit 0 if a multiplier exceeds 1 in magnitude, bit 1 on a zero / non-finite pivot.
-// Warp 0 keeps one column ahead: it updates and scales the next column while the
-// other warps finish the step's update.
-__device__ void lu32(double (*a)[PB + 1], int kb, int* flag) {
+// |x| > |piv|, as a pivot search sees it (bit 0), or x not finite (bit 1); piv by its bits
+// without the sign
+__device__ __forceinline__ int exceeds(double x, long long piv) {
+    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffll;
+    return b > piv ? (b < 0x7ff0000000000000ll ? 1 : 2) : 0;
+}
+
+// LU without exchanges of a 32 x 32 block by 128 threads, lane = row, v[u] = column w + 4 u of
+// warp w; the first kb columns are factored (the rest of the block: identity).  flag bit 0
+// if a multiplier exceeds 1 in magnitude, bit 1 on a zero / non-finite pivot.  The
+// finished columns go to out (leading dimension ldo; kb rows and columns).
+// Column j belongs to warp j & 3: it publishes the column's multipliers through shared
+// memory and a barrier that only the other warps wait on, before its own updates of the step.
+__device__ void lu32(double (&v)[8], double (*lc)[PB], int kb, double* out, long long ldo, int* flag) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (w == 0) {
-        const double piv = a[0][0], v = lane < kb ? a[lane][0] : 0.0;
-        if (lane == 0 && !(piv != 0.0 && isfinite(piv))) atomicOr(flag, 2);
-        if (lane > 0 && lane < kb) {
-            if (!(fabs(v) <= fabs(piv))) atomicOr(flag, isfinite(v) ? 1 : 2);
-            a[lane][0] = v * recip(piv);
+    int bad = 0;
+    auto publish = [&](int j) {  // by the warp that holds column j in v[0]
+        const double piv = __shfl_sync(0xffffffffu, v[0], j);
+        const long long pb = __double_as_longlong(piv) & 0x7fffffffffffffffll;
+        if (pb == 0 || pb >= 0x7ff0000000000000ll) bad |= 2;
+        const double l = v[0] * recip(piv);
+        if (lane > j) {
+            bad |= exceeds(v[0], pb);
+            v[0] = l;
         }
-    }
-    __syncthreads();
-    for (int j = 0; j + 1 < kb; ++j) {
-        const double l = lane > j && lane < kb ? a[lane][j] : 0.0;
-        if (w == 0) {
-            const int c = j + 1;
-            double v = lane > j && lane < kb ? fma(-l, a[j][c], a[lane][c]) : 0.0;
-            const double piv = __shfl_sync(0xffffffffu, v, c);
-            const double r = recip(piv);
-            if (lane == c && !(piv != 0.0 && isfinite(piv))) atomicOr(flag, 2);
-            if (lane > c && lane < kb) {
-                if (!(fabs(v) <= fabs(piv))) atomicOr(flag, isfinite(v) ? 1 : 2);
-                v *= r;
+        lc[j & 3][lane] = lane > j ? l : 0.0;
+        __threadfence_block();
+        asm volatile("barrier.cta.arrive %0, 128;" ::"r"(1 + (j & 3)) : "memory");
+    };
+    if (w == 0) publish(0);
+    for (int t = 0; 4 * t < kb; ++t) {
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const int j = 4 * t + s;
+            if (w != s) asm volatile("barrier.cta.sync %0, 128;" ::"r"(1 + s) : "memory");
+            const double l = lc[s][lane];
+            if (w > s) v[0] = fma(-l, __shfl_sync(0xffffffffu, v[0], j), v[0]);
+            if (s < 3 && w == s + 1) publish(j + 1);
+#pragma unroll
+            for (int u = 1; u < 8; ++u) {
+                if (4 * (t + u) < kb) v[u] = fma(-l, __shfl_sync(0xffffffffu, v[u], j), v[u]);
+                if (u == 1 && s == 3 && w == 0 && j + 1 < PB) {  // column j + 1 is next in line: v[1] of warp 0
+                    const double keep = v[0];
+                    v[0] = v[1];
+                    publish(j + 1);
+                    v[1] = v[0];
+                    v[0] = keep;
+                }
             }
-            if (lane > j && lane < kb) a[lane][c] = v;
-        } else if (lane > j && lane < kb) {
-            for (int c = j + 1 + w; c < kb; c += 3) a[lane][c] = fma(-l, a[j][c], a[lane][c]);
         }
-        __syncthreads();
+        if (lane < kb && w + 4 * t < kb) out[lane + (w + 4 * t) * ldo] = v[0];
+#pragma unroll
+        for (int u = 0; u < 7; ++u) v[u] = v[u + 1];
     }
+    // the last publication has no readers: take the barrier back to its start
+    if (((kb + 3) & ~3) < PB && w != 0) asm volatile("barrier.cta.sync %0, 128;" ::"r"(1) : "memory");
+    if (bad) atomicOr(flag, bad);
 }
 
 __global__ void __launch_bounds__(128) lu_diag_kernel(double* A, long long lda, int kb, int* flag) {
-    __shared__ double a[PB][PB + 1];
-    for (int e = threadIdx.x; e < kb * kb; e += 128) a[e % kb][e / kb] = A[(e % kb) + (e / kb) * lda];
-    __syncthreads();
-    lu32(a, kb, flag);
-    for (int e = threadIdx.x; e < kb * kb; e += 128) A[(e % kb) + (e / kb) * lda] = a[e % kb][e / kb];
+    __shared__ double lc[4][PB];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const int c = w + 4 * u;
+        v[u] = lane < kb && c < kb ? A[lane + c * lda] : (lane == c ? 1.0 : 0.0);
+    }
+    lu32(v, lc, kb, A, lda, flag);
 }
 
 // A points at the factored kb x kb diagonal block (kb <= 32); m rows below it, w columns
-// right of it.  CTAs 0 .. ceil(m / 32) - 1 take rows, the others columns; four lanes
-// share a row (column), each holding every fourth of its 32 entries.
+// right of it.  CTAs 0 .. ceil(m / 16) - 1 take rows, the others columns; eight lanes
+// share a row (column), each holding every eighth of its 32 entries.  A row's substitution
+// carries y_j = x_j u_jj and the scaled factor u_jk / u_jj, so that the divisions come
+// once at the end.
 __global__ void __launch_bounds__(128) lu_trsm32_kernel(double* A, long long lda, int kb, int m, int w, int* flag) {
-    __shared__ double t[PB][PB + 1];  // rows: U11 by [j][k]; columns: L11^T by [j][i]
-    __shared__ double rd[PB], ad[PB];
-    const int nrow = (m + 31) >> 5;
+    __shared__ double t[PB][PB + 1];  // rows: U11 by [j][k] over u_jj; columns: L11^T by [j][i]; 0 for k <= j
+    __shared__ double rd[PB];
+    __shared__ long long ad[PB];
+    const int nrow = (m + 15) >> 4;
     const bool rows = (int)blockIdx.x < nrow;
-    for (int e = threadIdx.x; e < PB * PB; e += 128) {
-        const int i = e & 31, j = e >> 5;
-        const double v = i < kb && j < kb ? A[i + j * lda] : (i == j ? 1.0 : 0.0);
-        if (rows) t[i][j] = v;
-        else t[j][i] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < PB) {
-        rd[threadIdx.x] = rows ? recip(t[threadIdx.x][threadIdx.x]) : 1.0;
-        ad[threadIdx.x] = fabs(t[threadIdx.x][threadIdx.x]);
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, q = lane & 3;
-    const int idx = (rows ? blockIdx.x : blockIdx.x - nrow) * 32 + (threadIdx.x >> 2);
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, q = lane & 7;
+    const int idx = (rows ? blockIdx.x : blockIdx.x - nrow) * 16 + (threadIdx.x >> 3);
     const bool in = idx < (rows ? m : w);
     // entry k of this row (column)
     double* const p = rows ? A + kb + idx : A + (kb + idx) * lda;
     const long long s = rows ? lda : 1;
-    double v[8];
+    double v[4];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = in && q + 4 * u < kb ? p[(q + 4 * u) * s] : 0.0;
+    for (int u = 0; u < 4; ++u) v[u] = in && q + 8 * u < kb ? p[(q + 8 * u) * s] : 0.0;
+    double e[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const int c = g + 4 * u;
+        e[u] = lane < kb && c < kb ? A[lane + c * lda] : (lane == c ? 1.0 : 0.0);
+    }
+    double piv = 1.0;  // of column lane, where this warp holds it
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+        if (lane == g + 4 * u) piv = e[u];
+    piv = (lane & 3) == g ? piv : 1.0;
+    const double rp = recip(piv);
+    if ((lane & 3) == g) {
+        rd[lane] = rp;
+        ad[lane] = __double_as_longlong(piv) & 0x7fffffffffffffffll;
+    }
+    __syncthreads();
+    if (rows) {
+        const double r = rd[lane];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t[lane][g + 4 * u] = g + 4 * u > lane ? e[u] * r : 0.0;
+    } else {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t[g + 4 * u][lane] = lane > g + 4 * u ? e[u] : 0.0;
+    }
+    __syncthreads();
     int bad = 0;
 #pragma unroll
     for (int j = 0; j < PB; ++j) {
-        const double x0 = __shfl_sync(0xffffffffu, v[j >> 2], (lane & ~3) | (j & 3));
-        if (rows && !(fabs(x0) <= ad[j])) bad |= isfinite(x0) ? 1 : 2;
-        const double x = x0 * rd[j];
-        if (q == (j & 3)) v[j >> 2] = x;
-        else if (q > (j & 3)) v[j >> 2] = fma(-x, t[j][q + (j & ~3)], v[j >> 2]);
+        const double y = __shfl_sync(0xffffffffu, v[j >> 3], (lane & ~7) | (j & 7));
+        if (rows) bad |= exceeds(y, ad[j]);
 #pragma unroll
-        for (int u = (j >> 2) + 1; u < 8; ++u) v[u] = fma(-x, t[j][q + 4 * u], v[u]);
+        for (int u = j >> 3; u < 4; ++u)
+            if (j != 8 * u + 7) v[u] = fma(-y, t[j][q + 8 * u], v[u]);
     }
-    if (in && bad) atomicOr(flag, bad);
-    if (in)
+    if (!in) return;
+    if (bad) atomicOr(flag, bad);
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (q + 4 * u < kb) p[(q + 4 * u) * s] = v[u];
+    for (int u = 0; u < 4; ++u)
+        if (q + 8 * u < kb) p[(q + 8 * u) * s] = rows ? v[u] * rd[q + 8 * u] : v[u];
 }
 
 // A22 -= L21 U12 for the m rows and w <= 96 columns past a full 32 x 32 diagonal block
@@ -395,7 +440,7 @@ __global__ void __launch_bounds__(128) lu_update32_kernel(double* A, long long l
             const int c = wp + 4 * u;
             L[c][lane] = lane < nb ? A[PB + lane + c * lda] : 0.0;
             U[lane][c] = c < nb ? A[lane + (PB + c) * lda] : 0.0;
-            acc[u] = lane < nb && c < nb ? A[PB + lane + (PB + c) * lda] : 0.0;
+            acc[u] = lane < nb && c < nb ? A[PB + lane + (PB + c) * lda] : (lane == c ? 1.0 : 0.0);
         }
         __syncthreads();
 #pragma unroll 8
@@ -405,26 +450,22 @@ __global__ void __launch_bounds__(128) lu_update32_kernel(double* A, long long l
             for (int u = 0; u < 8; ++u) acc[u] = fma(-l, U[k][wp + 4 * u], acc[u]);
         }
         __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 8; ++u) L[lane][wp + 4 * u] = acc[u];
-        __syncthreads();
-        lu32(L, nb, flag);
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (lane < nb && wp + 4 * u < nb) A[PB + lane + (PB + wp + 4 * u) * lda] = L[lane][wp + 4 * u];
+        lu32(acc, reinterpret_cast<double (*)[PB]>(&L[0][0]), nb, A + PB + PB * lda, lda, flag);
         return;
     }
     const int row = (blockIdx.x - 1) * 16 + (lane & 15), g = wp * 2 + (lane >> 4);
     const int c0 = row < nb ? nb : 0;
+#pragma unroll
     for (int k = g; k < PB; k += 8) L[k][lane & 15] = row < m ? A[PB + row + k * lda] : 0.0;
+#pragma unroll 8
     for (int c = wp; c < w; c += 4) U[lane][c] = A[lane + (PB + c) * lda];
-    __syncthreads();
     double acc[12];
 #pragma unroll
     for (int u = 0; u < 12; ++u) {
         const int c = g + 8 * u;
         acc[u] = row < m && c < w ? A[PB + row + (PB + c) * lda] : 0.0;
     }
+    __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < PB; ++k) {
         const double l = L[k][lane & 15];
@@ -439,14 +480,14 @@ __global__ void __launch_bounds__(128) lu_update32_kernel(double* A, long long l
     }
 }
 
-// X <- L^{-1} X or U^{-1} X for the diagonal blocks (nbk wide) of a factored matrix, four
-// columns per CTA, a thread per row, one barrier per step.  The triangle's column for a
-// step does not depend on the steps before, so eight are loaded ahead (waiting for
-// each one's L2 round trip took 64 us for 128 steps).
+// X <- L^{-1} X or U^{-1} X for the diagonal blocks of a factored matrix, two columns per
+// CTA, a thread per row, one barrier per step; warps whose rows are finished skip the
+// step's FMAs.  The triangle's column for a step does not depend on the steps before, so
+// eight are loaded ahead (waiting for each one's L2 round trip took 64 us for 128 steps).
 //   lu_lower_kernel    X = columns of the matrix right of block A (in place)
-//   lu_inverse_kernel  X = identity: Linv and Uinv of block blockIdx.x, column-major with
-//                      leading dimension LU_NB, zero padded; blockIdx.y < LU_NB / 4: L.
-constexpr int INV_C = 4, INV_AHEAD = 8;
+//   lu_inverse_kernel  X = identity: the inverse of block blockIdx.x's triangle, column-major
+//                      with leading dimension LU_NB, zero padded.
+constexpr int INV_C = 2, INV_AHEAD = 8;
 template <bool LOWER>
 __device__ void tri_solve(const double* a, long long lda, int rows, int first, int steps, double rd,
                           double (&r)[INV_C], double (*x)[INV_C]) {
@@ -473,8 +514,9 @@ __device__ void tri_solve(const double* a, long long lda, int rows, int first, i
                     x[j][c] = r[c];
                 }
             __syncthreads();
+            if (LOWER ? (i | 31) > j : (i & ~31) < j)
 #pragma unroll
-            for (int c = 0; c < INV_C; ++c) r[c] = fma(-t[u], x[j][c], r[c]);
+                for (int c = 0; c < INV_C; ++c) r[c] = fma(-t[u], x[j][c], r[c]);
         }
 #pragma unroll
         for (int u = 0; u < INV_AHEAD; ++u) t[u] = nx[u];
@@ -495,22 +537,20 @@ __global__ void __launch_bounds__(HB) lu_lower_kernel(double* A, long long lda, 
 }
 
 __global__ void __launch_bounds__(LU_NB) lu_inverse_kernel(const double* __restrict__ A, long long lda, int n,
-                                                           double* __restrict__ Linv, double* __restrict__ Uinv) {
+                                                           bool upper, double* __restrict__ inv) {
     __shared__ double x[LU_NB][INV_C];
     const int k0 = blockIdx.x * LU_NB, kb = min(LU_NB, n - k0), i = threadIdx.x;
-    const bool lower = blockIdx.y < LU_NB / INV_C;
-    const int c0 = (lower ? blockIdx.y : blockIdx.y - LU_NB / INV_C) * INV_C;
+    const int c0 = blockIdx.y * INV_C;
     const double* a = A + k0 + (long long)k0 * lda;
     double r[INV_C];
 #pragma unroll
     for (int c = 0; c < INV_C; ++c) r[c] = i == c0 + c && i < kb ? 1.0 : 0.0;
     if (c0 < kb) {
         const int last = min(kb, c0 + INV_C) - 1;
-        // rows past the block hold zeros and read none of its entries
-        if (lower) tri_solve<true>(a, lda, kb, c0, kb - c0, 1.0, r, x);
+        if (!upper) tri_solve<true>(a, lda, kb, c0, kb - c0, 1.0, r, x);
         else tri_solve<false>(a, lda, kb, last, last + 1, i < kb ? recip(a[i + (long long)i * lda]) : 0.0, r, x);
     }
-    double* o = (lower ? Linv : Uinv) + (long long)blockIdx.x * LU_NB * LU_NB + i;
+    double* o = inv + (long long)blockIdx.x * LU_NB * LU_NB + i;
 #pragma unroll
     for (int c = 0; c < INV_C; ++c) o[(c0 + c) * LU_NB] = i < kb ? r[c] : 0.0;
 }
@@ -599,7 +639,7 @@ static void factor_panel(double* A, long long ld, int n, int k0, int kb, int* fl
     for (int j = 0; j < kb; j += PB) {
         const int jb = std::min(PB, kb - j), m = n - k0 - j - jb, w = kb - j - jb;
         double* D = A11 + j + j * ld;
-        if (m > 0) LAUNCH(lu_trsm32_kernel, ceil_div(m, 32) + ceil_div(w, 32), 128, 0, st, D, ld, jb, m, w, flag);
+        if (m > 0) LAUNCH(lu_trsm32_kernel, ceil_div(m, 16) + ceil_div(w, 16), 128, 0, st, D, ld, jb, m, w, flag);
         if (w > 0) LAUNCH(lu_update32_kernel, 1 + ceil_div(m, 16), 128, 0, st, D, ld, m, w, std::min(PB, w), flag);
     }
 }
@@ -623,12 +663,16 @@ static void run_fast(double* A, long long ld, int n, double* Linv, double* Uinv,
         double* A21 = A + (k0 + kb) + k0 * ld;
         double* A22 = A + (k0 + kb) + (k0 + kb) * ld;
         // U12 = L11^{-1} A12
-        LAUNCH(lu_inverse_kernel, dim3(1, LU_NB / INV_C), LU_NB, 0, st, A11, ld, kb, Li, (double*)nullptr);
+        LAUNCH(lu_inverse_kernel, dim3(1, LU_NB / INV_C), LU_NB, 0, st, A11, ld, kb, false, Li);
         tensor_product(Li, LU_NB, A12, ld, kb, n2, kb, 1.0, 0.0, A12, ld, err, st);
         // A22 -= L21 U12
         tensor_product(A21, ld, A12, ld, n2, n2, kb, -1.0, 1.0, A22, ld, err, st);
     }
-    LAUNCH(lu_inverse_kernel, dim3(ceil_div(n, LU_NB), 2 * LU_NB / INV_C), LU_NB, 0, st, A, ld, n, Linv, Uinv);
+    // L^{-1} of the last block, and U^{-1} of all
+    const int last = (n - 1) / LU_NB, k0 = last * LU_NB;
+    LAUNCH(lu_inverse_kernel, dim3(1, LU_NB / INV_C), LU_NB, 0, st, A + k0 + k0 * ld, ld, n - k0, false,
+           Linv + (long long)last * LU_NB * LU_NB);
+    LAUNCH(lu_inverse_kernel, dim3(last + 1, LU_NB / INV_C), LU_NB, 0, st, A, ld, n, true, Uinv);
 }
 
 static void run_pivoted(double* A, long long ld, int n, int* ipiv, double* Linv, double* Uinv, int* flag,
@@ -641,7 +685,9 @@ static void run_pivoted(double* A, long long ld, int n, int* ipiv, double* Linv,
             LAUNCH(scale_col_kernel, ceil_div(n - j - 1, 256), 256, 0, st, A, ld, n, j);
         }
     }
-    LAUNCH(lu_inverse_kernel, dim3(ceil_div(n, LU_NB), 2 * LU_NB / INV_C), LU_NB, 0, st, A, ld, n, Linv, Uinv);
+    for (int up = 0; up < 2; ++up)
+        LAUNCH(lu_inverse_kernel, dim3(ceil_div(n, LU_NB), LU_NB / INV_C), LU_NB, 0, st, A, ld, n, up != 0,
+               up ? Uinv : Linv);
 }
 
 // [0]: the certificate, [1]: a bounded wait of the tensor-core products expired
