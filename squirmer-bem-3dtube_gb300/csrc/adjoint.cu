@@ -63,7 +63,7 @@ void sqbem_swimmer::adjoint(int nrhs, const double* slips, double* U, double* Om
     ls.upload(g.data(), g.size());
     luM.solve_transpose(ls.get(), n, 6, st);
     gemm64(true, false, nt, 6, ns, -1.0, D.get(), ns, ls.get(), n, 0.0, lt.get(), nt, st);
-    tube->lu.solve_transpose(lt.get(), nt, 6, st);
+    tube->solve64_transpose(lt.get(), nt, 6, st);
     DevBuf<double> dfs(fs.size(), st), dft(ft.size(), st), dv(v.size(), st), out(6 * ADJ_MAX_MODES * 3, st);
     dfs.upload(fs.data(), fs.size());
     dft.upload(ft.data(), ft.size());

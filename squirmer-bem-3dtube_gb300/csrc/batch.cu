@@ -415,7 +415,8 @@ void run_fp64(int n, const sqbem_instance* inst, const std::vector<Prepared>& pr
     std::vector<double> bytes;
     for (int k : order) {
         const double t = 3.0 * (prep[k].bounded ? prep[k].tube.P() : 0), s = 3.0 * prep[k].sphere.P();
-        bytes.push_back(1.25 * 8.0 * (3.0 * t * t + 6.0 * t * s + 6.0 * s * s));
+        // with the digits (two doubles an entry) of the Schur product's operands
+        bytes.push_back(1.25 * 8.0 * (3.0 * t * t + 10.0 * t * s + 8.0 * s * s));
     }
     run_concurrent((size_t)n, bytes, bs, [&](size_t j, cudaStream_t st) {
         const int k = order[j];
@@ -484,7 +485,7 @@ extern "C" int sqbem_adjoint_batch(int n, const sqbem_instance* inst, int precis
         std::vector<double> bytes;
         for (int k = 0; k < n; ++k) {
             const double t = 3.0 * (prep[k].bounded ? prep[k].tube.P() : 0), sp = 3.0 * prep[k].sphere.P();
-            bytes.push_back(1.25 * 8.0 * (3.0 * t * t + 7.0 * t * sp + 6.0 * sp * sp));
+            bytes.push_back(1.25 * 8.0 * (3.0 * t * t + 11.0 * t * sp + 8.0 * sp * sp));
         }
         run_concurrent((size_t)n, bytes, bs, [&](size_t kk, cudaStream_t st) {
             const int k = (int)kk;

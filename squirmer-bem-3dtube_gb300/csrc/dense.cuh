@@ -41,6 +41,13 @@ void gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const double* A
             const double* B, long long ldb, double beta, double* C, long long ldc, cudaStream_t st,
             int* err = nullptr);
 
+// The same for at most SK_N columns and tb = false, for a batch of matrices at the strides
+// sa, sb, sc.
+constexpr int SK_N = 8;
+void gemm64_few(bool ta, int M, int N, int K, double alpha, const double* A, long long lda, const double* B,
+                long long ldb, double beta, double* C, long long ldc, cudaStream_t st, int batch = 1,
+                long long sa = 0, long long sb = 0, long long sc = 0);
+
 // LU factorisation (dgetrf semantics) of an n x n column-major matrix, kept on
 // the device with the inverses of its diagonal blocks (used by the solves).
 struct LU64 {

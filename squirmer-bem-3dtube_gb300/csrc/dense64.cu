@@ -86,15 +86,20 @@ __global__ void __launch_bounds__(256) dgemm_kernel(int M, int N, int K, double 
 // Products with up to 8 columns (right-hand sides).  Reading A is the work: 8 bytes
 // per 2 n FP64 operations, so above n = 2 the FP64 pipe bounds it.  The 64 x 64
 // tiles above put such a product on a handful of CTAs, each walking all of K.
-constexpr int SK_N = 8;
+struct Strides {
+    long long a = 0, b = 0, c = 0;  // from one matrix of a batch (blockIdx.y) to the next
+};
 
 // C = alpha A B + beta C, A column-major: 32 rows per CTA, 8 warps split K, each
 // lane one row (a column's 32 rows are one 256-byte read).
 template <int N>
 __global__ void __launch_bounds__(256) skinny_n_kernel(int M, int K, double alpha, const double* __restrict__ A,
                                                        long long lda, const double* __restrict__ B, long long ldb,
-                                                       double beta, double* __restrict__ C, long long ldc) {
+                                                       double beta, double* __restrict__ C, long long ldc, Strides bs) {
     __shared__ double part[8][N][32];
+    A += blockIdx.y * bs.a;
+    B += blockIdx.y * bs.b;
+    C += blockIdx.y * bs.c;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int m = blockIdx.x * 32 + lane;
     double acc[N];
@@ -125,7 +130,10 @@ __global__ void __launch_bounds__(256) skinny_n_kernel(int M, int K, double alph
 template <int N>
 __global__ void __launch_bounds__(256) skinny_t_kernel(int M, int K, double alpha, const double* __restrict__ A,
                                                        long long lda, const double* __restrict__ B, long long ldb,
-                                                       double beta, double* __restrict__ C, long long ldc) {
+                                                       double beta, double* __restrict__ C, long long ldc, Strides bs) {
+    A += blockIdx.y * bs.a;
+    B += blockIdx.y * bs.b;
+    C += blockIdx.y * bs.c;
     const int lane = threadIdx.x & 31, m = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (m >= M) return;
     double acc[N];
@@ -152,14 +160,31 @@ __global__ void __launch_bounds__(256) skinny_t_kernel(int M, int K, double alph
 
 template <int N>
 static void skinny(bool ta, int M, int K, double alpha, const double* A, long long lda, const double* B, long long ldb,
-                   double beta, double* C, long long ldc, cudaStream_t st) {
-    const double fl = 2.0 * M * N * K, by = 8.0 * ((double)M * K + (double)K * N + (beta == 0.0 ? 1.0 : 2.0) * M * N);
+                   double beta, double* C, long long ldc, cudaStream_t st, int batch, Strides bs) {
+    const double fl = 2.0 * batch * M * N * K, by = batch * 8.0 * ((double)M * K + (double)K * N + (beta == 0.0 ? 1.0 : 2.0) * M * N);
     if (ta)
-        TIMED_LAUNCH("dgemm", fl, by, skinny_t_kernel<N>, ceil_div(M, 8), 256, 0, st, M, K, alpha, A, lda, B, ldb, beta,
-                     C, ldc);
+        TIMED_LAUNCH("dgemm", fl, by, skinny_t_kernel<N>, dim3(ceil_div(M, 8), batch), 256, 0, st, M, K, alpha, A, lda, B,
+                     ldb, beta, C, ldc, bs);
     else
-        TIMED_LAUNCH("dgemm", fl, by, skinny_n_kernel<N>, ceil_div(M, 32), 256, 0, st, M, K, alpha, A, lda, B, ldb, beta,
-                     C, ldc);
+        TIMED_LAUNCH("dgemm", fl, by, skinny_n_kernel<N>, dim3(ceil_div(M, 32), batch), 256, 0, st, M, K, alpha, A, lda, B,
+                     ldb, beta, C, ldc, bs);
+}
+
+void gemm64_few(bool ta, int M, int N, int K, double alpha, const double* A, long long lda, const double* B,
+                long long ldb, double beta, double* C, long long ldc, cudaStream_t st, int batch, long long sa,
+                long long sb, long long sc) {
+    const Strides bs{sa, sb, sc};
+    switch (N) {
+        case 1: return skinny<1>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st, batch, bs);
+        case 2: return skinny<2>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st, batch, bs);
+        case 3: return skinny<3>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st, batch, bs);
+        case 4: return skinny<4>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st, batch, bs);
+        case 5: return skinny<5>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st, batch, bs);
+        case 6: return skinny<6>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st, batch, bs);
+        case 7: return skinny<7>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st, batch, bs);
+        case 8: return skinny<8>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st, batch, bs);
+        default: fail(SQBEM_ERR_ARG, "gemm64_few: %d columns", N);
+    }
 }
 
 // The digit products need about 60 us whatever the size (two splits, a tile's 36
@@ -177,18 +202,7 @@ void gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const double* A
         if (beta == 1.0) return;
         K = 0;
     }
-    if (N <= SK_N && !tb) {
-        switch (N) {
-            case 1: return skinny<1>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
-            case 2: return skinny<2>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
-            case 3: return skinny<3>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
-            case 4: return skinny<4>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
-            case 5: return skinny<5>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
-            case 6: return skinny<6>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
-            case 7: return skinny<7>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
-            default: return skinny<8>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
-        }
-    }
+    if (N <= SK_N && !tb) return gemm64_few(ta, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
     if (use_tensor(M, N, K, err)) {
         OzMat a, b;
         a.split(A, ta ? lda : 1, ta ? 1 : lda, M, K, st);

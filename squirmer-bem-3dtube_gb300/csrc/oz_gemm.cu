@@ -47,7 +47,9 @@ constexpr uint32_t IDESC =
 
 // ---------------------------------------------------------------- digits
 __global__ void oz_exponent_rows(const double* __restrict__ a, long long rs, long long ks, int rows, int k, int kper,
-                                 int* __restrict__ ex) {
+                                 int* __restrict__ ex, long long bs, int eb) {
+    a += blockIdx.z * bs;
+    ex += (long long)blockIdx.z * eb;
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows) return;
     const int c1 = min(k, (int)(blockIdx.y + 1) * kper);
@@ -58,7 +60,10 @@ __global__ void oz_exponent_rows(const double* __restrict__ a, long long rs, lon
 }
 
 // contiguous along k: a warp per row
-__global__ void oz_exponent_cols(const double* __restrict__ a, long long rs, int rows, int k, int* __restrict__ ex) {
+__global__ void oz_exponent_cols(const double* __restrict__ a, long long rs, int rows, int k, int* __restrict__ ex,
+                                 long long bs, int eb) {
+    a += blockIdx.z * bs;
+    ex += (long long)blockIdx.z * eb;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= rows) return;
     int m = 0;
@@ -112,7 +117,11 @@ __device__ __forceinline__ void store_digits(const double (&x)[8], int E, uint4*
 // block.x = 128 rows, block.y = 2 halves of a k16 step; grid.x = row blocks,
 // grid.y strides over the k16 steps.
 __global__ void __launch_bounds__(256) oz_split(const double* __restrict__ a, long long rs, long long ks, int rows,
-                                                int k, int k16, const int* __restrict__ ex, uint4* __restrict__ out) {
+                                                int k, int k16, const int* __restrict__ ex, uint4* __restrict__ out,
+                                                long long bs, int eb) {
+    a += blockIdx.z * bs;
+    ex += (long long)blockIdx.z * eb;
+    out += (long long)blockIdx.z * (eb / TILE) * k16 * (BLOCK / 16);
     const int r = blockIdx.x * TILE + threadIdx.x;
     const int E = r < rows ? ex[r] : 0;
     const bool ok = r < rows && E != 0x7ff;
@@ -129,10 +138,14 @@ __global__ void __launch_bounds__(256) oz_split(const double* __restrict__ a, lo
 // and solves): a CTA holds 32 rows' values of all k in shared memory, so each is read
 // from global memory once.  About 90 integer operations per value bound it: with 128
 // rows per CTA a 3840 x 128 panel sat on 30 SMs for 20 us.
-constexpr int FUSED_K = 256;
+constexpr int FUSED_K = 512;
 constexpr int FUSED_SMEM = FUSED_K * 33 * 8;
 __global__ void __launch_bounds__(256) oz_split_fused(const double* __restrict__ a, long long rs, long long ks, int rows,
-                                                      int k, int k16, int* __restrict__ ex, uint4* __restrict__ out) {
+                                                      int k, int k16, int* __restrict__ ex, uint4* __restrict__ out,
+                                                      long long bs, int eb) {
+    a += blockIdx.z * bs;
+    ex += (long long)blockIdx.z * eb;
+    out += (long long)blockIdx.z * (eb / TILE) * k16 * (BLOCK / 16);
     extern __shared__ double xs[];  // [k][33]
     __shared__ int em[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r0 = blockIdx.x * 32;
@@ -182,6 +195,8 @@ struct OzArgs {
     long long ldc;
     const double *srcA, *srcB;  // rows with an infinity or a NaN are summed from these
     long long ars, aks, brs, bks;
+    int batch;
+    long long cb, abs, bbs;     // batch strides of C and of the sources
     long long* stash;           // 16384 sums per CTA
     int* err;
     long long wait;
@@ -206,7 +221,10 @@ __device__ __forceinline__ uint64_t oz_desc(uint32_t addr) {
 
 // C tiles in groups of 12 tile rows, the rows innermost: 152 CTAs then cover a patch
 // of about 12 x 13 tiles, whose operands are re-read from L2 and not from HBM.
-__device__ __forceinline__ void tile_at(const OzArgs& g, int t, int& tm, int& tn) {
+__device__ __forceinline__ void tile_at(const OzArgs& g, int t, int& b, int& tm, int& tn) {
+    const int one = g.tiles_m * g.tiles_n;
+    b = t / one;
+    t -= b * one;
     const int per = 12 * g.tiles_n, grp = t / per, r = t - grp * per;
     const int h = min(12, g.tiles_m - grp * 12);
     tn = r / h;
@@ -356,7 +374,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
     const uint32_t done_bar = smem_u32(bars + 2 * STAGES + 4);
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 5);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles = g.tiles_m * g.tiles_n, k16 = g.k16, ng = n_groups(k16);
+    const int tiles = g.tiles_m * g.tiles_n * g.batch, k16 = g.k16, ng = n_groups(k16);
     int* const err = g.err;
     const long long wait = g.wait;
 
@@ -390,10 +408,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
         int armed[STAGES] = {};
         bool ok = true;
         for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
-            int tm, tn;
-            tile_at(g, t, tm, tn);
-            const uint8_t* A = g.A + (long long)tm * k16 * BLOCK;
-            const uint8_t* B = g.B + (long long)tn * k16 * BLOCK;
+            int tb, tm, tn;
+            tile_at(g, t, tb, tm, tn);
+            const uint8_t* A = g.A + ((long long)tb * g.tiles_m + tm) * k16 * BLOCK;
+            const uint8_t* B = g.B + ((long long)tb * g.tiles_n + tn) * k16 * BLOCK;
             for (int q = 0; ok && q < ng; ++q) {
                 const Group G = group_at(q, k16);
                 const int sp = steps_per_stage(G.p);
@@ -469,16 +487,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
         uint32_t aph = 0;
         bool ok = true;
         for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
-            int tm, tn;
-            tile_at(g, t, tm, tn);
+            int tb, tm, tn;
+            tile_at(g, t, tb, tm, tn);
+            const int* const exA = g.exA + (long long)tb * g.tiles_m * TILE;
+            const int* const exB = g.exB + (long long)tb * g.tiles_n * TILE;
             const int m = tm * TILE + row, n0 = tn * TILE + col0, nc = min(64, g.N - n0);
             const bool mine = m < g.M;
             // exponents: this thread's row, and two of the warp's 64 columns per lane
-            const int Ea = mine ? g.exA[m] : 0;
-            const int Eb0 = lane < nc ? g.exB[n0 + lane] : 0, Eb1 = lane + 32 < nc ? g.exB[n0 + 32 + lane] : 0;
+            const int Ea = mine ? exA[m] : 0;
+            const int Eb0 = lane < nc ? exB[n0 + lane] : 0, Eb1 = lane + 32 < nc ? exB[n0 + 32 + lane] : 0;
             const bool special = __any_sync(0xffffffffu, Ea == 0x7ff || Eb0 == 0x7ff || Eb1 == 0x7ff);
             const int ea = max(Ea, 1);
-            double* const Cm = g.C + m + (long long)n0 * g.ldc;
+            double* const Cm = g.C + tb * g.cb + m + (long long)n0 * g.ldc;
             const double alpha = g.alpha, beta = g.beta;
             long long sum[64];
 #pragma unroll
@@ -590,7 +610,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
                     const long long n = n0 + c;
                     double r = g.srcB ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
                     for (int k = 0; g.srcB && k < g.K; ++k)
-                        r = fma(g.srcA[m * g.ars + k * g.aks], g.srcB[n * g.brs + k * g.bks], r);
+                        r = fma(g.srcA[tb * g.abs + m * g.ars + k * g.aks], g.srcB[tb * g.bbs + n * g.brs + k * g.bks], r);
                     double* const o = Cm + c * g.ldc;
                     *o = beta == 0.0 ? alpha * r : fma(alpha, r, beta * *o);
                 }
@@ -620,37 +640,42 @@ static void set_up() {
     });
 }
 
-void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int k_, cudaStream_t st) {
+void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int k_, cudaStream_t st, int batch_,
+                  long long bs_) {
     set_up();
     rows = rows_;
     k = k_;
     k16 = ceil_div(k, 16);
+    batch = batch_;
     src = a;
     rs = rs_;
     ks = ks_;
-    const int rb = ceil_div(rows, TILE);
-    d.alloc((size_t)rb * k16 * (BLOCK / 16), st);
-    ex.alloc(rows, st);
+    bs = bs_;
+    const int rb = ceil_div(rows, TILE), eb = rb * TILE;
+    d.alloc((size_t)batch * rb * k16 * (BLOCK / 16), st);
+    ex.alloc((size_t)batch * eb, st);
     if (k <= FUSED_K && (rs == 1 || ks == 1)) {
-        LAUNCH(oz_split_fused, ceil_div(rows, 32), 256, k16 * 16 * 33 * 8, st, a, rs, ks, rows, k, k16, ex.get(), d.get());
+        LAUNCH(oz_split_fused, dim3(ceil_div(rows, 32), 1, batch), 256, k16 * 16 * 33 * 8, st, a, rs, ks, rows, k, k16,
+               ex.get(), d.get(), bs, eb);
         return;
     }
     if (ks == 1) {
-        LAUNCH(oz_exponent_cols, ceil_div(rows, 8), 256, 0, st, a, rs, rows, k, ex.get());
+        LAUNCH(oz_exponent_cols, dim3(ceil_div(rows, 8), 1, batch), 256, 0, st, a, rs, rows, k, ex.get(), bs, eb);
     } else {
         ex.zero();
         const int kper = 32;
-        LAUNCH(oz_exponent_rows, dim3(rb, ceil_div(k, kper)), TILE, 0, st, a, rs, ks, rows, k, kper, ex.get());
+        LAUNCH(oz_exponent_rows, dim3(rb, ceil_div(k, kper), batch), TILE, 0, st, a, rs, ks, rows, k, kper, ex.get(), bs,
+               eb);
     }
     // about four CTAs per SM's worth of k16 steps
-    const int gy = std::max(1, std::min(k16, 152 * 8 / rb));
-    LAUNCH(oz_split, dim3(rb, gy), dim3(TILE, 2), 0, st, a, rs, ks, rows, k, k16, ex.get(), d.get());
+    const int gy = std::max(1, std::min(k16, 152 * 8 / (rb * batch)));
+    LAUNCH(oz_split, dim3(rb, gy, batch), dim3(TILE, 2), 0, st, a, rs, ks, rows, k, k16, ex.get(), d.get(), bs, eb);
 }
 
 void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* C, long long ldc, int* err,
-             cudaStream_t st) {
-    if (A.rows <= 0 || B.rows <= 0) return;
-    if (A.k != B.k || A.k <= 0 || ldc < A.rows || !err) fail(SQBEM_ERR_ARG, "oz_gemm: bad arguments");
+             cudaStream_t st, long long cb) {
+    if (A.rows <= 0 || B.rows <= 0 || A.batch <= 0) return;
+    if (A.k != B.k || A.k <= 0 || A.batch != B.batch || ldc < A.rows || !err) fail(SQBEM_ERR_ARG, "oz_gemm: bad arguments");
     set_up();
     OzArgs g;
     g.A = reinterpret_cast<const uint8_t*>(A.d.get());
@@ -670,18 +695,22 @@ void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* 
     g.srcA = A.src;
     g.ars = A.rs;
     g.aks = A.ks;
-    g.srcB = C == B.src ? nullptr : B.src;
+    g.srcB = C == B.src || C == A.src ? nullptr : B.src;
     g.brs = B.rs;
     g.bks = B.ks;
-    const int grid = std::min(g.tiles_m * g.tiles_n, g_sms);
+    g.batch = A.batch;
+    g.cb = cb;
+    g.abs = A.bs;
+    g.bbs = B.bs;
+    const int grid = std::min(g.tiles_m * g.tiles_n * g.batch, g_sms);
     const bool brief = g.k16 <= HI_CHUNK;
     DevBuf<long long> stash(brief ? 0 : (size_t)grid * TILE * TILE, st);
     g.stash = stash.get();
     g.err = err;
     g.wait = gemm_wait_cycles();
     // credited as BF16 tensor work: 36 digit products
-    const double fl = 72.0 * g.M * g.N * g.K,
-                 by = 16.0 * ((double)g.M + g.N) * g.K + (beta == 0.0 ? 8.0 : 16.0) * g.M * g.N;
+    const double fl = 72.0 * g.batch * g.M * g.N * g.K,
+                 by = g.batch * (16.0 * ((double)g.M + g.N) * g.K + (beta == 0.0 ? 8.0 : 16.0) * g.M * g.N);
     if (brief) TIMED_LAUNCH("oz_gemm", fl, by, oz_gemm_kernel<true>, grid, NTHREADS, SMEM_BYTES, st, g);
     else TIMED_LAUNCH("oz_gemm", fl, by, oz_gemm_kernel<false>, grid, NTHREADS, SMEM_BYTES, st, g);
 }

@@ -25,19 +25,22 @@ namespace sqbem {
 struct OzMat {
     DevBuf<uint4> d;
     DevBuf<int> ex;
-    int rows = 0, k = 0, k16 = 0;
+    int rows = 0, k = 0, k16 = 0, batch = 1;
     // the values' source, for rows that hold an infinity or a NaN
     const double* src = nullptr;
-    long long rs = 0, ks = 0;
-    // element (r, c) of the operand is a[r * rs + c * ks]
-    void split(const double* a, long long rs, long long ks, int rows, int k, cudaStream_t st);
+    long long rs = 0, ks = 0, bs = 0;
+    // element (r, c) of matrix b is a[r * rs + c * ks + b * bs]
+    void split(const double* a, long long rs, long long ks, int rows, int k, cudaStream_t st, int batch = 1,
+               long long bs = 0);
 };
 
 // C (M x N, column-major) = alpha A B + beta C for the digits of A (M rows) and of
-// B (N columns, given as rows) over the same k.  The sources of A and B must be
-// alive and unchanged until the launch has run, and C must not overlap them.
-// *err is set if a bounded wait expires (SQBEM_ERR_TIMEOUT to the caller).
+// B (N columns, given as rows) over the same k, for every matrix of the batch (C at
+// stride cb).  The sources of A and B must be alive and unchanged until the launch has
+// run; C may be one of them (its rows and columns with an infinity or a NaN then give
+// NaN), but must not overlap them otherwise.  *err is set if a bounded wait expires
+// (SQBEM_ERR_TIMEOUT to the caller).
 void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* C, long long ldc, int* err,
-             cudaStream_t st);
+             cudaStream_t st, long long cb = 0);
 
 }  // namespace sqbem

@@ -90,12 +90,31 @@ void sqbem_tube::build_device() {
         CUDA_CHECK(cudaStreamSynchronize(st));
         return;
     }
+    const TubeSymmetry sym = tube_symmetry(host_panels, n_theta);
+    if (circulant64_supported(sym)) {
+        DevBuf<double> T0((size_t)3 * sym.nb * n, st);
+        DevBuf<int> tie(1, st);
+        tie.zero();
+        assemble_sector0(host_panels, panels.rec.get(), sym, mu, T0.get(), nullptr, tie.get(), st);
+        deflate_sector0(T0.get(), panels.rec.get(), sym, Nt, 1.0 / (EIGHT_PI * mu * std::sqrt(panels.area_total)), st);
+        if (circ.build(sym, T0.get(), tie.get(), st)) return;
+    }
     DevBuf<double> T((size_t)n * n, st);
     auto job = block_job<double>(panels, panels, true, mu, T.get(), n, nullptr, 0);
     assemble_block(job, near_capacity(Nt, Nt), st, false);
     deflate(T.get(), 1, n, panels, mu, st);
     lu.factor_inplace(std::move(T), n, st, "dgetrf failed");
     CUDA_CHECK(cudaStreamSynchronize(st));
+}
+
+void sqbem_tube::solve64(double* B, long long ldb, int nrhs, cudaStream_t s, int* err) const {
+    if (circ.ready) circ.solve(B, ldb, nrhs, s, err);
+    else lu.solve(B, ldb, nrhs, s, err);
+}
+
+void sqbem_tube::solve64_transpose(double* B, long long ldb, int nrhs, cudaStream_t s) const {
+    if (circ.ready) circ.solve(B, ldb, nrhs, s, nullptr, true);
+    else lu.solve_transpose(B, ldb, nrhs, s);
 }
 
 // ---------------------------------------------------------------- SwimmerSolver
@@ -174,7 +193,7 @@ void sqbem_swimmer::build_fp64() {
     if (tube) {
         // Y = T^{-1} [B | Ct];  Gs = E - D Y_s;  Gc = Cs - D Y_c  (238-249)
         WaitError we;
-        tube->lu.solve(Y.get(), nt, ns + 6, st, we.get(st));
+        tube->solve64(Y.get(), nt, ns + 6, st, we.get(st));
         gemm64(false, false, ns, ns, nt, -1.0, D.get(), ns, Y.get(), nt, 1.0, Gs.get(), ns, st, we.get(st));
         gemm64(false, false, ns, 6, nt, -1.0, D.get(), ns, Y.get() + (size_t)nt * ns, nt, 1.0, Gc.get(), ns, st);
         clock2.stop(st);
@@ -224,7 +243,7 @@ void sqbem_swimmer::solve_free(int nrhs, const double* slips, double* U, double*
     if (tube) {
         rt.alloc((size_t)nt * nrhs, st);
         gemm64(false, false, nt, nrhs, ns, -1.0, AuBt.get(), nt, u.get(), ns, 0.0, rt.get(), nt, st);
-        tube->lu.solve(rt.get(), nt, nrhs, st);
+        tube->solve64(rt.get(), nt, nrhs, st);
         gemm64(false, false, ns, nrhs, nt, -1.0, D.get(), ns, rt.get(), nt, 1.0, Rh.get(), n, st);
     }
     luM.solve(Rh.get(), n, nrhs, st);
@@ -278,6 +297,48 @@ void sqbem_swimmer::solve_prescribed(const double* U, const double* Om, double* 
 }
 
 // ---------------------------------------------------------------- DuctFlow
+// The boundary data of every solve -- one pressure per cap, no slip -- is the same in every
+// sector, so the solution is too: only the part of the system that acts on vectors which
+// a rotation by a sector maps onto themselves is needed (order 3 nb instead of 3 P), and
+// its rows are those of sector 0.  False if a pair sits on a quadrature threshold.
+bool sqbem_duct::build_symmetric(const std::vector<PanelRec>& hp) {
+    const TubeSymmetry sym = tube_symmetry(hp, nth);
+    if (!circulant64_supported(sym)) return false;
+    const int n3 = 3 * sym.nb, n = 3 * P, ncap = (int)cap.size();
+    DevBuf<double> S((size_t)n3 * n, st), D((size_t)n3 * n, st), M((size_t)n3 * n3, st), rsum((size_t)n3 * 3, st);
+    DevBuf<int> tie(1, st), dp(sym.panel.size(), st), dz(std::max(ncap, 1), st);
+    tie.zero();
+    rsum.zero();
+    dp.upload(sym.panel.data(), sym.panel.size());
+    assemble_sector0(hp, panels.rec.get(), sym, mu, S.get(), D.get(), tie.get(), st);
+    add_rowsums(D.get(), 1, n3, n3, P, rsum.get(), st);
+    std::vector<int> zcols(ncap);
+    for (int k = 0; k < ncap; ++k) zcols[k] = 3 * cap[k] + 2;
+    if (ncap) dz.upload(zcols.data(), ncap);
+    Fk.alloc((size_t)n3 * std::max(ncap, 1), st);
+    if (ncap) {
+        LAUNCH(gather_cols_kernel, ceil_div((long long)n3 * ncap, 256), 256, 0, st, S.get(), n3, dz.get(), ncap, n3,
+               Fk.get(), n3);
+        LAUNCH(copy_cols_kernel, ceil_div((long long)n3 * ncap, 256), 256, 0, st, D.get(), n3, dz.get(), ncap, n3,
+               S.get(), n3);
+    }
+    fold_sector0(S.get(), dp.get(), sym.nth, sym.nb, M.get(), st);
+    std::vector<unsigned char> mask(sym.nb, 0);
+    for (int a = 0; a < sym.nb; ++a)
+        if (mesh.tags[sym.rep_panel[a]] != bem::WALL) mask[a] = 4;
+    DevBuf<unsigned char> dmask(sym.nb, st);
+    dmask.upload(mask.data(), sym.nb);
+    diag_complete(M.get(), 1, n3, sym.nb, rsum.get(), 0.0, dmask.get(), st);
+    int h = 0;
+    tie.download(&h, 1);
+    CUDA_CHECK(cudaStreamSynchronize(st));
+    if (h) return false;
+    lu.factor_inplace(std::move(M), n3, st, "dgetrf failed");
+    nb = sym.nb;
+    panel = sym.panel;
+    return true;
+}
+
 void sqbem_duct::build(double R_, double L_, int nth, int nz, int nr, double mu_, int prec) {
     R = R_; L = L_; mu = mu_; precision = prec;
     mesh = bem::tube_mesh(R, bem::uniform_z(0, L, nz), nth, nr);
@@ -290,6 +351,8 @@ void sqbem_duct::build(double R_, double L_, int nth, int nz, int nr, double mu_
     for (int p = 0; p < P; ++p)
         if (mesh.tags[p] != bem::WALL) cap.push_back(p);
     const int ncap = (int)cap.size();
+    this->nth = nth;
+    if (build_symmetric(hp)) return;
     // A_f = SL/(8 pi mu) into M, A_u = -DL/(8 pi) into Dsc   (duct_flow.hpp:373-397)
     DevBuf<double> M((size_t)n * n, st), Dsc((size_t)n * n, st);
     auto job = block_job<double>(panels, panels, true, mu, M.get(), n, Dsc.get(), n);
@@ -325,14 +388,28 @@ void sqbem_duct::solve(double p_in, double p_out, double* u, double* f, double* 
     const int n = 3 * P, ncap = (int)cap.size();
     std::vector<double> fk(ncap);
     for (int k = 0; k < ncap; ++k) fk[k] = mesh.tags[cap[k]] == bem::INLET ? p_in : -p_out;
-    DevBuf<double> dfk(std::max(ncap, 1), st), rhs((size_t)n, st);
+    const int rows = lu.n;
+    DevBuf<double> dfk(std::max(ncap, 1), st), rhs((size_t)rows, st);
     if (ncap) dfk.upload(fk.data(), ncap);
     // rhs = -Fk fk (known u are all zero), x = M^{-1} rhs   (duct_flow.hpp:41-63)
-    gemm64(false, false, n, 1, ncap, -1.0, Fk.get(), n, dfk.get(), std::max(ncap, 1), 0.0, rhs.get(), n, st);
-    lu.solve(rhs.get(), n, 1, st);
-    std::vector<double> x(n);
-    rhs.download(x.data(), n);
+    gemm64(false, false, rows, 1, ncap, -1.0, Fk.get(), rows, dfk.get(), std::max(ncap, 1), 0.0, rhs.get(), rows, st);
+    lu.solve(rhs.get(), rows, 1, st);
+    std::vector<double> x(rows);
+    rhs.download(x.data(), rows);
     CUDA_CHECK(cudaStreamSynchronize(st));
+    if (nb > 0) {  // sector 0's solution, rotated into every sector
+        const std::vector<double> x0 = std::move(x);
+        x.assign((size_t)n, 0.0);
+        for (int s = 0; s < nth; ++s) {
+            const double c = std::cos(2 * bem::PI * s / nth), sn = std::sin(2 * bem::PI * s / nth);
+            for (int a = 0; a < nb; ++a) {
+                double* o = x.data() + 3 * (size_t)panel[a * nth + s];
+                o[0] = c * x0[3 * a] - sn * x0[3 * a + 1];
+                o[1] = sn * x0[3 * a] + c * x0[3 * a + 1];
+                o[2] = x0[3 * a + 2];
+            }
+        }
+    }
     std::vector<double> uu((size_t)n, 0.0), ff((size_t)n, 0.0);
     for (int p = 0; p < P; ++p)
         for (int b = 0; b < 3; ++b) {

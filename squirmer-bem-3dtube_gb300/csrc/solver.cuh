@@ -7,6 +7,7 @@
 
 #include "assemble.cuh"
 #include "bem/utils/mesh.hpp"
+#include "circulant64.cuh"
 #include "common.cuh"
 #include "dense.cuh"
 #include "mixed.cuh"
@@ -82,11 +83,17 @@ struct sqbem_tube {
     int Nt = 0;
     std::vector<sqbem::PanelRec> host_panels;
     sqbem::DevPanels panels;
-    sqbem::LU64 lu;           // FP64 factor of the deflated T
+    // FP64: the deflated T through its Fourier blocks, or its factor where the mesh has no
+    // symmetry to use
+    sqbem::Circulant64 circ;
+    sqbem::LU64 lu;
     sqbem::MixedTube mt;      // mixed: FP32 T (for residuals) and its split-BF16 factor
     void build(double R, double L, double a, int n_theta, int n_r, double mu, int precision);
     void build_device();  // from `mesh` and the parameters already set
     void set_panels();    // panel records only (the grouped mixed build factors later)
+    // FP64: B <- T^{-1} B or T^{-T} B (3 Nt x nrhs); err as in gemm64
+    void solve64(double* B, long long ldb, int nrhs, cudaStream_t st, int* err = nullptr) const;
+    void solve64_transpose(double* B, long long ldb, int nrhs, cudaStream_t st) const;
 };
 
 // host slip field (kernels.hpp:107-111) at the panel centroids, packed xyz
@@ -149,8 +156,11 @@ struct sqbem_duct {
     int P = 0;
     std::vector<int> cap;  // cap panel indices (columns of Fk)
     sqbem::DevPanels panels;
-    sqbem::LU64 lu;
-    sqbem::DevBuf<double> Fk;
+    sqbem::LU64 lu;            // of the whole system, or (nb > 0) of its n_theta-fold symmetric part
+    sqbem::DevBuf<double> Fk;  // the cap columns of the rows of lu
+    int nb = 0, nth = 0;       // panels per sector, sectors
+    std::vector<int> panel;    // nb x nth: panel[a * nth + s]
+    bool build_symmetric(const std::vector<sqbem::PanelRec>& hp);
     void build(double R, double L, int n_theta, int n_z, int n_r, double mu, int precision);
     void solve(double p_in, double p_out, double* u, double* f, double* Q);
 };

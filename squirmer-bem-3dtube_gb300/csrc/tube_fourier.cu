@@ -596,6 +596,23 @@ bool fourier_supported(const TubeSymmetry& sym) {
            gj_cluster(3 * sym.nb) > 0;
 }
 
+void gauss_jordan_blocks(float2* C, int nblk, int n3, int* flag, cudaStream_t st) {
+    const int cl = gj_cluster(n3);
+    if (!cl) fail(SQBEM_ERR_ARG, "Gauss-Jordan: block order %d too large", n3);
+    set_smem_limits();
+    for (int b0 = 0; b0 < nblk; b0 += GJ_MAXB) {
+        GjArgs g;
+        g.n = n3;
+        g.w = (n3 + cl - 1) / cl;
+        g.nblk = std::min(GJ_MAXB, nblk - b0);
+        g.flag = flag;
+        for (int b = 0; b < g.nblk; ++b) g.C[b] = C + (size_t)(b0 + b) * n3 * n3;
+        const double fl = 8.0 * g.nblk * (double)n3 * n3 * n3, by = 16.0 * g.nblk * (double)n3 * n3;
+        if (cl == 2) TIMED_LAUNCH("fourier_inverse", fl, by, gj_kernel<2>, 2 * g.nblk, GJ_THREADS, gj_smem(n3, cl), st, g);
+        else TIMED_LAUNCH("fourier_inverse", fl, by, gj_kernel<4>, 4 * g.nblk, GJ_THREADS, gj_smem(n3, cl), st, g);
+    }
+}
+
 void fourier_build(const std::vector<FourierTube*>& fts, const std::vector<const TubeSymmetry*>& syms,
                    const std::vector<const float*>& T0s, const MixedCtx& cx) {
     // tubes of equal sector count and block order go through the same launches

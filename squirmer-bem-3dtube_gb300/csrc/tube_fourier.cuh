@@ -39,6 +39,10 @@ struct FourierTube {
     DevBuf<bf16> Ah, Al;          // nf real forms of the block inverses, m2 x m2 row-major (ld ldk), split
 };
 
+// In-place inverses of nblk complex blocks of order n3 (column-major, one after the
+// other) by Gauss-Jordan with partial pivoting in FP32; a zero pivot sets bit 1 of *flag.
+void gauss_jordan_blocks(float2* C, int nblk, int n3, int* flag, cudaStream_t st);
+
 // Whether a tube with this symmetry takes the Fourier path (n_theta and block
 // order within the kernels' limits).
 bool fourier_supported(const TubeSymmetry& sym);
