@@ -29,6 +29,7 @@
 // rounded once; the far (7) and near (28/112) rules are evaluated in FP32 from
 // them, while the 448-point near-singular rule and the Duffy self integrals stay
 // FP64, with a reciprocal square root refined from an FP32 seed (rsqrt_nr).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,6 +40,8 @@
 #include "assemble.cuh"
 #include "bem/utils/quadrature.hpp"
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace sqbem {
 
@@ -798,103 +801,368 @@ void panel_pairs(int n, const PanelRec* P, const double* x0, const int* self, do
 
 // ---------------------------------------------------------------- field
 // u_j(x0) = sum_p [SL_p,ij f_p,i / (8 pi mu) - DL_p,ij u_p,i / (8 pi)]  (field.hpp:18-34)
-// One warp per point: pass 1, the lanes take the panels round-robin and apply the
-// 7-point rule to far panels while near panels (d < 3) are collected in shared
-// memory; pass 2, the whole warp integrates each near panel (lanes split the
-// rule points).  Fixed order, hence deterministic.
-constexpr int FIELD_WARPS = 4;
+//
+// The lanes of a warp take panels, a warp PPW points (so that a staged panel serves
+// several), or, for few points, the eight warps of a CTA (and the CTAs of a cluster)
+// one point.  Pass 1 applies the 7-point rule to far panels while near ones (d < 3) are
+// collected, in panel order, in shared memory; in pass 2 the warp integrates each near
+// panel, its lanes splitting the rule's points.  Fixed order, hence deterministic.
+//
+// What bounds it is the FP64 pipe (64 cycles a warp instruction), so each panel's share of
+// a tile is prepared once in shared memory, and
+//   FP64    a flat panel's r.m is the same at all its nodes, and the node sums are formed
+//           contracted: sum_q w f / r and sum_q (..) r, 27 FP64 operations a node;
+//   mixed   nothing per pair is FP64: the rule by the bands of far_kernel_f32, the vertex
+//           offsets V - x0 from FP32 pairs (TwoDiff, rounded as the FP64 difference's
+//           conversion is but for one in 10^7), the products with f and u as FP32 pairs
+//           (Dot2) within a tile's common power of two.
+// 18 k points x 1712 panels in mixed precision: 12.5 ms with FP64 offsets, rule tests and
+// products per pair.
+constexpr int FIELD_WARPS = 8;
 constexpr int FIELD_NEAR_CAP = 256;
+constexpr int FT32 = 47, FT64 = 35;  // words per staged panel (odd: lanes on different banks)
 
+__device__ __forceinline__ void two_diff(float a, float b, float& s, float& e) {
+    s = __fsub_rn(a, b);
+    const float t = __fsub_rn(s, a);
+    e = __fsub_rn(__fsub_rn(a, __fsub_rn(s, t)), __fadd_rn(b, t));
+}
+// (s, c) += a (bh + bl)
+__device__ __forceinline__ void dot2_add(float& s, float& c, float a, float bh, float bl) {
+    const float p = __fmul_rn(a, bh), e = __fmaf_rn(a, bh, -p);
+    const float t = __fadd_rn(s, p), z = __fsub_rn(t, s);
+    c = __fadd_rn(c, __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(p, z)), __fmaf_rn(a, bl, e)));
+    s = t;
+}
+
+struct FieldPoint {
+    double x, y, z, u[3];
+    int near;
+};
+
+// The panel-independent state of a point and its far sum over the panels of a tile, for both
+// arithmetics: stage() writes one panel's record, pair() returns the rule and adds the
+// panel if it is far, flush() moves the tile's sum to FP64.
 template <class TC>
-__global__ void __launch_bounds__(FIELD_WARPS * 32) field_kernel(FieldJob job) {
-    __shared__ int near_p[FIELD_WARPS][FIELD_NEAR_CAP];
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const int pt = blockIdx.x * FIELD_WARPS + wl;
-    if (pt >= job.npts) return;
-    const double x = job.pts[3 * pt], y = job.pts[3 * pt + 1], z = job.pts[3 * pt + 2];
-    double ux = 0, uy = 0, uz = 0;
-    int nnear = 0;
-    int overflow = 0;
-    for (int base = 0; base < job.P; base += 32) {
-        const int p = base + lane;
-        int rule = -1;
-        PanelRec P;
-        if (p < job.P) {
-            P = job.panels[p];
-            rule = rule_of(P, x, y, z);
-        }
-        const unsigned nearmask = __ballot_sync(0xffffffffu, rule > 0);
-        if (rule > 0) {
-            const int slot = nnear + __popc(nearmask & ((1u << lane) - 1));
-            if (slot < FIELD_NEAR_CAP) near_p[wl][slot] = p;
-        }
-        nnear += __popc(nearmask);
-        if (rule == 0) {
-            Acc<TC> A;
-            A.zero();
-            const TC e0x = (TC)(P.v[0] - x), e0y = (TC)(P.v[1] - y), e0z = (TC)(P.v[2] - z);
-            const TC e1x = (TC)(P.v[3] - x), e1y = (TC)(P.v[4] - y), e1z = (TC)(P.v[5] - z);
-            const TC e2x = (TC)(P.v[6] - x), e2y = (TC)(P.v[7] - y), e2z = (TC)(P.v[8] - z);
-            const TC mx = (TC)P.n[0], my = (TC)P.n[1], mz = (TC)P.n[2], area = (TC)P.area;
-#pragma unroll
-            for (int q = 0; q < 7; ++q) {
-                TC l0, l1, l2, w;
-                if constexpr (sizeof(TC) == 8) {
-                    l0 = c_rule7[q].l0; l1 = c_rule7[q].l1; l2 = c_rule7[q].l2; w = c_rule7[q].w;
-                } else {
-                    l0 = c_rule7f[q].l0; l1 = c_rule7f[q].l1; l2 = c_rule7f[q].l2; w = c_rule7f[q].w;
-                }
-                accum<TC, true>(A, l0 * e0x + l1 * e1x + l2 * e2x, l0 * e0y + l1 * e1y + l2 * e2y,
-                                l0 * e0z + l1 * e1z + l2 * e2z, w * area, mx, my, mz);
-            }
-            const double* f = job.f + 3 * p;
-            const double* u = job.u + 3 * p;
-            for (int j = 0; j < 3; ++j) {
-                double s = 0;
-                for (int i = 0; i < 3; ++i)
-                    s += (double)sl_entry(A, i, j) * f[i] * job.sscale + (double)dl_entry(A, i, j) * u[i] * job.dscale;
-                (j == 0 ? ux : j == 1 ? uy : uz) += s;
-            }
-        }
-    }
-    if (nnear > FIELD_NEAR_CAP) overflow = 1;
-    __syncwarp();
-    // warp-reduce the far part (fixed butterfly order)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ux += __shfl_xor_sync(0xffffffffu, ux, o);
-        uy += __shfl_xor_sync(0xffffffffu, uy, o);
-        uz += __shfl_xor_sync(0xffffffffu, uz, o);
-    }
-    const int nn = min(nnear, FIELD_NEAR_CAP);
-    for (int k = 0; k < nn; ++k) {
-        const int p = near_p[wl][k];
+struct FieldArith;
+
+template <>
+struct FieldArith<double> {
+    static constexpr int WORDS = FT64;
+    static __device__ int exponent(const FieldJob&, int) { return 0; }
+    static __device__ void stage(double* d, const FieldJob& job, int p, const double*, int) {
         const PanelRec P = job.panels[p];
-        const int rule = rule_of(P, x, y, z);
-        double sl[9], dl[9];
-        if (job.mixed && rule < 3) {
-            Acc<float> A;
-            warp_rule_f32(A, job.panels + p, x, y, z, rule, lane);
-            for (int q = 0; q < 9; ++q) { sl[q] = sl_entry(A, q / 3, q % 3); dl[q] = dl_entry(A, q / 3, q % 3); }
-        } else {
-            Acc<double> A;
-            if (job.mixed) warp_rule<double, true>(A, P, x, y, z, rule, lane);
-            else warp_rule<double, false>(A, P, x, y, z, rule, lane);
-            for (int q = 0; q < 9; ++q) { sl[q] = sl_entry(A, q / 3, q % 3); dl[q] = dl_entry(A, q / 3, q % 3); }
+        double v[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v[k] = P.v[k] - P.c[k % 3];
+#pragma unroll
+        for (int q = 0; q < 7; ++q)
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                d[3 * q + k] = c_rule7[q].l0 * v[k] + c_rule7[q].l1 * v[3 + k] + c_rule7[q].l2 * v[6 + k];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            d[21 + k] = P.n[k];
+            d[24 + k] = P.c[k];
+            d[28 + k] = job.f[3 * p + k] * (job.sscale * P.area);
+            d[31 + k] = job.u[3 * p + k] * (-6.0 * job.dscale * P.area);
         }
-        const double* f = job.f + 3 * p;
-        const double* u = job.u + 3 * p;
-        for (int j = 0; j < 3; ++j) {
-            double s = 0;
-            for (int i = 0; i < 3; ++i) s += sl[3 * i + j] * f[i] * job.sscale + dl[3 * i + j] * u[i] * job.dscale;
-            (j == 0 ? ux : j == 1 ? uy : uz) += s;
+        d[27] = 9.0 * P.h * P.h * (1.0 + 1e-12);
+    }
+    double a[3];
+    __device__ void point(const FieldPoint&, const double*) {}
+    __device__ void begin() { a[0] = a[1] = a[2] = 0.0; }
+    __device__ int pair(const double* d, const FieldJob& job, int p, const FieldPoint& X, bool) {
+        const double bx = d[24] - X.x, by = d[25] - X.y, bz = d[26] - X.z;
+        // within 1e-12 of the threshold and below: the exact test
+        if (!(bx * bx + by * by + bz * bz > d[27])) {
+            const int rule = rule_of(job.panels[p], X.x, X.y, X.z);
+            if (rule != 0) return rule;
+        }
+        const double rm = bx * d[21] + by * d[22] + bz * d[23];
+        const double fx = d[28], fy = d[29], fz = d[30], gx = d[31] * rm, gy = d[32] * rm, gz = d[33] * rm;
+        double al = 0.0;
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            const double rx = bx + d[3 * q], ry = by + d[3 * q + 1], rz = bz + d[3 * q + 2];
+            const double ir = rsqrt(rx * rx + ry * ry + rz * rz), ir2 = ir * ir, t = c_rule7[q].w * ir;
+            al += t;
+            const double fr = rx * fx + ry * fy + rz * fz, gr = rx * gx + ry * gy + rz * gz;
+            const double be = t * ir2 * fma(gr, ir2, fr);
+            a[0] = fma(be, rx, a[0]);
+            a[1] = fma(be, ry, a[1]);
+            a[2] = fma(be, rz, a[2]);
+        }
+        a[0] = fma(al, fx, a[0]);
+        a[1] = fma(al, fy, a[1]);
+        a[2] = fma(al, fz, a[2]);
+        return 0;
+    }
+    __device__ void flush(FieldPoint& X, double) const {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) X.u[k] += a[k];
+    }
+};
+
+template <>
+struct FieldArith<float> {
+    static constexpr int WORDS = FT32;
+    // the largest biased exponent of f / (8 pi mu) and u / (8 pi) on a panel; 0x7ff: not finite
+    static __device__ int exponent(const FieldJob& job, int p) {
+        int m = 0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            m = max(m, __double2hiint(job.f[3 * p + k] * job.sscale) & 0x7ff00000);
+            m = max(m, __double2hiint(job.u[3 * p + k] * job.dscale) & 0x7ff00000);
+        }
+        return m >> 20;
+    }
+    // lengths relative to the origin o (a point of the CTA); f and u over 2^(ex - 1023)
+    static __device__ void stage(float* d, const FieldJob& job, int p, const double* o, int ex) {
+        const PanelRec P = job.panels[p];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) split2(P.v[k] - o[k % 3], d[k], d[9 + k]);
+        const double h2 = P.h * P.h, sc = ex > 0 && ex < 0x7ff ? scalbn(1.0, 1023 - ex) : 1.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double t = (k == 0 ? 0.5625 : k == 1 ? 2.25 : 9.0) * h2;
+            d[18 + k] = (float)P.n[k];
+            split2(P.c[k] - o[k], d[22 + k], d[25 + k]);
+            d[28 + k] = (float)(t * (1.0 - 1e-5));
+            d[31 + k] = (float)(t * (1.0 + 1e-5));
+            split2(job.f[3 * p + k] * job.sscale * sc, d[34 + k], d[37 + k]);
+            split2(job.u[3 * p + k] * job.dscale * sc, d[40 + k], d[43 + k]);
+        }
+        d[21] = (float)P.area;
+    }
+    float xh[3], xl[3], s[3], c[3];
+    __device__ void point(const FieldPoint& X, const double* o) {
+        split2(X.x - o[0], xh[0], xl[0]);
+        split2(X.y - o[1], xh[1], xl[1]);
+        split2(X.z - o[2], xh[2], xl[2]);
+    }
+    __device__ void begin() {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s[k] = c[k] = 0.f;
+    }
+    __device__ int pair(const float* d, const FieldJob& job, int p, FieldPoint& X, bool special) {
+        const float bx = (d[22] - xh[0]) + (d[25] - xl[0]), by = (d[23] - xh[1]) + (d[26] - xl[1]),
+                    bz = (d[24] - xh[2]) + (d[27] - xl[2]);
+        const float d2 = bx * bx + by * by + bz * bz;
+        if (!(d2 > d[33])) {
+            int rule;
+            if (d2 < d[30] && d2 > d[32]) rule = 1;
+            else if (d2 < d[29] && d2 > d[31]) rule = 2;
+            else if (d2 < d[28]) rule = 3;
+            else rule = rule_of(job.panels[p], X.x, X.y, X.z);
+            if (rule != 0) return rule;
+        }
+        float e[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            float hi, lo;
+            two_diff(d[k], xh[k % 3], hi, lo);
+            e[k] = __fadd_rn(hi, __fadd_rn(lo, __fsub_rn(d[9 + k], xl[k % 3])));
+        }
+        Acc<float> A;
+        A.zero();
+        const float mx = d[18], my = d[19], mz = d[20], area = d[21];
+#pragma unroll
+        for (int q = 0; q < 7; ++q) {
+            const float l0 = c_rule7f[q].l0, l1 = c_rule7f[q].l1, l2 = c_rule7f[q].l2, w = c_rule7f[q].w;
+            accum<float, true>(A, l0 * e[0] + l1 * e[3] + l2 * e[6], l0 * e[1] + l1 * e[4] + l2 * e[7],
+                               l0 * e[2] + l1 * e[5] + l2 * e[8], w * area, mx, my, mz);
+        }
+        if (special) {  // an infinity or a NaN among the tile's f and u: plain products
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    X.u[j] += (double)sl_entry(A, i, j) * job.f[3 * p + i] * job.sscale +
+                              (double)dl_entry(A, i, j) * job.u[3 * p + i] * job.dscale;
+            return 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                dot2_add(s[j], c[j], sl_entry(A, i, j), d[34 + i], d[37 + i]);
+                dot2_add(s[j], c[j], dl_entry(A, i, j), d[40 + i], d[43 + i]);
+            }
+        return 0;
+    }
+    __device__ void flush(FieldPoint& X, double scale) const {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) X.u[k] = fma((double)s[k] + (double)c[k], scale, X.u[k]);
+    }
+};
+
+// One near panel of one point by a warp, added to lane 0 .. 2's u (component = lane).
+template <bool MIXED>
+__device__ void field_near(const FieldJob& job, int p, int rule, const FieldPoint& X, int lane, double& u) {
+    if (MIXED && rule < 3) {
+        Acc<float> A;
+        warp_rule_f32(A, job.panels + p, X.x, X.y, X.z, rule, lane);
+        // lane 3 i + j: the (i, j) terms; lane j collects its column
+        const int i = lane / 3, j = lane - 3 * i;
+        double t = 0.0;
+        if (lane < 9)
+            t = (double)sl_entry(A, i, j) * job.f[3 * p + i] * job.sscale +
+                (double)dl_entry(A, i, j) * job.u[3 * p + i] * job.dscale;
+        t += __shfl_down_sync(0xffffffffu, t, 3) + __shfl_down_sync(0xffffffffu, t, 6);
+        u += t;
+        return;
+    }
+    const PanelRec& P = job.panels[p];
+    const double e0x = P.v[0] - X.x, e0y = P.v[1] - X.y, e0z = P.v[2] - X.z;
+    const double e1x = P.v[3] - X.x, e1y = P.v[4] - X.y, e1z = P.v[5] - X.z;
+    const double e2x = P.v[6] - X.x, e2y = P.v[7] - X.y, e2z = P.v[8] - X.z;
+    const double rm = -6.0 * ((P.c[0] - X.x) * P.n[0] + (P.c[1] - X.y) * P.n[1] + (P.c[2] - X.z) * P.n[2]);
+    const double ss = job.sscale * P.area, ds = job.dscale * P.area * rm;
+    const double fx = job.f[3 * p] * ss, fy = job.f[3 * p + 1] * ss, fz = job.f[3 * p + 2] * ss;
+    const double gx = job.u[3 * p] * ds, gy = job.u[3 * p + 1] * ds, gz = job.u[3 * p + 2] * ds;
+    double al = 0.0, a0 = 0.0, a1 = 0.0, a2 = 0.0;
+    const int q1 = rule_off(rule + 1);
+    for (int q = rule_off(rule) + lane; q < q1; q += 32) {
+        const QPoint Q = d_rule[q];
+        const double rx = Q.l0 * e0x + Q.l1 * e1x + Q.l2 * e2x;
+        const double ry = Q.l0 * e0y + Q.l1 * e1y + Q.l2 * e2y;
+        const double rz = Q.l0 * e0z + Q.l1 * e1z + Q.l2 * e2z;
+        const double ir = rsqrt(rx * rx + ry * ry + rz * rz), ir2 = ir * ir, t = Q.w * ir;
+        al += t;
+        const double be = t * ir2 * fma(rx * gx + ry * gy + rz * gz, ir2, rx * fx + ry * fy + rz * fz);
+        a0 = fma(be, rx, a0);
+        a1 = fma(be, ry, a1);
+        a2 = fma(be, rz, a2);
+    }
+    a0 = fma(al, fx, a0);
+    a1 = fma(al, fy, a1);
+    a2 = fma(al, fz, a2);
+    // three sums over the warp: lane groups 0, 1 mod 4 and 2 mod 4 end with one component each
+    const double k0 = __shfl_xor_sync(0xffffffffu, a0, 1), k1 = __shfl_xor_sync(0xffffffffu, a1, 1),
+                 k2 = __shfl_xor_sync(0xffffffffu, a2, 1);
+    double v = (lane & 1) ? a1 + k1 : a0 + k0, w = a2 + k2;
+    const double vw = __shfl_xor_sync(0xffffffffu, v, 2), ww = __shfl_xor_sync(0xffffffffu, w, 2);
+    v = (lane & 2) ? w + ww : v + vw;  // lanes 0, 1, 2 (mod 4): components 0, 1, 2 (3: 2 again)
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    u += v;
+}
+
+// PPW points per warp, each warp all panels; or (SHARED) one point per CTA -- per
+// cluster -- whose warps and CTAs share the panels.
+template <class TC, int PPW, bool SHARED>
+__global__ void __launch_bounds__(FIELD_WARPS * 32) field_kernel(FieldJob job) {
+    constexpr int TP = SHARED ? 256 : 128;  // panels per tile
+    constexpr int W = FieldArith<TC>::WORDS;
+    extern __shared__ __align__(16) unsigned char field_smem[];
+    TC* const tile = reinterpret_cast<TC*>(field_smem);
+    int* const lists = reinterpret_cast<int*>(tile + TP * W);
+    __shared__ int tex;
+    __shared__ double part[FIELD_WARPS][3];
+    __shared__ int pnear[FIELD_WARPS];
+    __shared__ double clsum[3];
+    __shared__ int clnear;
+    cg::cluster_group cl = cg::this_cluster();
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const int ncl = SHARED ? (int)cl.num_blocks() : 1, rank = SHARED ? (int)cl.block_rank() : 0;
+    const int pt0 = SHARED ? blockIdx.x / ncl : (blockIdx.x * FIELD_WARPS + wl) * PPW;
+    const double* const o = job.pts + 3LL * (SHARED ? pt0 : blockIdx.x * FIELD_WARPS * PPW);
+    FieldPoint X[PPW];
+    FieldArith<TC> F[PPW];
+#pragma unroll
+    for (int k = 0; k < PPW; ++k) {
+        const int pt = min(pt0 + k, job.npts - 1);
+        X[k].x = job.pts[3 * pt];
+        X[k].y = job.pts[3 * pt + 1];
+        X[k].z = job.pts[3 * pt + 2];
+        X[k].u[0] = X[k].u[1] = X[k].u[2] = 0.0;
+        X[k].near = 0;
+        F[k].point(X[k], o);
+    }
+    int* const list = lists + wl * PPW * FIELD_NEAR_CAP;
+    for (int base = rank * TP; base < job.P; base += ncl * TP) {
+        const int np = min(TP, job.P - base);
+        __syncthreads();
+        if (threadIdx.x == 0) tex = 0;
+        __syncthreads();
+        if (sizeof(TC) == 4 && (int)threadIdx.x < np) {
+            const int e = FieldArith<TC>::exponent(job, base + threadIdx.x);
+            if (e) atomicMax(&tex, e);
+        }
+        __syncthreads();
+        const int ex = tex;
+        if ((int)threadIdx.x < np)
+            FieldArith<TC>::stage(tile + threadIdx.x * W, job, base + threadIdx.x, o, ex);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < PPW; ++k) F[k].begin();
+        for (int s = SHARED ? wl * 32 : 0; s < (SHARED ? min(np, wl * 32 + 32) : np); s += 32) {
+            const int q = s + lane, p = base + q;
+#pragma unroll
+            for (int k = 0; k < PPW; ++k) {
+                int rule = 0;
+                if (q < np) rule = F[k].pair(tile + q * W, job, p, X[k], ex == 0x7ff);
+                const unsigned m = __ballot_sync(0xffffffffu, rule > 0);
+                if (rule > 0) {
+                    const int slot = X[k].near + __popc(m & ((1u << lane) - 1));
+                    if (slot < FIELD_NEAR_CAP) list[k * FIELD_NEAR_CAP + slot] = p | (rule << 28);
+                }
+                X[k].near += __popc(m);
+            }
+        }
+        const double scale = ex > 0 && ex < 0x7ff ? scalbn(1.0, ex - 1023) : 1.0;
+#pragma unroll
+        for (int k = 0; k < PPW; ++k) F[k].flush(X[k], scale);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < PPW; ++k) {
+        // the far part: warp sums (fixed butterfly order), component j to lane j
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) X[k].u[j] += __shfl_xor_sync(0xffffffffu, X[k].u[j], d);
+        double u = lane == 0 ? X[k].u[0] : lane == 1 ? X[k].u[1] : X[k].u[2];
+        const int nn = min(X[k].near, FIELD_NEAR_CAP);
+        if (SHARED || pt0 + k < job.npts)
+            for (int n = 0; n < nn; ++n) {
+                const int e = list[k * FIELD_NEAR_CAP + n];
+                field_near<sizeof(TC) == 4>(job, e & 0x0fffffff, e >> 28, X[k], lane, u);
+            }
+        if (!SHARED && pt0 + k < job.npts) {
+            if (lane < 3) job.out[3 * (pt0 + k) + lane] = u;
+            if (lane == 0 && X[k].near > FIELD_NEAR_CAP) atomicExch(job.overflow, 1);
+        }
+        if (SHARED) {
+            if (lane < 3) part[wl][lane] = u;
+            if (lane == 0) pnear[wl] = X[k].near;
         }
     }
-    if (lane == 0) {
-        job.out[3 * pt] = ux;
-        job.out[3 * pt + 1] = uy;
-        job.out[3 * pt + 2] = uz;
-        if (overflow) atomicExch(job.overflow, 1);
+    if (SHARED) {
+        __syncthreads();
+        if (threadIdx.x < 3) {
+            double u = 0.0;
+            for (int w = 0; w < FIELD_WARPS; ++w) u += part[w][threadIdx.x];
+            clsum[threadIdx.x] = u;
+        }
+        if (threadIdx.x == 3) {
+            int n = 0;
+            for (int w = 0; w < FIELD_WARPS; ++w) n += pnear[w];
+            clnear = n;
+        }
+        cl.sync();
+        if (rank == 0 && threadIdx.x < 4) {
+            double u = 0.0;
+            int n = 0;
+            for (int c = 0; c < ncl; ++c) {
+                if (threadIdx.x < 3) u += cl.map_shared_rank(clsum, c)[threadIdx.x];
+                else n += *cl.map_shared_rank(&clnear, c);
+            }
+            if (threadIdx.x < 3) job.out[3 * pt0 + threadIdx.x] = u;
+            else if (n > FIELD_NEAR_CAP) atomicExch(job.overflow, 1);
+        }
+        cl.sync();
     }
 }
 
@@ -907,11 +1175,47 @@ void rsqrt_nr_eval(int n, const double* x, double* y, cudaStream_t st) {
     if (n > 0) LAUNCH(rsqrt_nr_kernel, ceil_div(n, 256), 256, 0, st, n, x, y);
 }
 
+namespace {
+template <class TC, int PPW, bool SHARED>
+void field_launch(const FieldJob& job, int cluster, cudaStream_t st) {
+    constexpr int TP = SHARED ? 256 : 128;
+    constexpr size_t smem =
+        sizeof(TC) * TP * FieldArith<TC>::WORDS + sizeof(int) * FIELD_WARPS * PPW * FIELD_NEAR_CAP;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        CUDA_CHECK(cudaFuncSetAttribute((const void*)field_kernel<TC, PPW, SHARED>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    });
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute at[1];
+    c.gridDim = dim3(SHARED ? (unsigned)job.npts * cluster : (unsigned)ceil_div(job.npts, FIELD_WARPS * PPW));
+    c.blockDim = dim3(FIELD_WARPS * 32);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    CUDA_CHECK(cudaLaunchKernelEx(&c, field_kernel<TC, PPW, SHARED>, job));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+}
+
+// Four points per warp once every SM has its 32 points; below that one per warp, and a few
+// points share a CTA or a cluster of four each, which costs staging every panel per point.
+template <class TC>
+void field_dispatch(const FieldJob& job, cudaStream_t st) {
+    if (job.npts >= 152 * FIELD_WARPS * 4) field_launch<TC, 4, false>(job, 1, st);
+    else if (job.npts >= 152 * FIELD_WARPS) field_launch<TC, 1, false>(job, 1, st);
+    else field_launch<TC, 1, true>(job, job.npts < 152 * 2 ? 4 : 1, st);
+}
+}  // namespace
+
 void field_eval(const FieldJob& job, cudaStream_t st) {
     if (job.npts <= 0) return;
     init_tables();
-    if (job.mixed) LAUNCH(field_kernel<float>, ceil_div(job.npts, FIELD_WARPS), FIELD_WARPS * 32, 0, st, job);
-    else LAUNCH(field_kernel<double>, ceil_div(job.npts, FIELD_WARPS), FIELD_WARPS * 32, 0, st, job);
+    if (job.mixed) field_dispatch<float>(job, st);
+    else field_dispatch<double>(job, st);
 }
 
 }  // namespace sqbem
