@@ -223,11 +223,12 @@ __device__ void warp_rule(Acc<T>& A, const PanelRec& P, double x, double y, doub
 // per lane (GB300's FP64 pipe runs at about 1/64 of the FP32 rate).
 __device__ void warp_rule_f32(Acc<float>& A, const PanelRec* Pg, double x, double y, double z, int rule, int lane) {
     A.zero();
-    float val = 0.f;
-    if (lane < 9) val = (float)(Pg->v[lane] - Pg->c[lane % 3]);
-    else if (lane < 12) val = (float)(Pg->c[lane - 9] - (lane == 9 ? x : lane == 10 ? y : z));
-    else if (lane < 15) val = (float)Pg->n[lane - 12];
-    else if (lane == 15) val = (float)Pg->area;
+    // minuend: v (9), c, n, area (words 0 .. 8, 12 .. 14, 9 .. 11, 15 of the record);
+    // subtrahend: c, x0, 0: one FP64 subtraction and one conversion for the warp
+    const double* const w = reinterpret_cast<const double*>(Pg);
+    const double hi = w[lane < 9 ? lane : lane < 12 ? lane + 3 : lane < 15 ? lane - 3 : 15];
+    const double lo = lane < 9 ? w[12 + lane % 3] : lane == 9 ? x : lane == 10 ? y : lane == 11 ? z : 0.0;
+    const float val = (float)(hi - lo);
     float d[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) d[k] = __shfl_sync(0xffffffffu, val, k);
@@ -997,20 +998,19 @@ struct FieldArith<float> {
     }
 };
 
-// One near panel of one point by a warp, added to lane 0 .. 2's u (component = lane).
+// One near panel of one point by a warp.  u: lanes 0 .. 2 hold the component of their
+// number; t (mixed, 28 and 112 points): lane 3 i + j holds the sum of its (i, j) terms,
+// collected once per point.
 template <bool MIXED>
-__device__ void field_near(const FieldJob& job, int p, int rule, const FieldPoint& X, int lane, double& u) {
+__device__ void field_near(const FieldJob& job, int p, int rule, const FieldPoint& X, int lane, double& u, double& t) {
     if (MIXED && rule < 3) {
         Acc<float> A;
         warp_rule_f32(A, job.panels + p, X.x, X.y, X.z, rule, lane);
-        // lane 3 i + j: the (i, j) terms; lane j collects its column
         const int i = lane / 3, j = lane - 3 * i;
-        double t = 0.0;
-        if (lane < 9)
-            t = (double)sl_entry(A, i, j) * job.f[3 * p + i] * job.sscale +
-                (double)dl_entry(A, i, j) * job.u[3 * p + i] * job.dscale;
-        t += __shfl_down_sync(0xffffffffu, t, 3) + __shfl_down_sync(0xffffffffu, t, 6);
-        u += t;
+        if (lane < 9) {
+            t = fma((double)sl_entry(A, i, j), job.f[3 * p + i] * job.sscale, t);
+            t = fma((double)dl_entry(A, i, j), job.u[3 * p + i] * job.dscale, t);
+        }
         return;
     }
     const PanelRec& P = job.panels[p];
@@ -1052,7 +1052,7 @@ __device__ void field_near(const FieldJob& job, int p, int rule, const FieldPoin
 // PPW points per warp, each warp all panels; or (SHARED) one point per CTA -- per
 // cluster -- whose warps and CTAs share the panels.
 template <class TC, int PPW, bool SHARED>
-__global__ void __launch_bounds__(FIELD_WARPS * 32) field_kernel(FieldJob job) {
+__global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job) {
     constexpr int TP = SHARED ? 256 : 128;  // panels per tile
     constexpr int W = FieldArith<TC>::WORDS;
     extern __shared__ __align__(16) unsigned char field_smem[];
@@ -1125,11 +1125,13 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32) field_kernel(FieldJob job) {
             for (int d = 16; d > 0; d >>= 1) X[k].u[j] += __shfl_xor_sync(0xffffffffu, X[k].u[j], d);
         double u = lane == 0 ? X[k].u[0] : lane == 1 ? X[k].u[1] : X[k].u[2];
         const int nn = min(X[k].near, FIELD_NEAR_CAP);
+        double t = 0.0;
         if (SHARED || pt0 + k < job.npts)
             for (int n = 0; n < nn; ++n) {
                 const int e = list[k * FIELD_NEAR_CAP + n];
-                field_near<sizeof(TC) == 4>(job, e & 0x0fffffff, e >> 28, X[k], lane, u);
+                field_near<sizeof(TC) == 4>(job, e & 0x0fffffff, e >> 28, X[k], lane, u, t);
             }
+        if (sizeof(TC) == 4) u += t + __shfl_down_sync(0xffffffffu, t, 3) + __shfl_down_sync(0xffffffffu, t, 6);
         if (!SHARED && pt0 + k < job.npts) {
             if (lane < 3) job.out[3 * (pt0 + k) + lane] = u;
             if (lane == 0 && X[k].near > FIELD_NEAR_CAP) atomicExch(job.overflow, 1);
@@ -1225,123 +1227,227 @@ namespace sqbem {
 
 constexpr int ADJ_TT = 32;   // targets per CTA (one per lane)
 constexpr int ADJ_ST = 32;   // source panels per CTA (staged in shared memory)
+constexpr int ADJ_W = 4;     // warps, each a quarter of the sources
 constexpr int ADJ_OUT = 6 * ADJ_MAX_MODES * 3;
+constexpr int ADJ_WORDS = 41;  // staged words per source
 
 // Gradients with respect to r of  phi_G = lam.G(r).f = (lam.f)/|r| + (lam.r)(f.r)/|r|^3
 //   grad phi_G = [lam (f.r) + f (lam.r) - (lam.f) r] / |r|^3 - 3 (lam.r)(f.r) r / |r|^5
 // and of phi_T = lam.(T(r).m).v = -6 (r.m)(lam.r)(v.r) / |r|^5
 //   grad phi_T = -6 [m (lam.r)(v.r) + lam (r.m)(v.r) + v (r.m)(lam.r)] / |r|^5
 //                + 30 (r.m)(lam.r)(v.r) r / |r|^7
-// (kernels.hpp:8-9 differentiated), accumulated with the weights gs w, ts w.
-__global__ void __launch_bounds__(6 * ADJ_TT) adjoint_pairs_kernel(AdjTerm J, int nm, double* partial) {
-    __shared__ PanelRec sp[ADJ_ST];
-    __shared__ double sf[ADJ_ST][ADJ_MAX_MODES][3];
-    __shared__ double sv[ADJ_ST][ADJ_MAX_MODES][3];
-    const int tid = threadIdx.x, o = tid / ADJ_TT, lt = tid % ADJ_TT;
-    const int t = blockIdx.x * ADJ_TT + lt;
-    const int s0 = blockIdx.y * ADJ_ST, ns = min(ADJ_ST, J.nS - s0);
-    {
-        const double* srcd = reinterpret_cast<const double*>(J.src + s0);
-        double* dstd = reinterpret_cast<double*>(sp);
-        for (int e = tid; e < ns * 18; e += blockDim.x) dstd[e] = srcd[e];
-        for (int e = tid; e < ns * ADJ_MAX_MODES * 3; e += blockDim.x) {
-            const int s = e / (ADJ_MAX_MODES * 3), j = (e / 3) % ADJ_MAX_MODES, a = e % 3;
-            sf[s][j][a] = j < nm ? J.f[3 * (long long)(s0 + s) + a + j * J.f_ld] : 0.0;
-            sv[s][j][a] = (J.v_src && j < nm) ? J.v[3 * (long long)(s0 + s) + a + j * J.v_ld] : 0.0;
+// (kernels.hpp:8-9 differentiated).  Both are lam.C(f, v) with a 3 x 3 matrix C that does not
+// know the adjoint vector, and C is linear in a few moments of the quadrature nodes.  So a
+// pair sums its nodes into the moments
+//   p = sum w r/|r|^3, y = sum w r/|r|^5, W = sum w r r/|r|^5, Q = sum w r r r/|r|^5,
+//   Z = sum w r r r/|r|^7
+// (symmetric; the zz. entries of Q and Z follow from the traces p and y), forms C per
+// solution, and a target's C is summed over its sources before it meets the six adjoint
+// vectors: 625 FP64 operations a far pair where the gradient per node, adjoint vector
+// and solution took 5000 (FP64-bound, 10.6 ms for 1392 x 320 panels both ways).
+struct AdjMoments {
+    double p[3], y[3], W[6], Q[7], Z[7];  // W: xx xy xz yy yz zz; Q, Z: xxx xxy xxz xyy xyz yyy yyz
+    __device__ void zero() {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p[k] = y[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) W[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 7; ++k) Q[k] = Z[k] = 0.0;
+    }
+    __device__ void node(double rx, double ry, double rz, double w) {
+        const double ir = rsqrt(rx * rx + ry * ry + rz * rz), ir2 = ir * ir;
+        const double a3 = w * ir * ir2, a5 = a3 * ir2, a7 = a5 * ir2;
+        const double xx = rx * rx, xy = rx * ry, xz = rx * rz, yy = ry * ry, yz = ry * rz;
+        p[0] = fma(a3, rx, p[0]); p[1] = fma(a3, ry, p[1]); p[2] = fma(a3, rz, p[2]);
+        y[0] = fma(a5, rx, y[0]); y[1] = fma(a5, ry, y[1]); y[2] = fma(a5, rz, y[2]);
+        W[0] = fma(a5, xx, W[0]); W[1] = fma(a5, xy, W[1]); W[2] = fma(a5, xz, W[2]);
+        W[3] = fma(a5, yy, W[3]); W[4] = fma(a5, yz, W[4]); W[5] = fma(a5, rz * rz, W[5]);
+        const double t[7] = {xx * rx, xx * ry, xx * rz, xy * ry, xy * rz, yy * ry, yy * rz};
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {
+            Q[k] = fma(a5, t[k], Q[k]);
+            Z[k] = fma(a7, t[k], Z[k]);
         }
+    }
+};
+
+// H = sum_b f_b Q_ab. as xx xy xz yy yz zz, the entries Q_zz. from the trace tr
+__device__ __forceinline__ void adj_contract(const double (&Q)[7], const double (&tr)[3], double fx, double fy, double fz,
+                                             double (&H)[6]) {
+    const double xzz = tr[0] - Q[0] - Q[3], yzz = tr[1] - Q[1] - Q[5], zzz = tr[2] - Q[2] - Q[6];
+    H[0] = Q[0] * fx + Q[1] * fy + Q[2] * fz;
+    H[1] = Q[1] * fx + Q[3] * fy + Q[4] * fz;
+    H[2] = Q[2] * fx + Q[4] * fy + xzz * fz;
+    H[3] = Q[3] * fx + Q[5] * fy + Q[6] * fz;
+    H[4] = Q[4] * fx + Q[6] * fy + yzz * fz;
+    H[5] = xzz * fx + yzz * fy + zzz * fz;
+}
+
+// C[3 a + k] += the pair's matrix for (f, v); s = r.m, m the normal
+__device__ __forceinline__ void adj_matrix(double* C, const AdjMoments& M, const double* f, const double* v, double mx,
+                                           double my, double mz, double s, double gs, double ts) {
+    double H[6];
+    {
+        const double fx = gs * f[0], fy = gs * f[1], fz = gs * f[2];
+        adj_contract(M.Q, M.p, fx, fy, fz, H);
+        const double d = fx * M.p[0] + fy * M.p[1] + fz * M.p[2];
+        // antisymmetric part p_a f_k - f_a p_k
+        const double axy = M.p[0] * fy - fx * M.p[1], axz = M.p[0] * fz - fx * M.p[2], ayz = M.p[1] * fz - fy * M.p[2];
+        C[0] += fma(-3.0, H[0], d); C[1] += fma(-3.0, H[1], axy); C[2] += fma(-3.0, H[2], axz);
+        C[3] += fma(-3.0, H[1], -axy); C[4] += fma(-3.0, H[3], d); C[5] += fma(-3.0, H[4], ayz);
+        C[6] += fma(-3.0, H[2], -axz); C[7] += fma(-3.0, H[4], -ayz); C[8] += fma(-3.0, H[5], d);
+    }
+    const double c = -6.0 * ts, vx = c * v[0], vy = c * v[1], vz = c * v[2];
+    const double s5 = -5.0 * s;
+    adj_contract(M.Z, M.y, s5 * vx, s5 * vy, s5 * vz, H);
+    const double wx = M.W[0] * vx + M.W[1] * vy + M.W[2] * vz, wy = M.W[1] * vx + M.W[3] * vy + M.W[4] * vz,
+                 wz = M.W[2] * vx + M.W[4] * vy + M.W[5] * vz;
+    const double d = s * (vx * M.y[0] + vy * M.y[1] + vz * M.y[2]);
+    const double yx = s * M.y[0], yy = s * M.y[1], yz = s * M.y[2];
+    C[0] += H[0] + d + wx * mx + yx * vx; C[1] += H[1] + wx * my + yx * vy; C[2] += H[2] + wx * mz + yx * vz;
+    C[3] += H[1] + wy * mx + yy * vx; C[4] += H[3] + d + wy * my + yy * vy; C[5] += H[4] + wy * mz + yy * vz;
+    C[6] += H[2] + wz * mx + yz * vx; C[7] += H[4] + wz * my + yz * vy; C[8] += H[5] + d + wz * mz + yz * vz;
+}
+
+__global__ void __launch_bounds__(32 * ADJ_W) adjoint_pairs_kernel(AdjTerm J, int nm, double* partial) {
+    constexpr int NC = 9 * ADJ_MAX_MODES;
+    __shared__ double sp[ADJ_ST][ADJ_WORDS];  // o (21), c, n, 9 h^2, area, f, v
+    __shared__ unsigned char list[ADJ_W][ADJ_TT * ADJ_ST / ADJ_W][2];  // near pairs: lane, source
+    __shared__ double sC[ADJ_W][NC][ADJ_TT];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int t = blockIdx.x * ADJ_TT + lane;
+    const int s0 = blockIdx.y * ADJ_ST, ns = min(ADJ_ST, J.nS - s0);
+    for (int s = threadIdx.x; s < ns; s += 32 * ADJ_W) {
+        const PanelRec P = J.src[s0 + s];
+        double* d = sp[s];
+#pragma unroll
+        for (int q = 0; q < 7; ++q)
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                d[3 * q + k] = c_rule7[q].l0 * (P.v[k] - P.c[k]) + c_rule7[q].l1 * (P.v[3 + k] - P.c[k]) +
+                               c_rule7[q].l2 * (P.v[6 + k] - P.c[k]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            d[21 + k] = P.c[k];
+            d[24 + k] = P.n[k];
+        }
+        d[27] = 9.0 * P.h * P.h * (1.0 + 1e-12);
+        d[28] = P.area;
+        for (int j = 0; j < ADJ_MAX_MODES; ++j)
+            for (int a = 0; a < 3; ++a) {
+                d[29 + 3 * j + a] = j < nm ? J.f[3 * (long long)(s0 + s) + a + j * J.f_ld] : 0.0;
+                d[35 + 3 * j + a] = J.v_src && j < nm ? J.v[3 * (long long)(s0 + s) + a + j * J.v_ld] : 0.0;
+            }
     }
     __syncthreads();
-    double acc[ADJ_MAX_MODES][3];
-#pragma unroll
-    for (int j = 0; j < ADJ_MAX_MODES; ++j) acc[j][0] = acc[j][1] = acc[j][2] = 0.0;
-    if (t < J.nT) {
-        const double x = J.tgt[3 * t], y = J.tgt[3 * t + 1], z = J.tgt[3 * t + 2];
-        const double* lp = J.lam + 3 * (long long)t + o * J.lam_ld;
-        const double lx = lp[0], ly = lp[1], lz = lp[2];
-        double tv[ADJ_MAX_MODES][3];
-#pragma unroll
-        for (int j = 0; j < ADJ_MAX_MODES; ++j)
-#pragma unroll
-            for (int a = 0; a < 3; ++a) tv[j][a] = (!J.v_src && j < nm) ? J.v[3 * (long long)t + a + j * J.v_ld] : 0.0;
-        for (int s = 0; s < ns; ++s) {
-            const PanelRec& P = sp[s];
-            const int rule = rule_of(P, x, y, z);
-            const double e0x = P.v[0] - x, e0y = P.v[1] - y, e0z = P.v[2] - z;
-            const double e1x = P.v[3] - x, e1y = P.v[4] - y, e1z = P.v[5] - z;
-            const double e2x = P.v[6] - x, e2y = P.v[7] - y, e2z = P.v[8] - z;
-            const double mx = P.n[0], my = P.n[1], mz = P.n[2];
-            double fv[ADJ_MAX_MODES][3], vv[ADJ_MAX_MODES][3], lf[ADJ_MAX_MODES];
-#pragma unroll
-            for (int j = 0; j < ADJ_MAX_MODES; ++j) {
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    fv[j][a] = sf[s][j][a];
-                    vv[j][a] = J.v_src ? sv[s][j][a] : tv[j][a];
-                }
-                lf[j] = lx * fv[j][0] + ly * fv[j][1] + lz * fv[j][2];
-            }
-            const int q0 = rule_off(rule), q1 = rule_off(rule + 1);
-            for (int q = q0; q < q1; ++q) {
-                const QPoint Q = d_rule[q];
-                const double rx = Q.l0 * e0x + Q.l1 * e1x + Q.l2 * e2x;
-                const double ry = Q.l0 * e0y + Q.l1 * e1y + Q.l2 * e2y;
-                const double rz = Q.l0 * e0z + Q.l1 * e1z + Q.l2 * e2z;
-                const double w = Q.w * P.area;
-                const double r2 = rx * rx + ry * ry + rz * rz;
-                const double ir = rsqrt(r2), ir2 = ir * ir, ir3 = ir * ir2, ir5 = ir3 * ir2, ir7 = ir5 * ir2;
-                const double sm = rx * mx + ry * my + rz * mz;
-                const double sl = rx * lx + ry * ly + rz * lz;
-                const double wg = w * J.gs, wt = w * J.ts;
-#pragma unroll
-                for (int j = 0; j < ADJ_MAX_MODES; ++j) {
-                    if (j >= nm) break;
-                    const double sfj = rx * fv[j][0] + ry * fv[j][1] + rz * fv[j][2];
-                    const double svj = rx * vv[j][0] + ry * vv[j][1] + rz * vv[j][2];
-                    // grad phi_G = (lam sf + f sl - lf r) ir3 + cg r
-                    const double cg = -3.0 * sl * sfj * ir5;
-                    // grad phi_T = -6 ir5 (m sl sv + lam sm sv + v sm sl) + ct r
-                    const double a1 = sl * svj, a2 = sm * svj, a3 = sm * sl;
-                    const double ct = 30.0 * a3 * svj * ir7, m6 = -6.0 * ir5;
-                    const double gx = (lx * sfj + fv[j][0] * sl - lf[j] * rx) * ir3 + cg * rx;
-                    const double gy = (ly * sfj + fv[j][1] * sl - lf[j] * ry) * ir3 + cg * ry;
-                    const double gz = (lz * sfj + fv[j][2] * sl - lf[j] * rz) * ir3 + cg * rz;
-                    const double tx = m6 * (mx * a1 + lx * a2 + vv[j][0] * a3) + ct * rx;
-                    const double ty = m6 * (my * a1 + ly * a2 + vv[j][1] * a3) + ct * ry;
-                    const double tz = m6 * (mz * a1 + lz * a2 + vv[j][2] * a3) + ct * rz;
-                    acc[j][0] += wg * gx + wt * tx;
-                    acc[j][1] += wg * gy + wt * ty;
-                    acc[j][2] += wg * gz + wt * tz;
-                }
-            }
-        }
-    }
-    // the 32 lanes of a warp share o: reduce over targets, lane 0 writes
+    const bool in = t < J.nT;
+    const int tt = in ? t : J.nT - 1;
+    const double x = J.tgt[3 * tt], y = J.tgt[3 * tt + 1], z = J.tgt[3 * tt + 2];
+    double tv[ADJ_MAX_MODES][3];
 #pragma unroll
     for (int j = 0; j < ADJ_MAX_MODES; ++j)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            double v = acc[j][a];
+        for (int a = 0; a < 3; ++a) tv[j][a] = !J.v_src && j < nm ? J.v[3 * (long long)tt + a + j * J.v_ld] : 0.0;
+    double C[NC];
 #pragma unroll
-            for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-            acc[j][a] = v;
+    for (int k = 0; k < NC; ++k) C[k] = 0.0;
+    int nnear = 0;
+    AdjMoments M;
+    for (int s = w; s < ns; s += ADJ_W) {
+        const double* d = sp[s];
+        const double bx = d[21] - x, by = d[22] - y, bz = d[23] - z;
+        bool near = false;
+        // within 1e-12 of the threshold and below: the exact test
+        if (!(bx * bx + by * by + bz * bz > d[27])) near = rule_of(J.src[s0 + s], x, y, z) != 0;
+        near = near && in;
+        const unsigned m = __ballot_sync(0xffffffffu, near);
+        if (near) {
+            unsigned char* e = list[w][nnear + __popc(m & ((1u << lane) - 1))];
+            e[0] = (unsigned char)lane;
+            e[1] = (unsigned char)s;
         }
-    if (lt == 0) {
-        const long long cta = blockIdx.x + (long long)gridDim.x * blockIdx.y;
-        double* out = partial + cta * ADJ_OUT + o * ADJ_MAX_MODES * 3;
+        nnear += __popc(m);
+        if (near || !in) continue;
+        M.zero();
+#pragma unroll
+        for (int q = 0; q < 7; ++q) M.node(bx + d[3 * q], by + d[3 * q + 1], bz + d[3 * q + 2], c_rule7[q].w);
+        const double sm = bx * d[24] + by * d[25] + bz * d[26], gs = J.gs * d[28], ts = J.ts * d[28];
 #pragma unroll
         for (int j = 0; j < ADJ_MAX_MODES; ++j)
+            if (j < nm)
+                adj_matrix(C + 9 * j, M, d + 29 + 3 * j, J.v_src ? d + 35 + 3 * j : tv[j], d[24], d[25], d[26], sm, gs, ts);
+    }
+    __syncwarp();
+    // near pairs by the whole warp: the lanes split the nodes, the sum goes to the target's lane
+    for (int n = 0; n < nnear; ++n) {
+        const int tl = list[w][n][0], s = list[w][n][1];
+        const PanelRec& P = J.src[s0 + s];
+        const double* d = sp[s];
+        const double X = __shfl_sync(0xffffffffu, x, tl), Y = __shfl_sync(0xffffffffu, y, tl),
+                     Zc = __shfl_sync(0xffffffffu, z, tl);
+        const double e0x = P.v[0] - X, e0y = P.v[1] - Y, e0z = P.v[2] - Zc;
+        const double e1x = P.v[3] - X, e1y = P.v[4] - Y, e1z = P.v[5] - Zc;
+        const double e2x = P.v[6] - X, e2y = P.v[7] - Y, e2z = P.v[8] - Zc;
+        const int rule = rule_of(P, X, Y, Zc), q1 = rule_off(rule + 1);
+        M.zero();
+        for (int q = rule_off(rule) + lane; q < q1; q += 32) {
+            const QPoint R = d_rule[q];
+            M.node(R.l0 * e0x + R.l1 * e1x + R.l2 * e2x, R.l0 * e0y + R.l1 * e1y + R.l2 * e2y,
+                   R.l0 * e0z + R.l1 * e1z + R.l2 * e2z, R.w);
+        }
+        const double sm = (d[21] - X) * d[24] + (d[22] - Y) * d[25] + (d[23] - Zc) * d[26];
+        double D[NC];
 #pragma unroll
-            for (int a = 0; a < 3; ++a) out[j * 3 + a] = acc[j][a];
+        for (int k = 0; k < NC; ++k) D[k] = 0.0;
+#pragma unroll
+        for (int j = 0; j < ADJ_MAX_MODES; ++j) {
+            double vv[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) vv[a] = J.v_src ? d[35 + 3 * j + a] : __shfl_sync(0xffffffffu, tv[j][a], tl);
+            if (j < nm) adj_matrix(D + 9 * j, M, d + 29 + 3 * j, vv, d[24], d[25], d[26], sm, J.gs * d[28], J.ts * d[28]);
+        }
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) D[k] += __shfl_xor_sync(0xffffffffu, D[k], o);
+            if (lane == tl) C[k] += D[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NC; ++k) sC[w][k][lane] = in ? C[k] : 0.0;
+    __syncthreads();
+    // the six adjoint vectors: warp w takes outputs w, w + 4, .. of the 6 x modes x 3
+    const long long cta = blockIdx.x + (long long)gridDim.x * blockIdx.y;
+    for (int e = w; e < ADJ_OUT; e += ADJ_W) {
+        const int o = e / (ADJ_MAX_MODES * 3), j = (e / 3) % ADJ_MAX_MODES, k = e % 3;
+        const double* lp = J.lam + 3 * (long long)tt + o * J.lam_ld;
+        double v = 0.0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            double c = 0.0;
+#pragma unroll
+            for (int q = 0; q < ADJ_W; ++q) c += sC[q][9 * j + 3 * a + k][lane];
+            v = fma(lp[a], c, v);
+        }
+        if (!in) v = 0.0;
+#pragma unroll
+        for (int q = 16; q > 0; q >>= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
+        if (lane == 0) partial[cta * ADJ_OUT + e] = v;
     }
 }
 
-// out[k] = sum over the ncta partial records, in order
-__global__ void adjoint_reduce_kernel(const double* __restrict__ partial, long long ncta, double* __restrict__ out) {
-    const int k = threadIdx.x;
-    if (k >= ADJ_OUT) return;
-    double s = 0.0;
-    for (long long c = 0; c < ncta; ++c) s += partial[c * ADJ_OUT + k];
-    out[k] = s;
+// out[k] = sum over the ncta partial records in a fixed order: a warp per output
+__global__ void __launch_bounds__(1024) adjoint_reduce_kernel(const double* __restrict__ partial, long long ncta,
+                                                              double* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < ADJ_OUT; k += 32) {
+        double s = 0.0;
+        for (long long c = lane; c < ncta; c += 32) s += partial[c * ADJ_OUT + k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) out[k] = s;
+    }
 }
 
 void adjoint_pairs(const AdjTerm* terms, int nterms, int nm, double* out, cudaStream_t st) {
@@ -1357,14 +1463,14 @@ void adjoint_pairs(const AdjTerm* terms, int nterms, int nm, double* out, cudaSt
         const AdjTerm& J = terms[k];
         if (J.nT <= 0 || J.nS <= 0) continue;
         const dim3 grid(ceil_div(J.nT, ADJ_TT), ceil_div(J.nS, ADJ_ST));
-        // far-rule estimate: per node and adjoint vector 54 + 81 nm flops
-        const double fl = (double)J.nT * J.nS * 7.0 * 6.0 * (54.0 + 81.0 * nm);
+        // far-rule estimate: 83 flops per node for the moments, 160 per solution for its matrix
+        const double fl = (double)J.nT * J.nS * (7.0 * 83.0 + 160.0 * nm);
         const double by = (double)J.nS * sizeof(PanelRec) * grid.x + (double)J.nT * 8.0 * 3.0 * 7.0;
-        TIMED_LAUNCH("adjoint_pairs", fl, by, adjoint_pairs_kernel, grid, 6 * ADJ_TT, 0, st, J, nm,
+        TIMED_LAUNCH("adjoint_pairs", fl, by, adjoint_pairs_kernel, grid, 32 * ADJ_W, 0, st, J, nm,
                      partial.get() + off * ADJ_OUT);
         off += (long long)grid.x * grid.y;
     }
-    LAUNCH(adjoint_reduce_kernel, 1, 64, 0, st, partial.get(), total, out);
+    LAUNCH(adjoint_reduce_kernel, 1, 1024, 0, st, partial.get(), total, out);
 }
 
 }  // namespace sqbem
