@@ -216,6 +216,46 @@ __device__ void warp_rule(Acc<T>& A, const PanelRec& P, double x, double y, doub
     warp_reduce(A);
 }
 
+// The FP64 sums of a rule for the FP64 mode, v[0 .. 5] = sum w rr/|r|^3, v[6 .. 11] = sum w
+// rr/|r|^5, v[12] = sum w/|r| over this lane's points: r.m is the same at every point of a
+// flat panel and, with the area, enters once per entry.
+__device__ __forceinline__ void lane_rule64(double (&v)[16], const PanelRec& P, double x, double y, double z, int rule,
+                                            int lane) {
+    const double e0x = P.v[0] - x, e0y = P.v[1] - y, e0z = P.v[2] - z;
+    const double e1x = P.v[3] - x, e1y = P.v[4] - y, e1z = P.v[5] - z;
+    const double e2x = P.v[6] - x, e2y = P.v[7] - y, e2z = P.v[8] - z;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = 0.0;
+    const int q1 = rule_off(rule + 1);
+    for (int q = rule_off(rule) + lane; q < q1; q += 32) {
+        const QPoint Q = d_rule[q];
+        const double rx = Q.l0 * e0x + Q.l1 * e1x + Q.l2 * e2x;
+        const double ry = Q.l0 * e0y + Q.l1 * e1y + Q.l2 * e2y;
+        const double rz = Q.l0 * e0z + Q.l1 * e1z + Q.l2 * e2z;
+        const double ir = rsqrt(rx * rx + ry * ry + rz * rz), ir2 = ir * ir, t = Q.w * ir, a3 = t * ir2, a5 = a3 * ir2;
+        const double rr[6] = {rx * rx, rx * ry, rx * rz, ry * ry, ry * rz, rz * rz};
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            v[k] = fma(a3, rr[k], v[k]);
+            v[6 + k] = fma(a5, rr[k], v[6 + k]);
+        }
+        v[12] += t;
+    }
+}
+// Warp sums of 16 values by halving: lane l ends with value l & 15 (15 + 1 FP64 additions
+// instead of 5 per value).
+__device__ __forceinline__ double warp_sum16(double (&v)[16], int lane) {
+#pragma unroll
+    for (int h = 8; h >= 1; h >>= 1)
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const bool up = lane & h;
+            const double give = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+        }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+
 // FP32 evaluation of a 7/28/112-point rule from centroid-relative offsets:
 // r = (c - x0) + sum_k l_k (V_k - c).  The FP64 differences and their FP32
 // roundings are spread over lanes 0..15 (one value each) and broadcast by
@@ -292,18 +332,36 @@ __device__ __forceinline__ void near_append(const BlockJob<TO>& job, int i, int 
 constexpr int FAR_TGT = 64;   // targets per CTA (threads)
 constexpr int FAR_SRC = 16;   // source panels per CTA
 
-// FP64 mode: one thread per target, the CTA's source panels staged in shared
-// memory; the exact rule test per pair, then the 7-point rule in FP64.
+// FP64 mode: one thread per target.  The FP64 pipe (one warp instruction per 64 cycles and SM
+// quarter) bounds it, so the CTA stages what depends on the source panel alone -- the 7 nodes'
+// offsets from the centroid, 9 h^2 -- and a pair takes (c - x0) + o_q per node, r.m once (the
+// panel is flat), the signs and the area once per entry, and a rule test without square
+// root or division unless it lies within 1e-12 of the threshold or below: 270 FP64
+// operations a pair instead of 400 (1392 x 1280 panels both ways and 1280 x 1280: 4.0 ms before).
+constexpr int FAR64_WORDS = 30;
 template <class TO>
 __global__ void __launch_bounds__(FAR_TGT) far_kernel(BlockJob<TO> job) {
-    __shared__ PanelRec sp[FAR_SRC];
+    __shared__ double sp[FAR_SRC][FAR64_WORDS];  // o (21), c, n, 9 h^2, S scale, D scale
     const int p0 = blockIdx.y * FAR_SRC;
     const int ns = min(FAR_SRC, job.nS - p0);
-    {
-        const double* src = reinterpret_cast<const double*>(job.src + p0);
-        double* dst = reinterpret_cast<double*>(sp);
-        const int nd = ns * (int)(sizeof(PanelRec) / sizeof(double));
-        for (int k = threadIdx.x; k < nd; k += blockDim.x) dst[k] = src[k];
+    for (int e = threadIdx.x; e < ns * 10; e += FAR_TGT) {
+        const int s = e / 10, q = e - 10 * s;
+        const PanelRec& P = job.src[p0 + s];
+        double* d = sp[s];
+        if (q < 7) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                d[3 * q + k] = c_rule7[q].l0 * (P.v[k] - P.c[k]) + c_rule7[q].l1 * (P.v[3 + k] - P.c[k]) +
+                               c_rule7[q].l2 * (P.v[6 + k] - P.c[k]);
+        } else if (q == 7) {
+            for (int k = 0; k < 3; ++k) d[21 + k] = P.c[k];
+        } else if (q == 8) {
+            for (int k = 0; k < 3; ++k) d[24 + k] = P.n[k];
+        } else {
+            d[27] = 9.0 * P.h * P.h * (1.0 + 1e-12);
+            d[28] = P.area * job.sscale;
+            d[29] = -6.0 * P.area * job.dscale;
+        }
     }
     __syncthreads();
     const int i = blockIdx.x * FAR_TGT + threadIdx.x;
@@ -311,34 +369,44 @@ __global__ void __launch_bounds__(FAR_TGT) far_kernel(BlockJob<TO> job) {
     const int self_p = job.same_mesh ? i : (job.self_of ? job.self_of[i] : -1);
     const double x = job.tgt[3 * i], y = job.tgt[3 * i + 1], z = job.tgt[3 * i + 2];
     for (int s = 0; s < ns; ++s) {
-        const PanelRec& P = sp[s];
+        const double* d = sp[s];
         const int p = p0 + s;
-        const int rule = p == self_p ? 4 : rule_of(P, x, y, z);
+        const double bx = d[21] - x, by = d[22] - y, bz = d[23] - z;
+        int rule = p == self_p ? 4 : 0;
+        if (rule == 0 && !(bx * bx + by * by + bz * bz > d[27])) rule = rule_of(job.src[p], x, y, z);
         if (rule != 0) {
             near_append(job, i, p, rule);
             if (job.rule_count) atomicAdd(job.rule_count + rule, 1);
             continue;
         }
-        Acc<double> A;
-        A.zero();
-        const double e0x = P.v[0] - x, e0y = P.v[1] - y, e0z = P.v[2] - z;
-        const double e1x = P.v[3] - x, e1y = P.v[4] - y, e1z = P.v[5] - z;
-        const double e2x = P.v[6] - x, e2y = P.v[7] - y, e2z = P.v[8] - z;
-        const double mx = P.n[0], my = P.n[1], mz = P.n[2], area = P.area;
+        double dg = 0, sxx = 0, sxy = 0, sxz = 0, syy = 0, syz = 0, szz = 0;
+        double dxx = 0, dxy = 0, dxz = 0, dyy = 0, dyz = 0, dzz = 0;
 #pragma unroll
         for (int q = 0; q < 7; ++q) {
-            const double l0 = c_rule7[q].l0, l1 = c_rule7[q].l1, l2 = c_rule7[q].l2, w = c_rule7[q].w;
-            accum<double, true>(A, l0 * e0x + l1 * e1x + l2 * e2x, l0 * e0y + l1 * e1y + l2 * e2y,
-                                l0 * e0z + l1 * e1z + l2 * e2z, w * area, mx, my, mz);
-        }
-#pragma unroll
-        for (int b = 0; b < 3; ++b)
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const long long r = 3LL * i + a, c = 3LL * p + b;
-                if (job.S) job.S[r * job.s_rs + c * job.s_cs] = (TO)(sl_entry(A, a, b) * job.sscale);
-                if (job.D) job.D[r * job.d_rs + c * job.d_cs] = (TO)(dl_entry(A, a, b) * job.dscale);
+            const double rx = bx + d[3 * q], ry = by + d[3 * q + 1], rz = bz + d[3 * q + 2];
+            const double ir = rsqrt(rx * rx + ry * ry + rz * rz), ir2 = ir * ir, t = c_rule7[q].w * ir;
+            const double a3 = t * ir2, a5 = a3 * ir2;
+            dg += t;
+            const double xx = rx * rx, xy = rx * ry, xz = rx * rz, yy = ry * ry, yz = ry * rz, zz = rz * rz;
+            sxx = fma(a3, xx, sxx); sxy = fma(a3, xy, sxy); sxz = fma(a3, xz, sxz);
+            syy = fma(a3, yy, syy); syz = fma(a3, yz, syz); szz = fma(a3, zz, szz);
+            if (job.D) {
+                dxx = fma(a5, xx, dxx); dxy = fma(a5, xy, dxy); dxz = fma(a5, xz, dxz);
+                dyy = fma(a5, yy, dyy); dyz = fma(a5, yz, dyz); dzz = fma(a5, zz, dzz);
             }
+        }
+        const long long r0 = 3LL * i, c0 = 3LL * p;
+        auto put = [&](TO* o, long long rs, long long cs, double f, double xx, double xy, double xz, double yy, double yz,
+                       double zz) {
+            TO* e = o + r0 * rs + c0 * cs;
+            const TO vxy = (TO)(f * xy), vxz = (TO)(f * xz), vyz = (TO)(f * yz);
+            e[0] = (TO)(f * xx); e[rs] = vxy; e[2 * rs] = vxz;
+            e[cs] = vxy; e[cs + rs] = (TO)(f * yy); e[cs + 2 * rs] = vyz;
+            e[2 * cs] = vxz; e[2 * cs + rs] = vyz; e[2 * cs + 2 * rs] = (TO)(f * zz);
+        };
+        if (job.S) put(job.S, job.s_rs, job.s_cs, d[28], sxx + dg, sxy, sxz, syy + dg, syz, szz + dg);
+        if (job.D)
+            put(job.D, job.d_rs, job.d_cs, d[29] * (bx * d[24] + by * d[25] + bz * d[26]), dxx, dxy, dxz, dyy, dyz, dzz);
     }
 }
 
@@ -581,10 +649,22 @@ __global__ void __launch_bounds__(32, 24) near_kernel(BlockJob<TO> job) {
             Acc<float> A;
             warp_rule_f32(A, job.src + p, x, y, z, rule, lane);
             if (lane < 9) { sl = sl_entry(A, a, b); dl = dl_entry(A, a, b); }
-        } else {
+        } else if (MIXED) {
             Acc<double> A;
             warp_rule<double, MIXED>(A, P, x, y, z, rule, lane);
             if (lane < 9) { sl = sl_entry(A, a, b); dl = dl_entry(A, a, b); }
+        } else {
+            double v[16];
+            lane_rule64(v, P, x, y, z, rule, lane);
+            const double t = warp_sum16(v, lane);
+            // entry (a, b): symmetric index into xx xy xz yy yz zz
+            const int lo = min(a, b), hi = max(a, b), k = (lo == 0 ? 0 : lo == 1 ? 2 : 3) + hi;
+            const double dg = __shfl_sync(0xffffffffu, t, 12);
+            sl = __shfl_sync(0xffffffffu, t, k & 31);
+            dl = __shfl_sync(0xffffffffu, t, (6 + k) & 31);
+            if (a == b) sl += dg;
+            sl *= P.area;
+            dl *= -6.0 * P.area * ((P.c[0] - x) * P.n[0] + (P.c[1] - y) * P.n[1] + (P.c[2] - z) * P.n[2]);
         }
         if (lane < 9) {
             const long long r = 3LL * i + a, c = 3LL * p + b;

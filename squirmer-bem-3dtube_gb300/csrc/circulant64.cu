@@ -94,9 +94,14 @@ __global__ void identity_kernel(double* __restrict__ R, int m2) {
 // bound; shared-memory traffic is not).
 __global__ void __launch_bounds__(256) fdft64_kernel(const double* __restrict__ x, long long ldx,
                                                      const int* __restrict__ panel, int nth, int nb, int nf, int nc,
-                                                     const __grid_constant__ Twiddles tw, double* __restrict__ xh) {
+                                                     const __grid_constant__ Twiddles tw, double* __restrict__ xh,
+                                                     int per) {
     extern __shared__ double sm[];
     __shared__ double2 tws[FT_MAX_SECTORS];
+    // this CTA's representatives: per of them from a0 on, rows r0 .. of the column's transform
+    const int a0 = blockIdx.y * per, r0 = 3 * a0, all3 = 3 * nb;
+    nb = min(per, nb - a0);
+    panel += a0 * nth;
     const int n3 = 3 * nb, ld = nth | 1, hn = nth / 2, j = blockIdx.x;
     const bool even = (nth & 1) == 0;
     if (threadIdx.x < nth) tws[threadIdx.x] = tw.t[threadIdx.x];
@@ -167,9 +172,9 @@ __global__ void __launch_bounds__(256) fdft64_kernel(const double* __restrict__ 
                 im = fma(v[nth - s], -tws[k].y, im);
             }
         }
-        double* o = xh + ((long long)f * nc + j) * 2 * n3 + r;
+        double* o = xh + ((long long)f * nc + j) * 2 * all3 + r0 + r;
         o[0] = re * scale;
-        o[n3] = im * scale;
+        o[all3] = im * scale;
     }
 }
 
@@ -178,9 +183,12 @@ __global__ void __launch_bounds__(256) fdft64_kernel(const double* __restrict__ 
 __global__ void __launch_bounds__(256) idft64_kernel(const double* __restrict__ yh, const int* __restrict__ panel,
                                                      int nth, int nb, int nf, int nc,
                                                      const __grid_constant__ Twiddles tw, double* __restrict__ y,
-                                                     long long ldy) {
+                                                     long long ldy, int per) {
     extern __shared__ double sm[];
     __shared__ double2 tws[FT_MAX_SECTORS];
+    const int a0 = blockIdx.y * per, r0 = 3 * a0, all3 = 3 * nb;
+    nb = min(per, nb - a0);
+    panel += a0 * nth;
     const int n3 = 3 * nb, ld = nth | 1, lf = 2 * nf + 1, hn = nth / 2, j = blockIdx.x;
     const bool even = (nth & 1) == 0;
     double* const v = sm;             // n3 x ld: sectors
@@ -188,10 +196,10 @@ __global__ void __launch_bounds__(256) idft64_kernel(const double* __restrict__ 
     if (threadIdx.x < nth) tws[threadIdx.x] = tw.t[threadIdx.x];
     for (int e = threadIdx.x; e < n3 * nf; e += blockDim.x) {
         const int f = e / n3, r = e - f * n3;
-        const double* o = yh + ((long long)f * nc + j) * 2 * n3 + r;
+        const double* o = yh + ((long long)f * nc + j) * 2 * all3 + r0 + r;
         const double g = f == 0 || 2 * f == nth ? 1.0 : 2.0;
         w[r * lf + 2 * f] = g * o[0];
-        w[r * lf + 2 * f + 1] = g * o[n3];
+        w[r * lf + 2 * f + 1] = g * o[all3];
     }
     __syncthreads();
     const int ns = even ? hn / 2 + 1 : hn + 1;  // s = 0 .. ns - 1
@@ -415,9 +423,13 @@ void Circulant64::solve(double* B, long long ldb, int nrhs, cudaStream_t st, int
     }
     const Twiddles tw = twiddles(nth);
     const long long one = (long long)m2 * m2, plane = (long long)m2 * nrhs;
+    // a CTA per column, or, for few columns, per 4 representatives of one (their transforms are
+    // independent): one column on one SM took 100 us
+    const int per = nrhs < 304 ? 4 : nb;
+    const dim3 grid(nrhs, ceil_div(nb, per));
     DevBuf<double> xh((size_t)nf * plane, st);
-    TIMED_LAUNCH("fourier_dft", 0.0, 8.0 * nrhs * (nt + (double)nf * m2), fdft64_kernel, nrhs, 256, fdft_smem(nth, nb), st,
-                 B, ldb, panel.get(), nth, nb, nf, nrhs, tw, xh.get());
+    TIMED_LAUNCH("fourier_dft", 0.0, 8.0 * nrhs * (nt + (double)nf * m2), fdft64_kernel, grid, 256, fdft_smem(nth, per), st,
+                 B, ldb, panel.get(), nth, nb, nf, nrhs, tw, xh.get(), per);
     if (nrhs <= SK_N) {
         DevBuf<double> yh((size_t)nf * plane, st);
         gemm64_few(transpose, m2, nrhs, m2, 1.0, inv.get(), m2, xh.get(), m2, 0.0, yh.get(), m2, st, nf, one, plane,
@@ -428,8 +440,8 @@ void Circulant64::solve(double* B, long long ldb, int nrhs, cudaStream_t st, int
         x.split(xh.get(), m2, 1, nrhs, m2, st, nf, plane);
         oz_gemm(digits, x, 1.0, 0.0, xh.get(), m2, err, st, plane);
     }
-    TIMED_LAUNCH("fourier_dft", 0.0, 8.0 * nrhs * (nt + (double)nf * m2), idft64_kernel, nrhs, 256, idft_smem(nth, nb), st,
-                 xh.get(), panel.get(), nth, nb, nf, nrhs, tw, B, ldb);
+    TIMED_LAUNCH("fourier_dft", 0.0, 8.0 * nrhs * (nt + (double)nf * m2), idft64_kernel, grid, 256, idft_smem(nth, per), st,
+                 xh.get(), panel.get(), nth, nb, nf, nrhs, tw, B, ldb, per);
 }
 
 }  // namespace sqbem

@@ -48,6 +48,10 @@ void gemm64_few(bool ta, int M, int N, int K, double alpha, const double* A, lon
                 long long ldb, double beta, double* C, long long ldc, cudaStream_t st, int batch = 1,
                 long long sa = 0, long long sb = 0, long long sc = 0);
 
+// C (m x 6) = A K, K the rigid-body map of np panels with the offsets r (3 per panel) from the
+// centre; A is m x 3 np.
+void rigid64(int m, int np, const double* A, long long lda, const double* r, double* C, long long ldc, cudaStream_t st);
+
 // LU factorisation (dgetrf semantics) of an n x n column-major matrix, kept on
 // the device with the inverses of its diagonal blocks (used by the solves).
 struct LU64 {
@@ -66,6 +70,8 @@ struct LU64 {
     void factor_inplace(DevBuf<double>&& M, int n, cudaStream_t st, const char* what);
     // B <- A^{-1} B for B (n x nrhs, leading dimension ldb, device); err as in gemm64
     void solve(double* B, long long ldb, int nrhs, cudaStream_t st, int* err = nullptr) const;
+    // B <- (leading m x m block of A)^{-1} B from the same factor; not after exchanges
+    void solve_leading(int m, double* B, long long ldb, int nrhs, cudaStream_t st) const;
     // B <- A^{-T} B (dgetrs 'T'): U^T then L^T solves, then the row exchanges undone
     void solve_transpose(double* B, long long ldb, int nrhs, cudaStream_t st) const;
 };

@@ -6,6 +6,7 @@
 // products therefore run as digit products on the BF16 tensor cores with FP64
 // results (oz_gemm.cu); what stays on the FP64 pipe is the work around them: the
 // 128-wide panels of the LU, and products with a few columns.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -14,6 +15,8 @@
 #include "common.cuh"
 #include "dense.cuh"
 #include "oz_gemm.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace sqbem {
 
@@ -158,12 +161,56 @@ __global__ void __launch_bounds__(256) skinny_t_kernel(int M, int K, double alph
         }
 }
 
+// The same with 8 rows per CTA and 32 slices of K: a 256 x 256 block inverse on 32 SMs instead
+// of 8 (18 us before).
+template <int N>
+__global__ void __launch_bounds__(256) skinny_n8_kernel(int M, int K, double alpha, const double* __restrict__ A,
+                                                        long long lda, const double* __restrict__ B, long long ldb,
+                                                        double beta, double* __restrict__ C, long long ldc, Strides bs) {
+    __shared__ double part[8][N][8];
+    A += blockIdx.y * bs.a;
+    B += blockIdx.y * bs.b;
+    C += blockIdx.y * bs.c;
+    const int r = threadIdx.x & 7, q = threadIdx.x >> 3, w = threadIdx.x >> 5;
+    const int m = blockIdx.x * 8 + r;
+    double acc[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) acc[j] = 0.0;
+    if (m < M) {
+#pragma unroll 8
+        for (int k = q; k < K; k += 32) {
+            const double a = A[m + k * lda];
+#pragma unroll
+            for (int j = 0; j < N; ++j) acc[j] = fma(a, B[k + j * ldb], acc[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 8);
+        acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 16);
+        if ((threadIdx.x & 31) < 8) part[w][j][r] = acc[j];
+    }
+    __syncthreads();
+    if (threadIdx.x < 8 * N) {
+        const int j = threadIdx.x >> 3;
+        if (m >= M) return;
+        double s = 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += part[u][j][r];
+        double* c = C + m + j * ldc;
+        *c = beta == 0.0 ? alpha * s : fma(alpha, s, beta * *c);
+    }
+}
+
 template <int N>
 static void skinny(bool ta, int M, int K, double alpha, const double* A, long long lda, const double* B, long long ldb,
                    double beta, double* C, long long ldc, cudaStream_t st, int batch, Strides bs) {
     const double fl = 2.0 * batch * M * N * K, by = batch * 8.0 * ((double)M * K + (double)K * N + (beta == 0.0 ? 1.0 : 2.0) * M * N);
     if (ta)
         TIMED_LAUNCH("dgemm", fl, by, skinny_t_kernel<N>, dim3(ceil_div(M, 8), batch), 256, 0, st, M, K, alpha, A, lda, B,
+                     ldb, beta, C, ldc, bs);
+    else if ((long long)M * batch <= 152 * 8 * 2)  // 32-row CTAs would leave most SMs idle
+        TIMED_LAUNCH("dgemm", fl, by, skinny_n8_kernel<N>, dim3(ceil_div(M, 8), batch), 256, 0, st, M, K, alpha, A, lda, B,
                      ldb, beta, C, ldc, bs);
     else
         TIMED_LAUNCH("dgemm", fl, by, skinny_n_kernel<N>, dim3(ceil_div(M, 32), batch), 256, 0, st, M, K, alpha, A, lda, B,
@@ -185,6 +232,45 @@ void gemm64_few(bool ta, int M, int N, int K, double alpha, const double* A, lon
         case 8: return skinny<8>(ta, M, K, alpha, A, lda, B, ldb, beta, C, ldc, st, batch, bs);
         default: fail(SQBEM_ERR_ARG, "gemm64_few: %d columns", N);
     }
+}
+
+// C (m x 6) = A K for the rigid-body map K of np panels (swimmer.hpp:224-231): row 3p + b of K
+// is a unit vector and r_p x e_b, so a panel's three columns take 9 FP64 operations where
+// the dense product takes 18.  32 rows per CTA, 8 warps split the panels.
+__global__ void __launch_bounds__(256) rigid64_kernel(int m, int np, const double* __restrict__ A, long long lda,
+                                                      const double* __restrict__ r, double* __restrict__ C,
+                                                      long long ldc) {
+    __shared__ double part[8][6][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    double c[6] = {0, 0, 0, 0, 0, 0};
+    if (i < m) {
+#pragma unroll 4
+        for (int p = w; p < np; p += 8) {
+            const double* a = A + i + 3LL * p * lda;
+            const double a0 = a[0], a1 = a[lda], a2 = a[2 * lda];
+            const double rx = r[3 * p], ry = r[3 * p + 1], rz = r[3 * p + 2];
+            c[0] += a0;
+            c[1] += a1;
+            c[2] += a2;
+            c[3] = fma(a2, ry, fma(-a1, rz, c[3]));
+            c[4] = fma(a0, rz, fma(-a2, rx, c[4]));
+            c[5] = fma(a1, rx, fma(-a0, ry, c[5]));
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) part[w][j][lane] = c[j];
+    __syncthreads();
+    if (w >= 6 || i >= m) return;
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s += part[q][w][lane];
+    C[i + w * ldc] = s;
+}
+
+void rigid64(int m, int np, const double* A, long long lda, const double* r, double* C, long long ldc, cudaStream_t st) {
+    if (m <= 0) return;
+    TIMED_LAUNCH("dgemm", 9.0 * m * np, 24.0 * m * np, rigid64_kernel, ceil_div(m, 32), 256, 0, st, m, np, A, lda, r, C,
+                 ldc);
 }
 
 // The digit products need about 60 us whatever the size (two splits, a tile's 36
@@ -294,17 +380,17 @@ void max_abs64(const double* A, long long lda, int rows, int cols, double* out, 
 // (integers order like the magnitudes), no per-step divisions.
 constexpr int PB = 32, HB = 128;
 
-// 1/x from an FP32 reciprocal y of the significand m (relative error e = 1 - m y about
-// 2^-23): 1/m = y / (1 - e) = y (1 + e + e^2 + ..), cut after e^2, so 2^-69 and the
-// rounding.  Three FP64 operations where the full division (430 cycles) is on the
-// factorisation's serial chain.
+// 1/x from the hardware's approximate reciprocal y (relative error e = 1 - x y about 2^-20):
+// 1/x = y / (1 - e) = y (1 + e + e^2 + ..), cut after e^2, so 2^-60 and the rounding.  Three
+// FP64 operations where the full division (430 cycles) is on the factorisation's
+// serial chain.
 __device__ __forceinline__ double recip(double x) {
-    const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
     if (e < 64 || e > 1980) return 1.0 / x;
-    const double m = __hiloint2double((hi & 0x800fffff) | 0x3ff00000, __double2loint(x));
-    const double y = (double)(1.0f / (float)m), d = fma(-m, y, 1.0);
-    const double r = fma(y, fma(d, d, d), y);
-    return __hiloint2double(__double2hiint(r) + ((1023 - e) << 20), __double2loint(r));
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double d = fma(-x, y, 1.0);
+    return fma(y, fma(d, d, d), y);
 }
 
 // |x| > |piv|, as a pivot search sees it (bit 0), or x not finite (bit 1); piv by its bits
@@ -441,18 +527,25 @@ __global__ void __launch_bounds__(128) lu_trsm32_kernel(double* A, long long lda
 }
 
 // A22 -= L21 U12 for the m rows and w <= 96 columns past a full 32 x 32 diagonal block
-// at A.  CTA 0 takes the next diagonal block (nb x nb) and factors it; the others 16 rows
-// each, without that block's columns in its rows.
-__global__ void __launch_bounds__(128) lu_update32_kernel(double* A, long long lda, int m, int w, int nb, int* flag) {
+// at A.  The first cluster of four CTAs takes the next diagonal block (nb x nb), eight
+// columns each (one SM alone took 10 us for it), and its first CTA factors it; the other
+// CTAs 16 rows each, without that block's columns in its rows.
+constexpr int UPD_CL = 4;
+__global__ void __cluster_dims__(UPD_CL, 1, 1) __launch_bounds__(128)
+    lu_update32_kernel(double* A, long long lda, int m, int w, int nb, int* flag) {
     __shared__ double L[PB][PB + 1];      // [k][row]
     __shared__ double U[PB][3 * PB + 1];  // [k][column]
+    __shared__ double lc[4][PB];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    if (blockIdx.x == 0) {
-        double acc[8];
+    if (blockIdx.x < UPD_CL) {
+        cg::cluster_group cl = cg::this_cluster();
+        const int cb = 8 * blockIdx.x + 2 * wp;
+        double acc[2];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int c = wp + 4 * u;
-            L[c][lane] = lane < nb ? A[PB + lane + c * lda] : 0.0;
+        for (int u = 0; u < 8; ++u) L[wp + 4 * u][lane] = lane < nb ? A[PB + lane + (wp + 4 * u) * lda] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int c = cb + u;
             U[lane][c] = c < nb ? A[lane + (PB + c) * lda] : 0.0;
             acc[u] = lane < nb && c < nb ? A[PB + lane + (PB + c) * lda] : (lane == c ? 1.0 : 0.0);
         }
@@ -461,13 +554,23 @@ __global__ void __launch_bounds__(128) lu_update32_kernel(double* A, long long l
         for (int k = 0; k < PB; ++k) {
             const double l = L[k][lane];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) acc[u] = fma(-l, U[k][wp + 4 * u], acc[u]);
+            for (int u = 0; u < 2; ++u) acc[u] = fma(-l, U[k][cb + u], acc[u]);
         }
-        __syncthreads();
-        lu32(acc, reinterpret_cast<double (*)[PB]>(&L[0][0]), nb, A + PB + PB * lda, lda, flag);
+        // gathered in the first CTA's U, by [column][row]
+        cl.sync();
+        double (*const G)[PB + 1] = reinterpret_cast<double (*)[PB + 1]>(cl.map_shared_rank(&U[0][0], 0));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) G[cb + u][lane] = acc[u];
+        cl.sync();
+        if (blockIdx.x != 0) return;
+        double v[8];
+        const double (*const g)[PB + 1] = reinterpret_cast<const double (*)[PB + 1]>(&U[0][0]);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = g[wp + 4 * u][lane];
+        lu32(v, lc, nb, A + PB + PB * lda, lda, flag);
         return;
     }
-    const int row = (blockIdx.x - 1) * 16 + (lane & 15), g = wp * 2 + (lane >> 4);
+    const int row = (blockIdx.x - UPD_CL) * 16 + (lane & 15), g = wp * 2 + (lane >> 4);
     const int c0 = row < nb ? nb : 0;
 #pragma unroll
     for (int k = g; k < PB; k += 8) L[k][lane & 15] = row < m ? A[PB + row + k * lda] : 0.0;
@@ -494,15 +597,15 @@ __global__ void __launch_bounds__(128) lu_update32_kernel(double* A, long long l
     }
 }
 
-// X <- L^{-1} X or U^{-1} X for the diagonal blocks of a factored matrix, two columns per
-// CTA, a thread per row, one barrier per step; warps whose rows are finished skip the
+// X <- L^{-1} X or U^{-1} X for the diagonal blocks of a factored matrix, C columns per CTA
+// (one where a single block's latency counts, two for all blocks of a matrix), a thread per row, one barrier per step; warps whose rows are finished skip the
 // step's FMAs.  The triangle's column for a step does not depend on the steps before, so
 // eight are loaded ahead (waiting for each one's L2 round trip took 64 us for 128 steps).
 //   lu_lower_kernel    X = columns of the matrix right of block A (in place)
 //   lu_inverse_kernel  X = identity: the inverse of block blockIdx.x's triangle, column-major
 //                      with leading dimension LU_NB, zero padded.
-constexpr int INV_C = 2, INV_AHEAD = 8;
-template <bool LOWER>
+constexpr int INV_AHEAD = 8;
+template <bool LOWER, int INV_C>
 __device__ void tri_solve(const double* a, long long lda, int rows, int first, int steps, double rd,
                           double (&r)[INV_C], double (*x)[INV_C]) {
     const int i = threadIdx.x, d = LOWER ? 1 : -1;
@@ -537,19 +640,22 @@ __device__ void tri_solve(const double* a, long long lda, int rows, int first, i
     }
 }
 
+constexpr int LOWER_C = 1;
 __global__ void __launch_bounds__(HB) lu_lower_kernel(double* A, long long lda, int w) {
+    constexpr int INV_C = LOWER_C;
     __shared__ double x[HB][INV_C];
     const int i = threadIdx.x, c0 = blockIdx.x * INV_C;
     double* X = A + (long long)(HB + c0) * lda + i;
     double r[INV_C];
 #pragma unroll
     for (int c = 0; c < INV_C; ++c) r[c] = c0 + c < w ? X[c * lda] : 0.0;
-    tri_solve<true>(A, lda, HB, 0, HB, 1.0, r, x);
+    tri_solve<true, INV_C>(A, lda, HB, 0, HB, 1.0, r, x);
 #pragma unroll
     for (int c = 0; c < INV_C; ++c)
         if (c0 + c < w) X[c * lda] = r[c];
 }
 
+template <int INV_C>
 __global__ void __launch_bounds__(LU_NB) lu_inverse_kernel(const double* __restrict__ A, long long lda, int n,
                                                            bool upper, double* __restrict__ inv) {
     __shared__ double x[LU_NB][INV_C];
@@ -561,8 +667,8 @@ __global__ void __launch_bounds__(LU_NB) lu_inverse_kernel(const double* __restr
     for (int c = 0; c < INV_C; ++c) r[c] = i == c0 + c && i < kb ? 1.0 : 0.0;
     if (c0 < kb) {
         const int last = min(kb, c0 + INV_C) - 1;
-        if (!upper) tri_solve<true>(a, lda, kb, c0, kb - c0, 1.0, r, x);
-        else tri_solve<false>(a, lda, kb, last, last + 1, i < kb ? recip(a[i + (long long)i * lda]) : 0.0, r, x);
+        if (!upper) tri_solve<true, INV_C>(a, lda, kb, c0, kb - c0, 1.0, r, x);
+        else tri_solve<false, INV_C>(a, lda, kb, last, last + 1, i < kb ? recip(a[i + (long long)i * lda]) : 0.0, r, x);
     }
     double* o = inv + (long long)blockIdx.x * LU_NB * LU_NB + i;
 #pragma unroll
@@ -654,7 +760,8 @@ static void factor_panel(double* A, long long ld, int n, int k0, int kb, int* fl
         const int jb = std::min(PB, kb - j), m = n - k0 - j - jb, w = kb - j - jb;
         double* D = A11 + j + j * ld;
         if (m > 0) LAUNCH(lu_trsm32_kernel, ceil_div(m, 16) + ceil_div(w, 16), 128, 0, st, D, ld, jb, m, w, flag);
-        if (w > 0) LAUNCH(lu_update32_kernel, 1 + ceil_div(m, 16), 128, 0, st, D, ld, m, w, std::min(PB, w), flag);
+        if (w > 0) LAUNCH(lu_update32_kernel, UPD_CL * (1 + ceil_div(m, 16 * UPD_CL)), 128, 0, st, D, ld, m, w,
+                          std::min(PB, w), flag);
     }
 }
 
@@ -667,7 +774,7 @@ static void run_fast(double* A, long long ld, int n, double* Linv, double* Uinv,
         factor_panel(A, ld, n, k0, h, flag, st);
         if (h2 > 0) {
             double* right = A11 + h * ld;
-            LAUNCH(lu_lower_kernel, ceil_div(h2, INV_C), HB, 0, st, A11, ld, h2);
+            LAUNCH(lu_lower_kernel, ceil_div(h2, LOWER_C), HB, 0, st, A11, ld, h2);
             tensor_product(A11 + h, ld, right, ld, n - k0 - h, h2, h, -1.0, 1.0, right + h, ld, err, st);
             factor_panel(A, ld, n, k0 + h, h2, flag, st);
         }
@@ -677,16 +784,16 @@ static void run_fast(double* A, long long ld, int n, double* Linv, double* Uinv,
         double* A21 = A + (k0 + kb) + k0 * ld;
         double* A22 = A + (k0 + kb) + (k0 + kb) * ld;
         // U12 = L11^{-1} A12
-        LAUNCH(lu_inverse_kernel, dim3(1, LU_NB / INV_C), LU_NB, 0, st, A11, ld, kb, false, Li);
+        LAUNCH(lu_inverse_kernel<1>, dim3(1, LU_NB), LU_NB, 0, st, A11, ld, kb, false, Li);
         tensor_product(Li, LU_NB, A12, ld, kb, n2, kb, 1.0, 0.0, A12, ld, err, st);
         // A22 -= L21 U12
         tensor_product(A21, ld, A12, ld, n2, n2, kb, -1.0, 1.0, A22, ld, err, st);
     }
     // L^{-1} of the last block, and U^{-1} of all
     const int last = (n - 1) / LU_NB, k0 = last * LU_NB;
-    LAUNCH(lu_inverse_kernel, dim3(1, LU_NB / INV_C), LU_NB, 0, st, A + k0 + k0 * ld, ld, n - k0, false,
+    LAUNCH(lu_inverse_kernel<1>, dim3(1, LU_NB), LU_NB, 0, st, A + k0 + k0 * ld, ld, n - k0, false,
            Linv + (long long)last * LU_NB * LU_NB);
-    LAUNCH(lu_inverse_kernel, dim3(last + 1, LU_NB / INV_C), LU_NB, 0, st, A, ld, n, true, Uinv);
+    LAUNCH(lu_inverse_kernel<2>, dim3(last + 1, LU_NB / 2), LU_NB, 0, st, A, ld, n, true, Uinv);
 }
 
 static void run_pivoted(double* A, long long ld, int n, int* ipiv, double* Linv, double* Uinv, int* flag,
@@ -700,7 +807,7 @@ static void run_pivoted(double* A, long long ld, int n, int* ipiv, double* Linv,
         }
     }
     for (int up = 0; up < 2; ++up)
-        LAUNCH(lu_inverse_kernel, dim3(ceil_div(n, LU_NB), LU_NB / INV_C), LU_NB, 0, st, A, ld, n, up != 0,
+        LAUNCH(lu_inverse_kernel<2>, dim3(ceil_div(n, LU_NB), LU_NB / 2), LU_NB, 0, st, A, ld, n, up != 0,
                up ? Uinv : Linv);
 }
 
@@ -748,8 +855,8 @@ void LU64::factor(const double* M, int n_, long long ldm, cudaStream_t st, const
 
 // Few right-hand sides: per block one product with the block's inverse and one update of
 // the rows past it, between B and a second buffer (no copies).
-static void solve_few(const LU64& lu, double* B, long long ldb, int nrhs, cudaStream_t st) {
-    const int n = lu.n, nblk = ceil_div(n, LU_NB);
+static void solve_few(const LU64& lu, int n, double* B, long long ldb, int nrhs, cudaStream_t st) {
+    const int nblk = ceil_div(n, LU_NB);
     const long long ld = lu.ld;
     const double* A = lu.A.get();
     // per-call scratch (stream-ordered), so handles sharing one factor on
@@ -771,11 +878,18 @@ static void solve_few(const LU64& lu, double* B, long long ldb, int nrhs, cudaSt
     }
 }
 
+// Without exchanges the factor of a leading block is the leading block of the factor, and so
+// are the inverses of its diagonal blocks.
+void LU64::solve_leading(int m, double* B, long long ldb, int nrhs, cudaStream_t st) const {
+    if (pivoted || m > n) fail(SQBEM_ERR_ARG, "LU: no factor of the leading block");
+    for (int c = 0; c < nrhs; c += SK_N) solve_few(*this, m, B + c * ldb, ldb, std::min(SK_N, nrhs - c), st);
+}
+
 void LU64::solve(double* B, long long ldb, int nrhs, cudaStream_t st, int* err) const {
     if (nrhs <= 0 || n == 0) return;
     if (pivoted) LAUNCH(laswp_kernel, ceil_div(nrhs, 128), 128, 0, st, B, ldb, n, nrhs, ipiv.get());
     if (nrhs < 64 || !err) {
-        for (int c = 0; c < nrhs; c += SK_N) solve_few(*this, B + c * ldb, ldb, std::min(SK_N, nrhs - c), st);
+        for (int c = 0; c < nrhs; c += SK_N) solve_few(*this, n, B + c * ldb, ldb, std::min(SK_N, nrhs - c), st);
         return;
     }
     // many: the block inverses and the updates as tensor-core products

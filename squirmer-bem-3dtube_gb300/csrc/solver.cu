@@ -181,12 +181,14 @@ void sqbem_swimmer::build_fp64() {
     diag_complete(AuBs.get(), 1, ns, Ns, rsum.get(), tube ? 0.0 : 1.0, nullptr, st);
     deflate(E.get(), 1, ns, panels, mu, st);
     // rigid-body map and C = A_u K (222-234)
-    const auto Kh = rigid_map(host_panels, xc);
-    DevBuf<double> K((size_t)ns * 6, st);
-    K.upload(Kh.data(), Kh.size());
+    std::vector<double> off(ns);
+    for (int p = 0; p < Ns; ++p)
+        for (int k = 0; k < 3; ++k) off[3 * p + k] = host_panels[p].c[k] - xc[k];
+    DevBuf<double> r((size_t)ns, st);
+    r.upload(off.data(), off.size());
     Gc.alloc((size_t)ns * 6, st);
-    gemm64(false, false, ns, 6, ns, 1.0, AuBs.get(), ns, K.get(), ns, 0.0, Gc.get(), ns, st);
-    if (tube) gemm64(false, false, nt, 6, ns, 1.0, AuBt.get(), nt, K.get(), ns, 0.0, Y.get() + (size_t)nt * ns, nt, st);
+    rigid64(ns, Ns, AuBs.get(), ns, r.get(), Gc.get(), ns, st);
+    if (tube) rigid64(nt, Ns, AuBt.get(), nt, r.get(), Y.get() + (size_t)nt * ns, nt, st);
     clock.stop(st);
     clock2.start(st);
     Gs = std::move(E);
@@ -276,7 +278,10 @@ void sqbem_swimmer::solve_prescribed(const double* U, const double* Om, double* 
         solve_mixed(true, 1, w, Uo, Oo, f_sphere, f_tube);
         return;
     }
-    if (!haveGs) {
+    // Gs is the leading block of M (factor_M), so M's factor serves where it is there and its
+    // rows were not exchanged
+    const bool leading = haveM && !luM.pivoted;
+    if (!leading && !haveGs) {
         luGs.factor(Gs.get(), ns, ns, st, "dgesv failed");
         haveGs = true;
     }
@@ -285,7 +290,8 @@ void sqbem_swimmer::solve_prescribed(const double* U, const double* Om, double* 
     DevBuf<double> dw(6, st), x((size_t)n, st);
     dw.upload(w, 6);
     gemm64(false, false, ns, 1, 6, -1.0, Gc.get(), ns, dw.get(), 6, 0.0, x.get(), n, st);
-    luGs.solve(x.get(), n, 1, st);
+    if (leading) luM.solve_leading(ns, x.get(), n, 1, st);
+    else luGs.solve(x.get(), n, 1, st);
     CUDA_CHECK(cudaMemcpyAsync(x.get() + ns, dw.get(), sizeof(double) * 6, cudaMemcpyDeviceToDevice, st));
     if (f_sphere) x.download(f_sphere, ns);
     if (tube && f_tube) {
