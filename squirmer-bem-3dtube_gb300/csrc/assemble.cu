@@ -438,9 +438,8 @@ __device__ __forceinline__ void split2(double v, float& hi, float& lo) {
 
 // FarF of every source panel and the hi + lo split (x, y, z hi; x, y, z lo) of
 // every target: the only FP64 work of the mixed far field.
-__global__ void far_prep_kernel(const PanelRec* __restrict__ src, int nS, const double* __restrict__ tgt, int nT,
-                                FarF* __restrict__ srcf, float* __restrict__ tgtf) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void far_prep(const PanelRec* __restrict__ src, int nS, const double* __restrict__ tgt,
+                                         int nT, FarF* __restrict__ srcf, float* __restrict__ tgtf, int k) {
     if (k < nS) {
         const PanelRec& P = src[k];
         FarF F;
@@ -469,6 +468,27 @@ __global__ void far_prep_kernel(const PanelRec* __restrict__ src, int nS, const 
         for (int q = 0; q < 3; ++q) split2(tgt[3 * k + q], tgtf[6 * k + q], tgtf[6 * k + 3 + q]);
 }
 
+__global__ void far_prep_kernel(const PanelRec* __restrict__ src, int nS, const double* __restrict__ tgt, int nT,
+                                FarF* __restrict__ srcf, float* __restrict__ tgtf) {
+    far_prep(src, nS, tgt, nT, srcf, tgtf, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// blockIdx.y: one of several panel sets or target sets
+constexpr int PREP_MAX = 96;
+struct PrepArgs {
+    struct {
+        const PanelRec* src;
+        const double* tgt;
+        FarF* srcf;
+        float* tgtf;
+        int nS, nT;
+    } j[PREP_MAX];
+};
+__global__ void far_prep_group(const __grid_constant__ PrepArgs g) {
+    const auto& j = g.j[blockIdx.y];
+    far_prep(j.src, j.nS, j.tgt, j.nT, j.srcf, j.tgtf, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 // Mixed mode: as far_kernel, all in FP32.  c - x0 comes from the hi + lo pairs
 // (relative error <= ~2.5 ulp per component, so d2 is within ~5e-7 of the exact
 // value), and the rule from comparing d2 with the thresholds' 1e-5 bands: a
@@ -480,9 +500,10 @@ __global__ void far_prep_kernel(const PanelRec* __restrict__ src, int nS, const 
 // so no thread waits on a global atomic inside the pair loop.
 // SRC: source panels per CTA (FAR_SRC, or fewer for blocks with few targets,
 // such as the tube's sector-0 rows, so that the grid still fills the GPU).
+// tag goes into the upper bits of a near entry's target (the job of a grouped launch).
 template <class TO, int SRC>
-__global__ void __launch_bounds__(FAR_TGT, 8) far_kernel_f32(BlockJob<TO> job, const FarF* __restrict__ srcf,
-                                                          const float* __restrict__ tgtf) {
+__device__ __forceinline__ void far_f32(const BlockJob<TO>& job, const FarF* __restrict__ srcf,
+                                        const float* __restrict__ tgtf, int tag) {
     constexpr int FAR_PAIRS = FAR_TGT * SRC;
     __shared__ FarF sf[SRC];
     __shared__ int2 nl[FAR_PAIRS];
@@ -531,7 +552,7 @@ __global__ void __launch_bounds__(FAR_TGT, 8) far_kernel_f32(BlockJob<TO> job, c
         if (rule != 0) {
             const bool heavy = rule >= 3;
             const int slot = atomicAdd(&ncount[heavy ? 0 : 1], 1);  // at most FAR_PAIRS in total
-            nl[heavy ? slot : FAR_PAIRS - 1 - slot] = make_int2(i, p | (rule << 28));
+            nl[heavy ? slot : FAR_PAIRS - 1 - slot] = make_int2(i | tag, p | (rule << 28));
             if (job.rule_count) atomicAdd(&rcount[rule], 1);
             continue;
         }
@@ -604,16 +625,42 @@ __global__ void __launch_bounds__(FAR_TGT, 8) far_kernel_f32(BlockJob<TO> job, c
     }
 }
 
+template <class TO, int SRC>
+__global__ void __launch_bounds__(FAR_TGT, 8) far_kernel_f32(BlockJob<TO> job, const FarF* __restrict__ srcf,
+                                                          const float* __restrict__ tgtf) {
+    far_f32<TO, SRC>(job, srcf, tgtf, 0);
+}
+
+// Several blocks of one kind (every swimmer's tube rows, or sphere rows) per launch,
+// blockIdx.z the block.  One by one a 1248 x 320 block took 9.5 us to prepare, 12.5 us for
+// its 1600 short CTAs and 6.7 us for its near pairs, most of it launch and tail.
+constexpr int GROUP_MAX = 48;
+constexpr int TAG_SHIFT = 24;  // near entries: target below, block above
+struct GroupArgs {
+    int n;
+    BlockJob<float> job[GROUP_MAX];
+    const FarF* srcf[GROUP_MAX];
+    const float* tgtf[GROUP_MAX];
+};
+
+template <int SRC>
+__global__ void __launch_bounds__(FAR_TGT, 8) far_group_kernel(const __grid_constant__ GroupArgs g) {
+    const BlockJob<float>& job = g.job[blockIdx.z];
+    if ((int)(blockIdx.x * FAR_TGT) >= job.nT || (int)(blockIdx.y * SRC) >= job.nS) return;
+    far_f32<float, SRC>(job, g.srcf[blockIdx.z], g.tgtf[blockIdx.z], (int)blockIdx.z << TAG_SHIFT);
+}
+
 // ---------------------------------------------------------------- near kernel
 // Warps take pairs from a shared counter, heavy pairs first (a heavy pair costs
 // up to 16x a light one; static striding left SMs idle for a third of the run).
 // Each pair is computed whole by one warp, so the result does not depend on the
 // order.
-template <class TO, bool MIXED>
-__global__ void __launch_bounds__(32, 24) near_kernel(BlockJob<TO> job) {
+// list: the job that holds the near list; of(e): the job of a list entry.
+template <class TO, bool MIXED, class Of>
+__device__ __forceinline__ void near_pairs(const BlockJob<TO>& list, int imask, Of of) {
     const int lane = threadIdx.x & 31;
-    const int nh = job.near_count[0], nl = job.near_count[1];
-    if (nh + nl > job.near_cap) return;  // overflow: reported by the host
+    const int nh = list.near_count[0], nl = list.near_count[1];
+    if (nh + nl > list.near_cap) return;  // overflow: reported by the host
     // heavy pairs (448-point rule, self integrals) by warp index: warp g takes
     // g, g + W, ...; one-warp CTAs are dispatched round-robin over the SMs, so
     // consecutive heavy pairs run on different SMs' FP64 pipes (a shared counter
@@ -629,13 +676,14 @@ __global__ void __launch_bounds__(32, 24) near_kernel(BlockJob<TO> job) {
             kh += W;
         } else {
             int t = 0;
-            if (lane == 0) t = atomicAdd(job.near_count + 2, 1);
+            if (lane == 0) t = atomicAdd(list.near_count + 2, 1);
             t = __shfl_sync(0xffffffffu, t, 0);
             if (t >= nl) break;
             k = nh + t;
         }
-        const int2 e = job.near_list[k < nh ? k : job.near_cap - 1 - (k - nh)];
-        const int i = e.x, p = e.y & 0x0fffffff;
+        const int2 e = list.near_list[k < nh ? k : list.near_cap - 1 - (k - nh)];
+        const BlockJob<TO>& job = of(e.x);
+        const int i = e.x & imask, p = e.y & 0x0fffffff;
         const PanelRec P = job.src[p];
         const double x = job.tgt[3 * i], y = job.tgt[3 * i + 1], z = job.tgt[3 * i + 2];
         const int rule = e.y >> 28;  // exact rule (4 = self), decided by the far kernel
@@ -672,6 +720,30 @@ __global__ void __launch_bounds__(32, 24) near_kernel(BlockJob<TO> job) {
             if (job.D) job.D[r * job.d_rs + c * job.d_cs] = (TO)(dl * job.dscale);
         }
     }
+}
+
+template <class TO, bool MIXED>
+__global__ void __launch_bounds__(32, 24) near_kernel(BlockJob<TO> job) {
+    near_pairs<TO, MIXED>(job, 0x7fffffff, [&](int) -> const BlockJob<TO>& { return job; });
+}
+
+__global__ void __launch_bounds__(32, 24) near_group_kernel(const __grid_constant__ GroupArgs g) {
+    near_pairs<float, true>(g.job[0], (1 << TAG_SHIFT) - 1,
+                            [&](int x) -> const BlockJob<float>& { return g.job[x >> TAG_SHIFT]; });
+}
+
+// 24 one-warp CTAs per SM (80 registers per thread): consecutive pairs of the list -- the heavy
+// 448-point and self pairs come first -- go to warps of different SMs, so they do not queue
+// on a few SMs' FP64 pipes
+static int near_warps() {
+    static int sms = 0;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        int dev = 0;
+        CUDA_CHECK(cudaGetDevice(&dev));
+        CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    });
+    return sms * 24;
 }
 
 template <class TO>
@@ -712,17 +784,7 @@ void assemble_block(const BlockJob<TO>& job0, int near_cap, cudaStream_t st, boo
     } else {
         TIMED_LAUNCH("assemble_far", fl, by, far_kernel<TO>, grid, FAR_TGT, 0, st, job);
     }
-    static int sms = 0;
-    static std::once_flag sms_once;
-    std::call_once(sms_once, [] {
-        int dev = 0;
-        CUDA_CHECK(cudaGetDevice(&dev));
-        CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    });
-    // 24 one-warp CTAs per SM (80 registers per thread): consecutive pairs of the
-    // list -- the heavy 448-point and self pairs come first -- go to warps of
-    // different SMs, so they do not queue on a few SMs' FP64 pipes
-    const int warps = sms * 24;
+    const int warps = near_warps();
     // credited FP64-pipe work of the near kernel (kernel statistics only, which
     // count the pairs per rule on the device): the 448-point rule and the self
     // integral, plus in FP64 mode the 28- and 112-point rules (FP32 in mixed mode)
@@ -753,6 +815,107 @@ void assemble_block(const BlockJob<TO>& job0, int near_cap, cudaStream_t st, boo
     }
 }
 
+// FP32 blocks of the mixed path, column-major, by grouped launches.  Panel sets and target sets
+// that several blocks share (the tube of an ensemble) are prepared once.  The near list of
+// a launch holds every pair of its blocks, so it cannot overflow: launches of up to
+// GROUP_MAX blocks and 32 M pairs.
+void assemble_group(const std::vector<BlockJob<float>>& jobs, cudaStream_t st) {
+    init_tables();
+    for (size_t i0 = 0; i0 < jobs.size();) {
+        GroupArgs g;
+        PrepArgs pr;
+        long long pairs = 0;
+        int mt = 0, ms = 0, mp = 0, np = 0;
+        std::vector<size_t> so, to;  // offsets into the prepared arrays
+        size_t ns = 0, nt = 0;
+        g.n = 0;
+        while (i0 < jobs.size() && g.n < GROUP_MAX) {
+            const BlockJob<float>& J = jobs[i0];
+            if (J.nT <= 0 || J.nS <= 0) {
+                ++i0;
+                continue;
+            }
+            const long long p = (long long)J.nT * J.nS;
+            if (J.nT >= 1 << TAG_SHIFT || p > 32LL << 20) {  // outside the group's forms
+                if (g.n > 0) break;
+                assemble_block(J, (int)std::min<long long>(p, 64LL << 20), st, true);
+                ++i0;
+                continue;
+            }
+            if (g.n > 0 && pairs + p > 32LL << 20) break;
+            pairs += p;
+            // this block's panel set and target set, or an earlier block's
+            size_t a = ns, b = nt;
+            for (int k = 0; k < g.n; ++k) {
+                if (g.job[k].src == J.src && g.job[k].nS == J.nS) a = so[k];
+                if (g.job[k].tgt == J.tgt && g.job[k].nT == J.nT) b = to[k];
+            }
+            const bool newS = a == ns, newT = b == nt;
+            if (newS || newT) {
+                pr.j[np].src = J.src;
+                pr.j[np].tgt = J.tgt;
+                pr.j[np].nS = newS ? J.nS : 0;
+                pr.j[np].nT = newT ? J.nT : 0;
+                pr.j[np].srcf = reinterpret_cast<FarF*>(a);
+                pr.j[np].tgtf = reinterpret_cast<float*>(b);
+                mp = std::max({mp, pr.j[np].nS, pr.j[np].nT});
+                ++np;
+            }
+            so.push_back(a);
+            to.push_back(b);
+            if (newS) ns += J.nS;
+            if (newT) nt += J.nT;
+            g.job[g.n++] = J;
+            mt = std::max(mt, J.nT);
+            ms = std::max(ms, J.nS);
+            ++i0;
+        }
+        if (g.n == 0) continue;
+        DevBuf<FarF> srcf(ns, st);
+        DevBuf<float> tgtf(6 * nt, st);
+        DevBuf<int2> list((size_t)pairs, st);
+        DevBuf<int> count(3, st), rc;
+        count.zero();
+        if (kstats_on()) {
+            rc.alloc(5, st);
+            rc.zero();
+        }
+        for (int k = 0; k < np; ++k) {
+            pr.j[k].srcf = srcf.get() + reinterpret_cast<size_t>(pr.j[k].srcf);
+            pr.j[k].tgtf = tgtf.get() + 6 * reinterpret_cast<size_t>(pr.j[k].tgtf);
+        }
+        for (int k = 0; k < g.n; ++k) {
+            g.srcf[k] = srcf.get() + so[k];
+            g.tgtf[k] = tgtf.get() + 6 * to[k];
+            g.job[k].near_list = list.get();
+            g.job[k].near_count = count.get();
+            g.job[k].near_cap = (int)pairs;
+            g.job[k].rule_count = rc.get();
+        }
+        double by = 0;
+        for (int k = 0; k < g.n; ++k)
+            by += 36.0 * g.job[k].nT * g.job[k].nS * ((g.job[k].S ? 1 : 0) + (g.job[k].D ? 1 : 0));
+        LAUNCH(far_prep_group, dim3(ceil_div(mp, 128), np), 128, 0, st, pr);
+        const dim3 grid(ceil_div(mt, FAR_TGT), ceil_div(ms, FAR_SRC), g.n), grid4(grid.x, ceil_div(ms, 4), g.n);
+        // few CTAs (a swimmer or two): 4 sources each, as for one block
+        if ((long long)grid.x * grid.y * grid.z < 2LL * 152 * 4)
+            TIMED_LAUNCH("assemble_far", 7.0 * FLOPS_PER_EVAL * pairs, by, far_group_kernel<4>, grid4, FAR_TGT, 0, st, g);
+        else
+            TIMED_LAUNCH("assemble_far", 7.0 * FLOPS_PER_EVAL * pairs, by, far_group_kernel<FAR_SRC>, grid, FAR_TGT, 0, st,
+                         g);
+        if (kstats_on()) {
+            int* counts = kstat_pinned_ints(5);
+            CUDA_CHECK(cudaMemcpyAsync(counts, rc.get(), 5 * sizeof(int), cudaMemcpyDeviceToHost, st));
+            const double w[5] = {0.0, 0.0, 0.0, 448.0 * FLOPS_PER_EVAL, 300.0 * FLOPS_PER_EVAL_SL};
+            const int ks = kstat_begin(st);
+            LAUNCH(near_group_kernel, near_warps(), 32, 0, st, g);
+            kstat_end_counted(ks, "assemble_near", st, counts, w, 5, 0.0);
+        } else {
+            LAUNCH(near_group_kernel, near_warps(), 32, 0, st, g);
+        }
+    }
+}
+
 template void assemble_block<double>(const BlockJob<double>&, int, cudaStream_t, bool);
 template void assemble_block<float>(const BlockJob<float>&, int, cudaStream_t, bool);
 
@@ -772,8 +935,8 @@ __device__ __forceinline__ void two_sum_f(float& s, float& c, float x) {
 }
 
 template <class T>
-__global__ void rowsum_kernel(const T* __restrict__ D, long long rs, long long cs, int nrows, int ncolpanels,
-                              int chunk, double* __restrict__ partial) {
+__device__ __forceinline__ void rowsum_chunk(const T* __restrict__ D, long long rs, long long cs, int nrows,
+                                             int ncolpanels, int chunk, double* __restrict__ partial) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= nrows) return;
     const int c = blockIdx.y;
@@ -802,11 +965,19 @@ __global__ void rowsum_kernel(const T* __restrict__ D, long long rs, long long c
     }
 }
 
-// Add the chunked row sums (fixed order) to out[row * 3 + b]
-__global__ void rowsum_finish(const double* __restrict__ partial, int nchunk, int nrows, double* __restrict__ out) {
+template <class T>
+__global__ void rowsum_kernel(const T* __restrict__ D, long long rs, long long cs, int nrows, int ncolpanels,
+                              int chunk, double* __restrict__ partial) {
+    rowsum_chunk(D, rs, cs, nrows, ncolpanels, chunk, partial);
+}
+
+// Add the chunked row sums (fixed order) to out[row * 3 + b]; the loads of eight chunks at once
+__device__ __forceinline__ void rowsum_add(const double* __restrict__ partial, int nchunk, int nrows,
+                                           double* __restrict__ out) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= nrows) return;
     double s0 = 0, s1 = 0, s2 = 0;
+#pragma unroll 8
     for (int c = 0; c < nchunk; ++c) {
         const double* o = partial + ((long long)c * nrows + row) * 3;
         s0 += o[0]; s1 += o[1]; s2 += o[2];
@@ -814,6 +985,10 @@ __global__ void rowsum_finish(const double* __restrict__ partial, int nchunk, in
     out[row * 3] += s0;
     out[row * 3 + 1] += s1;
     out[row * 3 + 2] += s2;
+}
+
+__global__ void rowsum_finish(const double* __restrict__ partial, int nchunk, int nrows, double* __restrict__ out) {
+    rowsum_add(partial, nchunk, nrows, out);
 }
 
 template <class T>
@@ -828,6 +1003,48 @@ void add_rowsums(const T* D, long long rs, long long cs, int nrows, int ncolpane
 }
 template void add_rowsums<double>(const double*, long long, long long, int, int, double*, cudaStream_t);
 template void add_rowsums<float>(const float*, long long, long long, int, int, double*, cudaStream_t);
+
+// The FP32 row sums and the diagonal completion of several blocks per launch (blockIdx.z / .y
+// the block; the same chunks and order as above).
+struct SumArgs {
+    RowsumJob j[GROUP_MAX];
+    double* partial[GROUP_MAX];
+};
+__global__ void rowsum_group_kernel(const __grid_constant__ SumArgs g, int chunk) {
+    const RowsumJob& J = g.j[blockIdx.z];
+    if ((int)(blockIdx.y * chunk) >= J.npanels) return;
+    rowsum_chunk(J.D, 1, J.ld, J.nrows, J.npanels, chunk, g.partial[blockIdx.z]);
+}
+__global__ void rowsum_finish_group(const __grid_constant__ SumArgs g, int chunk) {
+    const RowsumJob& J = g.j[blockIdx.y];
+    rowsum_add(g.partial[blockIdx.y], (J.npanels + chunk - 1) / chunk, J.nrows, J.out);
+}
+
+void add_rowsums_group(const std::vector<RowsumJob>& jobs, cudaStream_t st) {
+    const int chunk = 32;
+    for (size_t i0 = 0; i0 < jobs.size(); i0 += GROUP_MAX) {
+        SumArgs g;
+        const int n = (int)std::min<size_t>(GROUP_MAX, jobs.size() - i0);
+        size_t total = 0;
+        int mr = 0, mc = 0;
+        for (int k = 0; k < n; ++k) {
+            g.j[k] = jobs[i0 + k];
+            const int nc = ceil_div(g.j[k].npanels, chunk);
+            total += (size_t)nc * g.j[k].nrows * 3;
+            mr = std::max(mr, g.j[k].nrows);
+            mc = std::max(mc, nc);
+        }
+        if (mr <= 0 || mc <= 0) continue;
+        DevBuf<double> part(total, st);
+        size_t off = 0;
+        for (int k = 0; k < n; ++k) {
+            g.partial[k] = part.get() + off;
+            off += (size_t)ceil_div(g.j[k].npanels, chunk) * g.j[k].nrows * 3;
+        }
+        LAUNCH(rowsum_group_kernel, dim3(ceil_div(mr, 128), mc, n), 128, 0, st, g, chunk);
+        LAUNCH(rowsum_finish_group, dim3(ceil_div(mr, 128), n), 128, 0, st, g, chunk);
+    }
+}
 
 // A(3i+a, 3i+b) -= rsum[(3i+a)*3 + b] (+ ext * delta_ab) for columns b with
 // colmask bit b of mask[i] set (all three when mask == nullptr).

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <vector>
+
 namespace sqbem {
 
 // One source panel as the kernels read it (144 bytes): vertices, unit normal
@@ -62,6 +64,15 @@ struct FieldJob {
 void init_tables();
 template <class TO>
 void assemble_block(const BlockJob<TO>& job, int near_cap, cudaStream_t st, bool mixed);
+void assemble_group(const std::vector<BlockJob<float>>& jobs, cudaStream_t st);
+// add_rowsums for several column-major FP32 blocks (leading dimension ld)
+struct RowsumJob {
+    const float* D = nullptr;
+    long long ld = 0;
+    int nrows = 0, npanels = 0;
+    double* out = nullptr;
+};
+void add_rowsums_group(const std::vector<RowsumJob>& jobs, cudaStream_t st);
 template <class T>
 void add_rowsums(const T* D, long long rs, long long cs, int nrows, int ncolpanels, double* out, cudaStream_t st);
 template <class T>

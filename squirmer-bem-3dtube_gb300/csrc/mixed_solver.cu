@@ -221,23 +221,29 @@ void mixed_build_tubes(const std::vector<sqbem_tube*>& tubes, const MixedCtx& cx
         four = fourier_supported(syms[k]);
     }
     if (four) {
-        std::vector<DevBuf<float>> T0(G);
+        std::vector<DevBuf<float>> T0;
         std::vector<FourierTube*> fts;
         std::vector<const TubeSymmetry*> sp;
         std::vector<const float*> t0p;
+        std::vector<const sqbem_tube*> ct;
+        std::vector<float*> Tp;
+        std::vector<long long> ld;
         for (size_t k = 0; k < G; ++k) {
             sqbem_tube* t = tubes[k];
             MixedTube& M = t->mt;
             M.nt = 3 * t->Nt;
             M.ntp = pad128(M.nt);
             M.T.alloc((size_t)M.nt * M.nt, cx.st);
-            assemble_tube_symmetric(t, syms[k], M.T.get(), M.nt, cx.st, &T0[k]);
             M.lu.reset();
             M.ft = std::make_unique<FourierTube>();
             fts.push_back(M.ft.get());
             sp.push_back(&syms[k]);
-            t0p.push_back(T0[k].get());
+            ct.push_back(t);
+            Tp.push_back(M.T.get());
+            ld.push_back(M.nt);
         }
+        assemble_tubes_symmetric(ct, sp, Tp, ld, T0, cx.st);
+        for (size_t k = 0; k < G; ++k) t0p.push_back(T0[k].get());
         fourier_build(fts, sp, t0p, cx);
         check_ctx(cx, "mixed tube (Fourier blocks)");
         // A tube shared by many swimmers could also keep T^{-1} (solving the identity
@@ -343,6 +349,10 @@ void mixed_build_swimmers(const std::vector<sqbem_swimmer*>& sw, const MixedCtx&
     std::vector<RigidJob> rj;
     std::vector<DevBuf<double>> tmp;
     tmp.reserve(3 * G);
+    std::vector<BlockJob<float>> tube_rows, sphere_rows;
+    std::vector<RowsumJob> sums;
+    std::vector<DevBuf<float>> Dt;
+    std::vector<DevBuf<double>> rsums;
     for (sqbem_swimmer* s : sw) {
         MixedSwimmer& M = s->mx;
         const int Ns = s->Ns, Nt = s->Nt;
@@ -367,21 +377,31 @@ void mixed_build_swimmers(const std::vector<sqbem_swimmer*>& sw, const MixedCtx&
         if (bounded) {
             M.B.alloc((size_t)nt * ns, cx.st);
             M.AuBt.alloc((size_t)nt * ns, cx.st);
-            auto j1 = fjob(s->tube->panels, s->panels, false, s->mu, M.B.get(), nt, M.AuBt.get(), nt);
-            assemble_block(j1, cap_pairs(Nt, Ns), cx.st, true);
+            tube_rows.push_back(fjob(s->tube->panels, s->panels, false, s->mu, M.B.get(), nt, M.AuBt.get(), nt));
             M.D.alloc((size_t)ns * nt, cx.st);
-            DevBuf<float> Dt((size_t)ns * nt, cx.st);
-            auto j2 = fjob(s->panels, s->tube->panels, false, s->mu, M.D.get(), ns, Dt.get(), ns);
-            assemble_block(j2, cap_pairs(Ns, Nt), cx.st, true);
-            add_rowsums<float>(Dt.get(), 1, ns, ns, Nt, rsum.get(), cx.st);
+            Dt.emplace_back((size_t)ns * nt, cx.st);
+            sphere_rows.push_back(fjob(s->panels, s->tube->panels, false, s->mu, M.D.get(), ns, Dt.back().get(), ns));
+            sums.push_back({Dt.back().get(), ns, ns, Nt, rsum.get()});
         }
-        if (!shared) {
+        rsums.push_back(std::move(rsum));
+    }
+    // tube rows <- sphere and sphere rows <- tube of every member, in two grouped assemblies
+    assemble_group(tube_rows, cx.st);
+    assemble_group(sphere_rows, cx.st);
+    add_rowsums_group(sums, cx.st);
+    Dt.clear();
+    for (size_t g = 0; g < G; ++g) {
+        sqbem_swimmer* s = sw[g];
+        MixedSwimmer& M = s->mx;
+        const int Ns = s->Ns, ns = M.ns, nt = M.nt;
+        double* const rsum = rsums[g].get();
+        if (!M.sphere) {
             auto j3 = fjob(s->panels, s->panels, true, s->mu, M.E.get(), ns, M.AuBs.get(), ns);
             assemble_block(j3, cap_pairs(Ns, Ns), cx.st, true);
-            add_rowsums<float>(M.AuBs.get(), 1, ns, ns, Ns, rsum.get(), cx.st);
+            add_rowsums<float>(M.AuBs.get(), 1, ns, ns, Ns, rsum, cx.st);
             deflate<float>(M.E.get(), 1, ns, s->panels, s->mu, cx.st);
         }
-        diag_complete<float>(M.AuBs.get(), 1, ns, Ns, rsum.get(), bounded ? 0.0 : 1.0, nullptr, cx.st);
+        diag_complete<float>(M.AuBs.get(), 1, ns, Ns, rsum, bounded ? 0.0 : 1.0, nullptr, cx.st);
         // rigid-body map, C = A_u K (accumulated in FP64, stored FP32)   (swimmer.hpp:222-234)
         const auto Kh = rigid_map(s->host_panels, s->xc);
         M.K.alloc(Kh.size(), cx.st);

@@ -122,50 +122,71 @@ __global__ void deflate_rows_kernel(float* __restrict__ T0, int ld0, const int* 
 
 }  // namespace
 
-void assemble_tube_symmetric(const sqbem_tube* t, const TubeSymmetry& sym, float* T, long long ld,
-                             cudaStream_t st, DevBuf<float>* T0_out) {
-    const int Nt = t->Nt, nb = sym.nb, nth = sym.nth;
-    if (!sym.ok || nb * nth != Nt) fail(SQBEM_ERR_ARG, "tube assembly: the panels have no rotational symmetry");
+void assemble_tubes_symmetric(const std::vector<const sqbem_tube*>& tubes, const std::vector<const TubeSymmetry*>& syms,
+                              const std::vector<float*>& T, const std::vector<long long>& ld,
+                              std::vector<DevBuf<float>>& T0, cudaStream_t st) {
+    const size_t G = tubes.size();
+    std::vector<DevBuf<double>> tc(G);
+    std::vector<DevBuf<int>> self(G);
+    std::vector<BlockJob<float>> jobs(G);
+    T0.clear();
+    T0.resize(G);
     // rows of sector 0: targets are the representatives' centroids, sources all panels
-    std::vector<double> hc(3 * (size_t)nb);
-    for (int a = 0; a < nb; ++a)
-        for (int k = 0; k < 3; ++k) hc[3 * a + k] = t->host_panels[sym.rep_panel[a]].c[k];
-    DevBuf<double> tc(hc.size(), st);
-    tc.upload(hc.data(), hc.size());
-    DevBuf<int> self(nb, st);
-    self.upload(sym.rep_panel.data(), nb);
-    const int ld0 = 3 * nb;
-    DevBuf<float> T0((size_t)ld0 * 3 * Nt, st);
-    T0.zero();
-    BlockJob<float> j;
-    j.tgt = tc.get();
-    j.nT = nb;
-    j.src = t->panels.rec.get();
-    j.nS = Nt;
-    j.self_of = self.get();
-    j.S = T0.get();
-    j.s_rs = 1;
-    j.s_cs = ld0;
-    j.sscale = 1.0 / (EIGHT_PI * t->mu);
-    j.dscale = -1.0 / EIGHT_PI;
-    assemble_block(j, (int)std::min<long long>((long long)nb * Nt, 64LL << 20), st, true);
-    const double sc = 1.0 / (EIGHT_PI * t->mu * std::sqrt(t->panels.area_total));
-    LAUNCH(deflate_rows_kernel, dim3(ceil_div(ld0, 128), 3 * Nt), 128, 0, st, T0.get(), ld0, self.get(), nb,
-           t->panels.rec.get(), Nt, sc);
-    // the rotation of every sector and the panel maps
-    std::vector<float2> hr(nth);
-    const double al = 2.0 * 3.14159265358979323846 / nth;
-    for (int s = 0; s < nth; ++s) hr[s] = make_float2((float)std::cos(s * al), (float)std::sin(s * al));
-    DevBuf<float2> rot(nth, st);
-    rot.upload(hr.data(), nth);
-    DevBuf<int> sector(Nt, st), rep(Nt, st), panel((size_t)nb * nth, st);
-    sector.upload(sym.sector.data(), Nt);
-    rep.upload(sym.rep.data(), Nt);
-    panel.upload(sym.panel.data(), (size_t)nb * nth);
-    const double bytes = 4.0 * 9.0 * Nt * (double)Nt;
-    TIMED_LAUNCH("tube_fill", 0.0, bytes, tube_fill_kernel, dim3(ceil_div(Nt, 128), Nt), 128, 0, st, T, ld, T0.get(),
-                 ld0, Nt, nth, sector.get(), rep.get(), panel.get(), rot.get());
-    if (T0_out) *T0_out = std::move(T0);
+    for (size_t g = 0; g < G; ++g) {
+        const sqbem_tube* t = tubes[g];
+        const TubeSymmetry& sym = *syms[g];
+        const int Nt = t->Nt, nb = sym.nb, ld0 = 3 * nb;
+        if (!sym.ok || nb * sym.nth != Nt) fail(SQBEM_ERR_ARG, "tube assembly: the panels have no rotational symmetry");
+        std::vector<double> hc(3 * (size_t)nb);
+        for (int a = 0; a < nb; ++a)
+            for (int k = 0; k < 3; ++k) hc[3 * a + k] = t->host_panels[sym.rep_panel[a]].c[k];
+        tc[g].alloc(hc.size(), st);
+        tc[g].upload(hc.data(), hc.size());
+        self[g].alloc(nb, st);
+        self[g].upload(sym.rep_panel.data(), nb);
+        T0[g].alloc((size_t)ld0 * 3 * Nt, st);
+        T0[g].zero();
+        BlockJob<float>& j = jobs[g];
+        j.tgt = tc[g].get();
+        j.nT = nb;
+        j.src = t->panels.rec.get();
+        j.nS = Nt;
+        j.self_of = self[g].get();
+        j.S = T0[g].get();
+        j.s_rs = 1;
+        j.s_cs = ld0;
+        j.sscale = 1.0 / (EIGHT_PI * t->mu);
+        j.dscale = -1.0 / EIGHT_PI;
+    }
+    assemble_group(jobs, st);
+    for (size_t g = 0; g < G; ++g) {
+        const sqbem_tube* t = tubes[g];
+        const TubeSymmetry& sym = *syms[g];
+        const int Nt = t->Nt, nb = sym.nb, nth = sym.nth, ld0 = 3 * nb;
+        const double sc = 1.0 / (EIGHT_PI * t->mu * std::sqrt(t->panels.area_total));
+        LAUNCH(deflate_rows_kernel, dim3(ceil_div(ld0, 128), 3 * Nt), 128, 0, st, T0[g].get(), ld0, self[g].get(), nb,
+               t->panels.rec.get(), Nt, sc);
+        // the rotation of every sector and the panel maps
+        std::vector<float2> hr(nth);
+        const double al = 2.0 * 3.14159265358979323846 / nth;
+        for (int s = 0; s < nth; ++s) hr[s] = make_float2((float)std::cos(s * al), (float)std::sin(s * al));
+        DevBuf<float2> rot(nth, st);
+        rot.upload(hr.data(), nth);
+        DevBuf<int> sector(Nt, st), rep(Nt, st), panel((size_t)nb * nth, st);
+        sector.upload(sym.sector.data(), Nt);
+        rep.upload(sym.rep.data(), Nt);
+        panel.upload(sym.panel.data(), (size_t)nb * nth);
+        const double bytes = 4.0 * 9.0 * Nt * (double)Nt;
+        TIMED_LAUNCH("tube_fill", 0.0, bytes, tube_fill_kernel, dim3(ceil_div(Nt, 128), Nt), 128, 0, st, T[g], ld[g],
+                     T0[g].get(), ld0, Nt, nth, sector.get(), rep.get(), panel.get(), rot.get());
+    }
+}
+
+void assemble_tube_symmetric(const sqbem_tube* t, const TubeSymmetry& sym, float* T, long long ld, cudaStream_t st,
+                             DevBuf<float>* T0_out) {
+    std::vector<DevBuf<float>> T0;
+    assemble_tubes_symmetric({t}, {&sym}, {T}, {ld}, T0, st);
+    if (T0_out) *T0_out = std::move(T0[0]);
 }
 
 }  // namespace sqbem

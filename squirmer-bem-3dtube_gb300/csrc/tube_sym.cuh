@@ -45,4 +45,10 @@ TubeSymmetry tube_symmetry(const std::vector<PanelRec>& P, int nth);
 void assemble_tube_symmetric(const sqbem_tube* t, const TubeSymmetry& sym, float* T, long long ld,
                              cudaStream_t st, DevBuf<float>* T0_out = nullptr);
 
+// The same for several tubes, their sector-0 rows assembled by grouped launches (T0: one
+// buffer per tube).
+void assemble_tubes_symmetric(const std::vector<const sqbem_tube*>& tubes, const std::vector<const TubeSymmetry*>& syms,
+                              const std::vector<float*>& T, const std::vector<long long>& ld,
+                              std::vector<DevBuf<float>>& T0, cudaStream_t st);
+
 }  // namespace sqbem
