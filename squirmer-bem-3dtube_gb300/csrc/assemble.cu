@@ -339,11 +339,11 @@ constexpr int FAR_SRC = 16;   // source panels per CTA
 // root or division unless it lies within 1e-12 of the threshold or below: 270 FP64
 // operations a pair instead of 400 (1392 x 1280 panels both ways and 1280 x 1280: 4.0 ms before).
 constexpr int FAR64_WORDS = 30;
-template <class TO>
+template <class TO, int SRC>
 __global__ void __launch_bounds__(FAR_TGT) far_kernel(BlockJob<TO> job) {
-    __shared__ double sp[FAR_SRC][FAR64_WORDS];  // o (21), c, n, 9 h^2, S scale, D scale
-    const int p0 = blockIdx.y * FAR_SRC;
-    const int ns = min(FAR_SRC, job.nS - p0);
+    __shared__ double sp[SRC][FAR64_WORDS];  // o (21), c, n, 9 h^2, S scale, D scale
+    const int p0 = blockIdx.y * SRC;
+    const int ns = min(SRC, job.nS - p0);
     for (int e = threadIdx.x; e < ns * 10; e += FAR_TGT) {
         const int s = e / 10, q = e - 10 * s;
         const PanelRec& P = job.src[p0 + s];
@@ -782,7 +782,15 @@ void assemble_block(const BlockJob<TO>& job0, int near_cap, cudaStream_t st, boo
             TIMED_LAUNCH("assemble_far", fl, by, (far_kernel_f32<TO, FAR_SRC>), grid, FAR_TGT, 0, st, job, srcf.get(),
                          tgtf.get());
     } else {
-        TIMED_LAUNCH("assemble_far", fl, by, far_kernel<TO>, grid, FAR_TGT, 0, st, job);
+        // a pair takes a warp 270 x 64 cycles, so 16 sources one after the other are 140 us: fewer
+        // per CTA until every SM quarter has a warp (80 x 80 panels: 168 us with 16)
+        const long long ctas = (long long)grid.x * grid.y;
+        if (ctas >= 304) TIMED_LAUNCH("assemble_far", fl, by, (far_kernel<TO, FAR_SRC>), grid, FAR_TGT, 0, st, job);
+        else if (ctas >= 76)
+            TIMED_LAUNCH("assemble_far", fl, by, (far_kernel<TO, 4>), dim3(grid.x, ceil_div(job.nS, 4)), FAR_TGT, 0, st,
+                         job);
+        else
+            TIMED_LAUNCH("assemble_far", fl, by, (far_kernel<TO, 1>), dim3(grid.x, job.nS), FAR_TGT, 0, st, job);
     }
     const int warps = near_warps();
     // credited FP64-pipe work of the near kernel (kernel statistics only, which
@@ -1378,28 +1386,34 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
         F[k].point(X[k], o);
     }
     int* const list = lists + wl * PPW * FIELD_NEAR_CAP;
-    for (int base = rank * TP; base < job.P; base += ncl * TP) {
-        const int np = min(TP, job.P - base);
+    // SHARED: consecutive panels go to different CTAs and warps, so that the near ones, which are
+    // neighbours, are shared out too (by whole tiles one warp had them all: 200 us for 60
+    // points)
+    auto index = [&](int base, int q) {
+        return SHARED ? base + (q & 31) * (FIELD_WARPS * ncl) + (q >> 5) * ncl + rank : base + q;
+    };
+    for (int base = 0; base < job.P; base += ncl * TP) {
+        const int mine = index(base, threadIdx.x);
+        const bool has = (int)threadIdx.x < TP && mine < job.P;
         __syncthreads();
         if (threadIdx.x == 0) tex = 0;
         __syncthreads();
-        if (sizeof(TC) == 4 && (int)threadIdx.x < np) {
-            const int e = FieldArith<TC>::exponent(job, base + threadIdx.x);
+        if (sizeof(TC) == 4 && has) {
+            const int e = FieldArith<TC>::exponent(job, mine);
             if (e) atomicMax(&tex, e);
         }
         __syncthreads();
         const int ex = tex;
-        if ((int)threadIdx.x < np)
-            FieldArith<TC>::stage(tile + threadIdx.x * W, job, base + threadIdx.x, o, ex);
+        if (has) FieldArith<TC>::stage(tile + threadIdx.x * W, job, mine, o, ex);
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < PPW; ++k) F[k].begin();
-        for (int s = SHARED ? wl * 32 : 0; s < (SHARED ? min(np, wl * 32 + 32) : np); s += 32) {
-            const int q = s + lane, p = base + q;
+        for (int s = SHARED ? wl * 32 : 0; s < (SHARED ? wl * 32 + 32 : min(TP, job.P - base)); s += 32) {
+            const int q = s + lane, p = index(base, q);
 #pragma unroll
             for (int k = 0; k < PPW; ++k) {
                 int rule = 0;
-                if (q < np) rule = F[k].pair(tile + q * W, job, p, X[k], ex == 0x7ff);
+                if (p < job.P) rule = F[k].pair(tile + q * W, job, p, X[k], ex == 0x7ff);
                 const unsigned m = __ballot_sync(0xffffffffu, rule > 0);
                 if (rule > 0) {
                     const int slot = X[k].near + __popc(m & ((1u << lane) - 1));
@@ -1501,12 +1515,13 @@ void field_launch(const FieldJob& job, int cluster, cudaStream_t st) {
 }
 
 // Four points per warp once every SM has its 32 points; below that one per warp, and a few
-// points share a CTA or a cluster of four each, which costs staging every panel per point.
+// points share a CTA or a cluster of four or eight each, which costs staging every panel
+// per point.
 template <class TC>
 void field_dispatch(const FieldJob& job, cudaStream_t st) {
     if (job.npts >= 152 * FIELD_WARPS * 4) field_launch<TC, 4, false>(job, 1, st);
     else if (job.npts >= 152 * FIELD_WARPS) field_launch<TC, 1, false>(job, 1, st);
-    else field_launch<TC, 1, true>(job, job.npts < 152 * 2 ? 4 : 1, st);
+    else field_launch<TC, 1, true>(job, job.npts < 152 ? 8 : job.npts < 152 * 2 ? 4 : 1, st);
 }
 }  // namespace
 

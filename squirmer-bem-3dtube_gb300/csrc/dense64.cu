@@ -793,7 +793,8 @@ static void run_fast(double* A, long long ld, int n, double* Linv, double* Uinv,
     const int last = (n - 1) / LU_NB, k0 = last * LU_NB;
     LAUNCH(lu_inverse_kernel<1>, dim3(1, LU_NB), LU_NB, 0, st, A + k0 + k0 * ld, ld, n - k0, false,
            Linv + (long long)last * LU_NB * LU_NB);
-    LAUNCH(lu_inverse_kernel<2>, dim3(last + 1, LU_NB / 2), LU_NB, 0, st, A, ld, n, true, Uinv);
+    if (last == 0) LAUNCH(lu_inverse_kernel<1>, dim3(1, LU_NB), LU_NB, 0, st, A, ld, n, true, Uinv);
+    else LAUNCH(lu_inverse_kernel<2>, dim3(last + 1, LU_NB / 2), LU_NB, 0, st, A, ld, n, true, Uinv);
 }
 
 static void run_pivoted(double* A, long long ld, int n, int* ipiv, double* Linv, double* Uinv, int* flag,
