@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <map>
 #include <mutex>
 #include <vector>
 
@@ -888,7 +889,165 @@ __global__ void __cluster_dims__(TS_CL, 1, 1) __launch_bounds__(TS_THREADS)
     cl.sync();
 }
 
+// The same solve for a few members: a cluster of 16 CTAs per member, 8 rows of a block each, so
+// that four times the SMs read the factor.  A warp copies its row of the next block into
+// shared memory (cp.async) and every thread its part of the block inverse into registers
+// while the cluster exchanges the sums of this one, so no step waits for memory.  Two columns;
+// the operations and their order are trsv_kernel's, the results the same bits.
+// 3840 unknowns, one member: 420 us with four CTAs, whose 128 warps kept too few loads in flight.
+constexpr int TW_CL = 16, TW_THREADS = 512, TW_ROWS = MX_NB / TW_CL;
+inline size_t trsv_wide_smem(int n) {
+    return sizeof(float) * 2 * ((size_t)trsv_npad(n) + 2 * MX_NB + TS_PARTS * MX_NB) + (size_t)TW_ROWS * 4 * n;
+}
+
+__global__ void __launch_bounds__(TW_THREADS) trsv_wide_kernel(const __grid_constant__ TrsvArgs args) {
+    constexpr int R = 2, PER = MX_NB * TS_PARTS / TW_THREADS, QN = MX_NB / TS_PARTS;
+    extern __shared__ __align__(16) float tsm[];
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank();
+    const TrsvJob& J = args.j[blockIdx.x / TW_CL];
+    const int n = args.n, nt = J.n_true, r = args.r;
+    const int npad = (n + 255) & ~255;
+    bf16* const rows = reinterpret_cast<bf16*>(tsm);               // per row: n of hi, n of lo
+    float* const x = tsm + (size_t)TW_ROWS * n;                    // column c: x[c * npad + xpos(row)]
+    float* const sb = x + (size_t)npad * R;
+    float* const part = sb + 2 * MX_NB * R;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int e = tid; e < n * R; e += TW_THREADS) {
+        const int row = e / R, c = e % R;
+        x[c * npad + xpos(row)] = (row < nt && c < r) ? (float)J.in[row + c * J.ldi] : 0.f;
+    }
+    __syncthreads();
+    const int nb = n / MX_NB, steps = 2 * nb;
+    auto block = [&](int st) { return st < nb ? st : steps - 1 - st; };
+    // this warp's row of step st into shared memory, 16 bytes per lane and copy
+    auto fetch = [&](int st) {
+        if (warp >= TW_ROWS || st >= steps) return;
+        const int b = block(st), k0 = st < nb ? 0 : (b + 1) * MX_NB, k1 = st < nb ? b * MX_NB : n;
+        const long long base = (long long)(b * MX_NB + rank * TW_ROWS + warp) * n;
+        bf16* const h = rows + (size_t)warp * 2 * n;
+        for (int k = k0 + 8 * lane; k < k1; k += 256) {
+            const uint32_t dh = (uint32_t)__cvta_generic_to_shared(h + k), dl = (uint32_t)__cvta_generic_to_shared(h + n + k);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dh), "l"(J.Rh + base + k) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dl), "l"(J.Rl + base + k) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    int buf = 0;
+    for (int st = 0; st < steps; ++st) {
+        const int b = block(st), k0 = st < nb ? 0 : (b + 1) * MX_NB, k1 = st < nb ? b * MX_NB : n;
+        // this thread's entries of the block inverse: (h, rl) for h = tid / 128 and + 4
+        const float* Inv = (st < nb ? J.Li : J.Ui) + (size_t)b * MX_NB * MX_NB + tid % MX_NB;
+        float iv[PER][QN];
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+#pragma unroll
+            for (int q = 0; q < QN; ++q)
+                iv[u][q] = __ldg(Inv + (((tid / MX_NB) + u * (TW_THREADS / MX_NB)) * QN + q) * MX_NB);
+        if (warp < TW_ROWS) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+            const int rl = rank * TW_ROWS + warp, row = b * MX_NB + rl;
+            const bf16* const h = rows + (size_t)warp * 2 * n;
+            float acc[R];
+#pragma unroll
+            for (int c = 0; c < R; ++c) acc[c] = 0.f;
+#pragma unroll 2
+            for (int k = k0 + 8 * lane; k < k1; k += 256) {
+                const uint4 hv = *reinterpret_cast<const uint4*>(h + k);
+                const uint4 lv = *reinterpret_cast<const uint4*>(h + n + k);
+                const bf16* hp = reinterpret_cast<const bf16*>(&hv);
+                const bf16* lp = reinterpret_cast<const bf16*>(&lv);
+                const int xp = xpos(k);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const float a = __bfloat162float(hp[q]) + __bfloat162float(lp[q]);
+#pragma unroll
+                    for (int c = 0; c < R; ++c) acc[c] = fmaf(a, x[c * npad + xp + 32 * q], acc[c]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < R; ++c) {
+                float v = acc[c];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                acc[c] = x[c * npad + xpos(row)] - v;
+            }
+            if (lane < TW_CL) {
+                float* dst = cl.map_shared_rank(sb, lane) + buf * MX_NB * R + rl * R;
+#pragma unroll
+                for (int c = 0; c < R; ++c) dst[c] = acc[c];
+            }
+            __syncwarp();  // the row is read before the next one takes its place
+            fetch(st + 1);
+        }
+        cl.sync();
+        const float* s = sb + buf * MX_NB * R;
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int rl = tid % MX_NB, hh = tid / MX_NB + u * (TW_THREADS / MX_NB);
+            float v[R];
+#pragma unroll
+            for (int c = 0; c < R; ++c) v[c] = 0.f;
+#pragma unroll
+            for (int q = 0; q < QN; ++q)
+#pragma unroll
+                for (int c = 0; c < R; ++c) v[c] = fmaf(iv[u][q], s[(hh * QN + q) * R + c], v[c]);
+#pragma unroll
+            for (int c = 0; c < R; ++c) part[(hh * MX_NB + rl) * R + c] = v[c];
+        }
+        __syncthreads();
+        if (tid < MX_NB * R) {
+            const int rl = tid % MX_NB, c = tid / MX_NB;
+            float v = 0.f;
+#pragma unroll
+            for (int h = 0; h < TS_PARTS; ++h) v += part[(h * MX_NB + rl) * R + c];
+            x[c * npad + xpos(b * MX_NB + rl)] = v;
+        }
+        __syncthreads();
+        buf ^= 1;
+    }
+    for (int e = tid + rank * TW_THREADS; e < nt * R; e += TW_THREADS * TW_CL) {
+        const int row = e / R, c = e % R;
+        if (c < r) J.out[row + c * J.ldo] = (double)x[c * npad + xpos(row)];
+    }
+    cl.sync();  // no CTA leaves while a peer could still address its shared memory
+}
+
 namespace {
+// Whether m members of order n go through trsv_wide_kernel: clusters of 16 take most of a GPC
+// each, so up to 8 members; beyond that the narrow clusters fill the GPU.  The GPU has to
+// place such a cluster at all (asked once per size).
+bool trsv_wide_fits(int n, int m) {
+    if (m > 8 || trsv_wide_smem(n) > 227 * 1024) return false;
+    static std::mutex mu;
+    static std::map<int, bool> known;
+    static bool usable = true;
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find(n);
+    if (it != known.end()) return it->second;
+    if (known.empty())
+        usable = cudaFuncSetAttribute(trsv_wide_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                 cudaFuncSetAttribute(trsv_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) ==
+                     cudaSuccess;
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute at[1];
+    c.gridDim = dim3(TW_CL);
+    c.blockDim = dim3(TW_THREADS);
+    c.dynamicSmemBytes = trsv_wide_smem(n);
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = TW_CL;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    int clusters = 0;
+    const bool ok = usable && cudaOccupancyMaxActiveClusters(&clusters, trsv_wide_kernel, &c) == cudaSuccess && clusters > 0;
+    (void)cudaGetLastError();
+    known[n] = ok;
+    return ok;
+}
+
 template <int R>
 void trsv_launch(const std::vector<const MixedLU*>& g, const std::vector<TrsvIO>& io, int c0, int r, cudaStream_t st) {
     const int n = g[0]->n;
@@ -909,6 +1068,24 @@ void trsv_launch(const std::vector<const MixedLU*>& g, const std::vector<TrsvIO>
                       q.out + (long long)c0 * q.ldo, q.ldo, q.n_true};
         }
         const double by = (double)m * ((double)n * n * 4.0 + 2.0 * n * r * 8.0);
+        if (R == 2 && trsv_wide_fits(n, m)) {
+            cudaLaunchConfig_t c = {};
+            cudaLaunchAttribute at[1];
+            c.gridDim = dim3((unsigned)(m * TW_CL));
+            c.blockDim = dim3(TW_THREADS);
+            c.dynamicSmemBytes = trsv_wide_smem(n);
+            c.stream = st;
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = TW_CL;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            c.attrs = at;
+            c.numAttrs = 1;
+            const int ks = kstats_on() ? kstat_begin(st) : -1;
+            CUDA_CHECK(cudaLaunchKernelEx(&c, trsv_wide_kernel, a));
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+            if (ks >= 0) kstat_end(ks, "trsv", st, 0.0, by);
+            continue;
+        }
         TIMED_LAUNCH("trsv", 0.0, by, trsv_kernel<R>, m * TS_CL, TS_THREADS, smem, st, a);
     }
 }
@@ -924,7 +1101,9 @@ void trsv_group_io(const std::vector<const MixedLU*>& g, const std::vector<TrsvI
         if (nt < 1 || nt > n || io[k].ldi < nt || io[k].ldo < nt) fail(SQBEM_ERR_ARG, "trsv: bad row count");
     }
     if (trsv_smem(n, 2) > 227 * 1024) fail(SQBEM_ERR_ARG, "trsv: %d unknowns exceed shared memory", n);
-    if (r > 2 && trsv_smem(n, 8) <= 227 * 1024) {
+    // eight columns at once, or (few members) two at a time on wide clusters: 3840 unknowns and six
+    // columns took 860 us at once
+    if (r > 2 && trsv_smem(n, 8) <= 227 * 1024 && !trsv_wide_fits(n, (int)g.size())) {
         trsv_launch<8>(g, io, 0, r, st);
         return;
     }

@@ -560,7 +560,10 @@ __global__ void chat_nth(const __grid_constant__ ChatArgs args, const __grid_con
     for (int f = 0; f < NF; ++f) J.C[(long long)f * n3 * n3 + (long long)c * n3 + r] = make_float2(re[f], im[f]);
 }
 
-int gj_cluster(int n) {
+int gj_cluster(int n, int nblk = 1 << 20) {
+    // one tube's blocks (13 for 24 sectors): eight CTAs each still leave SMs free, and a step's
+    // elimination is a quarter as long
+    if (nblk * 8 <= 152) return 8;
     // shared memory of one CTA: its columns, two pivot columns and the index
     // arrays; two CTAs per block where they fit (measured faster than four)
     for (int cl : {2, 4}) {
@@ -586,6 +589,7 @@ void set_smem_limits() {
     std::call_once(once, [] {
         CUDA_CHECK(cudaFuncSetAttribute(gj_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_MAX));
         CUDA_CHECK(cudaFuncSetAttribute(gj_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_MAX));
+        CUDA_CHECK(cudaFuncSetAttribute(gj_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_MAX));
     });
 }
 
@@ -597,7 +601,7 @@ bool fourier_supported(const TubeSymmetry& sym) {
 }
 
 void gauss_jordan_blocks(float2* C, int nblk, int n3, int* flag, cudaStream_t st) {
-    const int cl = gj_cluster(n3);
+    const int cl = gj_cluster(n3, nblk);
     if (!cl) fail(SQBEM_ERR_ARG, "Gauss-Jordan: block order %d too large", n3);
     set_smem_limits();
     for (int b0 = 0; b0 < nblk; b0 += GJ_MAXB) {
@@ -608,7 +612,8 @@ void gauss_jordan_blocks(float2* C, int nblk, int n3, int* flag, cudaStream_t st
         g.flag = flag;
         for (int b = 0; b < g.nblk; ++b) g.C[b] = C + (size_t)(b0 + b) * n3 * n3;
         const double fl = 8.0 * g.nblk * (double)n3 * n3 * n3, by = 16.0 * g.nblk * (double)n3 * n3;
-        if (cl == 2) TIMED_LAUNCH("fourier_inverse", fl, by, gj_kernel<2>, 2 * g.nblk, GJ_THREADS, gj_smem(n3, cl), st, g);
+        if (cl == 8) TIMED_LAUNCH("fourier_inverse", fl, by, gj_kernel<8>, 8 * g.nblk, GJ_THREADS, gj_smem(n3, cl), st, g);
+        else if (cl == 2) TIMED_LAUNCH("fourier_inverse", fl, by, gj_kernel<2>, 2 * g.nblk, GJ_THREADS, gj_smem(n3, cl), st, g);
         else TIMED_LAUNCH("fourier_inverse", fl, by, gj_kernel<4>, 4 * g.nblk, GJ_THREADS, gj_smem(n3, cl), st, g);
     }
 }
@@ -663,9 +668,9 @@ void fourier_build(const std::vector<FourierTube*>& fts, const std::vector<const
             else if (nth == 36) TIMED_LAUNCH("fourier_inverse", 0.0, cby, chat_nth<36>, cg3, 64, 0, cx.st, a, tw);
             else TIMED_LAUNCH("fourier_inverse", 0.0, cby, chat_kernel, cg3, 64, 0, cx.st, a);
         }
-        const int cl = gj_cluster(n3);
-        const size_t smem = gj_smem(n3, cl);
         const int nblk_all = (int)(ids.size() * nf);
+        const int cl = gj_cluster(n3, nblk_all);
+        const size_t smem = gj_smem(n3, cl);
         for (int b0 = 0; b0 < nblk_all; b0 += GJ_MAXB) {
             GjArgs g;
             g.n = n3;
@@ -688,7 +693,8 @@ void fourier_build(const std::vector<FourierTube*>& fts, const std::vector<const
             // credited: 8 n^3 FP32 flops per complex inversion; bytes: the block read and written
             const double gfl = 8.0 * g.nblk * (double)n3 * n3 * n3, gby = 16.0 * g.nblk * (double)n3 * n3;
             set_smem_limits();
-            if (cl == 2) TIMED_LAUNCH("fourier_inverse", gfl, gby, gj_kernel<2>, 2 * g.nblk, GJ_THREADS, smem, cx.st, g);
+            if (cl == 8) TIMED_LAUNCH("fourier_inverse", gfl, gby, gj_kernel<8>, 8 * g.nblk, GJ_THREADS, smem, cx.st, g);
+            else if (cl == 2) TIMED_LAUNCH("fourier_inverse", gfl, gby, gj_kernel<2>, 2 * g.nblk, GJ_THREADS, smem, cx.st, g);
             else TIMED_LAUNCH("fourier_inverse", gfl, gby, gj_kernel<4>, 4 * g.nblk, GJ_THREADS, smem, cx.st, g);
             const int t = ceil_div(2 * n3, 32);
             TIMED_LAUNCH("fourier_inverse", 0.0, g.nblk * (8.0 * n3 * n3 + 16.0 * n3 * n3), realform_kernel,
