@@ -308,7 +308,7 @@ extern "C" int sqbem_gemm64(int route, int ta, int tb, int M, int N, int K, doub
         if (route == 1) {
             OzMat a, b;
             a.split(dA.get(), ta ? lda : 1, ta ? 1 : lda, M, K, s);
-            b.split(dB.get(), tb ? 1 : ldb, tb ? ldb : 1, N, K, s);
+            b.split(dB.get(), tb ? 1 : ldb, tb ? ldb : 1, N, K, s, true);
             oz_gemm(a, b, alpha, beta, dC.get(), ldc, we.get(s), s);
         } else {
             gemm64(ta, tb, M, N, K, alpha, dA.get(), lda, dB.get(), ldb, beta, dC.get(), ldc, s,

@@ -380,19 +380,19 @@ bool Circulant64::build(const TubeSymmetry& sym, const double* T0, const int* ti
     gauss_jordan_blocks(c32.get(), nf, n3, flag.get(), st);
     LAUNCH(realform64_kernel, dim3(gb.x, gb.y, nf), 64, 0, st, c32.get(), n3, inv.get());
     OzMat a, x, r;
-    a.split(C.get(), 1, m2, m2, m2, st, nf, one);
+    a.split(C.get(), 1, m2, m2, m2, st, false, nf, one);
     for (int it = 0; it < NEWTON_STEPS; ++it) {
         LAUNCH(identity_kernel, dim3(ceil_div(m2, 128), m2, nf), 128, 0, st, R.get(), m2);
-        x.split(inv.get(), m2, 1, m2, m2, st, nf, one);
+        x.split(inv.get(), m2, 1, m2, m2, st, true, nf, one);
         oz_gemm(a, x, -1.0, 1.0, R.get(), m2, flag.get() + 1, st, one);
         if (it + 1 == NEWTON_STEPS)
             LAUNCH(max_abs_bits_kernel, 152, 256, 0, st, R.get(), all,
                    reinterpret_cast<unsigned long long*>(flag.get() + 2));
-        x.split(inv.get(), 1, m2, m2, m2, st, nf, one);
-        r.split(R.get(), m2, 1, m2, m2, st, nf, one);
+        x.split(inv.get(), 1, m2, m2, m2, st, false, nf, one);
+        r.split(R.get(), m2, 1, m2, m2, st, true, nf, one);
         oz_gemm(x, r, 1.0, 1.0, inv.get(), m2, flag.get() + 1, st, one);
     }
-    digits.split(inv.get(), 1, m2, m2, m2, st, nf, one);
+    digits.split(inv.get(), 1, m2, m2, m2, st, false, nf, one);
     int h[4], htie = 0;
     flag.download(h, 4);
     if (tie) {
@@ -437,7 +437,7 @@ void Circulant64::solve(double* B, long long ldb, int nrhs, cudaStream_t st, int
         xh = std::move(yh);
     } else {
         OzMat x;
-        x.split(xh.get(), m2, 1, nrhs, m2, st, nf, plane);
+        x.split(xh.get(), m2, 1, nrhs, m2, st, true, nf, plane);
         oz_gemm(digits, x, 1.0, 0.0, xh.get(), m2, err, st, plane);
     }
     TIMED_LAUNCH("fourier_dft", 0.0, 8.0 * nrhs * (nt + (double)nf * m2), idft64_kernel, grid, 256, idft_smem(nth, per), st,

@@ -292,7 +292,7 @@ void gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const double* A
     if (use_tensor(M, N, K, err)) {
         OzMat a, b;
         a.split(A, ta ? lda : 1, ta ? 1 : lda, M, K, st);
-        b.split(B, tb ? 1 : ldb, tb ? ldb : 1, N, K, st);
+        b.split(B, tb ? 1 : ldb, tb ? ldb : 1, N, K, st, true);
         oz_gemm(a, b, alpha, beta, C, ldc, err, st);
         return;
     }
@@ -748,7 +748,7 @@ static void tensor_product(const double* A, long long lda, const double* B, long
                            double alpha, double beta, double* C, long long ldc, int* err, cudaStream_t st) {
     OzMat a, b;
     a.split(A, 1, lda, M, K, st);
-    b.split(B, ldb, 1, N, K, st);
+    b.split(B, ldb, 1, N, K, st, true);
     oz_gemm(a, b, alpha, beta, C, ldc, err, st);
 }
 

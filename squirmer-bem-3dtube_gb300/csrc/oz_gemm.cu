@@ -4,22 +4,23 @@
 // about 1900, so the 36 digit products of an FP64 product still leave room for a
 // factor of forty.
 //
-// Tile 128 x 128 of C per CTA, one persistent CTA per SM:
-//   warp 0     producer: bulk copies of the digits' blocks into a 3-stage ring of
-//              64 KB stages (the blocks are stored in the order the MMA reads, so
-//              the digits a pass needs of one k16 step are one copy per operand);
-//   warp 1     MMA issuer: passes of two weights (d, d + 1) into the two halves of a
-//              256-column accumulator, double-buffered over the 512 TMEM columns;
-//   warps 2-9  epilogue: the accumulators as integers into 64-bit sums held in
-//              registers (64 per thread), the rounding to FP64, C.
+// One persistent CTA per SM:
+//   producer   a warp: bulk copies of the digits' blocks into a ring of 192 KB (the blocks are
+//              stored in the order the MMA reads, so the digits a pass needs of one k16 step
+//              are one copy per operand);
+//   issuers    one warp or two: passes of two weights (d, d + 1), which are the two halves of
+//              an accumulator in tensor memory;
+//   epilogue   eight warps: the accumulators as integers into 64-bit sums held in registers,
+//              the rounding to FP64, C.
 // Four passes: weights 0, 1 (digits 0-1) and 2, 3 (digits 0-3) in chunks of 256 k,
 // where every sum is exact (4 * 256 * 2^14 = 2^24); then weights 4, 5 and 6, 7
 // in chunks of 1024 k, whose rounding past 2^24 lies 2^-56 below the product
 // of the largest entries.
-//   K <= 256 (the panels' updates): the 64-bit sums also take weights 4 and 5 (2^62 at
-//   most), and the last pass goes straight into the rounding.
-//   K > 256: the sums of the leading passes wait in global scratch (L2) for the others,
-//   since both sets do not fit in the registers together.
+//   K <= 256 (the panels' updates): tiles of 128 x 64, an accumulator per pass; the 64-bit
+//   sums also take weights 4 and 5 (2^62 at most), and the last pass goes straight into the
+//   rounding.
+//   K > 256: tiles of 128 x 128, two accumulators; the sums of the leading passes wait in
+//   global scratch (L2) for the others, since both sets do not fit in the registers together.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -37,13 +38,31 @@ constexpr int TILE = 128;
 constexpr int DIGITS = 8;
 constexpr int PLANE = TILE * 16 * 2;       // one digit of a 128 x 16 block: 4 KB
 constexpr int BLOCK = DIGITS * PLANE;      // 32 KB
-constexpr int STAGES = 3, STAGE = 64 * 1024;
-// past the ring: room for the descriptors' strides, never read
-constexpr int SMEM_BYTES = STAGES * STAGE + 1024 + 256;
-constexpr int NTHREADS = 320;              // producer, issuer, 8 epilogue warps
+constexpr int SMEM_BYTES = 192 * 1024 + 1024 + 256;
 constexpr int HI_CHUNK = 16, LO_CHUNK = 64;  // k16 steps between read-outs
-constexpr uint32_t IDESC =
-    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
+
+// Tiles of 128 x TN.  TN = 128 has the widest instructions and suits a long K.  With K <= 256
+// a 128 x 128 tile's read-out (20 us) was as long as its multiplication, and with tensor memory
+// for two accumulators it ran after it; TN = 64 has all four, so that a tile is multiplied
+// during the read-out of the one before, and twice the tiles for products of a few.  Its
+// instructions are bound by their issue, hence two issuers (4096 x 4096 over K = 256: 286 us
+// with TN = 128, 252 with TN = 64, 217 with two issuers; over K = 128: 204, 178, 153; one row
+// of tiles, K = 256: 49, 28, 26).
+template <int TN_>
+struct OzTile {
+    static constexpr int TN = TN_, COLS = TN / 2;            // columns per epilogue warp
+    // one producer, eight epilogue warps, and the issuers: for TN = 64 two, of a pass each
+    static constexpr int ISSUERS = TN == 128 ? 1 : 2, NTHREADS = 32 * (9 + ISSUERS);
+    static constexpr int STAGES = TN == 128 ? 3 : 4, STAGE = 192 * 1024 / STAGES;
+    static constexpr int PLANE_B = TN * 32;                  // one digit of B in a stage
+    static constexpr int NBUF = 512 / (2 * TN);              // accumulators: two weights of TN columns each
+    // one weight's columns, and two weights' side by side
+    static constexpr uint32_t IDESC1 =
+        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
+    static constexpr uint32_t IDESC2 = IDESC1 + ((uint32_t)(TN >> 3) << 17);
+    // bytes of nd digits of both operands for a k16 step
+    __device__ static constexpr uint32_t step_bytes(int nd) { return (uint32_t)nd * (PLANE + PLANE_B); }
+};
 
 // ---------------------------------------------------------------- digits
 __global__ void oz_exponent_rows(const double* __restrict__ a, long long rs, long long ks, int rows, int k, int kper,
@@ -89,7 +108,7 @@ __device__ __forceinline__ long long fixed64(double x, int E) {
 }
 
 // The digits of eight values of one row: 16 bytes of each of the eight planes.
-__device__ __forceinline__ void store_digits(const double (&x)[8], int E, uint4* o) {
+__device__ __forceinline__ void store_digits(const double (&x)[8], int E, uint4* o, int digit) {
     uint32_t w[DIGITS][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -110,7 +129,13 @@ __device__ __forceinline__ void store_digits(const double (&x)[8], int E, uint4*
         }
     }
 #pragma unroll
-    for (int s = 0; s < DIGITS; ++s) o[s * (PLANE / 16)] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+    for (int s = 0; s < DIGITS; ++s) o[s * digit] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+}
+
+// Where the first digit of row r's half h of k16 step kb goes, in blocks of rb rows.
+__device__ __forceinline__ long long digit_at(int r, int kb, int h, int k16, int rb) {
+    const int i = r & (rb - 1);
+    return ((long long)(rb == TILE ? r >> 7 : r >> 6) * k16 + kb) * (rb * 16) + (i >> 3) * 16 + h * 8 + (i & 7);
 }
 
 // Eight values along k of one row per thread -> 16 bytes of each digit plane.
@@ -118,7 +143,7 @@ __device__ __forceinline__ void store_digits(const double (&x)[8], int E, uint4*
 // grid.y strides over the k16 steps.
 __global__ void __launch_bounds__(256) oz_split(const double* __restrict__ a, long long rs, long long ks, int rows,
                                                 int k, int k16, const int* __restrict__ ex, uint4* __restrict__ out,
-                                                long long bs, int eb) {
+                                                long long bs, int eb, int rb) {
     a += blockIdx.z * bs;
     ex += (long long)blockIdx.z * eb;
     out += (long long)blockIdx.z * (eb / TILE) * k16 * (BLOCK / 16);
@@ -130,7 +155,7 @@ __global__ void __launch_bounds__(256) oz_split(const double* __restrict__ a, lo
         double x[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = ok && c0 + j < k ? a[r * rs + (c0 + j) * ks] : 0.0;
-        store_digits(x, E, out + ((long long)blockIdx.x * k16 + kb) * (BLOCK / 16) + threadIdx.y * (PLANE / 32) + threadIdx.x);
+        store_digits(x, E, out + digit_at(r, kb, threadIdx.y, k16, rb), rb * 2);
     }
 }
 
@@ -142,7 +167,7 @@ constexpr int FUSED_K = 512;
 constexpr int FUSED_SMEM = FUSED_K * 33 * 8;
 __global__ void __launch_bounds__(256) oz_split_fused(const double* __restrict__ a, long long rs, long long ks, int rows,
                                                       int k, int k16, int* __restrict__ ex, uint4* __restrict__ out,
-                                                      long long bs, int eb) {
+                                                      long long bs, int eb, int rb) {
     a += blockIdx.z * bs;
     ex += (long long)blockIdx.z * eb;
     out += (long long)blockIdx.z * (eb / TILE) * k16 * (BLOCK / 16);
@@ -175,12 +200,11 @@ __global__ void __launch_bounds__(256) oz_split_fused(const double* __restrict__
     __syncthreads();
     const int E = em[lane];
     if (w == 0 && r0 + lane < rows) ex[r0 + lane] = E;
-    uint4* const o = out + (long long)(blockIdx.x >> 2) * k16 * (BLOCK / 16) + (blockIdx.x & 3) * 32 + lane;
     for (int o8 = w; o8 < 2 * k16; o8 += 8) {
         double x[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = E != 0x7ff ? xs[(o8 * 8 + j) * 33 + lane] : 0.0;
-        store_digits(x, E, o + (o8 >> 1) * (BLOCK / 16) + (o8 & 1) * (PLANE / 32));
+        store_digits(x, E, out + digit_at(r0 + lane, o8 >> 1, o8 & 1, k16, rb), rb * 2);
     }
 }
 
@@ -212,10 +236,11 @@ __device__ __forceinline__ void red_add(double* p, double v) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 
-// K-major, no swizzle: 8-row core matrices of 128 bytes, the next 8 rows 128 bytes
-// on (SBO), the second half of the 16 k 2048 bytes on (LBO); descriptor version 1.
+// K-major, no swizzle: 8-row core matrices of 128 bytes, the second half of the 16 k 128 bytes
+// on (LBO), the next 8 rows 256 bytes on (SBO), so that half a block's rows are one piece;
+// descriptor version 1.
 __device__ __forceinline__ uint64_t oz_desc(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(2048 >> 4) << 16) | ((uint64_t)(128 >> 4) << 32) |
+    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
            (1ull << 46);
 }
 
@@ -231,45 +256,46 @@ __device__ __forceinline__ void tile_at(const OzArgs& g, int t, int& b, int& tm,
     tm = grp * 12 + r - tn * h;
 }
 
-// One accumulation between two read-outs: pass p (weights 2p, 2p + 1) over the k16
-// steps [k0, k1).  The leading passes 0, 1 alternate over HI_CHUNK steps, then 2, 3
-// over LO_CHUNK.
+// What runs over the k16 steps [k0, k1) with nd digits of both operands in the stages: pass p
+// (the weights 2p, 2p + 1), for SHORT also p + 1.  The long kernel has one pass
+// between two read-outs: the leading passes 0, 1 alternate over HI_CHUNK steps, then 2, 3 over
+// LO_CHUNK.  SHORT has accumulators for all four and loads a step's digits twice, not four
+// times: four digits for passes 0 and 1, then all eight for 2 and 3.
 struct Group {
-    int p, k0, k1;
-    bool last_hi, last;
+    int p, nd, k0, k1;
+    bool last_hi;
 };
+template <bool SHORT>
 __device__ __forceinline__ int n_groups(int k16) {
+    if (SHORT) return 2;
     return 2 * ((k16 + HI_CHUNK - 1) / HI_CHUNK) + 2 * ((k16 + LO_CHUNK - 1) / LO_CHUNK);
 }
+template <bool SHORT>
 __device__ __forceinline__ Group group_at(int q, int k16) {
-    const int nh = 2 * ((k16 + HI_CHUNK - 1) / HI_CHUNK), nl = 2 * ((k16 + LO_CHUNK - 1) / LO_CHUNK);
-    Group g;
+    if (SHORT) return Group{2 * q, 4 * q + 4, 0, k16, false};
+    const int nh = 2 * ((k16 + HI_CHUNK - 1) / HI_CHUNK);
     const bool hi = q < nh;
-    const int c = hi ? HI_CHUNK : LO_CHUNK, i = hi ? q : q - nh;
-    g.p = (hi ? 0 : 2) + (i & 1);
-    g.k0 = (i >> 1) * c;
-    g.k1 = min(k16, g.k0 + c);
-    g.last_hi = q == nh - 1;
-    g.last = q == nh + nl - 1;
-    return g;
+    const int c = hi ? HI_CHUNK : LO_CHUNK, i = hi ? q : q - nh, p = (hi ? 0 : 2) + (i & 1), k0 = (i >> 1) * c;
+    return Group{p, 2 * p + 2, k0, min(k16, k0 + c), q == nh - 1};
 }
-// k16 steps per stage of pass p (2, 4, 6, 8 digits of both operands)
-__device__ __forceinline__ int steps_per_stage(int p) { return p == 0 ? 4 : p == 1 ? 2 : 1; }
 
-template <int P>
-__device__ __forceinline__ void issue_step(uint32_t a0, uint32_t d, bool first) {
+// The products of one k16 step of pass P.  Digit i of A goes with B's digits 2P - i and
+// 2P - i + 1 in one instruction: these lie one behind the other in the stage, as the two
+// weights' accumulators do in tensor memory, so the pair is one operand of 2 TN rows.  36
+// instructions of TN columns per step issued at 93 clocks each, whatever TN; these 20 (16 of
+// them of 2 TN) keep the tensor core busy and read A's digits from shared memory half as often.
+template <int P, class T>
+__device__ __forceinline__ void issue_step(uint32_t a0, uint32_t b0, uint32_t d, bool first) {
     constexpr int ND = 2 * P + 2;
-    const uint64_t da = oz_desc(a0), db = oz_desc(a0 + ND * PLANE);
+    const uint64_t da = oz_desc(a0), db = oz_desc(b0);
+    if (elect_one()) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        constexpr int D0 = 2 * P;
-#pragma unroll
-        for (int i = 0; i <= D0 + h; ++i) {
-            const int j = D0 + h - i;
-            mma_bf16(d + h * TILE, da + (uint64_t)(i * (PLANE >> 4)), db + (uint64_t)(j * (PLANE >> 4)), IDESC,
+        for (int i = 0; i < ND - 1; ++i)
+            mma_bf16(d, da + (uint64_t)(i * (PLANE >> 4)), db + (uint64_t)((ND - 2 - i) * (T::PLANE_B >> 4)), T::IDESC2,
                      first && i == 0 ? 0u : 1u);
-        }
+        mma_bf16(d + T::TN, da + (uint64_t)((ND - 1) * (PLANE >> 4)), db, T::IDESC1, 1u);
     }
+    __syncwarp();
 }
 
 // m 2^(e - 1075) where that is not a normal number (kept out of line: the read-out's code
@@ -310,84 +336,93 @@ __device__ __forceinline__ double round96(long long hi, long long lo, int Eab) {
     return __hiloint2double(__double2hiint(r) ^ (int)(neg & 0x80000000u), __double2loint(r));
 }
 
-// (s 2^16 + q) 2^(56 + Ea + Eb - 2170) to nearest even, |q| < 2^35: the high 32 bits and the
-// low 48 each put into the significand of a power of two, whose removal and sum are two
-// FP64 operations, the first exact.
-__device__ __forceinline__ double significand80(long long s, long long q) {
+// s 2^16 + q, |q| < 2^35, as hi 2^32 + lo.
+__device__ __forceinline__ void parts80(long long s, long long q, long long& hi, uint32_t& lo) {
     const long long x = (long long)((unsigned long long)(uint32_t)s << 16) + q;
-    const uint32_t top = (uint32_t)(s >> 32) + (uint32_t)(x >> 48);
-    const double B = __hiloint2double(0x46300000, (int)(top ^ 0x80000000u));
-    const double A = __hiloint2double(0x43300000 | (int)((x >> 32) & 0xffff), (int)x);
-    return (B - 0x1.000008000001p+100) + A;  // 2^100 + 2^79 + 2^52
+    lo = (uint32_t)x;
+    hi = ((long long)(int)(s >> 32) << 16) + (int)(x >> 32);
 }
-// r 2^(E - 2114) where r is 0 or the result leaves the normal numbers
-__device__ __noinline__ double scale80_far(double r, int E) {
-    const int hi = __double2hiint(r), e = (hi >> 20) & 0x7ff;
-    if (e == 0) return 0.0;
-    const double f = scale_far(((unsigned long long)__double_as_longlong(r) & 0xfffffffffffffull) | (1ull << 52),
-                               e + E - 2114);
-    return hi < 0 ? -f : f;
+__device__ __noinline__ double round80_far(long long s, float v0, float v1, int Eab) {
+    long long hi;
+    uint32_t lo;
+    parts80(s, (long long)__float2int_rn(v0) * 256 + __float2int_rn(v1), hi, lo);
+    return round96(hi, lo, Eab);
 }
-// Eight of them.  Branch-free but for one rare test of all eight: a branch per element kept
-// the elements' latencies from overlapping (750 cycles each).
+// (s 2^16 + v0 2^8 + v1) 2^(56 + Ea + Eb - 2170) to nearest even for eight elements: integer
+// arithmetic (two FP64 operations per element took a 128 x 128 tile 9 us), branch-free but for
+// one rare test of all eight (a branch per element kept their latencies from overlapping, 750
+// cycles each).
 __device__ __forceinline__ void round80(const long long* s, const float (&v0)[8], const float (&v1)[8],
                                         const int (&E)[8], double (&r)[8]) {
     uint32_t far = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-        r[j] = significand80(s[j], (long long)__float2int_rn(v0[j]) * 256 + __float2int_rn(v1[j]));
-    double n[8];
-#pragma unroll
     for (int j = 0; j < 8; ++j) {
-        const int hi = __double2hiint(r[j]), e = (hi >> 20) & 0x7ff;
-        far |= (uint32_t)(e + E[j] - 2115) >= 2046u || e == 0 ? 1u << j : 0u;
-        n[j] = __hiloint2double(hi + ((E[j] - 2114) << 20), __double2loint(r[j]));
+        long long h;
+        uint32_t l;
+        parts80(s[j], (long long)__float2int_rn(v0[j]) * 256 + __float2int_rn(v1[j]), h, l);
+        const uint32_t neg = (uint32_t)((int)(h >> 32) >> 31);
+        const unsigned long long a =
+            ((unsigned long long)h ^ ((unsigned long long)neg << 32 | neg)) + ((neg & 1) & (uint32_t)(l == 0));
+        l = (l ^ neg) - neg;
+        const int z = __clzll((long long)a) & 63;
+        const unsigned long long L = (unsigned long long)l << 32;
+        const unsigned long long T = (a << z) | ((L >> 1) >> (63 - z));
+        unsigned long long m = T >> 11;
+        const uint32_t rb = (uint32_t)T & 0x7ff, sticky = (uint32_t)((L << z) != 0) | (uint32_t)(m & 1);
+        m += rb + sticky > 0x400 ? 1 : 0;
+        const int e = E[j] - z - 996;
+        far |= (uint32_t)(e - 1) >= 2045u || a == 0 ? 1u << j : 0u;
+        m += (unsigned long long)(uint32_t)(e - 1) << 52;
+        r[j] = __hiloint2double((int)(m >> 32) ^ (int)(neg & 0x80000000u), (int)m);
     }
     if (far) {
 #pragma unroll 1
         for (int j = 0; j < 8; ++j) {
             if (!(far >> j & 1)) continue;
-            double x = r[0];
+            long long x = s[0];
+            float f0 = v0[0], f1 = v1[0];
             int Ej = E[0];
 #pragma unroll
             for (int u = 1; u < 8; ++u) {
-                x = j == u ? r[u] : x;
+                x = j == u ? s[u] : x;
+                f0 = j == u ? v0[u] : f0;
+                f1 = j == u ? v1[u] : f1;
                 Ej = j == u ? E[u] : Ej;
             }
-            const double f = scale80_far(x, Ej);
+            const double f = round80_far(x, f0, f1, Ej);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) n[u] = j == u ? f : n[u];
+            for (int u = 0; u < 8; ++u) r[u] = j == u ? f : r[u];
         }
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) r[j] = n[j];
 }
 
 // SHORT: k16 <= HI_CHUNK
-template <bool SHORT>
-__global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_constant__ OzArgs g) {
+template <bool SHORT, class T>
+__global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_constant__ OzArgs g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    constexpr int STAGES = T::STAGES, STAGE = T::STAGE, TN = T::TN, COLS = T::COLS, NBUF = T::NBUF;
+    static_assert(!SHORT || (NBUF == 4 && T::ISSUERS == 2), "SHORT has an accumulator and, of two, an issuer per pass");
     uint64_t* bars = (uint64_t*)(smem + STAGES * STAGE);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
-    const uint32_t tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + 2);
-    const uint32_t done_bar = smem_u32(bars + 2 * STAGES + 4);
-    uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 5);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles = g.tiles_m * g.tiles_n * g.batch, k16 = g.k16, ng = n_groups(k16);
+    const uint32_t tfull0 = smem_u32(bars + 2 * STAGES), tempty0 = smem_u32(bars + 2 * STAGES + NBUF);
+    const uint32_t done_bar = smem_u32(bars + 2 * STAGES + 2 * NBUF);
+    uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 2 * NBUF + 1);
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int tiles = g.tiles_m * g.tiles_n * g.batch, k16 = g.k16, ng = n_groups<SHORT>(k16);
     int* const err = g.err;
     const long long wait = g.wait;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full0 + 8 * s, 1);
-            mbar_init(empty0 + 8 * s, 1);
+            mbar_init(empty0 + 8 * s, T::ISSUERS);
         }
-        for (int a = 0; a < 2; ++a) {
+        for (int a = 0; a < NBUF; ++a) {
             mbar_init(tfull0 + 8 * a, 1);
             mbar_init(tempty0 + 8 * a, 256);
         }
-        mbar_init(done_bar, 1);
+        mbar_init(done_bar, T::ISSUERS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -411,21 +446,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
             int tb, tm, tn;
             tile_at(g, t, tb, tm, tn);
             const uint8_t* A = g.A + ((long long)tb * g.tiles_m + tm) * k16 * BLOCK;
-            const uint8_t* B = g.B + ((long long)tb * g.tiles_n + tn) * k16 * BLOCK;
+            const long long bn = TN == TILE ? (long long)tb * g.tiles_n + tn : (long long)tb * ((g.tiles_n + 1) & ~1) + tn;
+            const uint8_t* B = g.B + bn * k16 * (DIGITS * T::PLANE_B);
             for (int q = 0; ok && q < ng; ++q) {
-                const Group G = group_at(q, k16);
-                const int sp = steps_per_stage(G.p);
-                const uint32_t nb = (uint32_t)(2 * G.p + 2) * PLANE;
+                const Group G = group_at<SHORT>(q, k16);
+                const int nd = G.nd, step = T::step_bytes(nd), sp = STAGE / step;
                 for (int k = G.k0; k < G.k1; k += sp) {
                     if (!mbar_wait(empty0 + 8 * s, ph ^ 1, err, wait)) { ok = false; break; }
                     const int n = min(sp, G.k1 - k);
                     uint32_t dst = smem_u32(smem + s * STAGE);
                     const uint32_t fb = full0 + 8 * s;
-                    mbar_expect_tx(fb, 2 * nb * n);
+                    mbar_expect_tx(fb, step * n);
                     for (int u = 0; u < n; ++u) {
-                        bulk_load(dst, A + (long long)(k + u) * BLOCK, nb, fb);
-                        bulk_load(dst + nb, B + (long long)(k + u) * BLOCK, nb, fb);
-                        dst += 2 * nb;
+                        bulk_load(dst, A + (long long)(k + u) * BLOCK, nd * PLANE, fb);
+                        bulk_load(dst + nd * PLANE, B + (long long)(k + u) * (DIGITS * T::PLANE_B), nd * T::PLANE_B, fb);
+                        dst += step;
                     }
                     armed[s] += 1;
                     if (++s == STAGES) { s = 0; ph ^= 1; }
@@ -440,47 +475,57 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
                 while (!mbar_try(full0 + 8 * q, par) && clock64() - t0 < DRAIN_CYCLES) {
                 }
             }
-    } else if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer
+    } else if (warp == 1 || warp >= 10) {
+        // ---------------- MMA issuer (of pass `mine` of a group): the whole warp runs the
+        // loop, so that the descriptors are uniform values, and one lane issues
+        const int mine = warp == 1 ? 0 : 1;
         int s = 0, acc = 0;
         uint32_t ph = 0, aph = 0;
         bool ok = true;
         for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
             for (int q = 0; ok && q < ng; ++q) {
-                const Group G = group_at(q, k16);
-                const int sp = steps_per_stage(G.p);
-                const uint32_t nb = (uint32_t)(2 * G.p + 2) * PLANE;
-                if (!mbar_wait(tempty0 + 8 * acc, aph ^ 1, err, wait)) { ok = false; break; }
+                const Group G = group_at<SHORT>(q, k16);
+                const int step = T::step_bytes(G.nd), sp = STAGE / step;
+                const int p = G.p + mine;
+                if (SHORT) acc = p;
+                ok = __all_sync(0xffffffffu, mbar_wait(tempty0 + 8 * acc, aph ^ 1, err, wait));
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t d = tmem_base + (uint32_t)(acc * 2 * TILE);
+                const uint32_t d = tmem_base + (uint32_t)(acc * 2 * TN);
                 for (int k = G.k0; k < G.k1; k += sp) {
-                    if (!mbar_wait(full0 + 8 * s, ph, err, wait)) { ok = false; break; }
+                    ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph, err, wait));
+                    if (!ok) break;
                     tc_fence_after();
                     const int n = min(sp, G.k1 - k);
                     uint32_t a0 = smem_u32(smem + s * STAGE);
-                    for (int u = 0; u < n; ++u, a0 += 2 * nb) {
+                    for (int u = 0; u < n; ++u, a0 += step) {
                         const bool first = k + u == G.k0;
-                        if (G.p == 0) issue_step<0>(a0, d, first);
-                        else if (G.p == 1) issue_step<1>(a0, d, first);
-                        else if (G.p == 2) issue_step<2>(a0, d, first);
-                        else issue_step<3>(a0, d, first);
+                        const uint32_t b0 = a0 + G.nd * PLANE;
+                        if (p == 0) issue_step<0, T>(a0, b0, d, first);
+                        else if (p == 1) issue_step<1, T>(a0, b0, d, first);
+                        else if (p == 2) issue_step<2, T>(a0, b0, d, first);
+                        else issue_step<3, T>(a0, b0, d, first);
                     }
-                    mma_commit(empty0 + 8 * s);
+                    if (elect_one()) mma_commit(empty0 + 8 * s);
+                    __syncwarp();
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
                 if (!ok) break;
-                mma_commit(tfull0 + 8 * acc);
-                if (++acc == 2) { acc = 0; aph ^= 1; }
+                if (elect_one()) mma_commit(tfull0 + 8 * acc);
+                __syncwarp();
+                if (!SHORT && ++acc == NBUF) { acc = 0; aph ^= 1; }
             }
+            if (SHORT) aph ^= 1;
         }
         // all MMAs issued by this CTA complete before TMEM is released
-        mma_commit(done_bar);
+        if (elect_one()) mma_commit(done_bar);
+        __syncwarp();
         const long long t0 = clock64();
         while (!mbar_try(done_bar, 0) && clock64() - t0 < DRAIN_CYCLES) {
         }
     } else if (warp >= 2) {
-        // ---------------- epilogue: row = TMEM lane, 64 columns per thread
-        const int quarter = warp & 3, row = quarter * 32 + lane, col0 = ((warp - 2) >> 2) * 64;
+        // ---------------- epilogue: row = TMEM lane, COLS columns per thread
+        const int quarter = warp & 3, row = quarter * 32 + lane, col0 = ((warp - 2) >> 2) * COLS;
         long long* const stash = SHORT ? nullptr : g.stash + (long long)blockIdx.x * (TILE * TILE) + col0 * TILE + row;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
         int acc = 0;
@@ -490,19 +535,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
             int tb, tm, tn;
             tile_at(g, t, tb, tm, tn);
             const int* const exA = g.exA + (long long)tb * g.tiles_m * TILE;
-            const int* const exB = g.exB + (long long)tb * g.tiles_n * TILE;
-            const int m = tm * TILE + row, n0 = tn * TILE + col0, nc = min(64, g.N - n0);
+            const int* const exB = g.exB + (long long)tb * ((g.N + TILE - 1) / TILE) * TILE;
+            const int m = tm * TILE + row, n0 = tn * TN + col0, nc = min(COLS, g.N - n0);
             const bool mine = m < g.M;
-            // exponents: this thread's row, and two of the warp's 64 columns per lane
+            // exponents: this thread's row, and one or two of the warp's columns per lane
             const int Ea = mine ? exA[m] : 0;
-            const int Eb0 = lane < nc ? exB[n0 + lane] : 0, Eb1 = lane + 32 < nc ? exB[n0 + 32 + lane] : 0;
+            const int Eb0 = lane < nc ? exB[n0 + lane] : 0, Eb1 = COLS > 32 && lane + 32 < nc ? exB[n0 + 32 + lane] : 0;
             const bool special = __any_sync(0xffffffffu, Ea == 0x7ff || Eb0 == 0x7ff || Eb1 == 0x7ff);
             const int ea = max(Ea, 1);
             double* const Cm = g.C + tb * g.cb + m + (long long)n0 * g.ldc;
             const double alpha = g.alpha, beta = g.beta;
-            long long sum[64];
+            long long sum[COLS];
 #pragma unroll
-            for (int j = 0; j < 64; ++j) sum[j] = 0;
+            for (int j = 0; j < COLS; ++j) sum[j] = 0;
             // The read-out walks the columns eight at a time in a rolled loop, the sums moving
             // down by eight registers each turn: unrolled it outgrew the instruction cache and
             // took 70 us a tile.
@@ -535,24 +580,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
                     }
                 }
             };
-            auto exps = [&](int c) { return ea + max(__shfl_sync(0xffffffffu, c < 32 ? Eb0 : Eb1, c & 31), 1); };
+            auto exps = [&](int c) { return ea + max(__shfl_sync(0xffffffffu, COLS <= 32 || c < 32 ? Eb0 : Eb1, c & 31), 1); };
             auto rotate = [&]() {
 #pragma unroll
-                for (int j = 0; j < 56; ++j) sum[j] = sum[j + 8];
+                for (int j = 0; j < COLS - 8; ++j) sum[j] = sum[j + 8];
             };
-            for (int q = 0; q < ng; ++q) {
-                const Group G = group_at(q, k16);
-                const bool straight = SHORT && G.last && !special;
+            for (int q = 0; q < (SHORT ? NBUF : ng); ++q) {
+                const Group G = group_at<SHORT>(SHORT ? q >> 1 : q, k16);
+                const int p = SHORT ? q : G.p;
+                const bool straight = SHORT && q == 3 && !special;
                 // the whole warp stays or leaves: tcgen05.ld is warp-collective
                 ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, aph, err, wait));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t base = tmem_base + lanes + (uint32_t)(acc * 2 * TILE + col0);
-                if (SHORT && G.last) {
+                const uint32_t base = tmem_base + lanes + (uint32_t)(acc * 2 * TN + col0);
+                if (SHORT && q == 3) {
 #pragma unroll 1
-                    for (int c = 0; straight && c < 64; c += 8) {
+                    for (int c = 0; straight && c < COLS; c += 8) {
                         float v0[8], v1[8];
-                        tmem_ld8x2(base + c, base + TILE + c, v0, v1);
+                        tmem_ld8x2(base + c, base + TN + c, v0, v1);
                         double r[8];
                         int E[8];
 #pragma unroll
@@ -562,28 +608,27 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
                         rotate();
                     }
                 } else {
-                    // weights of the two accumulators within the sums
-                    const int w1 = (G.p & 1) || (SHORT && G.p == 2) ? 1 : 1 << 16, w0 = w1 << 8;
-                    if (SHORT && G.p == 2)
+                    // weights of the two accumulators within the sums (SHORT: of 0 to 5 in units
+                    // of weight 5, below 2^63)
+                    const long long w1 = SHORT ? 1ll << (32 - 16 * p) : p & 1 ? 1 : 1 << 16;
+                    const long long w0 = w1 << 8;
 #pragma unroll
-                        for (int j = 0; j < 64; ++j) sum[j] <<= 16;
-#pragma unroll
-                    for (int c = 0; c < 64; c += 16) {
+                    for (int c = 0; c < COLS; c += 16) {
                         float v[16];
                         tmem_ld16(base + c, v);
 #pragma unroll
                         for (int j = 0; j < 16; ++j) sum[c + j] += (long long)__float2int_rn(v[j]) * w0;
-                        tmem_ld16(base + TILE + c, v);
+                        tmem_ld16(base + TN + c, v);
 #pragma unroll
                         for (int j = 0; j < 16; ++j) sum[c + j] += (long long)__float2int_rn(v[j]) * w1;
                     }
                 }
                 tc_fence_before();
                 mbar_arrive(tempty0 + 8 * acc);
-                if (++acc == 2) { acc = 0; aph ^= 1; }
+                if (++acc == NBUF) { acc = 0; aph ^= 1; }
                 if (!SHORT && G.last_hi) {
 #pragma unroll
-                    for (int j = 0; j < 64; ++j) {
+                    for (int j = 0; j < COLS; ++j) {
                         stash[j * TILE] = sum[j];
                         sum[j] = 0;
                     }
@@ -592,7 +637,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) oz_gemm_kernel(const __grid_const
             if (!ok) break;
             if (!SHORT && !special) {
 #pragma unroll 1
-                for (int c = 0; c < 64; c += 8) {
+                for (int c = 0; c < COLS; c += 8) {
                     double r[8];
                     long long h[8];
 #pragma unroll
@@ -634,14 +679,16 @@ static void set_up() {
         int dev = 0;
         CUDA_CHECK(cudaGetDevice(&dev));
         CUDA_CHECK(cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev));
-        CUDA_CHECK(cudaFuncSetAttribute(oz_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        CUDA_CHECK(cudaFuncSetAttribute(oz_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        CUDA_CHECK(cudaFuncSetAttribute(oz_gemm_kernel<true, OzTile<64>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        SMEM_BYTES));
+        CUDA_CHECK(cudaFuncSetAttribute(oz_gemm_kernel<false, OzTile<128>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        SMEM_BYTES));
         CUDA_CHECK(cudaFuncSetAttribute(oz_split_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
     });
 }
 
-void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int k_, cudaStream_t st, int batch_,
-                  long long bs_) {
+void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int k_, cudaStream_t st, bool right,
+                  int batch_, long long bs_) {
     set_up();
     rows = rows_;
     k = k_;
@@ -651,12 +698,13 @@ void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int 
     rs = rs_;
     ks = ks_;
     bs = bs_;
-    const int rb = ceil_div(rows, TILE), eb = rb * TILE;
-    d.alloc((size_t)batch * rb * k16 * (BLOCK / 16), st);
+    block = right && k16 <= HI_CHUNK ? 64 : TILE;
+    const int nb = ceil_div(rows, TILE), eb = nb * TILE;
+    d.alloc((size_t)batch * nb * k16 * (BLOCK / 16), st);
     ex.alloc((size_t)batch * eb, st);
     if (k <= FUSED_K && (rs == 1 || ks == 1)) {
         LAUNCH(oz_split_fused, dim3(ceil_div(rows, 32), 1, batch), 256, k16 * 16 * 33 * 8, st, a, rs, ks, rows, k, k16,
-               ex.get(), d.get(), bs, eb);
+               ex.get(), d.get(), bs, eb, block);
         return;
     }
     if (ks == 1) {
@@ -664,12 +712,12 @@ void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int 
     } else {
         ex.zero();
         const int kper = 32;
-        LAUNCH(oz_exponent_rows, dim3(rb, ceil_div(k, kper), batch), TILE, 0, st, a, rs, ks, rows, k, kper, ex.get(), bs,
+        LAUNCH(oz_exponent_rows, dim3(nb, ceil_div(k, kper), batch), TILE, 0, st, a, rs, ks, rows, k, kper, ex.get(), bs,
                eb);
     }
     // about four CTAs per SM's worth of k16 steps
-    const int gy = std::max(1, std::min(k16, 152 * 8 / (rb * batch)));
-    LAUNCH(oz_split, dim3(rb, gy, batch), dim3(TILE, 2), 0, st, a, rs, ks, rows, k, k16, ex.get(), d.get(), bs, eb);
+    const int gy = std::max(1, std::min(k16, 152 * 8 / (nb * batch)));
+    LAUNCH(oz_split, dim3(nb, gy, batch), dim3(TILE, 2), 0, st, a, rs, ks, rows, k, k16, ex.get(), d.get(), bs, eb, block);
 }
 
 void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* C, long long ldc, int* err,
@@ -687,7 +735,9 @@ void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* 
     g.K = A.k;
     g.k16 = A.k16;
     g.tiles_m = ceil_div(g.M, TILE);
-    g.tiles_n = ceil_div(g.N, TILE);
+    const bool brief = g.k16 <= HI_CHUNK;
+    if (A.block != TILE || B.block != (brief ? 64 : TILE)) fail(SQBEM_ERR_ARG, "oz_gemm: B was not split as the right operand");
+    g.tiles_n = ceil_div(g.N, B.block);
     g.alpha = alpha;
     g.beta = beta;
     g.C = C;
@@ -703,7 +753,6 @@ void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* 
     g.abs = A.bs;
     g.bbs = B.bs;
     const int grid = std::min(g.tiles_m * g.tiles_n * g.batch, g_sms);
-    const bool brief = g.k16 <= HI_CHUNK;
     DevBuf<long long> stash(brief ? 0 : (size_t)grid * TILE * TILE, st);
     g.stash = stash.get();
     g.err = err;
@@ -711,8 +760,10 @@ void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* 
     // credited as BF16 tensor work: 36 digit products
     const double fl = 72.0 * g.batch * g.M * g.N * g.K,
                  by = g.batch * (16.0 * ((double)g.M + g.N) * g.K + (beta == 0.0 ? 8.0 : 16.0) * g.M * g.N);
-    if (brief) TIMED_LAUNCH("oz_gemm", fl, by, oz_gemm_kernel<true>, grid, NTHREADS, SMEM_BYTES, st, g);
-    else TIMED_LAUNCH("oz_gemm", fl, by, oz_gemm_kernel<false>, grid, NTHREADS, SMEM_BYTES, st, g);
+    if (brief)
+        TIMED_LAUNCH("oz_gemm", fl, by, (oz_gemm_kernel<true, OzTile<64>>), grid, OzTile<64>::NTHREADS, SMEM_BYTES, st, g);
+    else
+        TIMED_LAUNCH("oz_gemm", fl, by, (oz_gemm_kernel<false, OzTile<128>>), grid, OzTile<128>::NTHREADS, SMEM_BYTES, st, g);
 }
 
 }  // namespace sqbem

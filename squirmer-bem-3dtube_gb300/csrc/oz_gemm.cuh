@@ -25,13 +25,14 @@ namespace sqbem {
 struct OzMat {
     DevBuf<uint4> d;
     DevBuf<int> ex;
-    int rows = 0, k = 0, k16 = 0, batch = 1;
+    int rows = 0, k = 0, k16 = 0, batch = 1, block = 128;
     // the values' source, for rows that hold an infinity or a NaN
     const double* src = nullptr;
     long long rs = 0, ks = 0, bs = 0;
-    // element (r, c) of matrix b is a[r * rs + c * ks + b * bs]
-    void split(const double* a, long long rs, long long ks, int rows, int k, cudaStream_t st, int batch = 1,
-               long long bs = 0);
+    // element (r, c) of matrix b is a[r * rs + c * ks + b * bs]; `right` where the operand is B
+    // (blocks of 64 rows then, while k <= 256)
+    void split(const double* a, long long rs, long long ks, int rows, int k, cudaStream_t st, bool right = false,
+               int batch = 1, long long bs = 0);
 };
 
 // C (M x N, column-major) = alpha A B + beta C for the digits of A (M rows) and of

@@ -71,6 +71,34 @@ def test_digit_product_of_integers_is_exact():
     np.testing.assert_array_equal(sqbem.gemm64(A, B, route=1), (A @ B).astype(float))
 
 
+@pytest.mark.parametrize("N", [1, 63, 64, 65, 128, 129, 192, 321])
+@pytest.mark.parametrize("K", [15, 33, 256])
+def test_short_digit_product_at_its_column_tiles(N, K):
+    # K <= 256: column tiles of 64, the whole 80-bit total rounded in integers.  Integers of 20
+    # bits with empty rows and columns, exact in FP64; then equal entries whose digits are the
+    # largest (sums of 2^62 before the last pass), sums that cancel to 2^-70 of the row's largest
+    # entry, and results beyond the normal numbers on either side
+    rng = np.random.default_rng([N, K])
+    A, B = rng.integers(-2 ** 20, 2 ** 20, (131, K)), rng.integers(-2 ** 20, 2 ** 20, (K, N))
+    A[::7] = 0
+    B[:, ::5] = 0
+    np.testing.assert_array_equal(sqbem.gemm64(A, B, route=1), (A @ B).astype(float))
+    for v in (255.0 / 256, 127.5 / 128, 2.0 ** 31 - 1):
+        A, B = np.full((131, K), v), np.full((K, N), -v)
+        ref = -float(K * int(v * 2 ** 40) * int(v * 2 ** 40) / 2 ** 80)
+        np.testing.assert_array_equal(sqbem.gemm64(A, B, route=1), np.full((131, N), ref))
+    A = np.ones((131, K))
+    A[:, 1] = -1.0
+    A[:, 2:] = 0.0
+    B = np.full((K, N), 0.75)
+    B[0] += 2.0 ** -53 * 64
+    np.testing.assert_array_equal(sqbem.gemm64(A, B, route=1), np.full((131, N), 2.0 ** -47))
+    for a, b in ((2.0 ** -600, 2.0 ** -460), (2.0 ** 600, 2.0 ** 460), (2.0 ** -512, 2.0 ** -510)):
+        A, B = np.zeros((131, K)), np.zeros((K, N))
+        A[:, 0], B[0] = a, -b
+        np.testing.assert_array_equal(sqbem.gemm64(A, B, route=1), np.full((131, N), -(a * b)))
+
+
 def test_digit_product_no_less_exact_than_the_fp64_pipe():
     # rows and columns whose entries span four orders of magnitude, as the blocks' do
     rng = np.random.default_rng(7)
