@@ -138,6 +138,114 @@ __global__ void __launch_bounds__(MV_ROWS) mv_partial32(const __grid_constant__ 
         if (k < r) o[k] = (double)s[k] + (double)cc[k];
 }
 
+// Two FP32 values in a 64-bit register, each operation rounded like its scalar form.
+__device__ __forceinline__ uint64_t pack2(float x, float y) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& x, float& y) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// The compensated sums of one or two columns, the two as one packed operand: dot2_step's
+// eleven operations per element once for both (the rounding of each half is the scalar one;
+// the product's error enters with its sign turned, which needs the matrix entry negated and not
+// the product), and the vector's four parts in one shared-memory load.  The scalar kernel
+// issued about 30 instructions per element, 22 of them FP32 operations; packed operations take
+// two turns of the FP32 pipe but one issue.  48 products of 3888 x 3888 (some matrices shared,
+// in L2): 475 us scalar, 408 packed, 345 with two rows per thread.
+// ROWS = 2 (8-byte aligned columns) gives a thread rows 2t and 2t + 1: twice the independent
+// operations, and half the FP64 conversions of the vector per row.
+template <int ROWS>
+__global__ void __launch_bounds__(MV_ROWS) mv_pair32(const __grid_constant__ MvArgs args, double* __restrict__ part) {
+    constexpr int NB = MV_BATCH;
+    static_assert(MV_CHUNK % NB == 0, "matvec chunk must be a multiple of the load batch");
+    __shared__ ulonglong2 xs[MV_CHUNK];  // (xh of both columns, xl of both)
+    const int jb = blockIdx.z, c = blockIdx.y;
+    const int nchunk = args.j[jb].nchunk;
+    if (c >= nchunk) return;
+    const float* __restrict__ A = args.j[jb].j.A32;
+    const double* __restrict__ X = args.j[jb].j.x;
+    const long long lda = args.j[jb].j.lda, ldx = args.j[jb].j.ldx;
+    const int m = args.j[jb].j.m, n = args.j[jb].j.n, r = args.j[jb].j.r;
+    const long long poff = args.j[jb].part_off;
+    const int rstride = args.j[jb].rstride;
+    const int j0 = c * MV_CHUNK, nj = min(n, j0 + MV_CHUNK) - j0;
+    for (int j = threadIdx.x; j < MV_CHUNK; j += MV_ROWS) {
+        const double v0 = j < nj ? X[j0 + j] : 0.0, v1 = j < nj && r > 1 ? X[j0 + j + ldx] : 0.0;
+        const float h0 = (float)v0, h1 = (float)v1;
+        xs[j] = make_ulonglong2(pack2(h0, h1), pack2((float)(v0 - (double)h0), (float)(v1 - (double)h1)));
+    }
+    __syncthreads();
+    const int row = ROWS * (blockIdx.x * MV_ROWS + threadIdx.x);
+    if (row >= m) return;
+    const bool two = row + 1 < m;
+    uint64_t s[ROWS], cc[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) s[i] = cc[i] = 0;
+    const float* a = A + row + (long long)j0 * lda;
+    for (int j = 0; j < nj; j += NB) {
+        float av[NB][ROWS];
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+            const float* p = a + (long long)(j + u) * lda;
+            if (ROWS == 1) {
+                av[u][0] = j + u < nj ? __ldg(p) : 0.f;
+            } else {
+                const float2 q = j + u < nj ? (two ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(__ldg(p), 0.f))
+                                            : make_float2(0.f, 0.f);
+                av[u][0] = q.x;
+                av[u][ROWS - 1] = q.y;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+            const ulonglong2 x = xs[j + u];
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) {
+                const uint64_t v = pack2(av[u][i], av[u][i]), nv = pack2(-av[u][i], -av[u][i]);
+                const uint64_t p = mul2(v, x.x);
+                const uint64_t e = fma2(nv, x.x, p);  // exact: a * xh = p - e
+                const uint64_t t = add2(s[i], p), z = sub2(t, s[i]);
+                const uint64_t err = add2(sub2(s[i], sub2(t, z)), sub2(p, z));  // exact: s + p = t + err
+                s[i] = t;
+                cc[i] = fma2(v, x.y, add2(cc[i], sub2(err, e)));
+            }
+        }
+    }
+    double* o = part + poff + ((long long)c * m + row) * rstride;
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        if (i == 1 && !two) break;
+        float s0, s1, c0, c1;
+        unpack2(s[i], s0, s1);
+        unpack2(cc[i], c0, c1);
+        o[i * rstride] = (double)s0 + (double)c0;
+        if (r > 1) o[i * rstride + 1] = (double)s1 + (double)c1;
+    }
+}
+
 // PLAIN with two rows per thread: one 8-byte load gives a thread rows 2t and
 // 2t + 1 of a column, so a warp reads 256 contiguous bytes per load and the
 // load count halves.  Used when every job's base address and leading
@@ -493,20 +601,22 @@ static void matvec_launches(const std::vector<MvJob>& jobs, cudaStream_t st) {
         bool pairs_ok = true;
         for (int k = 0; k < a.n && pairs_ok; ++k)
             pairs_ok = a.j[k].j.A32 && ((uintptr_t)a.j[k].j.A32 % 8 == 0) && a.j[k].j.lda % 2 == 0;
+        const dim3 g2(ceil_div(maxm, 2 * MV_ROWS), maxc, (unsigned)a.n);
         if (few) {
             const dim3 g(1, maxc, (unsigned)a.n);
             if (maxr <= 2) TIMED_LAUNCH("matvec", 0.0, bytes, mv_few<2>, g, 32 * MV_FEW_WARPS, 0, st, a, part.get());
             else TIMED_LAUNCH("matvec", 0.0, bytes, mv_few<MV_RMAX>, g, 32 * MV_FEW_WARPS, 0, st, a, part.get());
         } else if (plain && pairs_ok && maxr <= 2) {
-            const dim3 g2(ceil_div(maxm, 2 * MV_ROWS), maxc, (unsigned)a.n);
             TIMED_LAUNCH("matvec", 0.0, bytes, mv_plain2<2>, g2, MV_ROWS, 0, st, a, part.get());
         } else if (plain) {
             if (maxr <= 2) TIMED_LAUNCH("matvec", 0.0, bytes, (mv_partial32<2, true>), grid, MV_ROWS, 0, st, a, part.get());
             else TIMED_LAUNCH("matvec", 0.0, bytes, (mv_partial32<MV_RMAX, true>), grid, MV_ROWS, 0, st, a, part.get());
         } else if (all32) {
             // the compensated sums are FP32-issue-bound, so the column count is a
-            // template parameter (2: refinement; 6: the rigid-body columns A_u K)
-            if (maxr <= 2) TIMED_LAUNCH("matvec", 0.0, bytes, (mv_partial32<2, false>), grid, MV_ROWS, 0, st, a, part.get());
+            // template parameter (6: the rigid-body columns A_u K), and one or two columns
+            // (refinement) have packed operations
+            if (maxr <= 2 && pairs_ok) TIMED_LAUNCH("matvec", 0.0, bytes, mv_pair32<2>, g2, MV_ROWS, 0, st, a, part.get());
+            else if (maxr <= 2) TIMED_LAUNCH("matvec", 0.0, bytes, mv_pair32<1>, grid, MV_ROWS, 0, st, a, part.get());
             else if (maxr <= 6) TIMED_LAUNCH("matvec", 0.0, bytes, (mv_partial32<6, false>), grid, MV_ROWS, 0, st, a, part.get());
             else TIMED_LAUNCH("matvec", 0.0, bytes, (mv_partial32<MV_RMAX, false>), grid, MV_ROWS, 0, st, a, part.get());
         } else if (maxr <= 2) {
