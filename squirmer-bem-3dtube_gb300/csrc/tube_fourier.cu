@@ -398,133 +398,187 @@ __global__ void __launch_bounds__(64) idft_kernel(const __grid_constant__ DftArg
     }
 }
 
-// Both transforms with a thread per representative a and column (blockIdx.x;
-// job: blockIdx.y), all three components of its rows in the thread: the rotation
-// R_s needs no exchange between lanes, every panel load and twiddle serves three
-// rows, and with the sector and frequency loops unrolled the twiddles are
-// constant operands of the multiply-adds.
+// Both transforms with the number of sectors known at compile time: the sector and frequency
+// loops unrolled, the twiddles constant operands of the multiply-adds.  A CTA holds one column
+// (blockIdx.x; job: blockIdx.y), whose rows by panel go through shared memory: they are
+// 12-byte pieces there, gathered at the panels' numbers, and whole lines in global memory.
+constexpr int FDFT_THREADS = 256, IDFT_THREADS = 96;
+static_assert(FDFT_THREADS >= FT_MAX_ORDER && 3 * IDFT_THREADS >= FT_MAX_ORDER, "a CTA holds one column");
+int fdft_threads(int nb) { return (3 * nb + 31) / 32 * 32; }
+int idft_threads(int nb) { return nb <= 64 ? 64 : IDFT_THREADS; }
+size_t dft_smem(int nth, int nb) { return (size_t)3 * nb * nth * sizeof(float); }
+
+// Forward: a thread per row (a, c) of the spectrum, so that the 2-byte stores of a warp are
+// contiguous.  A thread per representative with all three components held 164 registers for
+// twelve warps per SM, which waited on its gathers: 265 us for 24 sectors, 54 representatives
+// and 23040 columns, 206 here (111 at the copy's rate).
 template <int NTH, class TI>
-__global__ void __launch_bounds__(64) fdft_rep(const __grid_constant__ DftArgs args) {
+__global__ void __launch_bounds__(FDFT_THREADS) fdft_rep(const __grid_constant__ DftArgs args) {
     constexpr int NF = NTH / 2 + 1;
     const DftJob& J = args.j[blockIdx.y];
     const int j = blockIdx.x;
     if (j >= J.nc) return;
-    const int n3 = 3 * J.nb;
+    extern __shared__ __align__(16) float xs[];
+    const int n3 = 3 * J.nb, nt = n3 * NTH, r = threadIdx.x, bd = blockDim.x;
     const TI* x = reinterpret_cast<const TI*>(J.x) + (long long)j * J.ldx;
     const float scale = 1.f / (float)NTH;
-    for (int a = threadIdx.x; a < J.nb; a += blockDim.x) {
-        const int* pa = J.panel + a * NTH;
-        float v[3][NTH];  // R_s^T x_{panel(a, s)}
+    // eight loads in flight per thread (a rolled remainder waited for each)
+    int e0 = 0;
+    if (sizeof(TI) == 4 && ((uintptr_t)x & 15) == 0) {
+        for (int e = threadIdx.x; e < nt / 4; e += 8 * bd) {
+            float4 q[8];
 #pragma unroll
-        for (int s = 0; s < NTH; ++s) {
-            const TI* xp = x + 3LL * __ldg(pa + s);
-            const float x0 = (float)__ldg(xp), x1 = (float)__ldg(xp + 1);
-            const float c = args.tw[s].x, sn = args.tw[s].y;
-            v[0][s] = c * x0 + sn * x1;
-            v[1][s] = -sn * x0 + c * x1;
-            v[2][s] = (float)__ldg(xp + 2);
+            for (int u = 0; u < 8; ++u)
+                if (e + u * bd < nt / 4) q[u] = __ldg(reinterpret_cast<const float4*>(x) + e + u * bd);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (e + u * bd < nt / 4) reinterpret_cast<float4*>(xs)[e + u * bd] = q[u];
         }
+        e0 = nt & ~3;
+    }
+    for (int e = e0 + threadIdx.x; e < nt; e += 8 * bd) {
+        TI q[8];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int r = 3 * a + c;
-            float re[NF], im[NF];
+        for (int u = 0; u < 8; ++u)
+            if (e + u * bd < nt) q[u] = __ldg(x + e + u * bd);
 #pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                re[f] = v[c][0];
-                im[f] = 0.f;
-            }
-            // sectors s and NTH - s: shared cosines, opposite sines
+        for (int u = 0; u < 8; ++u)
+            if (e + u * bd < nt) xs[e + u * bd] = (float)q[u];
+    }
+    __syncthreads();
+    if (r >= n3) return;
+    const int a = r / 3, c = r - 3 * a;
+    const int* pa = J.panel + a * NTH;
+    float v[NTH];  // component c of R_s^T x_{panel(a, s)}
 #pragma unroll
-            for (int s = 1; 2 * s < NTH; ++s) {
-                const float sum = v[c][s] + v[c][NTH - s], dif = v[c][s] - v[c][NTH - s];
+    for (int s = 0; s < NTH; ++s) {
+        const float* xp = xs + 3 * __ldg(pa + s);
+        const float cs = args.tw[s].x, sn = args.tw[s].y;
+        // c = 0: cs x0 + sn x1; c = 1: cs x1 - sn x0
+        const float xa = xp[c], xb = xp[c == 0 ? 1 : 0];
+        const float w = __fmaf_rn(cs, xa, __fmul_rn(c == 0 ? sn : -sn, xb));
+        v[s] = c == 2 ? xa : w;
+    }
+    float re[NF], im[NF];
 #pragma unroll
-                for (int f = 0; f < NF; ++f) {
-                    re[f] += sum * args.tw[(f * s) % NTH].x;
-                    im[f] -= dif * args.tw[(f * s) % NTH].y;
-                }
-            }
-            if ((NTH & 1) == 0) {
+    for (int f = 0; f < NF; ++f) {
+        re[f] = v[0];
+        im[f] = 0.f;
+    }
+    // sectors s and NTH - s: shared cosines, opposite sines
 #pragma unroll
-                for (int f = 0; f < NF; ++f) re[f] += (f & 1) ? -v[c][NTH / 2] : v[c][NTH / 2];
-            }
+    for (int s = 1; 2 * s < NTH; ++s) {
+        const float sum = v[s] + v[NTH - s], dif = v[s] - v[NTH - s];
 #pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                const long long o = ((long long)f * J.nc + j) * J.ldk;
-                const float vr = re[f] * scale, vi = im[f] * scale;
-                const bf16 hr = __float2bfloat16_rn(vr), hi = __float2bfloat16_rn(vi);
-                J.h[o + r] = hr;
-                J.l[o + r] = __float2bfloat16_rn(vr - __bfloat162float(hr));
-                J.h[o + n3 + r] = hi;
-                J.l[o + n3 + r] = __float2bfloat16_rn(vi - __bfloat162float(hi));
-            }
+        for (int f = 0; f < NF; ++f) {
+            re[f] += sum * args.tw[(f * s) % NTH].x;
+            im[f] -= dif * args.tw[(f * s) % NTH].y;
         }
+    }
+    if ((NTH & 1) == 0) {
+#pragma unroll
+        for (int f = 0; f < NF; ++f) re[f] += (f & 1) ? -v[NTH / 2] : v[NTH / 2];
+    }
+    const long long step = (long long)J.nc * J.ldk;
+    bf16* h = J.h + (long long)j * J.ldk + r;
+    bf16* l = J.l + (long long)j * J.ldk + r;
+#pragma unroll
+    for (int f = 0; f < NF; ++f, h += step, l += step) {
+        const float vr = re[f] * scale, vi = im[f] * scale;
+        const bf16 hr = __float2bfloat16_rn(vr), hi = __float2bfloat16_rn(vi);
+        h[0] = hr;
+        l[0] = __float2bfloat16_rn(vr - __bfloat162float(hr));
+        h[n3] = hi;
+        l[n3] = __float2bfloat16_rn(vi - __bfloat162float(hi));
     }
 }
 
-// Thread per (representative a, component c) of one column: the 2 nf spectrum
-// values of its row in registers, the twiddles constant operands (NTH known at
-// compile time).  The rotation R_s mixes components 0 and 1, which sit on
-// neighbouring lanes: a warp takes 10 representatives on lanes 0 .. 29 (lanes
-// 30, 31 idle), so the pair never straddles two warps.
+// Inverse: a thread per representative a, whose three components' 6 NF spectrum values it
+// holds (the rotation R_s needs no exchange), and the sectors s and NTH - s from one pair of
+// sums,
+//   y~_s = A_s - B_s and y~_{NTH-s} = A_s + B_s with A_s = sum_f cos(2 pi f s / NTH) y^r_f and
+//   B_s = sum_f sin(2 pi f s / NTH) y^i_f.
+// With a thread per component and the sector loop rolled (twiddles by their index, partners by
+// shuffles) a column took 16,700 warp instructions, whose issue bound it: 443 us for the
+// columns above, 213 here (164 at the copy's rate).
 template <int NTH, class TO>
-__global__ void __launch_bounds__(192) idft_nth(const __grid_constant__ DftArgs args) {
+__global__ void __launch_bounds__(IDFT_THREADS) idft_rep(const __grid_constant__ DftArgs args) {
     constexpr int NF = NTH / 2 + 1;
     const DftJob& J = args.j[blockIdx.y];
     const int j = blockIdx.x;
     if (j >= J.nc) return;
-    const int n3 = 3 * J.nb;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    extern __shared__ __align__(16) float ys[];
+    const int nb = J.nb, n3 = 3 * nb, nt = n3 * NTH, a = threadIdx.x;
     const float* yh = reinterpret_cast<const float*>(J.x) + (long long)j * J.ldk;
     const long long plane = (long long)J.nc * J.ldk;
-    TO* y = reinterpret_cast<TO*>(J.y) + (long long)j * J.ldy;
-    const int c = lane % 3;
-    for (int a0 = 10 * warp; a0 < J.nb; a0 += 10 * nw) {
-        const int a = a0 + lane / 3;
-        const bool act = lane < 30 && a < J.nb;
-        const int r = 3 * a + c;
-        float yr[NF], yi[NF];
+    if (a < nb) {
+        float yr[3][NF], yi[3][NF];
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
             const float wgt = (f == 0 || 2 * f == NTH) ? 1.f : 2.f;
-            yr[f] = act ? wgt * yh[f * plane + r] : 0.f;
-            yi[f] = act ? wgt * yh[f * plane + n3 + r] : 0.f;
-        }
-        const int* pa = J.panel + (act ? a : 0) * NTH;
-        // the sector loop rolled: the twiddle index f s mod NTH is the same on
-        // every lane, so the twiddles are broadcast constant-cache loads, and the
-        // thread holds only its 2 NF spectrum values
-        // y~_s = A_s - B_s and y~_{NTH-s} = A_s + B_s with A_s = sum_f cos(2 pi f s / NTH) y^r_f and
-        // B_s = sum_f sin(2 pi f s / NTH) y^i_f: the two sectors from one pair of sums
-        auto emit = [&](int s, float v) {
-            // partner component: c = 0 <-> 1 (c = 2 keeps its own value)
-            const float w = __shfl_sync(0xffffffffu, v, c == 0 ? lane + 1 : (c == 1 ? lane - 1 : lane));
-            const float cs = args.tw[s].x, sn = args.tw[s].y;
-            const float o = c == 0 ? cs * v - sn * w : (c == 1 ? sn * w + cs * v : v);
-            if (act) {
-                const long long row = 3LL * __ldg(pa + s) + c;
-                y[row] = (TO)o;
-                if (J.h) {
-                    const long long e = row * J.hrs + (long long)j * J.hcs;
-                    const bf16 h = __float2bfloat16_rn(o);
-                    J.h[e] = h;
-                    J.l[e] = __float2bfloat16_rn(o - __bfloat162float(h));
-                }
-            }
-        };
-#pragma unroll 1
-        for (int s = 0; 2 * s <= NTH; ++s) {
-            float A = 0.f, B = 0.f;
-            int k = 0;
 #pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                const float2 t = args.tw[k];
-                A += t.x * yr[f];
-                B += t.y * yi[f];
-                k += s;
-                if (k >= NTH) k -= NTH;
+            for (int c = 0; c < 3; ++c) {
+                yr[c][f] = wgt * __ldg(yh + f * plane + 3 * a + c);
+                yi[c][f] = wgt * __ldg(yh + f * plane + n3 + 3 * a + c);
             }
-            emit(s, A - B);
-            if (s > 0 && 2 * s < NTH) emit(NTH - s, A + B);
+        }
+        const int* pa = J.panel + a * NTH;
+        auto emit = [&](int s, const float (&v)[3]) {
+            const float cs = args.tw[s].x, sn = args.tw[s].y;
+            float* const o = ys + 3 * __ldg(pa + s);
+            o[0] = cs * v[0] - sn * v[1];
+            o[1] = sn * v[0] + cs * v[1];
+            o[2] = v[2];
+        };
+#pragma unroll
+        for (int s = 0; 2 * s <= NTH; ++s) {
+            float A[3] = {}, B[3] = {};
+#pragma unroll
+            for (int f = 0; f < NF; ++f)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    A[c] += args.tw[(f * s) % NTH].x * yr[c][f];
+                    B[c] += args.tw[(f * s) % NTH].y * yi[c][f];
+                }
+            const float lo[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
+            emit(s, lo);
+            if (s > 0 && 2 * s < NTH) {
+                const float hi[3] = {A[0] + B[0], A[1] + B[1], A[2] + B[2]};
+                emit(NTH - s, hi);
+            }
+        }
+    }
+    __syncthreads();
+    TO* const y = reinterpret_cast<TO*>(J.y) + (long long)j * J.ldy;
+    bf16* const h = J.h ? J.h + (long long)j * J.hcs : nullptr;
+    bf16* const l = J.h ? J.l + (long long)j * J.hcs : nullptr;
+    int e0 = 0;
+    if (sizeof(TO) == 4 && ((uintptr_t)y & 15) == 0 && (!h || (J.hrs == 1 && (((uintptr_t)h | (uintptr_t)l) & 7) == 0))) {
+        e0 = nt & ~3;
+        for (int e = 4 * threadIdx.x; e < e0; e += 4 * blockDim.x) {
+            const float4 o = *reinterpret_cast<const float4*>(ys + e);
+            *reinterpret_cast<float4*>(y + e) = o;
+            if (h) {
+                const float q[4] = {o.x, o.y, o.z, o.w};
+                uint2 hv, lv;
+                bf16 *hp = reinterpret_cast<bf16*>(&hv), *lp = reinterpret_cast<bf16*>(&lv);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    hp[u] = __float2bfloat16_rn(q[u]);
+                    lp[u] = __float2bfloat16_rn(q[u] - __bfloat162float(hp[u]));
+                }
+                *reinterpret_cast<uint2*>(h + e) = hv;
+                *reinterpret_cast<uint2*>(l + e) = lv;
+            }
+        }
+    }
+    for (int e = e0 + threadIdx.x; e < nt; e += blockDim.x) {
+        const float o = ys[e];
+        y[e] = (TO)o;
+        if (h) {
+            const bf16 hv = __float2bfloat16_rn(o);
+            h[e * J.hrs] = hv;
+            l[e * J.hrs] = __float2bfloat16_rn(o - __bfloat162float(hv));
         }
     }
 }
@@ -775,16 +829,18 @@ void fourier_solve(const std::vector<FourierJob>& jobs, const MixedCtx& cx) {
         const int nth = jobs[i0].ft->nth;
         set_tw(a, nth);
         const double by = dft_bytes(i0, a.n, true);
-        const dim3 gd(maxnc, a.n);
+        int nb = 0;
+        for (int q = 0; q < a.n; ++q) nb = std::max(nb, a.j[q].nb);
+        const dim3 gd(maxnc, a.n), bs(fdft_threads(nb));
         if (in64) {
-            if (nth == 24) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<24, double>), gd, 64, 0, cx.st, a);
-            else if (nth == 30) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<30, double>), gd, 64, 0, cx.st, a);
-            else if (nth == 36) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<36, double>), gd, 64, 0, cx.st, a);
+            if (nth == 24) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<24, double>), gd, bs, dft_smem(24, nb), cx.st, a);
+            else if (nth == 30) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<30, double>), gd, bs, dft_smem(30, nb), cx.st, a);
+            else if (nth == 36) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<36, double>), gd, bs, dft_smem(36, nb), cx.st, a);
             else TIMED_LAUNCH("fourier_dft", 0.0, by, fdft_kernel<double>, gd, 192, 0, cx.st, a);
         } else {
-            if (nth == 24) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<24, float>), gd, 64, 0, cx.st, a);
-            else if (nth == 30) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<30, float>), gd, 64, 0, cx.st, a);
-            else if (nth == 36) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<36, float>), gd, 64, 0, cx.st, a);
+            if (nth == 24) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<24, float>), gd, bs, dft_smem(24, nb), cx.st, a);
+            else if (nth == 30) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<30, float>), gd, bs, dft_smem(30, nb), cx.st, a);
+            else if (nth == 36) TIMED_LAUNCH("fourier_dft", 0.0, by, (fdft_rep<36, float>), gd, bs, dft_smem(36, nb), cx.st, a);
             else TIMED_LAUNCH("fourier_dft", 0.0, by, fdft_kernel<float>, gd, 192, 0, cx.st, a);
         }
     }
@@ -816,17 +872,18 @@ void fourier_solve(const std::vector<FourierJob>& jobs, const MixedCtx& cx) {
         const int nth = jobs[i0].ft->nth;
         set_tw(a, nth);
         const double by = dft_bytes(i0, a.n, false);
-        const dim3 gs(maxnc, a.n), bs(192);
-        const size_t sm = 0;
+        int nb = 0;
+        for (int q = 0; q < a.n; ++q) nb = std::max(nb, a.j[q].nb);
+        const dim3 gs(maxnc, a.n), bs(idft_threads(nb));
         if (out64) {
-            if (nth == 24) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_nth<24, double>), gs, bs, sm, cx.st, a);
-            else if (nth == 30) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_nth<30, double>), gs, bs, sm, cx.st, a);
-            else if (nth == 36) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_nth<36, double>), gs, bs, sm, cx.st, a);
+            if (nth == 24) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_rep<24, double>), gs, bs, dft_smem(24, nb), cx.st, a);
+            else if (nth == 30) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_rep<30, double>), gs, bs, dft_smem(30, nb), cx.st, a);
+            else if (nth == 36) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_rep<36, double>), gs, bs, dft_smem(36, nb), cx.st, a);
             else TIMED_LAUNCH("fourier_dft", 0.0, by, idft_kernel<double>, dim3(maxnc, a.n), 64, 0, cx.st, a);
         } else {
-            if (nth == 24) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_nth<24, float>), gs, bs, sm, cx.st, a);
-            else if (nth == 30) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_nth<30, float>), gs, bs, sm, cx.st, a);
-            else if (nth == 36) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_nth<36, float>), gs, bs, sm, cx.st, a);
+            if (nth == 24) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_rep<24, float>), gs, bs, dft_smem(24, nb), cx.st, a);
+            else if (nth == 30) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_rep<30, float>), gs, bs, dft_smem(30, nb), cx.st, a);
+            else if (nth == 36) TIMED_LAUNCH("fourier_dft", 0.0, by, (idft_rep<36, float>), gs, bs, dft_smem(36, nb), cx.st, a);
             else TIMED_LAUNCH("fourier_dft", 0.0, by, idft_kernel<float>, dim3(maxnc, a.n), 64, 0, cx.st, a);
         }
     }
