@@ -8,10 +8,10 @@
 #include <cmath>
 #include <cstdlib>
 #include <map>
-#include <mutex>
 #include <vector>
 
 #include "common.cuh"
+#include "packed.cuh"
 #include "tc_gemm.cuh"
 #include "tube_fourier.cuh"
 
@@ -79,16 +79,20 @@ __global__ void chat_kernel(const __grid_constant__ ChatArgs args) {
 }
 
 // ---------------------------------------------------------------- inversion
-// In-place Gauss-Jordan inversion with partial pivoting of one n x n complex
-// block per cluster of CL CTAs: CTA q holds columns [q w, q w + w) in its
-// shared memory.  Step k: the CTA owning column k finds the pivot row p (largest
-// |a_ik|, i >= k) and writes p and the column into every CTA's shared memory
-// (double-buffered, so one cluster barrier per step suffices); every CTA swaps
-// rows k and p, scales row k by 1 / a_pk and eliminates column k from the other
-// rows of its own columns; column k itself becomes column k of the inverse.  The
-// row exchanges are undone as column exchanges in reverse order when the
-// columns are written back.  A zero pivot sets bit 1 of *flag.
-constexpr int GJ_THREADS = 512;
+// In-place Gauss-Jordan inversion with partial pivoting of one n x n complex block per
+// cluster of CL CTAs.  The block lives in registers: CTA q holds the columns
+// [q w, q w + w), warp v of it the columns q w + v + 16 j (j < CJ), lane l the rows
+// l + 32 i (i < RI).  Rows are not exchanged: the pivot row of step k is the row p_k with the
+// largest |a_ik| among those that have not been one, and the permutation is applied when the
+// inverse is written, A^-1[k, p_j] = a[p_k, j].
+//   Step k: column k and p_k come from the shared memory of the CTA, where the warp that holds
+// the column has put them in every CTA of the cluster; each warp passes its part of row p_k
+// around through shared memory and eliminates column k from its own columns.  The warp that
+// holds column k + 1 eliminates that one first, finds p_{k+1} and sends both off before it goes
+// on, so that the exchange runs during the elimination.  A zero pivot sets bit 1 of *flag.
+//   With the block in shared memory every step read and wrote all of it there (1900 clocks at
+// 128 bytes per clock for n = 174 in two CTAs, against 500 of FP32 arithmetic).
+constexpr int GJ_WARPS = 16, GJ_THREADS = 32 * GJ_WARPS;
 constexpr int GJ_MAXB = 1024;
 struct GjArgs {
     int n, w, nblk;
@@ -96,114 +100,216 @@ struct GjArgs {
     float2* C[GJ_MAXB];
 };
 
-template <int CL>
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// (re, im) -= (mr, mi) r for two rows; a negated half rounds like the product it replaces
+__device__ __forceinline__ void eliminate(uint64_t& re, uint64_t& im, uint64_t mr, uint64_t mi, float2 r) {
+    const uint64_t rx = pack2(r.x, r.x), ry = pack2(r.y, r.y), nry = pack2(-r.y, -r.y);
+    re = sub2(re, fma2(mr, rx, mul2(mi, nry)));
+    im = sub2(im, fma2(mr, ry, mul2(mi, rx)));
+}
+
+template <int RI, int CJ, int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(GJ_THREADS, 1) gj_kernel(const __grid_constant__ GjArgs args) {
     cg::cluster_group cl = cg::this_cluster();
-    extern __shared__ float2 gsm[];
-    const int n = args.n, w = args.w;
-    const int rank = (int)cl.block_rank();
-    const int blk = blockIdx.x / CL;
-    float2* A = gsm;                          // n x w, column-major, leading dimension n
-    float2* colk = gsm + (size_t)n * w;       // 2 x n: the pivot column of the step (double-buffered)
-    int* meta = reinterpret_cast<int*>(colk + 2 * n);  // [2]: pivot row per buffer (-1: zero pivot)
-    int* piv = meta + 2;                      // n: pivot row of every step
-    int* pos = piv + n;                       // n: output column of every stored column
-    float2* mk = reinterpret_cast<float2*>(pos + n);  // n: multipliers of the step (2 + 2 n ints: 8-byte aligned)
+    constexpr int RP = RI / 2, NR = 32 * RI;
+    __shared__ float2 colk[2][NR];           // column k, double-buffered
+    __shared__ int meta[2];                  // p_k (-1: zero pivot)
+    __shared__ float2 rowk[GJ_WARPS][CJ];    // a warp's part of row p_k
+    __shared__ int piv[NR], pos[NR];         // p_k, and its inverse
+    const int n = args.n, w = args.w, rank = (int)cl.block_rank();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c0 = rank * w, wl = max(0, min(w, n - c0));
-    float2* C = blk < args.nblk ? args.C[blk] : nullptr;
-    if (C)
-        for (int e = threadIdx.x; e < n * wl; e += blockDim.x) A[e] = C[(long long)c0 * n + e];
-    cl.sync();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    float2* const C = args.C[blockIdx.x / CL];
+    // packed by pairs of rows: lane + 64 i and lane + 64 i + 32
+    uint64_t re[RP][CJ], im[RP][CJ];
+    unsigned done = 0;  // bit i: row lane + 32 i has been a pivot row (or is past the block)
+#pragma unroll
+    for (int i = 0; i < RP; ++i) {
+        const int r = lane + 64 * i;
+        if (r >= n) done |= 1u << 2 * i;
+        if (r + 32 >= n) done |= 2u << 2 * i;
+#pragma unroll
+        for (int j = 0; j < CJ; ++j) {
+            const int c = warp + GJ_WARPS * j;
+            const float2* const src = C + (long long)(c0 + c) * n + r;
+            const float2 x = r < n && c < wl ? src[0] : make_float2(0.f, 0.f);
+            const float2 y = r + 32 < n && c < wl ? src[32] : make_float2(0.f, 0.f);
+            re[i][j] = pack2(x.x, y.x);
+            im[i][j] = pack2(x.y, y.y);
+        }
+    }
+    // column k (this lane's rows) and its pivot row into every CTA; by the whole warp that holds it
+    const auto publish = [&](int k, const uint64_t (&vr)[RP], const uint64_t (&vi)[RP]) {
+        float2 v[2 * RP];
+#pragma unroll
+        for (int i = 0; i < RP; ++i) {
+            const float2 x = unpack2(vr[i]), y = unpack2(vi[i]);
+            v[2 * i] = make_float2(x.x, y.x);
+            v[2 * i + 1] = make_float2(x.y, y.y);
+        }
+        unsigned best = 0;
+        unsigned mag[2 * RP];
+#pragma unroll
+        for (int i = 0; i < 2 * RP; ++i) {
+            const float m = v[i].x * v[i].x + v[i].y * v[i].y;
+            mag[i] = (done >> i & 1) || !(m > 0.f) ? 0u : __float_as_uint(m);
+            best = max(best, mag[i]);
+        }
+        best = __reduce_max_sync(0xffffffffu, best);
+        unsigned row = 0x7fffffffu;
+#pragma unroll
+        for (int i = 2 * RP - 1; i >= 0; --i)
+            if (mag[i] == best) row = lane + 32 * i;
+        row = __reduce_min_sync(0xffffffffu, row);
+#pragma unroll
+        for (int q = 0; q < CL; ++q) {
+            float2* const dst = cl.map_shared_rank(&colk[k & 1][0], q);
+#pragma unroll
+            for (int i = 0; i < 2 * RP; ++i) dst[lane + 32 * i] = v[i];
+        }
+        if (lane < CL) *cl.map_shared_rank(&meta[k & 1], lane) = best ? (int)row : -1;
+    };
+    cl.sync();  // every CTA of the cluster runs before its shared memory is written
+    if (rank == 0 && warp == 0) {
+        uint64_t vr[RP], vi[RP];
+#pragma unroll
+        for (int i = 0; i < RP; ++i) {
+            vr[i] = re[i][0];
+            vi[i] = im[i][0];
+        }
+        publish(0, vr, vi);
+    }
+    cluster_arrive();
     bool bad = false;
     for (int k = 0; k < n; ++k) {
-        const int buf = k & 1;
-        if (rank == k / w) {
-            const float2* ca = A + (size_t)(k - c0) * n;
-            // every thread copies a share of the column into every CTA; warp 0 also
-            // finds the pivot row
-            for (int e = threadIdx.x; e < CL * n; e += blockDim.x) {
-                const int q = e / n, i = e - q * n;
-                cl.map_shared_rank(colk, q)[buf * n + i] = ca[i];
-            }
-            if (warp == 0) {
-                float best = -1.f;
-                int bi = k;
-                for (int i = k + lane; i < n; i += 32) {
-                    const float2 v = ca[i];
-                    const float m = v.x * v.x + v.y * v.y;
-                    if (m > best) { best = m; bi = i; }
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                    if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-                }
-                if (lane < CL) cl.map_shared_rank(meta, lane)[buf] = best > 0.f ? bi : -1;
-            }
-        }
-        cl.sync();
-        const int p = meta[buf];
+        cluster_wait();
+        const int p = meta[k & 1];
         if (p < 0) { bad = true; break; }  // the same in every CTA of the cluster
+        const int lp = p & 31, ip = p >> 5;
+        const float2 pv = colk[k & 1][p];
+        uint64_t mr[RP], mi[RP];
+#pragma unroll
+        for (int i = 0; i < RP; ++i) {
+            const float2 x = colk[k & 1][lane + 64 * i], y = colk[k & 1][lane + 64 * i + 32];
+            mr[i] = pack2(x.x, y.x);
+            mi[i] = pack2(x.y, y.y);
+        }
         if (threadIdx.x == 0) piv[k] = p;
-        const float2* ck = colk + buf * n;  // column k before the exchange
-        const float2 pv = ck[p];
         const float s2 = 1.f / (pv.x * pv.x + pv.y * pv.y);
         const float2 d = make_float2(pv.x * s2, -pv.y * s2);  // 1 / pivot
-        // the multipliers after the exchange, row k's set to zero
-        for (int i = threadIdx.x; i < n; i += blockDim.x) mk[i] = i == k ? make_float2(0.f, 0.f) : ck[i == p ? k : i];
-        // exchange rows k and p and scale the new row k (one lane per column)
-        for (int jl = threadIdx.x; jl < wl; jl += blockDim.x) {
-            float2* col = A + (size_t)jl * n;
-            const float2 vk = col[k], vp = col[p];
-            col[p] = vk;
-            col[k] = c0 + jl == k ? d : cmul(vp, d);
-        }
-        __syncthreads();
-        // eliminate: column j -= m * (row k), row k itself untouched (m_k = 0);
-        // column k of the inverse: -m_i / pivot (row k: 1 / pivot)
-        for (int jl = warp; jl < wl; jl += nw) {
-            float2* col = A + (size_t)jl * n;
-            if (c0 + jl == k) {
-                for (int i = lane; i < n; i += 32)
-                    if (i != k) {
-                        const float2 t = cmul(mk[i], d);
-                        col[i] = make_float2(-t.x, -t.y);
-                    }
-            } else {
-                const float2 rk = col[k];
-                for (int i = lane; i < n; i += 32) {
-                    const float2 m = mk[i], c = col[i];
-                    col[i] = make_float2(c.x - (m.x * rk.x - m.y * rk.y), c.y - (m.x * rk.y + m.y * rk.x));
+        // column k of the inverse: -m_i / pivot, and 1 / pivot in row p: the elimination of zeros
+        const int own = k - c0, j0 = own >= 0 && own < wl && (own & (GJ_WARPS - 1)) == warp ? own / GJ_WARPS : -1;
+        if (j0 >= 0) {
+#pragma unroll
+            for (int j = 0; j < CJ; ++j)
+                if (j == j0) {
+#pragma unroll
+                    for (int i = 0; i < RP; ++i) re[i][j] = im[i][j] = 0;
                 }
-            }
         }
-        __syncthreads();
+        if (lane == lp) {
+#pragma unroll
+            for (int h = 0; h < 2 * RP; ++h)
+                if (h == ip) {
+                    const int i = h >> 1, odd = h & 1;
+#pragma unroll
+                    for (int j = 0; j < CJ; ++j) {
+                        const float2 x = unpack2(re[i][j]), y = unpack2(im[i][j]);
+                        float2 r = cmul(odd ? make_float2(x.y, y.y) : make_float2(x.x, y.x), d);
+                        if (j == j0) r = d;
+                        re[i][j] = odd ? pack2(x.x, r.x) : pack2(r.x, x.y);
+                        im[i][j] = odd ? pack2(y.x, r.y) : pack2(r.y, y.y);
+                        rowk[warp][j] = r;
+                    }
+                    const float2 x = unpack2(mr[i]), y = unpack2(mi[i]);
+                    mr[i] = odd ? pack2(x.x, 0.f) : pack2(0.f, x.y);
+                    mi[i] = odd ? pack2(y.x, 0.f) : pack2(0.f, y.y);
+                }
+            done |= 1u << ip;
+        }
+        __syncwarp();
+        if (k + 1 < n) {
+            const int nx = k + 1 - c0;
+            if (nx >= 0 && nx < wl && (nx & (GJ_WARPS - 1)) == warp) {
+                const int j1 = nx / GJ_WARPS;
+                const float2 rk = rowk[warp][j1];
+                uint64_t vr[RP], vi[RP];
+#pragma unroll
+                for (int j = 0; j < CJ; ++j)
+                    if (j == j1) {
+#pragma unroll
+                        for (int i = 0; i < RP; ++i) {
+                            vr[i] = re[i][j];
+                            vi[i] = im[i][j];
+                        }
+                    }
+#pragma unroll
+                for (int i = 0; i < RP; ++i) eliminate(vr[i], vi[i], mr[i], mi[i], rk);
+                publish(k + 1, vr, vi);
+            }
+            // this step's column has been read, the next one's sent: buffer k & 1 is free for k + 2
+            cluster_arrive();
+        }
+#pragma unroll
+        for (int j = 0; j < CJ; ++j) {
+            const float2 rk = rowk[warp][j];
+#pragma unroll
+            for (int i = 0; i < RP; ++i) eliminate(re[i][j], im[i][j], mr[i], mi[i], rk);
+        }
+        __syncwarp();  // rowk is written again in the next step
     }
     if (bad) {
         if (threadIdx.x == 0 && rank == 0) atomicOr(args.flag, 2);
         return;
     }
-    if (threadIdx.x == 0) {
-        // stored column cur[c] is output column c: the exchanges (k, piv[k]) in reverse order
-        int* cur = pos;  // built in place, then inverted below through colk's space
-        for (int c = 0; c < n; ++c) cur[c] = c;
-        for (int k = n - 1; k >= 0; --k) {
-            const int p = piv[k];
-            if (p != k) { const int t = cur[k]; cur[k] = cur[p]; cur[p] = t; }
-        }
-        int* inv = reinterpret_cast<int*>(colk);  // the pivot columns are no longer needed
-        for (int c = 0; c < n; ++c) inv[cur[c]] = c;
-        for (int c = 0; c < n; ++c) pos[c] = inv[c];
-    }
     __syncthreads();
-    if (C)
-        for (int jl = warp; jl < wl; jl += nw) {
-            float2* dst = C + (long long)pos[c0 + jl] * n;
-            const float2* src = A + (size_t)jl * n;
-            for (int i = lane; i < n; i += 32) dst[i] = src[i];
+    for (int k = threadIdx.x; k < n; k += GJ_THREADS) pos[piv[k]] = k;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < CJ; ++j) {
+        const int c = warp + GJ_WARPS * j;
+        if (c >= wl) continue;
+        float2* const dst = C + (long long)piv[c0 + c] * n;
+#pragma unroll
+        for (int i = 0; i < RP; ++i) {
+            const float2 x = unpack2(re[i][j]), y = unpack2(im[i][j]);
+            const int r = lane + 64 * i;
+            if (r < n) dst[pos[r]] = make_float2(x.x, y.x);
+            if (r + 32 < n) dst[pos[r + 32]] = make_float2(x.y, y.y);
         }
+    }
+}
+
+// Columns per CTA and CTAs per block for n <= 256: a thread's part of the block has to stay
+// in its registers (at most 36 complex entries).  One tube's blocks (13 for 24 sectors) go to
+// clusters of eight, which still leave SMs free.
+struct GjShape {
+    int ri, cl;
+};
+GjShape gj_shape(int n, int nblk) {
+    const int ri = n <= 128 ? 4 : n <= 192 ? 6 : 8;
+    return {ri, nblk * 8 <= 152 ? 8 : ri == 8 ? 4 : 2};
+}
+
+void launch_gj(GjArgs& g, cudaStream_t st) {
+    if (g.n > 256) fail(SQBEM_ERR_ARG, "Gauss-Jordan: block order %d too large", g.n);
+    const GjShape s = gj_shape(g.n, g.nblk);
+    g.w = (g.n + s.cl - 1) / s.cl;
+    // credited: 8 n^3 FP32 flops per complex inversion; bytes: the block read and written
+    const double fl = 8.0 * g.nblk * (double)g.n * g.n * g.n, by = 16.0 * g.nblk * (double)g.n * g.n;
+    const int grid = s.cl * g.nblk;
+#define GJ_LAUNCH(RI, CJ, CL) TIMED_LAUNCH("fourier_inverse", fl, by, (gj_kernel<RI, CJ, CL>), grid, GJ_THREADS, 0, st, g)
+    if (s.ri == 4 && s.cl == 8) GJ_LAUNCH(4, 1, 8);
+    else if (s.ri == 4) GJ_LAUNCH(4, 4, 2);
+    else if (s.ri == 6 && s.cl == 8) GJ_LAUNCH(6, 2, 8);
+    else if (s.ri == 6) GJ_LAUNCH(6, 6, 2);
+    else if (s.cl == 8) GJ_LAUNCH(8, 2, 8);
+    else GJ_LAUNCH(8, 4, 4);
+#undef GJ_LAUNCH
 }
 
 // The real form [[Re, -Im], [Im, Re]] of every inverse (n x n complex,
@@ -614,61 +720,20 @@ __global__ void chat_nth(const __grid_constant__ ChatArgs args, const __grid_con
     for (int f = 0; f < NF; ++f) J.C[(long long)f * n3 * n3 + (long long)c * n3 + r] = make_float2(re[f], im[f]);
 }
 
-int gj_cluster(int n, int nblk = 1 << 20) {
-    // one tube's blocks (13 for 24 sectors): eight CTAs each still leave SMs free, and a step's
-    // elimination is a quarter as long
-    if (nblk * 8 <= 152) return 8;
-    // shared memory of one CTA: its columns, two pivot columns and the index
-    // arrays; two CTAs per block where they fit (measured faster than four)
-    for (int cl : {2, 4}) {
-        const int w = (n + cl - 1) / cl;
-        const size_t bytes = (size_t)n * w * sizeof(float2) + 3 * n * sizeof(float2) + (2 + 2 * n) * sizeof(int);
-        if (bytes <= 220 * 1024) return cl;
-    }
-    return 0;
-}
-
-size_t gj_smem(int n, int cl) {
-    const int w = (n + cl - 1) / cl;
-    return (size_t)n * w * sizeof(float2) + 3 * n * sizeof(float2) + (2 + 2 * n) * sizeof(int);
-}
-
-// The dynamic shared memory limits of the kernels that need more than 48 KB, set
-// once per process to the largest size any launch asks for: concurrent host
-// threads launch blocks of different orders, and a per-launch setting could
-// lower the limit between another thread's setting and its launch.
-constexpr int FT_SMEM_MAX = 220 * 1024;
-void set_smem_limits() {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        CUDA_CHECK(cudaFuncSetAttribute(gj_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_MAX));
-        CUDA_CHECK(cudaFuncSetAttribute(gj_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_MAX));
-        CUDA_CHECK(cudaFuncSetAttribute(gj_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM_MAX));
-    });
-}
-
 }  // namespace
 
 bool fourier_supported(const TubeSymmetry& sym) {
-    return sym.ok && sym.nth >= 2 && sym.nth <= FT_MAX_SECTORS && 3 * sym.nb <= FT_MAX_ORDER &&
-           gj_cluster(3 * sym.nb) > 0;
+    return sym.ok && sym.nth >= 2 && sym.nth <= FT_MAX_SECTORS && 3 * sym.nb <= FT_MAX_ORDER;
 }
 
 void gauss_jordan_blocks(float2* C, int nblk, int n3, int* flag, cudaStream_t st) {
-    const int cl = gj_cluster(n3, nblk);
-    if (!cl) fail(SQBEM_ERR_ARG, "Gauss-Jordan: block order %d too large", n3);
-    set_smem_limits();
     for (int b0 = 0; b0 < nblk; b0 += GJ_MAXB) {
         GjArgs g;
         g.n = n3;
-        g.w = (n3 + cl - 1) / cl;
         g.nblk = std::min(GJ_MAXB, nblk - b0);
         g.flag = flag;
         for (int b = 0; b < g.nblk; ++b) g.C[b] = C + (size_t)(b0 + b) * n3 * n3;
-        const double fl = 8.0 * g.nblk * (double)n3 * n3 * n3, by = 16.0 * g.nblk * (double)n3 * n3;
-        if (cl == 8) TIMED_LAUNCH("fourier_inverse", fl, by, gj_kernel<8>, 8 * g.nblk, GJ_THREADS, gj_smem(n3, cl), st, g);
-        else if (cl == 2) TIMED_LAUNCH("fourier_inverse", fl, by, gj_kernel<2>, 2 * g.nblk, GJ_THREADS, gj_smem(n3, cl), st, g);
-        else TIMED_LAUNCH("fourier_inverse", fl, by, gj_kernel<4>, 4 * g.nblk, GJ_THREADS, gj_smem(n3, cl), st, g);
+        launch_gj(g, st);
     }
 }
 
@@ -723,12 +788,9 @@ void fourier_build(const std::vector<FourierTube*>& fts, const std::vector<const
             else TIMED_LAUNCH("fourier_inverse", 0.0, cby, chat_kernel, cg3, 64, 0, cx.st, a);
         }
         const int nblk_all = (int)(ids.size() * nf);
-        const int cl = gj_cluster(n3, nblk_all);
-        const size_t smem = gj_smem(n3, cl);
         for (int b0 = 0; b0 < nblk_all; b0 += GJ_MAXB) {
             GjArgs g;
             g.n = n3;
-            g.w = (n3 + cl - 1) / cl;
             g.nblk = std::min(GJ_MAXB, nblk_all - b0);
             g.flag = cx.flag;
             RfArgs r;
@@ -744,12 +806,7 @@ void fourier_build(const std::vector<FourierTube*>& fts, const std::vector<const
                 r.lo[b] = fts[k]->Al.get() + (size_t)f * fts[k]->m2 * fts[k]->ldk;
                 r.ldk = fts[k]->ldk;
             }
-            // credited: 8 n^3 FP32 flops per complex inversion; bytes: the block read and written
-            const double gfl = 8.0 * g.nblk * (double)n3 * n3 * n3, gby = 16.0 * g.nblk * (double)n3 * n3;
-            set_smem_limits();
-            if (cl == 8) TIMED_LAUNCH("fourier_inverse", gfl, gby, gj_kernel<8>, 8 * g.nblk, GJ_THREADS, smem, cx.st, g);
-            else if (cl == 2) TIMED_LAUNCH("fourier_inverse", gfl, gby, gj_kernel<2>, 2 * g.nblk, GJ_THREADS, smem, cx.st, g);
-            else TIMED_LAUNCH("fourier_inverse", gfl, gby, gj_kernel<4>, 4 * g.nblk, GJ_THREADS, smem, cx.st, g);
+            launch_gj(g, cx.st);
             const int t = ceil_div(2 * n3, 32);
             TIMED_LAUNCH("fourier_inverse", 0.0, g.nblk * (8.0 * n3 * n3 + 16.0 * n3 * n3), realform_kernel,
                          dim3(t, t, g.nblk), dim3(32, 8), 0, cx.st, r);

@@ -126,3 +126,22 @@ def test_concurrent_chunks_match_sequential(monkeypatch):
         for _ in range(2):
             r3, _ = sqbem.kinematics_batch(insts, prec)
             np.testing.assert_array_equal(r3[:, :12], r1[:, :12])
+
+
+# Orders of the tube's Fourier blocks on both sides of the inversion's register shapes (128,
+# 192, 256 rows), as four tubes' 28 blocks (two or four CTAs each) and as one tube's 7 (eight)
+@pytest.mark.parametrize("order,L,nr", [(54, 2.5, 1), (126, 9.0, 1), (186, 12.0, 4), (198, 13.5, 4), (246, 16.5, 6)])
+def test_fourier_block_inverses_at_their_orders(monkeypatch, order, L, nr):
+    rng = np.random.default_rng(order)
+    insts = [dict(a_over_R=0.5, beta=float(b), L_over_R=L, e=(0.6, 0.0, 0.8), n_theta=12, n_r=nr, sphere_level=1,
+                  towed=0) for b in rng.uniform(0.0, 0.3, 4)]
+    r64, _ = sqbem.kinematics_batch(insts, sqbem.FP64)
+    assert r64[0, 13] == 4 * order  # panels: twelve sectors of order / 3
+    rmx, _ = sqbem.kinematics_batch(insts, sqbem.MIXED)
+    one, _ = sqbem.kinematics_batch(insts[:1], sqbem.MIXED)
+    assert np.all(uo_err(rmx, r64) < 1e-6) and np.all(uo_err(one, r64[:1]) < 1e-6)
+    # an inverse that is a little off shows in the refinement: no more than one step past those
+    # of the tensor-core LU of the whole tube block
+    monkeypatch.setenv("SQBEM_TUBE_FOURIER", "0")
+    lu, _ = sqbem.kinematics_batch(insts, sqbem.MIXED)
+    assert np.all(rmx[:, 15] <= lu[:, 15] + 1) and np.all(one[:, 15] <= lu[:1, 15] + 1)
