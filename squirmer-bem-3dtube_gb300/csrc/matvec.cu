@@ -18,6 +18,8 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <map>
+#include <tuple>
 
 #include "common.cuh"
 #include "matvec.cuh"
@@ -276,6 +278,76 @@ __global__ void __launch_bounds__(MV_ROWS) mv_plain2(const __grid_constant__ MvA
         }
 }
 
+// PLAIN for MEM members of one matrix (the swimmers of an ensemble in one tube): every element is
+// read once for their 2 MEM columns.  mv_plain2 read the matrix, which fits L2, once per member.
+// 48 products of 3888 x 3888: 270 -> 144 us, now bound by the loads of x from shared memory
+// (a 16-byte load per two packed multiply-adds; the multiply-adds take 38 us).  Rows 2t and 2t + 1
+// are the halves of packed operands, each rounded as there, in the same order.
+template <int MEM>
+__global__ void __launch_bounds__(MV_ROWS) mv_plain_shared(const __grid_constant__ MvArgs args,
+                                                           double* __restrict__ part) {
+    constexpr int NB = 8, COLS = 2 * MEM;
+    static_assert(MV_CHUNK % NB == 0, "matvec chunk must be a multiple of the load batch");
+    // (x, x) of two neighbouring columns, the column pairs of one j side by side
+    __shared__ ulonglong2 xs[MV_CHUNK][MEM];
+    const int jb = blockIdx.z * MEM, nm = min(MEM, args.n - jb), c = blockIdx.y;
+    const MvJob& J = args.j[jb].j;
+    const float* __restrict__ A = J.A32;
+    const long long lda = J.lda;
+    const int m = J.m, n = J.n;
+    const int j0 = c * MV_CHUNK, nj = min(n, j0 + MV_CHUNK) - j0;
+#pragma unroll
+    for (int q = 0; q < MEM; ++q)
+        for (int j = threadIdx.x; j < MV_CHUNK; j += MV_ROWS) {
+            float x0 = 0.f, x1 = 0.f;
+            if (q < nm && j < nj) {
+                const MvJob& K = args.j[jb + q].j;
+                x0 = (float)K.x[j0 + j];
+                if (K.r > 1) x1 = (float)K.x[j0 + j + K.ldx];
+            }
+            xs[j][q] = make_ulonglong2(pack2(x0, x0), pack2(x1, x1));
+        }
+    __syncthreads();
+    const int row = 2 * (blockIdx.x * MV_ROWS + threadIdx.x);
+    if (row >= m) return;
+    const bool two = row + 1 < m;
+    uint64_t s[COLS];
+#pragma unroll
+    for (int k = 0; k < COLS; ++k) s[k] = 0;
+    const float* a = A + row + (long long)j0 * lda;
+    for (int j = 0; j < nj; j += NB) {
+        uint64_t av[NB];
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+            const float* p = a + (long long)(j + u) * lda;
+            const float2 q = j + u < nj ? (two ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(__ldg(p), 0.f))
+                                        : make_float2(0.f, 0.f);
+            av[u] = pack2(q.x, q.y);
+        }
+#pragma unroll
+        for (int u = 0; u < NB; ++u)
+#pragma unroll
+            for (int q = 0; q < MEM; ++q) {
+                const ulonglong2 x = xs[j + u][q];
+                s[2 * q] = fma2(av[u], x.x, s[2 * q]);
+                s[2 * q + 1] = fma2(av[u], x.y, s[2 * q + 1]);
+            }
+    }
+#pragma unroll
+    for (int q = 0; q < MEM; ++q) {
+        if (q >= nm) break;
+        const MvDev& D = args.j[jb + q];
+        double* o = part + D.part_off + ((long long)c * m + row) * D.rstride;
+        const float2 v0 = unpack2(s[2 * q]), v1 = unpack2(s[2 * q + 1]);
+        o[0] = (double)v0.x;
+        if (D.j.r > 1) o[1] = (double)v1.x;
+        if (two) {
+            o[D.rstride] = (double)v0.y;
+            if (D.j.r > 1) o[D.rstride + 1] = (double)v1.y;
+        }
+    }
+}
+
 template <int R>
 __global__ void __launch_bounds__(MV_ROWS) mv_partial(const __grid_constant__ MvArgs args, double* __restrict__ part) {
     const MvDev& D = args.j[blockIdx.z];
@@ -523,7 +595,8 @@ __global__ void sumsq_kernel(const __grid_constant__ NormArgs args) {
 static void matvec_launches(const std::vector<MvJob>& jobs, cudaStream_t st);
 
 // Compensated FP32, plain FP32 and FP64 jobs go to separate launches: one job
-// of another kind would move the whole launch onto its kernel.
+// of another kind would move the whole launch onto its kernel.  So do plain jobs
+// on the same matrix, which mv_plain_shared then reads once for several of them.
 void matvec_group(const std::vector<MvJob>& jobs_in, cudaStream_t st) {
     std::vector<MvJob> j32, j32p, j64;
     for (const MvJob& j : jobs_in)
@@ -532,7 +605,15 @@ void matvec_group(const std::vector<MvJob>& jobs_in, cudaStream_t st) {
             (j.A32 ? (j.plain ? j32p : j32) : j64).push_back(j);
         }
     matvec_launches(j32, st);
-    matvec_launches(j32p, st);
+    std::map<std::tuple<const float*, long long, int, int>, std::vector<MvJob>> by;
+    const auto key = [](const MvJob& j) { return std::make_tuple(j.A32, j.lda, j.m, j.n); };
+    for (const MvJob& j : j32p) by[key(j)].push_back(j);
+    std::vector<MvJob> one;
+    for (const MvJob& j : j32p)
+        if (by[key(j)].size() == 1) one.push_back(j);
+    for (const auto& kv : by)
+        if (kv.second.size() > 1) matvec_launches(kv.second, st);
+    matvec_launches(one, st);
     matvec_launches(j64, st);
 }
 
@@ -573,10 +654,19 @@ static void matvec_launches(const std::vector<MvJob>& jobs, cudaStream_t st) {
         for (int k = 0; k < a.n && pairs_ok; ++k)
             pairs_ok = a.j[k].j.A32 && ((uintptr_t)a.j[k].j.A32 % 8 == 0) && a.j[k].j.lda % 2 == 0;
         const dim3 g2(ceil_div(maxm, 2 * MV_ROWS), maxc, (unsigned)a.n);
+        // one matrix for every job of the launch
+        bool shared = a.n > 1;
+        for (int k = 1; k < a.n && shared; ++k)
+            shared = a.j[k].j.A32 == a.j[0].j.A32 && a.j[k].j.lda == a.j[0].j.lda && a.j[k].j.m == maxm &&
+                     a.j[0].j.m == maxm && a.j[k].j.n == a.j[0].j.n;
         if (few) {
             const dim3 g(1, maxc, (unsigned)a.n);
             if (maxr <= 2) TIMED_LAUNCH("matvec", 0.0, bytes, mv_few<2>, g, 32 * MV_FEW_WARPS, 0, st, a, part.get());
             else TIMED_LAUNCH("matvec", 0.0, bytes, mv_few<MV_RMAX>, g, 32 * MV_FEW_WARPS, 0, st, a, part.get());
+        } else if (plain && pairs_ok && maxr <= 2 && shared) {
+            const dim3 g(g2.x, maxc, (unsigned)ceil_div(a.n, a.n <= 4 ? 4 : 8));
+            if (a.n <= 4) TIMED_LAUNCH("matvec", 0.0, bytes, mv_plain_shared<4>, g, MV_ROWS, 0, st, a, part.get());
+            else TIMED_LAUNCH("matvec", 0.0, bytes, mv_plain_shared<8>, g, MV_ROWS, 0, st, a, part.get());
         } else if (plain && pairs_ok && maxr <= 2) {
             TIMED_LAUNCH("matvec", 0.0, bytes, mv_plain2<2>, g2, MV_ROWS, 0, st, a, part.get());
         } else if (plain) {
