@@ -118,17 +118,24 @@ struct DiagJob {
 };
 
 constexpr int DIAG_THREADS = 512;
-constexpr int DP = MX_NB + 1;  // padded row of the shared block
+constexpr int DP = MX_NB + 4;  // padded row of the shared block (16-byte aligned)
 
-__device__ __forceinline__ void put_split(bf16* h, bf16* l, long long i, float x) {
-    const bf16 a = __float2bfloat16_rn(x);
-    h[i] = a;
-    l[i] = __float2bfloat16_rn(x - __bfloat162float(a));
+// two neighbouring values as split BF16
+__device__ __forceinline__ void put_split2(bf16* h, bf16* l, long long i, float x, float y) {
+    const bf16 a = __float2bfloat16_rn(x), b = __float2bfloat16_rn(y);
+    *reinterpret_cast<__nv_bfloat162*>(h + i) = __halves2bfloat162(a, b);
+    *reinterpret_cast<__nv_bfloat162*>(l + i) =
+        __halves2bfloat162(__float2bfloat16_rn(x - __bfloat162float(a)), __float2bfloat16_rn(y - __bfloat162float(b)));
+}
+
+__device__ __forceinline__ void get4(float (&v)[4], const float* p) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
 }
 
 // LU of the block without exchanges, flagging |l| > 1 (bit 0) and a zero or
 // non-finite pivot (bit 1); then L^{-1} and U^{-1}.  The whole block lives in
-// shared memory (with both inverses: 3 x 128 x 129 floats).
+// shared memory with both inverses.
 //
 // LU, blocked right-looking with 16-column panels:
 //   diag    warp 0 factors the 16 x 16 diagonal block, a row per lane, the
@@ -140,9 +147,13 @@ __device__ __forceinline__ void put_split(bf16* h, bf16* l, long long i, float x
 //   U12     at the same time, by other threads: one column per thread solves
 //           with the unit-lower 16 x 16 block, the column in registers;
 //   A22     rank-16 update in 4 x 4 register tiles: a warp takes 4 rows, a lane
-//           4 columns 32 apart (conflict-free loads of the U12 row, broadcasts
-//           of the L21 column), half a shared load per multiply-add.
-// Inverses: blocked by 16 with 4 x 4 register tiles (see below).
+//           4 columns 32 apart.  Warp 0 updates the next diagonal block and factors it
+//           meanwhile (one after the other, the eight diagonal blocks took 1900 clocks each).
+// Inverses: blocked by 16 with 4 x 4 register tiles (see below), four k per shared load (one k per
+// load and the diagonal blocks in turn: 72 us per block, now 52).
+// CL = 2, for up to DG_PAIR blocks: a cluster of two CTAs per block, which both factor it and
+// form one inverse each: 45 us.  Many blocks stay on one: their other streams lack the SMs
+// (256 members in groups of 48: 186.5 ms, with pairs 188.6).
 struct DiagArgs {
     int* flag;
     DiagJob j[MAXJOBS];
@@ -150,306 +161,317 @@ struct DiagArgs {
 
 constexpr int DG_PW = 16;  // LU panel width
 
-__global__ void __launch_bounds__(DIAG_THREADS) diag_kernel(const __grid_constant__ DiagArgs args) {
-    extern __shared__ float sh[];
-    constexpr int N = MX_NB;
+constexpr int DG_PAIR = 16;
+
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(DIAG_THREADS) diag_kernel(const __grid_constant__ DiagArgs args) {
+    extern __shared__ __align__(16) float sh[];
+    constexpr int N = MX_NB, B = DG_PW, NBK = N / B;
     float(*a)[DP] = reinterpret_cast<float(*)[DP]>(sh);
-    float(*xl)[DP] = reinterpret_cast<float(*)[DP]>(sh + N * DP);
-    float(*xu)[DP] = reinterpret_cast<float(*)[DP]>(sh + 2 * N * DP);
-    float* rd = sh + 3 * N * DP;  // 1 / U(r, r)
-    float(*tl)[DP] = reinterpret_cast<float(*)[DP]>(sh + 3 * N * DP + N);            // 16 x N scratch (L^{-1})
-    float(*tu)[DP] = reinterpret_cast<float(*)[DP]>(sh + 3 * N * DP + N + DG_PW * DP);  // 16 x N scratch (U^{-1})
-    const DiagJob& J = args.j[blockIdx.x];
-    const int tid = threadIdx.x;
-    {
-        const float* A = J.A;
-        const long long lda = J.lda;
-        for (int e = tid; e < N * N; e += DIAG_THREADS) a[e % N][e / N] = A[(e % N) + (e / N) * lda];
-    }
+    float* rd = sh + 3 * N * DP + 2 * B * DP;  // 1 / U(r, r)
+    cg::cluster_group cl = cg::this_cluster();
+    const DiagJob& J = args.j[blockIdx.x / CL];
+    const int part = CL == 2 ? (int)cl.block_rank() : 0;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const long long lda = J.lda;
+#pragma unroll 16
+    for (int e = tid; e < N * N; e += DIAG_THREADS) a[e % N][e / N] = J.A[(e % N) + (e / N) * lda];
+    if (CL == 2) cl.barrier_arrive();  // J.A is overwritten when both CTAs have read it
     __syncthreads();
     int bad = 0;
-    __shared__ float rinv[DG_PW];  // 1 / U(j, j) of the current panel
-    for (int c0 = 0; c0 < N; c0 += DG_PW) {
-        if (tid < 32) {
-            // the 16 x 16 diagonal block by warp 0: lane t keeps row c0 + t in
-            // registers; the pivot row travels by shuffles (no barrier)
-            const int t = tid;
-            float row[DG_PW];
+    __shared__ float rinv[B];  // 1 / U(j, j) of the current panel
+    // the 16 x 16 diagonal block by one warp: lane t keeps row c0 + t in registers; the pivot
+    // row travels by shuffles (no barrier)
+    const auto factor = [&](int c0) {
+        const int t = lane;
+        float row[B];
 #pragma unroll
-            for (int cc = 0; cc < DG_PW; ++cc) row[cc] = t < DG_PW ? a[c0 + t][c0 + cc] : 0.f;
+        for (int cc = 0; cc < B; ++cc) row[cc] = t < B ? a[c0 + t][c0 + cc] : 0.f;
 #pragma unroll
-            for (int jj = 0; jj < DG_PW; ++jj) {
-                const float piv = __shfl_sync(0xffffffffu, row[jj], jj);
-                if (t == 0 && !(piv != 0.f && isfinite(piv))) bad |= 2;
-                const float rp = 1.f / piv;
-                float pr[DG_PW];
+        for (int jj = 0; jj < B; ++jj) {
+            const float piv = __shfl_sync(0xffffffffu, row[jj], jj);
+            if (t == 0 && !(piv != 0.f && isfinite(piv))) bad |= 2;
+            const float rp = 1.f / piv;
+            float pr[B];
 #pragma unroll
-                for (int cc = jj + 1; cc < DG_PW; ++cc) pr[cc] = __shfl_sync(0xffffffffu, row[cc], jj);
-                if (t > jj && t < DG_PW) {
-                    const float rj = row[jj];
-                    const float l = rj * rp;
-                    if (!(fabsf(rj) <= fabsf(piv))) bad |= isfinite(l) ? 1 : 2;
+            for (int cc = jj + 1; cc < B; ++cc) pr[cc] = __shfl_sync(0xffffffffu, row[cc], jj);
+            if (t > jj && t < B) {
+                const float rj = row[jj];
+                const float l = rj * rp;
+                if (!(fabsf(rj) <= fabsf(piv))) bad |= isfinite(l) ? 1 : 2;
 #pragma unroll
-                    for (int cc = jj + 1; cc < DG_PW; ++cc) row[cc] = fmaf(-l, pr[cc], row[cc]);
-                    row[jj] = l;
-                }
-            }
-            if (t < DG_PW) {
-                float d = row[0];
-#pragma unroll
-                for (int cc = 0; cc < DG_PW; ++cc) {
-                    a[c0 + t][c0 + cc] = row[cc];
-                    if (cc == t) d = row[cc];
-                }
-                rinv[t] = 1.f / d;
+                for (int cc = jj + 1; cc < B; ++cc) row[cc] = fmaf(-l, pr[cc], row[cc]);
+                row[jj] = l;
             }
         }
-        __syncthreads();
+        if (t < B) {
+            float d = row[0];
+#pragma unroll
+            for (int cc = 0; cc < B; ++cc) {
+                a[c0 + t][c0 + cc] = row[cc];
+                if (cc == t) d = row[cc];
+            }
+            rinv[t] = 1.f / d;
+        }
+    };
+    if (warp == 0) factor(0);
+    __syncthreads();
+    for (int c0 = 0; c0 + B < N; c0 += B) {
+        const int c1 = c0 + B, m = N - c1;
         if (tid < 128) {
             // L21: rows below the block, one per thread, independent of each other:
-            // l_ij = (a_ij - sum_{k<j} l_ik U_kj) / U_jj, certified |numerator| <= |U_jj|
-            const int i = c0 + DG_PW + tid;
+            // l_ij = (a_ij - sum_{k<j} l_ik U_kj) / U_jj, certified |numerator| <= |U_jj|;
+            // column by column, so that the sums of a row advance side by side
+            const int i = c1 + tid;
             if (i < N) {
-                float x[DG_PW];
+                float v[B];
 #pragma unroll
-                for (int j = 0; j < DG_PW; ++j) x[j] = a[i][c0 + j];
+                for (int j = 0; j < B; ++j) v[j] = a[i][c0 + j];
 #pragma unroll
-                for (int j = 0; j < DG_PW; ++j) {
+                for (int k = 0; k < B; ++k) {
+                    const float u = a[c0 + k][c0 + k];
+                    const float l = v[k] * rinv[k];
+                    if (!(fabsf(v[k]) <= fabsf(u))) bad |= isfinite(l) ? 1 : 2;
+                    v[k] = l;
 #pragma unroll
-                    for (int k = 0; k < j; ++k) x[j] = fmaf(-x[k], a[c0 + k][c0 + j], x[j]);
-                    const float u = a[c0 + j][c0 + j];
-                    const float l = x[j] * rinv[j];
-                    if (!(fabsf(x[j]) <= fabsf(u))) bad |= isfinite(l) ? 1 : 2;
-                    x[j] = l;
+                    for (int j = k + 1; j < B; ++j) v[j] = fmaf(-l, a[c0 + k][c0 + j], v[j]);
                 }
 #pragma unroll
-                for (int j = 0; j < DG_PW; ++j) a[i][c0 + j] = x[j];
+                for (int j = 0; j < B; ++j) a[i][c0 + j] = v[j];
             }
         } else if (tid < 256) {
             // U12 = L11^{-1} A12 at the same time, one column per thread, in registers
-            const int c = c0 + DG_PW + (tid - 128);
+            const int c = c1 + (tid - 128);
             if (c < N) {
-                float x[DG_PW];
+                float v[B];
 #pragma unroll
-                for (int r = 0; r < DG_PW; ++r) x[r] = a[c0 + r][c];
+                for (int r = 0; r < B; ++r) v[r] = a[c0 + r][c];
 #pragma unroll
-                for (int r = 1; r < DG_PW; ++r)
+                for (int k = 0; k < B; ++k)
 #pragma unroll
-                    for (int k = 0; k < r; ++k) x[r] = fmaf(-a[c0 + r][c0 + k], x[k], x[r]);
+                    for (int r = k + 1; r < B; ++r) v[r] = fmaf(-a[c0 + r][c0 + k], v[k], v[r]);
 #pragma unroll
-                for (int r = 1; r < DG_PW; ++r) a[c0 + r][c] = x[r];
+                for (int r = 1; r < B; ++r) a[c0 + r][c] = v[r];
             }
         }
         __syncthreads();
-        {  // A22 -= L21 U12 in 4 x 4 tiles: rows i0 .. i0 + 3 per warp, columns c1 + lane + 32 p
-            const int m = N - c0 - DG_PW, c1 = c0 + DG_PW;
-            const int warp = tid >> 5, lane = tid & 31;
-            for (int g = warp; g < m / 4; g += DIAG_THREADS / 32) {
-                const int i0 = c1 + 4 * g;
+        // A22 -= L21 U12
+        if (warp == 0) {
+            // the next diagonal block: row c1 + lane / 2, eight columns
+            const int i = c1 + (lane >> 1), cb = c1 + 8 * (lane & 1);
+            float acc[2][4];
+            get4(acc[0], &a[i][cb]);
+            get4(acc[1], &a[i][cb + 4]);
+#pragma unroll
+            for (int k = 0; k < B; k += 4) {
+                float lv[4];
+                get4(lv, &a[i][c0 + k]);
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float uv[4];
+                        get4(uv, &a[c0 + k + s][cb + 4 * h]);
+#pragma unroll
+                        for (int p = 0; p < 4; ++p) acc[h][p] = fmaf(-lv[s], uv[p], acc[h][p]);
+                    }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int p = 0; p < 4; ++p) a[i][cb + 4 * h + p] = acc[h][p];
+            __syncwarp();
+            factor(c1);
+        } else {
+            // the rest: rows i0 .. i0 + 3 per warp, columns c1 + lane + 32 p
+            for (int g = warp - 1; g < m / 4; g += DIAG_THREADS / 32 - 1) {
+                const int i0 = c1 + 4 * g, lo = g < B / 4 ? c1 + B : c1;  // first column that is not warp 0's
                 float acc[4][4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
 #pragma unroll
                     for (int p = 0; p < 4; ++p) {
                         const int c = c1 + lane + 32 * p;
-                        acc[q][p] = c < N ? a[i0 + q][c] : 0.f;
+                        acc[q][p] = c >= lo && c < N ? a[i0 + q][c] : 0.f;
                     }
 #pragma unroll
-                for (int k = 0; k < DG_PW; ++k) {
-                    float lv[4], uv[4];
+                for (int k = 0; k < B; k += 4) {
+                    float lv[4][4];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) lv[q] = a[i0 + q][c0 + k];
+                    for (int q = 0; q < 4; ++q) get4(lv[q], &a[i0 + q][c0 + k]);
 #pragma unroll
-                    for (int p = 0; p < 4; ++p) {
-                        const int c = c1 + lane + 32 * p;
-                        uv[p] = c < N ? a[c0 + k][c] : 0.f;
+                    for (int s = 0; s < 4; ++s) {
+                        float uv[4];
+#pragma unroll
+                        for (int p = 0; p < 4; ++p) {
+                            const int c = c1 + lane + 32 * p;
+                            uv[p] = c < N ? a[c0 + k + s][c] : 0.f;
+                        }
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+#pragma unroll
+                            for (int p = 0; p < 4; ++p) acc[q][p] = fmaf(-lv[q][s], uv[p], acc[q][p]);
                     }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-#pragma unroll
-                        for (int p = 0; p < 4; ++p) acc[q][p] = fmaf(-lv[q], uv[p], acc[q][p]);
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
 #pragma unroll
                     for (int p = 0; p < 4; ++p) {
                         const int c = c1 + lane + 32 * p;
-                        if (c < N) a[i0 + q][c] = acc[q][p];
+                        if (c >= lo && c < N) a[i0 + q][c] = acc[q][p];
                     }
             }
         }
         __syncthreads();
     }
     if (bad) atomicOr(args.flag, bad);
+    if (CL == 2) cl.barrier_wait();
     {
         float* A = J.A;
-        const long long lda = J.lda;
-        for (int e = tid; e < N * N; e += DIAG_THREADS) A[(e % N) + (e / N) * lda] = a[e % N][e / N];
+        const int h = part * (N / 2);  // first of this CTA's columns
+#pragma unroll 4
+        for (int e = tid; e < N * N / CL; e += DIAG_THREADS) A[(e % N) + (h + e / N) * lda] = a[e % N][h + e / N];
     }
-    for (int r = tid; r < N; r += DIAG_THREADS) rd[r] = 1.f / a[r][r];
-    __syncthreads();
-    for (int e = tid; e < N * N; e += DIAG_THREADS) {
-        const int r = e % N, c = e / N;
-        xl[r][c] = r == c ? 1.f : 0.f;
-        xu[r][c] = r == c ? rd[r] : 0.f;
-    }
+    if (tid < N) rd[tid] = 1.f / a[tid][tid];
+    for (int e = tid; e < 2 * N * N; e += DIAG_THREADS) sh[N * DP + (e / N) * DP + e % N] = 0.f;
     __syncthreads();
     // Inverses, blocked by 16: first the 16 x 16 diagonal blocks (a thread per
     // block column), then one block row at a time as two small GEMMs with 4 x 4
-    // register tiles (half a shared load per FMA instead of two):
+    // register tiles:
     //   L^{-1}: X_ij = -X_ii sum_{j <= k < i} L_ik X_kj      (block rows ascending)
     //   U^{-1}: X_ij = -X_ii sum_{i < k <= j} U_ik X_kj      (block rows descending)
-    // threads 0-255 form L^{-1}, 256-511 U^{-1}, each half with its own named barrier.
-    constexpr int B = DG_PW, NBK = N / DG_PW;
-    if (tid < N) {
-        const int blk = tid / B, c = tid % B, C = B * blk + c;
-        for (int r = c + 1; r < B; ++r) {
-            float v = 0.f;
-            for (int k = c; k < r; ++k) v = fmaf(a[B * blk + r][B * blk + k], xl[B * blk + k][C], v);
-            xl[B * blk + r][C] = -v;
+    // by four warps each, with a barrier of their own.
+    if (tid < 2 * N / CL) {
+        const bool upper = CL == 2 ? part == 1 : tid >= N;
+        const int u = tid & (N - 1), blk = u / B, c = u % B, C = B * blk + c;
+        float(*x)[DP] = reinterpret_cast<float(*)[DP]>(sh + (upper ? 2 : 1) * N * DP);
+        float(*tt)[DP] = reinterpret_cast<float(*)[DP]>(sh + 3 * N * DP + (upper ? B * DP : 0));  // 16 x N scratch
+        const auto sync = [&] {
+            if (upper) asm volatile("bar.sync 2, 128;" ::: "memory");
+            else asm volatile("bar.sync 1, 128;" ::: "memory");
+        };
+        float v[B];
+        if (!upper) {
+#pragma unroll
+            for (int r = 0; r < B; ++r) v[r] = 0.f;
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                v[k] = k == c ? 1.f : k < c ? 0.f : -v[k];
+#pragma unroll
+                for (int r = k + 1; r < B; ++r) v[r] = fmaf(a[B * blk + r][B * blk + k], v[k], v[r]);
+            }
+        } else {
+#pragma unroll
+            for (int r = B - 1; r >= 0; --r) {
+                float w = 0.f;
+#pragma unroll
+                for (int k = r + 1; k < B; ++k) w = fmaf(a[B * blk + r][B * blk + k], v[k], w);
+                v[r] = r == c ? rd[B * blk + r] : r > c ? 0.f : -w * rd[B * blk + r];
+            }
         }
-    } else if (tid >= 2 * N && tid < 3 * N) {
-        const int blk = (tid - 2 * N) / B, c = (tid - 2 * N) % B, C = B * blk + c;
-        for (int r = c - 1; r >= 0; --r) {
-            float v = 0.f;
-            for (int k = r + 1; k <= c; ++k) v = fmaf(a[B * blk + r][B * blk + k], xu[B * blk + k][C], v);
-            xu[B * blk + r][C] = -v * rd[B * blk + r];
-        }
-    }
-    __syncthreads();
-    if (tid < 2 * N) {
-        const int t = tid, tr = t % 4, tc = t / 4;
-        for (int i = 1; i < NBK; ++i) {
-            const bool act = t < B * i;  // 16 i tiles of 4 x 4 over the 16 x 16 i block row
+#pragma unroll
+        for (int r = 0; r < B; ++r) x[B * blk + r][C] = v[r];
+        sync();
+        const int tr = u % 4, tc = u / 4;
+        for (int s = 1; s < NBK; ++s) {
+            const int i = upper ? NBK - 1 - s : s;
+            const bool act = u < B * s;  // 16 s tiles of 4 x 4 over the 16 x 16 s block row
+            const int col0 = (upper ? B * (i + 1) : 0) + 4 * tc;
+            const int k0 = upper ? B * (i + 1) : B * (col0 / B), k1 = upper ? B * (col0 / B) + B : B * i;
             float acc[4][4];
             if (act) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
 #pragma unroll
                     for (int p = 0; p < 4; ++p) acc[q][p] = 0.f;
-                for (int k = B * ((4 * tc) / B); k < B * i; ++k) {
-                    float av[4], xv[4];
+#pragma unroll 2
+                for (int k = k0; k < k1; k += 4) {
+                    float av[4][4], xv[4][4];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) av[q] = a[B * i + 4 * tr + q][k];
+                    for (int q = 0; q < 4; ++q) get4(av[q], &a[B * i + 4 * tr + q][k]);
 #pragma unroll
-                    for (int p = 0; p < 4; ++p) xv[p] = xl[k][4 * tc + p];
+                    for (int t = 0; t < 4; ++t) get4(xv[t], &x[k + t][col0]);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
+                    for (int t = 0; t < 4; ++t)
 #pragma unroll
-                        for (int p = 0; p < 4; ++p) acc[q][p] = fmaf(av[q], xv[p], acc[q][p]);
+                        for (int q = 0; q < 4; ++q)
+#pragma unroll
+                            for (int p = 0; p < 4; ++p) acc[q][p] = fmaf(av[q][t], xv[t][p], acc[q][p]);
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) tl[4 * tr + q][4 * tc + p] = acc[q][p];
+                    *reinterpret_cast<float4*>(&tt[4 * tr + q][col0]) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
             }
-            asm volatile("bar.sync 2, 256;" ::: "memory");
+            sync();
             if (act) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
 #pragma unroll
                     for (int p = 0; p < 4; ++p) acc[q][p] = 0.f;
-#pragma unroll 4
-                for (int s2 = 0; s2 < B; ++s2) {
-                    float av[4], xv[4];
+#pragma unroll 2
+                for (int k = 0; k < B; k += 4) {
+                    float av[4][4], xv[4][4];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) av[q] = xl[B * i + 4 * tr + q][B * i + s2];
+                    for (int q = 0; q < 4; ++q) get4(av[q], &x[B * i + 4 * tr + q][B * i + k]);
 #pragma unroll
-                    for (int p = 0; p < 4; ++p) xv[p] = tl[s2][4 * tc + p];
+                    for (int t = 0; t < 4; ++t) get4(xv[t], &tt[k + t][col0]);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
+                    for (int t = 0; t < 4; ++t)
 #pragma unroll
-                        for (int p = 0; p < 4; ++p) acc[q][p] = fmaf(av[q], xv[p], acc[q][p]);
+                        for (int q = 0; q < 4; ++q)
+#pragma unroll
+                            for (int p = 0; p < 4; ++p) acc[q][p] = fmaf(av[q][t], xv[t][p], acc[q][p]);
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) xl[B * i + 4 * tr + q][4 * tc + p] = -acc[q][p];
+                    *reinterpret_cast<float4*>(&x[B * i + 4 * tr + q][col0]) =
+                        make_float4(-acc[q][0], -acc[q][1], -acc[q][2], -acc[q][3]);
             }
-            asm volatile("bar.sync 2, 256;" ::: "memory");
-        }
-    } else {
-        const int t = tid - 2 * N, tr = t % 4, tc = t / 4;
-        for (int i = NBK - 2; i >= 0; --i) {
-            const int ncol = N - B * (i + 1);
-            const bool act = t < ncol;  // ncol tiles of 4 x 4 over the 16 x ncol block row
-            const int col0 = B * (i + 1) + 4 * tc;
-            float acc[4][4];
-            if (act) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) acc[q][p] = 0.f;
-                for (int k = B * (i + 1); k < B * (col0 / B) + B; ++k) {
-                    float av[4], xv[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) av[q] = a[B * i + 4 * tr + q][k];
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) xv[p] = xu[k][col0 + p];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-#pragma unroll
-                        for (int p = 0; p < 4; ++p) acc[q][p] = fmaf(av[q], xv[p], acc[q][p]);
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) tu[4 * tr + q][col0 + p] = acc[q][p];
-            }
-            asm volatile("bar.sync 3, 256;" ::: "memory");
-            if (act) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) acc[q][p] = 0.f;
-#pragma unroll 4
-                for (int s2 = 0; s2 < B; ++s2) {
-                    float av[4], xv[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) av[q] = xu[B * i + 4 * tr + q][B * i + s2];
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) xv[p] = tu[s2][col0 + p];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-#pragma unroll
-                        for (int p = 0; p < 4; ++p) acc[q][p] = fmaf(av[q], xv[p], acc[q][p]);
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) xu[B * i + 4 * tr + q][col0 + p] = -acc[q][p];
-            }
-            asm volatile("bar.sync 3, 256;" ::: "memory");
+            sync();
         }
     }
     __syncthreads();
-    for (int e = tid; e < N * N; e += DIAG_THREADS) {
-        const int r = e % N, c = e / N;
-        J.Li[r + c * N] = xl[r][c];
-        J.Ui[r + c * N] = xu[r][c];
-        put_split(J.UiCh, J.UiCl, (long long)c * N + r, xu[r][c]);
-        put_split(J.LiCh, J.LiCl, (long long)c * N + r, xl[r][c]);
-    }
-    for (int e = tid; e < N * N; e += DIAG_THREADS) {
-        const int r = e / N, c = e % N;  // row-major: consecutive threads along a row
-        put_split(J.LiRh, J.LiRl, (long long)r * N + c, xl[r][c]);
-        put_split(J.UiRh, J.UiRl, (long long)r * N + c, xu[r][c]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (CL == 2 && h != part) continue;
+        float(*x)[DP] = reinterpret_cast<float(*)[DP]>(sh + (1 + h) * N * DP);
+        float* const F = h ? J.Ui : J.Li;
+        bf16 *const Ch = h ? J.UiCh : J.LiCh, *const Cl = h ? J.UiCl : J.LiCl;
+        bf16 *const Rh = h ? J.UiRh : J.LiRh, *const Rl = h ? J.UiRl : J.LiRl;
+        // column-major: two rows of four columns per thread, a warp 64 rows
+        for (int e = tid; e < N * N / 8; e += DIAG_THREADS) {
+            const int r = 2 * (e % (N / 2)), c = 4 * (e / (N / 2));
+            float u[4], v[4];
+            get4(u, &x[r][c]);
+            get4(v, &x[r + 1][c]);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                *reinterpret_cast<float2*>(F + r + (c + p) * N) = make_float2(u[p], v[p]);
+                put_split2(Ch, Cl, (long long)(c + p) * N + r, u[p], v[p]);
+            }
+        }
+        for (int e = tid; e < N * N / 2; e += DIAG_THREADS) {
+            const int r = e / (N / 2), c = 2 * (e % (N / 2));  // row-major: consecutive threads along a row
+            put_split2(Rh, Rl, (long long)r * N + c, x[r][c], x[r][c + 1]);
+        }
     }
 }
 
-constexpr int DIAG_SMEM = (3 * MX_NB * DP + MX_NB + 2 * DG_PW * DP) * (int)sizeof(float);
+constexpr int DIAG_SMEM = (3 * MX_NB * DP + 2 * DG_PW * DP + MX_NB) * (int)sizeof(float);
 
 void diag_group(const std::vector<DiagJob>& jobs, const MixedCtx& cx) {
     static std::once_flag attr;
     std::call_once(attr, [] {
-        CUDA_CHECK(cudaFuncSetAttribute(diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DIAG_SMEM));
+        CUDA_CHECK(cudaFuncSetAttribute(diag_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, DIAG_SMEM));
+        CUDA_CHECK(cudaFuncSetAttribute(diag_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, DIAG_SMEM));
     });
     for (size_t i0 = 0; i0 < jobs.size(); i0 += MAXJOBS) {
         DiagArgs a;
         a.flag = cx.flag;
         const int n = (int)std::min<size_t>(MAXJOBS, jobs.size() - i0);
         for (int k = 0; k < n; ++k) a.j[k] = jobs[i0 + k];
-        TIMED_LAUNCH("lu_diag", 0.0, 0.0, diag_kernel, n, DIAG_THREADS, DIAG_SMEM, cx.st, a);
+        if (n <= DG_PAIR) TIMED_LAUNCH("lu_diag", 0.0, 0.0, diag_kernel<2>, 2 * n, DIAG_THREADS, DIAG_SMEM, cx.st, a);
+        else TIMED_LAUNCH("lu_diag", 0.0, 0.0, diag_kernel<1>, n, DIAG_THREADS, DIAG_SMEM, cx.st, a);
     }
 }
 
