@@ -727,11 +727,52 @@ __global__ void __launch_bounds__(256) conv_direct_kernel(const __grid_constant_
     *reinterpret_cast<uint2*>(J.lo + o) = lv;
 }
 
+// Column-major FP32 -> row-major split with even, 4-byte aligned rows: 64 columns x 32 rows per
+// CTA, two neighbouring columns per store.  conv_kernel's 2-byte stores wrote 64 bytes per warp
+// and kept four loads in flight per thread: 3.9 TB/s; now 6.1 (48 blocks of 960 x 3888: 361 -> 235 us).
+constexpr int CT_C = 64;
+__global__ void __launch_bounds__(256) conv_transpose_kernel(const __grid_constant__ ConvArgs args) {
+    __shared__ float tile[CV_T][CT_C + 1];  // [row in tile][column in tile]
+    const ConvJob& J = args.j[blockIdx.y];
+    const int rows = J.rows, cols = J.cols;
+    const int ntr = (rows + CV_T - 1) / CV_T, ntc = (cols + CT_C - 1) / CT_C;
+    const int t = blockIdx.x;
+    if (t >= ntr * ntc) return;
+    const int r0 = (t % ntr) * CV_T, c0 = (t / ntr) * CT_C;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float v[CT_C / 8];
+#pragma unroll
+    for (int k = 0; k < CT_C / 8; ++k) {
+        const int r = r0 + lane, c = c0 + w + 8 * k;
+        v[k] = r < rows && c < cols ? __ldg(J.src + r + (long long)c * J.s_cs) : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < CT_C / 8; ++k) tile[lane][w + 8 * k] = v[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < CV_T; k += 8) {
+        const int r = r0 + w + k, c = c0 + 2 * lane;
+        if (r >= rows || c >= cols) continue;
+        const float x = tile[w + k][2 * lane], y = tile[w + k][2 * lane + 1];
+        const long long o = (long long)r * J.d_rs + c;
+        if (c + 1 < cols) {
+            put_split2(J.hi, J.lo, o, x, y);
+        } else {
+            const bf16 h = __float2bfloat16_rn(x);
+            J.hi[o] = h;
+            J.lo[o] = __float2bfloat16_rn(x - __bfloat162float(h));
+        }
+    }
+}
+
 namespace {
 bool direct_ok(const ConvJob& j) {
     return j.s_rs == 1 && j.d_rs == 1 && j.rows % 4 == 0 && j.s_cs % 4 == 0 && j.d_cs % 4 == 0 &&
            ((uintptr_t)j.src & 15) == 0 && ((uintptr_t)j.hi & 7) == 0 && ((uintptr_t)j.lo & 7) == 0 &&
            (long long)(j.rows / 4) * j.cols <= 0x7fffffffLL;
+}
+bool transpose_ok(const ConvJob& j) {
+    return j.s_rs == 1 && j.d_cs == 1 && j.d_rs % 2 == 0 && ((uintptr_t)j.hi & 3) == 0 && ((uintptr_t)j.lo & 3) == 0;
 }
 }  // namespace
 
@@ -740,15 +781,17 @@ void convert_group(const std::vector<ConvJob>& jobs, cudaStream_t st) {
     for (size_t i0 = 0; i0 < jobs.size(); i0 += MAXJOBS) {
         ConvArgs a;
         a.n = (int)std::min<size_t>(MAXJOBS, jobs.size() - i0);
-        long long mx = 0, mxd = 0;
+        long long mx = 0, mxd = 0, mxt = 0;
         double bytes = 0;
-        bool direct = true;
+        bool direct = true, transpose = true;
         for (int k = 0; k < a.n; ++k) {
             a.j[k] = jobs[i0 + k];
             const long long tiles = (long long)((a.j[k].rows + CV_T - 1) / CV_T) * ((a.j[k].cols + CV_T - 1) / CV_T);
             mx = std::max(mx, tiles);
             mxd = std::max(mxd, (long long)(a.j[k].rows / 4) * a.j[k].cols);
+            mxt = std::max(mxt, (long long)((a.j[k].rows + CV_T - 1) / CV_T) * ((a.j[k].cols + CT_C - 1) / CT_C));
             direct = direct && direct_ok(a.j[k]);
+            transpose = transpose && transpose_ok(a.j[k]);
             bytes += 8.0 * a.j[k].rows * a.j[k].cols;  // FP32 read, two BF16 written
         }
         if (mx == 0) continue;
@@ -756,6 +799,8 @@ void convert_group(const std::vector<ConvJob>& jobs, cudaStream_t st) {
         if (direct)
             TIMED_LAUNCH("convert", 0.0, bytes, conv_direct_kernel, dim3((unsigned)ceil_div(mxd, 256), (unsigned)a.n),
                          256, 0, st, a);
+        else if (transpose)
+            TIMED_LAUNCH("convert", 0.0, bytes, conv_transpose_kernel, dim3((unsigned)mxt, (unsigned)a.n), 256, 0, st, a);
         else
             TIMED_LAUNCH("convert", 0.0, bytes, conv_kernel, dim3((unsigned)mx, (unsigned)a.n), dim3(CV_T, CV_RY), 0,
                          st, a);
