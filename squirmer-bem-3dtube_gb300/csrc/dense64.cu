@@ -5,7 +5,7 @@
 // GB300 executes FP64 at roughly 1 TFLOP/s (CUDA-core DFMA and DMMA alike).  Large
 // products therefore run as digit products on the BF16 tensor cores with FP64
 // results (oz_gemm.cu); what stays on the FP64 pipe is the work around them: the
-// 128-wide panels of the LU, and products with a few columns.
+// panels of the LU, and products with a few columns.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
