@@ -91,7 +91,9 @@ __global__ void chat_kernel(const __grid_constant__ ChatArgs args) {
 // holds column k + 1 eliminates that one first, finds p_{k+1} and sends both off before it goes
 // on, so that the exchange runs during the elimination.  A zero pivot sets bit 1 of *flag.
 //   With the block in shared memory every step read and wrote all of it there (1900 clocks at
-// 128 bytes per clock for n = 174 in two CTAs, against 500 of FP32 arithmetic).
+// 128 bytes per clock for n = 174 in two CTAs, against 500 of FP32 arithmetic).  Now the
+// exchange bounds a step (about 1 us): 277 blocks of order 162 .. 174 in two CTAs each
+// 1575 -> 739 us, one tube's 13 blocks in eight 324 -> 158 us.
 constexpr int GJ_WARPS = 16, GJ_THREADS = 32 * GJ_WARPS;
 constexpr int GJ_MAXB = 1024;
 struct GjArgs {
