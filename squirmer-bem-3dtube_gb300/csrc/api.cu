@@ -306,10 +306,8 @@ extern "C" int sqbem_gemm64(int route, int ta, int tb, int M, int N, int K, doub
         dC.upload(C, (size_t)ldc * N);
         WaitError we;
         if (route == 1) {
-            OzMat a, b;
-            a.split(dA.get(), ta ? lda : 1, ta ? 1 : lda, M, K, s);
-            b.split(dB.get(), tb ? 1 : ldb, tb ? ldb : 1, N, K, s, true);
-            oz_gemm(a, b, alpha, beta, dC.get(), ldc, we.get(s), s);
+            oz_product(dA.get(), ta ? lda : 1, ta ? 1 : lda, dB.get(), tb ? 1 : ldb, tb ? ldb : 1, M, N, K, alpha, beta,
+                       dC.get(), ldc, we.get(s), s);
         } else {
             gemm64(ta, tb, M, N, K, alpha, dA.get(), lda, dB.get(), ldb, beta, dC.get(), ldc, s,
                    route == 0 ? nullptr : we.get(s));

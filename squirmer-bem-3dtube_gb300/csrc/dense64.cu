@@ -273,7 +273,7 @@ void rigid64(int m, int np, const double* A, long long lda, const double* r, dou
                  ldc);
 }
 
-// The digit products need about 60 us whatever the size (two splits, a tile's 36
+// The digit products need about 65 us whatever the size (the scales, two splits, a tile's 36
 // products and read-outs), in which the FP64 pipe does 6e7 operations; and a tile of
 // 128 x 128 with a K below 64 costs more to read out than to multiply.
 static bool use_tensor(int M, int N, int K, const int* err) {
@@ -290,10 +290,7 @@ void gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const double* A
     }
     if (N <= SK_N && !tb) return gemm64_few(ta, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, st);
     if (use_tensor(M, N, K, err)) {
-        OzMat a, b;
-        a.split(A, ta ? lda : 1, ta ? 1 : lda, M, K, st);
-        b.split(B, tb ? 1 : ldb, tb ? ldb : 1, N, K, st, true);
-        oz_gemm(a, b, alpha, beta, C, ldc, err, st);
+        oz_product(A, ta ? lda : 1, ta ? 1 : lda, B, tb ? 1 : ldb, tb ? ldb : 1, M, N, K, alpha, beta, C, ldc, err, st);
         return;
     }
     dim3 grid(ceil_div(M, GB_M), ceil_div(N, GB_N));
@@ -743,13 +740,10 @@ __global__ void laswp_kernel(double* B, long long ldb, int n, int nrhs, const in
 }
 
 // ---------------------------------------------------------------- LU64
-// C = alpha (op A) B + beta C where the operands' digits serve once.
+// C = alpha A B + beta C (column-major) by digit products; q: K words of zeros
 static void tensor_product(const double* A, long long lda, const double* B, long long ldb, int M, int N, int K,
-                           double alpha, double beta, double* C, long long ldc, int* err, cudaStream_t st) {
-    OzMat a, b;
-    a.split(A, 1, lda, M, K, st);
-    b.split(B, ldb, 1, N, K, st, true);
-    oz_gemm(a, b, alpha, beta, C, ldc, err, st);
+                           double alpha, double beta, double* C, long long ldc, int* err, cudaStream_t st, int* q) {
+    oz_product(A, 1, lda, B, ldb, 1, M, N, K, alpha, beta, C, ldc, err, st, q);
 }
 
 // The panel of columns [k0, k0 + kb), kb <= HB, of the n x n matrix, all rows below.
@@ -768,14 +762,18 @@ static void factor_panel(double* A, long long ld, int n, int k0, int kb, int* fl
 // Panels of LU_NB = 256 columns, each as two of 128.  With 256 the trailing update's tiles
 // multiply for longer (18 us) than they take to read out, which 128 do not.
 static void run_fast(double* A, long long ld, int n, double* Linv, double* Uinv, int* flag, int* err, cudaStream_t st) {
+    // the scales of up to three products per panel
+    DevBuf<int> scales(3 * (size_t)LU_NB * ceil_div(n, LU_NB), st);
+    scales.zero();
     for (int k0 = 0, b = 0; k0 < n; k0 += LU_NB, ++b) {
         const int kb = std::min(LU_NB, n - k0), n2 = n - k0 - kb, h = std::min(HB, kb), h2 = kb - h;
         double* A11 = A + k0 + k0 * ld;
+        int* const q = scales.get() + 3 * (size_t)LU_NB * b;
         factor_panel(A, ld, n, k0, h, flag, st);
         if (h2 > 0) {
             double* right = A11 + h * ld;
             LAUNCH(lu_lower_kernel, ceil_div(h2, LOWER_C), HB, 0, st, A11, ld, h2);
-            tensor_product(A11 + h, ld, right, ld, n - k0 - h, h2, h, -1.0, 1.0, right + h, ld, err, st);
+            tensor_product(A11 + h, ld, right, ld, n - k0 - h, h2, h, -1.0, 1.0, right + h, ld, err, st, q);
             factor_panel(A, ld, n, k0 + h, h2, flag, st);
         }
         if (n2 == 0) break;
@@ -785,9 +783,9 @@ static void run_fast(double* A, long long ld, int n, double* Linv, double* Uinv,
         double* A22 = A + (k0 + kb) + (k0 + kb) * ld;
         // U12 = L11^{-1} A12
         LAUNCH(lu_inverse_kernel<1>, dim3(1, LU_NB), LU_NB, 0, st, A11, ld, kb, false, Li);
-        tensor_product(Li, LU_NB, A12, ld, kb, n2, kb, 1.0, 0.0, A12, ld, err, st);
+        tensor_product(Li, LU_NB, A12, ld, kb, n2, kb, 1.0, 0.0, A12, ld, err, st, q + LU_NB);
         // A22 -= L21 U12
-        tensor_product(A21, ld, A12, ld, n2, n2, kb, -1.0, 1.0, A22, ld, err, st);
+        tensor_product(A21, ld, A12, ld, n2, n2, kb, -1.0, 1.0, A22, ld, err, st, q + 2 * LU_NB);
     }
     // L^{-1} of the last block, and U^{-1} of all
     const int last = (n - 1) / LU_NB, k0 = last * LU_NB;
@@ -895,20 +893,27 @@ void LU64::solve(double* B, long long ldb, int nrhs, cudaStream_t st, int* err) 
     }
     // many: the block inverses and the updates as tensor-core products
     const int nblk = ceil_div(n, LU_NB);
+    DevBuf<int> scales(4 * (size_t)LU_NB * nblk, st);
+    scales.zero();
+    int* q = scales.get();
     for (int b = 0; b < nblk; ++b) {  // forward: unit lower L
         const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0), n2 = n - k0 - kb;
         tensor_product(Linv.get() + (long long)b * LU_NB * LU_NB, LU_NB, B + k0, ldb, kb, nrhs, kb, 1.0, 0.0, B + k0, ldb,
-                       err, st);
+                       err, st, q);
+        q += LU_NB;
         if (n2 > 0)
             tensor_product(A.get() + (k0 + kb) + k0 * ld, ld, B + k0, ldb, n2, nrhs, kb, -1.0, 1.0, B + k0 + kb, ldb, err,
-                           st);
+                           st, q);
+        q += LU_NB;
     }
     for (int b = nblk - 1; b >= 0; --b) {  // backward: U
         const int k0 = b * LU_NB, kb = std::min(LU_NB, n - k0);
         tensor_product(Uinv.get() + (long long)b * LU_NB * LU_NB, LU_NB, B + k0, ldb, kb, nrhs, kb, 1.0, 0.0, B + k0, ldb,
-                       err, st);
+                       err, st, q);
+        q += LU_NB;
         if (k0 > 0)
-            tensor_product(A.get() + k0 * ld, ld, B + k0, ldb, k0, nrhs, kb, -1.0, 1.0, B, ldb, err, st);
+            tensor_product(A.get() + k0 * ld, ld, B + k0, ldb, k0, nrhs, kb, -1.0, 1.0, B, ldb, err, st, q);
+        q += LU_NB;
     }
 }
 

@@ -65,54 +65,177 @@ struct OzTile {
 };
 
 // ---------------------------------------------------------------- digits
+// Exponents of rows as stored beside the digits: the largest e + EXB of a row, e the biased
+// exponent of a value after its scaling along k; 0 for a row of zeros.
+constexpr int EXB = 8192, SPECIAL = 1 << 20;  // SPECIAL: the row holds an infinity or a NaN
+// Scales along k: the largest (exponent of a value - largest of its column of B) + QB; 0: zeros
+constexpr int QB = 4096;
+
+// the biased exponent (1 for the subnormal numbers), 0 for zero, 0x7ff for an infinity or a NaN
+__device__ __forceinline__ int exponent_of(double x) {
+    const int hi = __double2hiint(x) & 0x7fffffff;
+    return hi >= 1 << 20 ? hi >> 20 : (hi | __double2loint(x)) != 0;
+}
+// + the shift of its k (below 0: dropped); 0 stays zero
+__device__ __forceinline__ int stored_exponent(double x, int shift) {
+    const int e = exponent_of(x);
+    return e == 0x7ff ? SPECIAL : e ? e + shift + EXB : 0;
+}
+// What the values at index k of an operand are shifted by: A (sign 1) down by as much as B
+// (sign -1) up, so that the largest values of every row of B are about the same.  Where B's row is
+// zero A's values do not matter, and DROP takes them below every other.
+constexpr int DROP = -(1 << 16);
+__device__ __forceinline__ int shift_at(const int* __restrict__ q, int k, int sign) {
+    const int v = q ? q[k] : QB;
+    return v ? sign * (v - QB) : sign > 0 ? DROP : 0;
+}
+
+// q[k] = the largest exponent of B's row k, each column taken relative to its own largest one (K
+// <= FUSED_K: 32 columns per CTA, their exponents in shared memory; columns with an infinity
+// or a NaN do not count).  Bound by the latency of its loads, hence eight in flight per thread:
+// 256 k x 3840 columns 6 us, 20 with one.
+constexpr int FUSED_K = 512, LOADS = 8;  // loads in flight per thread
+__global__ void __launch_bounds__(256) oz_scale_fused(const double* __restrict__ b, long long rs, long long ks, int rows,
+                                                      int k, int* __restrict__ q) {
+    extern __shared__ int xe[];  // [k][33]
+    __shared__ int em[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r0 = blockIdx.x * 32;
+    if (threadIdx.x < 32) em[lane] = 0;
+    __syncthreads();
+    if (ks == 1) {
+        for (int r = w; r < 32; r += 8) {
+            int m = 0;
+            for (int c0 = lane; c0 < k; c0 += 32 * LOADS) {
+                double x[LOADS];
+#pragma unroll
+                for (int u = 0; u < LOADS; ++u) x[u] = r0 + r < rows && c0 + 32 * u < k ? b[(r0 + r) * rs + c0 + 32 * u] : 0.0;
+#pragma unroll
+                for (int u = 0; u < LOADS; ++u) {
+                    const int e = exponent_of(x[u]);
+                    if (c0 + 32 * u < k) xe[(c0 + 32 * u) * 33 + r] = e;
+                    m = max(m, e);
+                }
+            }
+            m = __reduce_max_sync(0xffffffffu, m);
+            if (lane == 0) em[r] = m;
+        }
+    } else {
+        int m = 0;
+        for (int c0 = w; c0 < k; c0 += 8 * LOADS) {
+            double x[LOADS];
+#pragma unroll
+            for (int u = 0; u < LOADS; ++u) x[u] = r0 + lane < rows && c0 + 8 * u < k ? b[r0 + lane + (c0 + 8 * u) * ks] : 0.0;
+#pragma unroll
+            for (int u = 0; u < LOADS; ++u) {
+                const int e = exponent_of(x[u]);
+                if (c0 + 8 * u < k) xe[(c0 + 8 * u) * 33 + lane] = e;
+                m = max(m, e);
+            }
+        }
+        if (m) atomicMax(em + lane, m);
+    }
+    __syncthreads();
+    // a thread per k: its 32 columns
+    for (int c = threadIdx.x; c < k; c += 256) {
+        int m = 0;
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) {
+            const int e = xe[c * 33 + r], E = em[r];
+            m = max(m, e && E != 0x7ff ? e - E + QB : 0);
+        }
+        if (m) atomicMax(q + c, m);
+    }
+}
+
+// The same from the columns' exponents (unscaled, in ex): a thread per k and 32 columns where k is
+// contiguous, a thread per column and 32 k where the columns are.
+__global__ void __launch_bounds__(128) oz_scale(const double* __restrict__ b, long long rs, long long ks, int rows, int k,
+                                                const int* __restrict__ ex, int* __restrict__ q) {
+    if (ks == 1) {
+        const int c = blockIdx.x * 128 + threadIdx.x, r1 = min(rows, (int)(blockIdx.y + 1) * 32);
+        if (c >= k) return;
+        int m = 0;
+        for (int r0 = blockIdx.y * 32; r0 < r1; r0 += LOADS) {
+            double x[LOADS];
+#pragma unroll
+            for (int u = 0; u < LOADS; ++u) x[u] = r0 + u < r1 ? b[(r0 + u) * rs + c] : 0.0;
+#pragma unroll
+            for (int u = 0; u < LOADS; ++u) {
+                const int e = exponent_of(x[u]), E = r0 + u < r1 ? ex[r0 + u] : SPECIAL;
+                m = max(m, e && E != SPECIAL ? e + EXB - E + QB : 0);
+            }
+        }
+        if (m) atomicMax(q + c, m);
+    } else {
+        const int r = blockIdx.x * 128 + threadIdx.x, c1 = min(k, (int)(blockIdx.y + 1) * 32);
+        const int E = r < rows ? ex[r] : SPECIAL;
+#pragma unroll 4
+        for (int c = blockIdx.y * 32; c < c1; ++c) {
+            const int e = E != SPECIAL ? exponent_of(b[r * rs + c * ks]) : 0;
+            const int m = __reduce_max_sync(0xffffffffu, e ? e + EXB - E + QB : 0);
+            if ((threadIdx.x & 31) == 0 && m) atomicMax(q + c, m);
+        }
+    }
+}
+
 __global__ void oz_exponent_rows(const double* __restrict__ a, long long rs, long long ks, int rows, int k, int kper,
-                                 int* __restrict__ ex, long long bs, int eb) {
+                                 int* __restrict__ ex, long long bs, int eb, const int* __restrict__ q, int sign) {
     a += blockIdx.z * bs;
     ex += (long long)blockIdx.z * eb;
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows) return;
     const int c1 = min(k, (int)(blockIdx.y + 1) * kper);
     int m = 0;
-#pragma unroll 8
-    for (int c = blockIdx.y * kper; c < c1; ++c) m = max(m, __double2hiint(a[r * rs + c * ks]) & 0x7ff00000);
-    if (m) atomicMax(ex + r, m >> 20);
+    for (int c0 = blockIdx.y * kper; c0 < c1; c0 += LOADS) {
+        double x[LOADS];
+#pragma unroll
+        for (int u = 0; u < LOADS; ++u) x[u] = c0 + u < c1 ? a[r * rs + (c0 + u) * ks] : 0.0;
+#pragma unroll
+        for (int u = 0; u < LOADS; ++u) m = max(m, stored_exponent(x[u], c0 + u < c1 ? shift_at(q, c0 + u, sign) : 0));
+    }
+    if (m) atomicMax(ex + r, m);
 }
 
 // contiguous along k: a warp per row
 __global__ void oz_exponent_cols(const double* __restrict__ a, long long rs, int rows, int k, int* __restrict__ ex,
-                                 long long bs, int eb) {
+                                 long long bs, int eb, const int* __restrict__ q, int sign) {
     a += blockIdx.z * bs;
     ex += (long long)blockIdx.z * eb;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= rows) return;
     int m = 0;
-#pragma unroll 4
-    for (int c = lane; c < k; c += 32) m = max(m, __double2hiint(a[r * rs + c]) & 0x7ff00000);
+    for (int c0 = lane; c0 < k; c0 += 32 * LOADS) {
+        double x[LOADS];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) ex[r] = m >> 20;
+        for (int u = 0; u < LOADS; ++u) x[u] = c0 + 32 * u < k ? a[r * rs + c0 + 32 * u] : 0.0;
+#pragma unroll
+        for (int u = 0; u < LOADS; ++u)
+            m = max(m, stored_exponent(x[u], c0 + 32 * u < k ? shift_at(q, c0 + 32 * u, sign) : 0));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) ex[r] = m;
 }
 
-// x as a 64-bit fixed-point number in units of 2^(E - 1085), E the row's largest
-// biased exponent: |x| < 2^(E - 1022), so the magnitude stays below 2^63.
-__device__ __forceinline__ long long fixed64(double x, int E) {
+// x 2^shift as a 64-bit fixed-point number in units of 2^(E - EXB - 1085), E the row's stored
+// exponent: |x 2^shift| < 2^(E - EXB - 1022), so the magnitude stays below 2^63.
+__device__ __forceinline__ long long fixed64(double x, int shift, int E) {
     const long long b = __double_as_longlong(x);
     int e = (int)(b >> 52) & 0x7ff;
     unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
     if (e) m |= 1ull << 52;
     else e = 1;
     m <<= 10;
-    const int sh = max(E, 1) - e;
+    const int sh = E - (e + shift + EXB);
     if (sh > 0) m = sh > 63 ? 0 : (m + (1ull << (sh - 1))) >> sh;
     return b < 0 ? -(long long)m : (long long)m;
 }
 
 // The digits of eight values of one row: 16 bytes of each of the eight planes.
-__device__ __forceinline__ void store_digits(const double (&x)[8], int E, uint4* o, int digit) {
+__device__ __forceinline__ void store_digits(const double (&x)[8], const int (&shift)[8], int E, uint4* o, int digit) {
     uint32_t w[DIGITS][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        long long v = fixed64(x[j], E);
+        long long v = fixed64(x[j], shift[j], E);
 #pragma unroll
         for (int s = DIGITS - 1; s >= 0; --s) {
             int d;
@@ -143,19 +266,24 @@ __device__ __forceinline__ long long digit_at(int r, int kb, int h, int k16, int
 // grid.y strides over the k16 steps.
 __global__ void __launch_bounds__(256) oz_split(const double* __restrict__ a, long long rs, long long ks, int rows,
                                                 int k, int k16, const int* __restrict__ ex, uint4* __restrict__ out,
-                                                long long bs, int eb, int rb) {
+                                                long long bs, int eb, int rb, const int* __restrict__ q, int sign) {
     a += blockIdx.z * bs;
     ex += (long long)blockIdx.z * eb;
     out += (long long)blockIdx.z * (eb / TILE) * k16 * (BLOCK / 16);
     const int r = blockIdx.x * TILE + threadIdx.x;
     const int E = r < rows ? ex[r] : 0;
-    const bool ok = r < rows && E != 0x7ff;
+    const bool ok = r < rows && E != SPECIAL;
     for (int kb = blockIdx.y; kb < k16; kb += gridDim.y) {
         const int c0 = kb * 16 + threadIdx.y * 8;
         double x[8];
+        int sh[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = ok && c0 + j < k ? a[r * rs + (c0 + j) * ks] : 0.0;
-        store_digits(x, E, out + digit_at(r, kb, threadIdx.y, k16, rb), rb * 2);
+        for (int j = 0; j < 8; ++j) {
+            const bool in = ok && c0 + j < k;
+            x[j] = in ? a[r * rs + (c0 + j) * ks] : 0.0;
+            sh[j] = in ? shift_at(q, c0 + j, sign) : 0;
+        }
+        store_digits(x, sh, E, out + digit_at(r, kb, threadIdx.y, k16, rb), rb * 2);
     }
 }
 
@@ -163,48 +291,66 @@ __global__ void __launch_bounds__(256) oz_split(const double* __restrict__ a, lo
 // and solves): a CTA holds 32 rows' values of all k in shared memory, so each is read
 // from global memory once.  About 90 integer operations per value bound it: with 128
 // rows per CTA a 3840 x 128 panel sat on 30 SMs for 20 us.
-constexpr int FUSED_K = 512;
 constexpr int FUSED_SMEM = FUSED_K * 33 * 8;
 __global__ void __launch_bounds__(256) oz_split_fused(const double* __restrict__ a, long long rs, long long ks, int rows,
                                                       int k, int k16, int* __restrict__ ex, uint4* __restrict__ out,
-                                                      long long bs, int eb, int rb) {
+                                                      long long bs, int eb, int rb, const int* __restrict__ q, int sign) {
     a += blockIdx.z * bs;
     ex += (long long)blockIdx.z * eb;
     out += (long long)blockIdx.z * (eb / TILE) * k16 * (BLOCK / 16);
     extern __shared__ double xs[];  // [k][33]
-    __shared__ int em[32];
+    __shared__ int em[32], sk[FUSED_K];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r0 = blockIdx.x * 32;
-    if (threadIdx.x < 32) em[lane] = 0;
-    __syncthreads();
     const int kp = k16 * 16;
+    if (threadIdx.x < 32) em[lane] = 0;
+    for (int c = threadIdx.x; c < kp; c += 256) sk[c] = c < k ? shift_at(q, c, sign) : 0;
+    __syncthreads();
     if (ks == 1) {
         for (int r = w; r < 32; r += 8) {
             int m = 0;
-            for (int c = lane; c < kp; c += 32) {
-                const double x = r0 + r < rows && c < k ? a[(r0 + r) * rs + c] : 0.0;
-                xs[c * 33 + r] = x;
-                m = max(m, __double2hiint(x) & 0x7ff00000);
+            for (int c0 = lane; c0 < kp; c0 += 32 * LOADS) {
+                double x[LOADS];
+#pragma unroll
+                for (int u = 0; u < LOADS; ++u) x[u] = r0 + r < rows && c0 + 32 * u < k ? a[(r0 + r) * rs + c0 + 32 * u] : 0.0;
+#pragma unroll
+                for (int u = 0; u < LOADS; ++u) {
+                    const int c = c0 + 32 * u;
+                    if (c >= kp) break;
+                    xs[c * 33 + r] = x[u];
+                    m = max(m, stored_exponent(x[u], sk[c]));
+                }
             }
             m = __reduce_max_sync(0xffffffffu, m);
-            if (lane == 0) em[r] = m >> 20;
+            if (lane == 0) em[r] = m;
         }
     } else {
         int m = 0;
-        for (int c = w; c < kp; c += 8) {
-            const double x = r0 + lane < rows && c < k ? a[r0 + lane + c * ks] : 0.0;
-            xs[c * 33 + lane] = x;
-            m = max(m, __double2hiint(x) & 0x7ff00000);
+        for (int c0 = w; c0 < kp; c0 += 8 * LOADS) {
+            double x[LOADS];
+#pragma unroll
+            for (int u = 0; u < LOADS; ++u) x[u] = r0 + lane < rows && c0 + 8 * u < k ? a[r0 + lane + (c0 + 8 * u) * ks] : 0.0;
+#pragma unroll
+            for (int u = 0; u < LOADS; ++u) {
+                const int c = c0 + 8 * u;
+                if (c >= kp) break;
+                xs[c * 33 + lane] = x[u];
+                m = max(m, stored_exponent(x[u], sk[c]));
+            }
         }
-        if (m) atomicMax(em + lane, m >> 20);
+        if (m) atomicMax(em + lane, m);
     }
     __syncthreads();
     const int E = em[lane];
     if (w == 0 && r0 + lane < rows) ex[r0 + lane] = E;
     for (int o8 = w; o8 < 2 * k16; o8 += 8) {
         double x[8];
+        int sh[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = E != 0x7ff ? xs[(o8 * 8 + j) * 33 + lane] : 0.0;
-        store_digits(x, E, out + digit_at(r0 + lane, o8 >> 1, o8 & 1, k16, rb), rb * 2);
+        for (int j = 0; j < 8; ++j) {
+            x[j] = E != SPECIAL ? xs[(o8 * 8 + j) * 33 + lane] : 0.0;
+            sh[j] = sk[o8 * 8 + j];
+        }
+        store_digits(x, sh, E, out + digit_at(r0 + lane, o8 >> 1, o8 & 1, k16, rb), rb * 2);
     }
 }
 
@@ -541,8 +687,8 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
             // exponents: this thread's row, and one or two of the warp's columns per lane
             const int Ea = mine ? exA[m] : 0;
             const int Eb0 = lane < nc ? exB[n0 + lane] : 0, Eb1 = COLS > 32 && lane + 32 < nc ? exB[n0 + 32 + lane] : 0;
-            const bool special = __any_sync(0xffffffffu, Ea == 0x7ff || Eb0 == 0x7ff || Eb1 == 0x7ff);
-            const int ea = max(Ea, 1);
+            const bool special = __any_sync(0xffffffffu, Ea == SPECIAL || Eb0 == SPECIAL || Eb1 == SPECIAL);
+            const int ea = Ea - 2 * EXB;
             double* const Cm = g.C + tb * g.cb + m + (long long)n0 * g.ldc;
             const double alpha = g.alpha, beta = g.beta;
             long long sum[COLS];
@@ -580,7 +726,7 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
                     }
                 }
             };
-            auto exps = [&](int c) { return ea + max(__shfl_sync(0xffffffffu, COLS <= 32 || c < 32 ? Eb0 : Eb1, c & 31), 1); };
+            auto exps = [&](int c) { return ea + __shfl_sync(0xffffffffu, COLS <= 32 || c < 32 ? Eb0 : Eb1, c & 31); };
             auto rotate = [&]() {
 #pragma unroll
                 for (int j = 0; j < COLS - 8; ++j) sum[j] = sum[j + 8];
@@ -683,12 +829,13 @@ static void set_up() {
                                         SMEM_BYTES));
         CUDA_CHECK(cudaFuncSetAttribute(oz_gemm_kernel<false, OzTile<128>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         SMEM_BYTES));
+        CUDA_CHECK(cudaFuncSetAttribute(oz_scale_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_K * 33 * 4));
         CUDA_CHECK(cudaFuncSetAttribute(oz_split_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, FUSED_SMEM));
     });
 }
 
 void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int k_, cudaStream_t st, bool right,
-                  int batch_, long long bs_) {
+                  int batch_, long long bs_, const int* q) {
     set_up();
     rows = rows_;
     k = k_;
@@ -699,25 +846,28 @@ void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int 
     ks = ks_;
     bs = bs_;
     block = right && k16 <= HI_CHUNK ? 64 : TILE;
+    const int sign = right ? -1 : 1;
     const int nb = ceil_div(rows, TILE), eb = nb * TILE;
     d.alloc((size_t)batch * nb * k16 * (BLOCK / 16), st);
     ex.alloc((size_t)batch * eb, st);
     if (k <= FUSED_K && (rs == 1 || ks == 1)) {
         LAUNCH(oz_split_fused, dim3(ceil_div(rows, 32), 1, batch), 256, k16 * 16 * 33 * 8, st, a, rs, ks, rows, k, k16,
-               ex.get(), d.get(), bs, eb, block);
+               ex.get(), d.get(), bs, eb, block, q, sign);
         return;
     }
     if (ks == 1) {
-        LAUNCH(oz_exponent_cols, dim3(ceil_div(rows, 8), 1, batch), 256, 0, st, a, rs, rows, k, ex.get(), bs, eb);
+        LAUNCH(oz_exponent_cols, dim3(ceil_div(rows, 8), 1, batch), 256, 0, st, a, rs, rows, k, ex.get(), bs, eb, q,
+               sign);
     } else {
         ex.zero();
         const int kper = 32;
         LAUNCH(oz_exponent_rows, dim3(nb, ceil_div(k, kper), batch), TILE, 0, st, a, rs, ks, rows, k, kper, ex.get(), bs,
-               eb);
+               eb, q, sign);
     }
     // about four CTAs per SM's worth of k16 steps
     const int gy = std::max(1, std::min(k16, 152 * 8 / (nb * batch)));
-    LAUNCH(oz_split, dim3(nb, gy, batch), dim3(TILE, 2), 0, st, a, rs, ks, rows, k, k16, ex.get(), d.get(), bs, eb, block);
+    LAUNCH(oz_split, dim3(nb, gy, batch), dim3(TILE, 2), 0, st, a, rs, ks, rows, k, k16, ex.get(), d.get(), bs,
+           eb, block, q, sign);
 }
 
 void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* C, long long ldc, int* err,
@@ -764,6 +914,39 @@ void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* 
         TIMED_LAUNCH("oz_gemm", fl, by, (oz_gemm_kernel<true, OzTile<64>>), grid, OzTile<64>::NTHREADS, SMEM_BYTES, st, g);
     else
         TIMED_LAUNCH("oz_gemm", fl, by, (oz_gemm_kernel<false, OzTile<128>>), grid, OzTile<128>::NTHREADS, SMEM_BYTES, st, g);
+}
+
+void oz_scales(const double* B, long long rs, long long ks, int N, int K, int* q, cudaStream_t st) {
+    set_up();
+    if (K <= FUSED_K && (rs == 1 || ks == 1)) {
+        LAUNCH(oz_scale_fused, ceil_div(N, 32), 256, K * 33 * 4, st, B, rs, ks, N, K, q);
+        return;
+    }
+    DevBuf<int> ex(N, st);
+    if (ks == 1) {
+        LAUNCH(oz_exponent_cols, ceil_div(N, 8), 256, 0, st, B, rs, N, K, ex.get(), 0, 0, nullptr, 0);
+        LAUNCH(oz_scale, dim3(ceil_div(K, 128), ceil_div(N, 32)), 128, 0, st, B, rs, ks, N, K, ex.get(), q);
+    } else {
+        ex.zero();
+        LAUNCH(oz_exponent_rows, dim3(ceil_div(N, TILE), ceil_div(K, 32)), TILE, 0, st, B, rs, ks, N, K, 32, ex.get(), 0,
+               0, nullptr, 0);
+        LAUNCH(oz_scale, dim3(ceil_div(N, 128), ceil_div(K, 32)), 128, 0, st, B, rs, ks, N, K, ex.get(), q);
+    }
+}
+
+void oz_product(const double* A, long long ars, long long aks, const double* B, long long brs, long long bks, int M, int N,
+                int K, double alpha, double beta, double* C, long long ldc, int* err, cudaStream_t st, int* q) {
+    DevBuf<int> own;
+    if (!q) {
+        own.alloc(K, st);
+        own.zero();
+        q = own.get();
+    }
+    oz_scales(B, brs, bks, N, K, q, st);
+    OzMat a, b;
+    a.split(A, ars, aks, M, K, st, false, 1, 0, q);
+    b.split(B, brs, bks, N, K, st, true, 1, 0, q);
+    oz_gemm(a, b, alpha, beta, C, ldc, err, st);
 }
 
 }  // namespace sqbem

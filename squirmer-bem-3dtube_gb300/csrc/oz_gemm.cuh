@@ -11,6 +11,15 @@
 // 96-bit total is rounded to FP64 once.  What is dropped lies below 2^-60 of the
 // row's largest entry times the column's, against the FP64 loop's rounding of
 // every partial sum.
+//
+// The FP64 loop does not see powers of two that move from A's column k to B's row k; a fixed
+// point does.  An LU of a matrix whose rows have different scales has small multipliers that
+// meet large entries, and kept 2^-62 of the largest multiplier: rows 2^-40 apart gave
+// solutions good to 1e-7.  So oz_product first scales every k by a power of two after which
+// the rows of B (its columns taken relative to their largest entries) have equal largest
+// exponents; the scales change the fixed points only, and cancel in the products.  It
+// takes one more pass over B; a product whose operands are known to be even (the Fourier blocks)
+// does without (split and oz_gemm).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -30,9 +39,9 @@ struct OzMat {
     const double* src = nullptr;
     long long rs = 0, ks = 0, bs = 0;
     // element (r, c) of matrix b is a[r * rs + c * ks + b * bs]; `right` where the operand is B
-    // (blocks of 64 rows then, while k <= 256)
+    // (blocks of 64 rows then, while k <= 256); q: scales along k (oz_scales), the same for A and B
     void split(const double* a, long long rs, long long ks, int rows, int k, cudaStream_t st, bool right = false,
-               int batch = 1, long long bs = 0);
+               int batch = 1, long long bs = 0, const int* q = nullptr);
 };
 
 // C (M x N, column-major) = alpha A B + beta C for the digits of A (M rows) and of
@@ -43,5 +52,14 @@ struct OzMat {
 // (SQBEM_ERR_TIMEOUT to the caller).
 void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* C, long long ldc, int* err,
              cudaStream_t st, long long cb = 0);
+
+// The scales along k of a product with B (element (k, n) at B[n * rs + k * ks]) into the K words
+// of q, which are zero before.
+void oz_scales(const double* B, long long rs, long long ks, int N, int K, int* q, cudaStream_t st);
+
+// C = alpha A B + beta C from the values, with scales along k: element (m, k) of A at A[m * ars + k * aks],
+// (k, n) of B at B[n * brs + k * bks]; C as in oz_gemm.  q (may be null): K words of zeros for the scales.
+void oz_product(const double* A, long long ars, long long aks, const double* B, long long brs, long long bks, int M, int N,
+                int K, double alpha, double beta, double* C, long long ldc, int* err, cudaStream_t st, int* q = nullptr);
 
 }  // namespace sqbem
