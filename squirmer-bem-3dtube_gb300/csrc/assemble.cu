@@ -218,7 +218,9 @@ __device__ void warp_rule(Acc<T>& A, const PanelRec& P, double x, double y, doub
 
 // The FP64 sums of a rule for the FP64 mode, v[0 .. 5] = sum w rr/|r|^3, v[6 .. 11] = sum w
 // rr/|r|^5, v[12] = sum w/|r| over this lane's points: r.m is the same at every point of a
-// flat panel and, with the area, enters once per entry.
+// flat panel and, with the area, enters once per entry.  (It comes from a vertex here, from a node
+// in the far kernels: the centroid lies off the plane by its own rounding, which grows with the
+// distance from the origin of the coordinates.)
 __device__ __forceinline__ void lane_rule64(double (&v)[16], const PanelRec& P, double x, double y, double z, int rule,
                                             int lane) {
     const double e0x = P.v[0] - x, e0y = P.v[1] - y, e0z = P.v[2] - z;
@@ -406,7 +408,8 @@ __global__ void __launch_bounds__(FAR_TGT) far_kernel(BlockJob<TO> job) {
         };
         if (job.S) put(job.S, job.s_rs, job.s_cs, d[28], sxx + dg, sxy, sxz, syy + dg, syz, szz + dg);
         if (job.D)
-            put(job.D, job.d_rs, job.d_cs, d[29] * (bx * d[24] + by * d[25] + bz * d[26]), dxx, dxy, dxz, dyy, dyz, dzz);
+            put(job.D, job.d_rs, job.d_cs, d[29] * ((bx + d[0]) * d[24] + (by + d[1]) * d[25] + (bz + d[2]) * d[26]), dxx,
+                dxy, dxz, dyy, dyz, dzz);
     }
 }
 
@@ -712,7 +715,7 @@ __device__ __forceinline__ void near_pairs(const BlockJob<TO>& list, int imask, 
             dl = __shfl_sync(0xffffffffu, t, (6 + k) & 31);
             if (a == b) sl += dg;
             sl *= P.area;
-            dl *= -6.0 * P.area * ((P.c[0] - x) * P.n[0] + (P.c[1] - y) * P.n[1] + (P.c[2] - z) * P.n[2]);
+            dl *= -6.0 * P.area * ((P.v[0] - x) * P.n[0] + (P.v[1] - y) * P.n[1] + (P.v[2] - z) * P.n[2]);
         }
         if (lane < 9) {
             const long long r = 3LL * i + a, c = 3LL * p + b;
@@ -1185,7 +1188,7 @@ struct FieldArith<double> {
             const int rule = rule_of(job.panels[p], X.x, X.y, X.z);
             if (rule != 0) return rule;
         }
-        const double rm = bx * d[21] + by * d[22] + bz * d[23];
+        const double rm = (bx + d[0]) * d[21] + (by + d[1]) * d[22] + (bz + d[2]) * d[23];
         const double fx = d[28], fy = d[29], fz = d[30], gx = d[31] * rm, gy = d[32] * rm, gz = d[33] * rm;
         double al = 0.0;
 #pragma unroll
@@ -1322,7 +1325,7 @@ __device__ void field_near(const FieldJob& job, int p, int rule, const FieldPoin
     const double e0x = P.v[0] - X.x, e0y = P.v[1] - X.y, e0z = P.v[2] - X.z;
     const double e1x = P.v[3] - X.x, e1y = P.v[4] - X.y, e1z = P.v[5] - X.z;
     const double e2x = P.v[6] - X.x, e2y = P.v[7] - X.y, e2z = P.v[8] - X.z;
-    const double rm = -6.0 * ((P.c[0] - X.x) * P.n[0] + (P.c[1] - X.y) * P.n[1] + (P.c[2] - X.z) * P.n[2]);
+    const double rm = -6.0 * (e0x * P.n[0] + e0y * P.n[1] + e0z * P.n[2]);
     const double ss = job.sscale * P.area, ds = job.dscale * P.area * rm;
     const double fx = job.f[3 * p] * ss, fy = job.f[3 * p + 1] * ss, fz = job.f[3 * p + 2] * ss;
     const double gx = job.u[3 * p] * ds, gy = job.u[3 * p + 1] * ds, gz = job.u[3 * p + 2] * ds;
@@ -1684,7 +1687,7 @@ __global__ void __launch_bounds__(32 * ADJ_W) adjoint_pairs_kernel(AdjTerm J, in
         M.zero();
 #pragma unroll
         for (int q = 0; q < 7; ++q) M.node(bx + d[3 * q], by + d[3 * q + 1], bz + d[3 * q + 2], c_rule7[q].w);
-        const double sm = bx * d[24] + by * d[25] + bz * d[26], gs = J.gs * d[28], ts = J.ts * d[28];
+        const double sm = (bx + d[0]) * d[24] + (by + d[1]) * d[25] + (bz + d[2]) * d[26], gs = J.gs * d[28], ts = J.ts * d[28];
 #pragma unroll
         for (int j = 0; j < ADJ_MAX_MODES; ++j)
             if (j < nm)
@@ -1708,7 +1711,7 @@ __global__ void __launch_bounds__(32 * ADJ_W) adjoint_pairs_kernel(AdjTerm J, in
             M.node(R.l0 * e0x + R.l1 * e1x + R.l2 * e2x, R.l0 * e0y + R.l1 * e1y + R.l2 * e2y,
                    R.l0 * e0z + R.l1 * e1z + R.l2 * e2z, R.w);
         }
-        const double sm = (d[21] - X) * d[24] + (d[22] - Y) * d[25] + (d[23] - Zc) * d[26];
+        const double sm = e0x * d[24] + e0y * d[25] + e0z * d[26];
         double D[NC];
 #pragma unroll
         for (int k = 0; k < NC; ++k) D[k] = 0.0;
