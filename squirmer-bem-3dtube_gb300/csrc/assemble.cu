@@ -1159,7 +1159,7 @@ template <>
 struct FieldArith<double> {
     static constexpr int WORDS = FT64;
     static __device__ int exponent(const FieldJob&, int) { return 0; }
-    static __device__ void stage(double* d, const FieldJob& job, int p, const double*, int) {
+    static __device__ bool stage(double* d, const FieldJob& job, int p, const double*, int) {
         const PanelRec P = job.panels[p];
         double v[9];
 #pragma unroll
@@ -1177,11 +1177,12 @@ struct FieldArith<double> {
             d[31 + k] = job.u[3 * p + k] * (-6.0 * job.dscale * P.area);
         }
         d[27] = 9.0 * P.h * P.h * (1.0 + 1e-12);
+        return false;
     }
     double a[3];
-    __device__ void point(const FieldPoint&, const double*) {}
+    __device__ void offset(int, double, double) {}
     __device__ void begin() { a[0] = a[1] = a[2] = 0.0; }
-    __device__ int pair(const double* d, const FieldJob& job, int p, const FieldPoint& X, bool) {
+    __device__ int pair(const double* d, const FieldJob& job, int p, const FieldPoint& X, bool, bool) {
         const double bx = d[24] - X.x, by = d[25] - X.y, bz = d[26] - X.z;
         // within 1e-12 of the threshold and below: the exact test
         if (!(bx * bx + by * by + bz * bz > d[27])) {
@@ -1226,11 +1227,16 @@ struct FieldArith<float> {
         }
         return m >> 20;
     }
-    // lengths relative to the origin o (a point of the CTA); f and u over 2^(ex - 1023)
-    static __device__ void stage(float* d, const FieldJob& job, int p, const double* o, int ex) {
+    // lengths relative to the origin o; f and u over 2^(ex - 1023).  True if the panel lies so far
+    // from o for its size that the pairs' 2^-48 would show beside FP32's rounding.
+    static __device__ bool stage(float* d, const FieldJob& job, int p, const double* o, int ex) {
         const PanelRec P = job.panels[p];
+        float ext = 0.f;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) split2(P.v[k] - o[k % 3], d[k], d[9 + k]);
+        for (int k = 0; k < 9; ++k) {
+            split2(P.v[k] - o[k % 3], d[k], d[9 + k]);
+            ext = fmaxf(ext, fabsf(d[k]));
+        }
         const double h2 = P.h * P.h, sc = ex > 0 && ex < 0x7ff ? scalbn(1.0, 1023 - ex) : 1.0;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -1243,24 +1249,27 @@ struct FieldArith<float> {
             split2(job.u[3 * p + k] * job.dscale * sc, d[40 + k], d[43 + k]);
         }
         d[21] = (float)P.area;
+        return ext > 4e6f * (float)P.h;
     }
     float xh[3], xl[3], s[3], c[3];
-    __device__ void point(const FieldPoint& X, const double* o) {
-        split2(X.x - o[0], xh[0], xl[0]);
-        split2(X.y - o[1], xh[1], xl[1]);
-        split2(X.z - o[2], xh[2], xl[2]);
+    // component k of the point's offset from the origin
+    __device__ void offset(int k, float hi, float lo) {
+        xh[k] = hi;
+        xl[k] = lo;
     }
     __device__ void begin() {
 #pragma unroll
         for (int k = 0; k < 3; ++k) s[k] = c[k] = 0.f;
     }
-    __device__ int pair(const float* d, const FieldJob& job, int p, FieldPoint& X, bool special) {
+    // wide: the offsets from the FP64 coordinates
+    __device__ int pair(const float* d, const FieldJob& job, int p, FieldPoint& X, bool special, bool wide) {
         const float bx = (d[22] - xh[0]) + (d[25] - xl[0]), by = (d[23] - xh[1]) + (d[26] - xl[1]),
                     bz = (d[24] - xh[2]) + (d[27] - xl[2]);
         const float d2 = bx * bx + by * by + bz * bz;
-        if (!(d2 > d[33])) {
+        if (wide || !(d2 > d[33])) {
             int rule;
-            if (d2 < d[30] && d2 > d[32]) rule = 1;
+            if (wide) rule = rule_of(job.panels[p], X.x, X.y, X.z);
+            else if (d2 < d[30] && d2 > d[32]) rule = 1;
             else if (d2 < d[29] && d2 > d[31]) rule = 2;
             else if (d2 < d[28]) rule = 3;
             else rule = rule_of(job.panels[p], X.x, X.y, X.z);
@@ -1272,6 +1281,10 @@ struct FieldArith<float> {
             float hi, lo;
             two_diff(d[k], xh[k % 3], hi, lo);
             e[k] = __fadd_rn(hi, __fadd_rn(lo, __fsub_rn(d[9 + k], xl[k % 3])));
+        }
+        if (wide) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) e[k] = (float)(job.panels[p].v[k] - (k % 3 == 0 ? X.x : k % 3 == 1 ? X.y : X.z));
         }
         Acc<float> A;
         A.zero();
@@ -1366,7 +1379,7 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
     extern __shared__ __align__(16) unsigned char field_smem[];
     TC* const tile = reinterpret_cast<TC*>(field_smem);
     int* const lists = reinterpret_cast<int*>(tile + TP * W);
-    __shared__ int tex;
+    __shared__ int tex, twide;
     __shared__ double part[FIELD_WARPS][3];
     __shared__ int pnear[FIELD_WARPS];
     __shared__ double clsum[3];
@@ -1375,7 +1388,6 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const int ncl = SHARED ? (int)cl.num_blocks() : 1, rank = SHARED ? (int)cl.block_rank() : 0;
     const int pt0 = SHARED ? blockIdx.x / ncl : (blockIdx.x * FIELD_WARPS + wl) * PPW;
-    const double* const o = job.pts + 3LL * (SHARED ? pt0 : blockIdx.x * FIELD_WARPS * PPW);
     FieldPoint X[PPW];
     FieldArith<TC> F[PPW];
 #pragma unroll
@@ -1386,8 +1398,9 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
         X[k].z = job.pts[3 * pt + 2];
         X[k].u[0] = X[k].u[1] = X[k].u[2] = 0.0;
         X[k].near = 0;
-        F[k].point(X[k], o);
     }
+    // lane 3 k + c: component c of point k, for the offsets from a tile's origin
+    const double xc = lane < 3 * PPW ? job.pts[3LL * min(pt0 + lane / 3, job.npts - 1) + lane % 3] : 0.0;
     int* const list = lists + wl * PPW * FIELD_NEAR_CAP;
     // SHARED: consecutive panels go to different CTAs and warps, so that the near ones, which are
     // neighbours, are shared out too (by whole tiles one warp had them all: 200 us for 60
@@ -1399,7 +1412,7 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
         const int mine = index(base, threadIdx.x);
         const bool has = (int)threadIdx.x < TP && mine < job.P;
         __syncthreads();
-        if (threadIdx.x == 0) tex = 0;
+        if (threadIdx.x == 0) tex = twide = 0;
         __syncthreads();
         if (sizeof(TC) == 4 && has) {
             const int e = FieldArith<TC>::exponent(job, mine);
@@ -1407,8 +1420,21 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
         }
         __syncthreads();
         const int ex = tex;
-        if (has) FieldArith<TC>::stage(tile + threadIdx.x * W, job, mine, o, ex);
+        // the origin of a tile's lengths: a vertex of its first panel (no point, which may be
+        // anything, has a say in another's result), or the one point of the CTA
+        const double* const o = SHARED ? job.pts + 3LL * pt0 : job.panels[base].v;
+        if (has && FieldArith<TC>::stage(tile + threadIdx.x * W, job, mine, o, ex)) twide = 1;
         __syncthreads();
+        const bool wide = !SHARED && twide != 0;
+        if (sizeof(TC) == 4) {
+            float hi, lo;
+            split2(xc - o[lane % 3], hi, lo);
+#pragma unroll
+            for (int k = 0; k < PPW; ++k)
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    F[k].offset(c, __shfl_sync(0xffffffffu, hi, 3 * k + c), __shfl_sync(0xffffffffu, lo, 3 * k + c));
+        }
 #pragma unroll
         for (int k = 0; k < PPW; ++k) F[k].begin();
         for (int s = SHARED ? wl * 32 : 0; s < (SHARED ? wl * 32 + 32 : min(TP, job.P - base)); s += 32) {
@@ -1416,7 +1442,7 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
 #pragma unroll
             for (int k = 0; k < PPW; ++k) {
                 int rule = 0;
-                if (p < job.P) rule = F[k].pair(tile + q * W, job, p, X[k], ex == 0x7ff);
+                if (p < job.P) rule = F[k].pair(tile + q * W, job, p, X[k], ex == 0x7ff, wide);
                 const unsigned m = __ballot_sync(0xffffffffu, rule > 0);
                 if (rule > 0) {
                     const int slot = X[k].near + __popc(m & ((1u << lane) - 1));
