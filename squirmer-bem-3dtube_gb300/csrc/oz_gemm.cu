@@ -700,7 +700,12 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
             // C += v goes to L2 as a reduction (one per element, IEEE rounding): reading C
             // here left the warps waiting on its loads for two thirds of the read-out.
             const int flip = alpha == -1.0 ? 0x80000000 : 0;
-            const bool plain = (alpha == 1.0 || alpha == -1.0) && (beta == 0.0 || beta == 1.0), add = beta == 1.0;
+            // Elements whose row or column holds an infinity or a NaN (zero digits) are left out here
+            // and follow below.
+            const bool plain = (alpha == 1.0 || alpha == -1.0) && (beta == 0.0 || beta == 1.0) && !special,
+                       add = beta == 1.0;
+            const uint32_t skip0 = __ballot_sync(0xffffffffu, Eb0 == SPECIAL), skip1 = __ballot_sync(0xffffffffu, Eb1 == SPECIAL);
+            auto left_out = [&](int c) { return Ea == SPECIAL || ((COLS <= 32 || c < 32 ? skip0 : skip1) >> (c & 31) & 1); };
             auto finish = [&](int c, const double (&r)[8]) {
                 if (plain && add) {
 #pragma unroll
@@ -718,6 +723,7 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
 #pragma unroll 1
                     for (int j = 0; j < 8; ++j) {
                         if (!mine || c + j >= nc) break;
+                        if (special && left_out(c + j)) continue;
                         double* const p = Cm + (long long)(c + j) * g.ldc;
                         double v = r[0];
 #pragma unroll
@@ -734,7 +740,6 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
             for (int q = 0; q < (SHORT ? NBUF : ng); ++q) {
                 const Group G = group_at<SHORT>(SHORT ? q >> 1 : q, k16);
                 const int p = SHORT ? q : G.p;
-                const bool straight = SHORT && q == 3 && !special;
                 // the whole warp stays or leaves: tcgen05.ld is warp-collective
                 ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, aph, err, wait));
                 if (!ok) break;
@@ -742,7 +747,7 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
                 const uint32_t base = tmem_base + lanes + (uint32_t)(acc * 2 * TN + col0);
                 if (SHORT && q == 3) {
 #pragma unroll 1
-                    for (int c = 0; straight && c < COLS; c += 8) {
+                    for (int c = 0; c < COLS; c += 8) {
                         float v0[8], v1[8];
                         tmem_ld8x2(base + c, base + TN + c, v0, v1);
                         double r[8];
@@ -781,7 +786,7 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
                 }
             }
             if (!ok) break;
-            if (!SHORT && !special) {
+            if (!SHORT) {
 #pragma unroll 1
                 for (int c = 0; c < COLS; c += 8) {
                     double r[8];
@@ -795,9 +800,9 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
                 }
             }
             if (special && mine) {
-                // an infinity or a NaN in these rows or columns: plain sums, or NaN where C
-                // takes the place of B
+                // plain sums, or NaN where C takes the place of B
                 for (int c = 0; c < nc; ++c) {
+                    if (!left_out(c)) continue;
                     const long long n = n0 + c;
                     double r = g.srcB ? 0.0 : __longlong_as_double(0x7ff8000000000000ll);
                     for (int k = 0; g.srcB && k < g.K; ++k)

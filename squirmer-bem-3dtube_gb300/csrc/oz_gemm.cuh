@@ -47,8 +47,9 @@ struct OzMat {
 // C (M x N, column-major) = alpha A B + beta C for the digits of A (M rows) and of
 // B (N columns, given as rows) over the same k, for every matrix of the batch (C at
 // stride cb).  The sources of A and B must be alive and unchanged until the launch has
-// run; C may be one of them (its rows and columns with an infinity or a NaN then give
-// NaN), but must not overlap them otherwise.  *err is set if a bounded wait expires
+// run; C may be one of them, but must not overlap them otherwise.  A row or a column with an
+// infinity or a NaN gives the plain sums of its elements, or NaN where C is a source, and leaves the
+// others as they are.  *err is set if a bounded wait expires
 // (SQBEM_ERR_TIMEOUT to the caller).
 void oz_gemm(const OzMat& A, const OzMat& B, double alpha, double beta, double* C, long long ldc, int* err,
              cudaStream_t st, long long cb = 0);
