@@ -12,13 +12,15 @@
 //              an accumulator in tensor memory;
 //   epilogue   eight warps: the accumulators as integers into 64-bit sums held in registers,
 //              the rounding to FP64, C.
-// Four passes: weights 0, 1 (digits 0-1) and 2, 3 (digits 0-3) in chunks of 256 k,
-// where every sum is exact (4 * 256 * 2^14 = 2^24); then weights 4, 5 and 6, 7
-// in chunks of 1024 k, whose rounding past 2^24 lies 2^-56 below the product
-// of the largest entries.
-//   K <= 256 (the panels' updates): tiles of 128 x 64, an accumulator per pass; the 64-bit
-//   sums also take weights 4 and 5 (2^62 at most), and the last pass goes straight into the
-//   rounding.
+// Four passes: weights 0, 1 (digits 0-1) and 2, 3 (digits 0-3) in chunks of 256 k and
+// weights 4, 5 in chunks of 160, where every sum is exact (4 * 256 * 2^14 = 2^24, 6 * 160 *
+// 2^14 < 2^24); then weights 6, 7 in chunks of 1024 k.  There a sum of weight 6, in units of
+// 2^-62 of the product of the largest entries, may reach 2^27 and lose up to 8 units at each of
+// its 448 accumulations: 2^-60 of K times that product at most.  (With weights 4, 5 in
+// chunks of 1024 too, digits of one sign lost up to 2^-46 of it.)
+//   K <= 256 (the panels' updates): tiles of 128 x 64, an accumulator per pass, that of weights
+//   4, 5 read out twice for K > 160; the 64-bit sums also take weights 4 and 5 (2^62 at
+//   most), and the last pass goes straight into the rounding.
 //   K > 256: tiles of 128 x 128, two accumulators; the sums of the leading passes wait in
 //   global scratch (L2) for the others, since both sets do not fit in the registers together.
 #include <cuda_runtime.h>
@@ -39,7 +41,7 @@ constexpr int DIGITS = 8;
 constexpr int PLANE = TILE * 16 * 2;       // one digit of a 128 x 16 block: 4 KB
 constexpr int BLOCK = DIGITS * PLANE;      // 32 KB
 constexpr int SMEM_BYTES = 192 * 1024 + 1024 + 256;
-constexpr int HI_CHUNK = 16, LO_CHUNK = 64;  // k16 steps between read-outs
+constexpr int HI_CHUNK = 16, MID_CHUNK = 10, LO_CHUNK = 64;  // k16 steps between read-outs: passes 0, 1; 2; 3
 
 // Tiles of 128 x TN.  TN = 128 has the widest instructions and suits a long K.  With K <= 256
 // a 128 x 128 tile's read-out (20 us) was as long as its multiplication, and with tensor memory
@@ -404,24 +406,26 @@ __device__ __forceinline__ void tile_at(const OzArgs& g, int t, int& b, int& tm,
 
 // What runs over the k16 steps [k0, k1) with nd digits of both operands in the stages: pass p
 // (the weights 2p, 2p + 1), for SHORT also p + 1.  The long kernel has one pass
-// between two read-outs: the leading passes 0, 1 alternate over HI_CHUNK steps, then 2, 3 over
-// LO_CHUNK.  SHORT has accumulators for all four and loads a step's digits twice, not four
-// times: four digits for passes 0 and 1, then all eight for 2 and 3.
+// between two read-outs: the leading passes 0, 1 alternate over HI_CHUNK steps, then 2 over
+// MID_CHUNK and 3 over LO_CHUNK.  SHORT has accumulators for all four and loads a step's digits
+// twice, not four times: four digits for passes 0 and 1, then all eight for 2 and 3.
 struct Group {
     int p, nd, k0, k1;
     bool last_hi;
 };
+__device__ __forceinline__ int n_chunks(int k16, int chunk) { return (k16 + chunk - 1) / chunk; }
 template <bool SHORT>
 __device__ __forceinline__ int n_groups(int k16) {
     if (SHORT) return 2;
-    return 2 * ((k16 + HI_CHUNK - 1) / HI_CHUNK) + 2 * ((k16 + LO_CHUNK - 1) / LO_CHUNK);
+    return 2 * n_chunks(k16, HI_CHUNK) + n_chunks(k16, MID_CHUNK) + n_chunks(k16, LO_CHUNK);
 }
 template <bool SHORT>
 __device__ __forceinline__ Group group_at(int q, int k16) {
     if (SHORT) return Group{2 * q, 4 * q + 4, 0, k16, false};
-    const int nh = 2 * ((k16 + HI_CHUNK - 1) / HI_CHUNK);
-    const bool hi = q < nh;
-    const int c = hi ? HI_CHUNK : LO_CHUNK, i = hi ? q : q - nh, p = (hi ? 0 : 2) + (i & 1), k0 = (i >> 1) * c;
+    const int nh = 2 * n_chunks(k16, HI_CHUNK), nm = n_chunks(k16, MID_CHUNK);
+    const int p = q < nh ? q & 1 : q < nh + nm ? 2 : 3;
+    const int c = q < nh ? HI_CHUNK : q < nh + nm ? MID_CHUNK : LO_CHUNK;
+    const int k0 = (q < nh ? q >> 1 : q < nh + nm ? q - nh : q - nh - nm) * c;
     return Group{p, 2 * p + 2, k0, min(k16, k0 + c), q == nh - 1};
 }
 
@@ -556,6 +560,10 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 2 * NBUF + 1);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int tiles = g.tiles_m * g.tiles_n * g.batch, k16 = g.k16, ng = n_groups<SHORT>(k16);
+    const bool halves = SHORT && k16 > MID_CHUNK;  // pass 2 read out after mid steps too
+    const int mid = (k16 + 1) / 2;
+    static_assert(!SHORT || (HI_CHUNK + 1) / 2 <= MID_CHUNK, "two halves suffice");
+    static_assert(!SHORT || T::step_bytes(DIGITS) == STAGE, "a stage per step in passes 2 and 3: mid starts one");
     int* const err = g.err;
     const long long wait = g.wait;
 
@@ -634,18 +642,27 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
                 const int step = T::step_bytes(G.nd), sp = STAGE / step;
                 const int p = G.p + mine;
                 if (SHORT) acc = p;
-                ok = __all_sync(0xffffffffu, mbar_wait(tempty0 + 8 * acc, aph ^ 1, err, wait));
+                // SHORT: pass 2's accumulator is used twice per tile, with the parities 0 and 1
+                const bool two = halves && p == 2;
+                ok = __all_sync(0xffffffffu, mbar_wait(tempty0 + 8 * acc, two ? 1u : aph ^ 1, err, wait));
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)(acc * 2 * TN);
                 for (int k = G.k0; k < G.k1; k += sp) {
+                    if (two && k == mid) {
+                        if (elect_one()) mma_commit(tfull0 + 8 * acc);
+                        __syncwarp();
+                        ok = __all_sync(0xffffffffu, mbar_wait(tempty0 + 8 * acc, 0, err, wait));
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
                     ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, ph, err, wait));
                     if (!ok) break;
                     tc_fence_after();
                     const int n = min(sp, G.k1 - k);
                     uint32_t a0 = smem_u32(smem + s * STAGE);
                     for (int u = 0; u < n; ++u, a0 += step) {
-                        const bool first = k + u == G.k0;
+                        const bool first = k + u == G.k0 || (two && k + u == mid);
                         const uint32_t b0 = a0 + G.nd * PLANE;
                         if (p == 0) issue_step<0, T>(a0, b0, d, first);
                         else if (p == 1) issue_step<1, T>(a0, b0, d, first);
@@ -737,15 +754,19 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
 #pragma unroll
                 for (int j = 0; j < COLS - 8; ++j) sum[j] = sum[j + 8];
             };
-            for (int q = 0; q < (SHORT ? NBUF : ng); ++q) {
-                const Group G = group_at<SHORT>(SHORT ? q >> 1 : q, k16);
-                const int p = SHORT ? q : G.p;
+            for (int q = 0; q < (SHORT ? NBUF + halves : ng); ++q) {
+                const int p = SHORT ? q - (halves && q > 2) : group_at<SHORT>(q, k16).p;
+                uint32_t par = aph;
+                if (SHORT) {
+                    acc = p;
+                    if (halves && p == 2) par = q - 2;
+                }
                 // the whole warp stays or leaves: tcgen05.ld is warp-collective
-                ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, aph, err, wait));
+                ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, par, err, wait));
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t base = tmem_base + lanes + (uint32_t)(acc * 2 * TN + col0);
-                if (SHORT && q == 3) {
+                if (SHORT && p == 3) {
 #pragma unroll 1
                     for (int c = 0; c < COLS; c += 8) {
                         float v0[8], v1[8];
@@ -776,8 +797,8 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
                 }
                 tc_fence_before();
                 mbar_arrive(tempty0 + 8 * acc);
-                if (++acc == NBUF) { acc = 0; aph ^= 1; }
-                if (!SHORT && G.last_hi) {
+                if (!SHORT && ++acc == NBUF) { acc = 0; aph ^= 1; }
+                if (!SHORT && group_at<SHORT>(q, k16).last_hi) {
 #pragma unroll
                     for (int j = 0; j < COLS; ++j) {
                         stash[j * TILE] = sum[j];
@@ -786,6 +807,7 @@ __global__ void __launch_bounds__(T::NTHREADS, 1) oz_gemm_kernel(const __grid_co
                 }
             }
             if (!ok) break;
+            if (SHORT) aph ^= 1;
             if (!SHORT) {
 #pragma unroll 1
                 for (int c = 0; c < COLS; c += 8) {

@@ -1,11 +1,41 @@
-"""Digit products (oz_gemm.cu) at the ends of what their sums and their read-out hold: rows and columns
-with infinities or NaN beside good ones."""
+"""Digit products (oz_gemm.cu) at the ends of what their sums and their read-out hold: digits of one
+sign, and rows and columns with infinities or NaN beside good ones."""
 import numpy as np
 import pytest
+
+from test_gpu_gemm64 import exact
 
 sqbem = pytest.importorskip("sqbem")
 
 pytestmark = pytest.mark.gpu
+
+
+def digits(rng, shape, lo, hi):
+    """Numbers whose six leading base-256 digits lie in [lo, hi], hence 48 bits."""
+    return sum(rng.integers(lo, hi + 1, shape).astype(float) * 2.0 ** (-8 * i) for i in range(6))
+
+
+def err(C, A, B):
+    hi, lo = exact(A, B)
+    return float(np.max(np.abs((C - hi) - lo)) / (A.shape[1] * np.abs(A).max() * np.abs(B).max()))
+
+
+# one chunk of the short kernel and its remainders, chunks of the long one
+@pytest.mark.parametrize("K", [96, 160, 161, 176, 240, 256, 257, 512, 1024, 1300, 4100])
+@pytest.mark.parametrize("lo,hi,sign", [(100, 127, 1.0), (100, 127, -1.0), (120, 127, 1.0), (127, 127, 1.0), (64, 127, 1.0)])
+def test_digits_of_one_sign(K, lo, hi, sign):
+    rng = np.random.default_rng([K, lo])
+    A, B = digits(rng, (130, K), lo, hi), sign * digits(rng, (K, 140), lo, hi)
+    # the result is rounded once, to 2^-53 of at most K times the largest product; below that the
+    # digits left out and the sums of weight 6
+    assert err(sqbem.gemm64(A, B, route=1), A, B) <= 2.0 ** -53 + 2.0 ** -59
+
+
+@pytest.mark.parametrize("K", [160, 256, 1024])
+def test_digits_of_both_signs(K):
+    rng = np.random.default_rng(K)
+    A, B = digits(rng, (130, K), -127, 127), digits(rng, (K, 140), -127, 127)
+    assert err(sqbem.gemm64(A, B, route=1), A, B) <= 2.0 ** -53 + 2.0 ** -59
 
 
 @pytest.mark.parametrize("n", [129, 300, 640])
