@@ -270,6 +270,21 @@ extern "C" int sqbem_test_rsqrt_nr(int n, const double* x, double* y) {
     });
 }
 
+// Test hook, not part of the public ABI: the LU kernels' reciprocal on n host values.
+extern "C" int sqbem_test_recip(int n, const double* x, double* y) {
+    return guarded([&] {
+        if (n < 0 || (n > 0 && (!x || !y))) fail(SQBEM_ERR_ARG, "test_recip: bad arguments");
+        if (n == 0) return;
+        require_device();
+        Stream s;
+        DevBuf<double> dx(n, s), dy(n, s);
+        dx.upload(x, n);
+        recip_eval(n, dx.get(), dy.get(), s);
+        dy.download(y, n);
+        CUDA_CHECK(cudaStreamSynchronize(s));
+    });
+}
+
 // ---------------------------------------------------------------- dense
 extern "C" int sqbem_solve_dense(int n, int nrhs, const double* A, double* B, int* pivoted) {
     return guarded([&] {

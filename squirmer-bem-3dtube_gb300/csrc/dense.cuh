@@ -48,6 +48,10 @@ void gemm64_few(bool ta, int M, int N, int K, double alpha, const double* A, lon
                 long long ldb, double beta, double* C, long long ldc, cudaStream_t st, int batch = 1,
                 long long sa = 0, long long sb = 0, long long sc = 0);
 
+// y = recip(x) elementwise on device arrays: the reciprocal of the LU kernels (tested through
+// sqbem_test_recip)
+void recip_eval(int n, const double* x, double* y, cudaStream_t st);
+
 // C (m x 6) = A K, K the rigid-body map of np panels with the offsets r (3 per panel) from the
 // centre; A is m x 3 np.
 void rigid64(int m, int np, const double* A, long long lda, const double* r, double* C, long long ldc, cudaStream_t st);

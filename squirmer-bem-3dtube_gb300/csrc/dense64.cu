@@ -378,8 +378,8 @@ void max_abs64(const double* A, long long lda, int rows, int cols, double* out, 
 constexpr int PB = 32, HB = 128;
 
 // 1/x from the hardware's approximate reciprocal y (relative error e = 1 - x y about 2^-20):
-// 1/x = y / (1 - e) = y (1 + e + e^2 + ..), cut after e^2, so 2^-60 and the rounding.  Three
-// FP64 operations where the full division (430 cycles) is on the factorisation's
+// 1/x = y / (1 - e) = y (1 + e + e^2 + ..), cut after e^2, so 2^-60 and the rounding: within one
+// unit in the last place of the division.  Three FP64 operations where the full division (430 cycles) is on the factorisation's
 // serial chain.
 __device__ __forceinline__ double recip(double x) {
     const int e = (__double2hiint(x) >> 20) & 0x7ff;
@@ -388,6 +388,15 @@ __device__ __forceinline__ double recip(double x) {
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double d = fma(-x, y, 1.0);
     return fma(y, fma(d, d, d), y);
+}
+
+__global__ void recip_kernel(int n, const double* __restrict__ x, double* __restrict__ y) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) y[i] = recip(x[i]);
+}
+
+void recip_eval(int n, const double* x, double* y, cudaStream_t st) {
+    if (n > 0) LAUNCH(recip_kernel, ceil_div(n, 256), 256, 0, st, n, x, y);
 }
 
 // |x| > |piv|, as a pivot search sees it (bit 0), or x not finite (bit 1); piv by its bits
