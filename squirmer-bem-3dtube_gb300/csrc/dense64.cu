@@ -276,8 +276,9 @@ void rigid64(int m, int np, const double* A, long long lda, const double* r, dou
 // The digit products need about 65 us whatever the size (the scales, two splits, a tile's 36
 // products and read-outs), in which the FP64 pipe does 6e7 operations; and a tile of
 // 128 x 128 with a K below 64 costs more to read out than to multiply.
+constexpr double PIPE_OPS = 6e7;
 static bool use_tensor(int M, int N, int K, const int* err) {
-    return err && K >= 64 && M >= 64 && N >= 64 && 2.0 * M * N * K > 6e7;
+    return err && K >= 64 && M >= 64 && N >= 64 && 2.0 * M * N * K > PIPE_OPS;
 }
 
 void gemm64(bool ta, bool tb, int M, int N, int K, double alpha, const double* A, long long lda, const double* B,
@@ -379,8 +380,8 @@ constexpr int PB = 32, HB = 128;
 
 // 1/x from the hardware's approximate reciprocal y (relative error e = 1 - x y about 2^-20):
 // 1/x = y / (1 - e) = y (1 + e + e^2 + ..), cut after e^2, so 2^-60 and the rounding: within one
-// unit in the last place of the division.  Three FP64 operations where the full division (430 cycles) is on the factorisation's
-// serial chain.
+// unit in the last place of the division.  Three FP64 operations where the full division (430
+// cycles) is on the factorisation's serial chain.
 __device__ __forceinline__ double recip(double x) {
     const int e = (__double2hiint(x) >> 20) & 0x7ff;
     if (e < 64 || e > 1980) return 1.0 / x;
@@ -772,8 +773,11 @@ static void factor_panel(double* A, long long ld, int n, int k0, int kb, int* fl
 // multiply for longer (18 us) than they take to read out, which 128 do not.
 static void run_fast(double* A, long long ld, int n, double* Linv, double* Uinv, int* flag, int* err, cudaStream_t st) {
     // the scales of up to three products per panel
-    DevBuf<int> scales(3 * (size_t)LU_NB * ceil_div(n, LU_NB), st);
-    scales.zero();
+    DevBuf<int> scales;
+    if (n > HB) {
+        scales.alloc(3 * (size_t)LU_NB * ceil_div(n, LU_NB), st);
+        scales.zero();
+    }
     for (int k0 = 0, b = 0; k0 < n; k0 += LU_NB, ++b) {
         const int kb = std::min(LU_NB, n - k0), n2 = n - k0 - kb, h = std::min(HB, kb), h2 = kb - h;
         double* A11 = A + k0 + k0 * ld;
@@ -886,6 +890,23 @@ static void solve_few(const LU64& lu, int n, double* B, long long ldb, int nrhs,
     }
 }
 
+// Many right-hand sides of a system of one block and few operations: two products with the
+// block's inverses, SK_N columns per CTA, all columns at once.  The digits take 130 us for the
+// two whatever the size.
+static void solve_one_block(const LU64& lu, double* B, long long ldb, int nrhs, cudaStream_t st) {
+    const int n = lu.n;
+    DevBuf<double> X((size_t)n * nrhs, st);
+    auto product = [&](const double* inv, const double* b, long long lb, double* c, long long lc) {
+        for (int j = 0, batch; j < nrhs; j += SK_N * batch) {
+            batch = std::max(1, std::min(65535, (nrhs - j) / SK_N));
+            gemm64_few(false, n, std::min(SK_N, nrhs - j), n, 1.0, inv, LU_NB, b + j * lb, lb, 0.0, c + j * lc, lc, st,
+                       batch, 0, SK_N * lb, SK_N * lc);
+        }
+    };
+    product(lu.Linv.get(), B, ldb, X.get(), n);
+    product(lu.Uinv.get(), X.get(), n, B, ldb);
+}
+
 // Without exchanges the factor of a leading block is the leading block of the factor, and so
 // are the inverses of its diagonal blocks.
 void LU64::solve_leading(int m, double* B, long long ldb, int nrhs, cudaStream_t st) const {
@@ -900,6 +921,7 @@ void LU64::solve(double* B, long long ldb, int nrhs, cudaStream_t st, int* err) 
         for (int c = 0; c < nrhs; c += SK_N) solve_few(*this, n, B + c * ldb, ldb, std::min(SK_N, nrhs - c), st);
         return;
     }
+    if (n <= LU_NB && 2.0 * n * n * nrhs <= PIPE_OPS) return solve_one_block(*this, B, ldb, nrhs, st);
     // many: the block inverses and the updates as tensor-core products
     const int nblk = ceil_div(n, LU_NB);
     DevBuf<int> scales(4 * (size_t)LU_NB * nblk, st);
