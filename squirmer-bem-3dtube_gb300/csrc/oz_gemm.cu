@@ -293,16 +293,30 @@ __global__ void __launch_bounds__(256) oz_split(const double* __restrict__ a, lo
 // and solves): a CTA holds 32 rows' values of all k in shared memory, so each is read
 // from global memory once.  About 90 integer operations per value bound it: with 128
 // rows per CTA a 3840 x 128 panel sat on 30 SMs for 20 us.
+// blockIdx.y: one of two operands.  A and B of a product take one launch, in which the smaller
+// one's CTAs run beside the other's (two launches: level 3 swimmer 21.50 ms, 20.98 with one;
+// n = 700 with 64 right-hand sides 2.58 and 2.39), which pays for the scales' pass.
 constexpr int FUSED_SMEM = FUSED_K * 33 * 8;
-__global__ void __launch_bounds__(256) oz_split_fused(const double* __restrict__ a, long long rs, long long ks, int rows,
-                                                      int k, int k16, int* __restrict__ ex, uint4* __restrict__ out,
-                                                      long long bs, int eb, int rb, const int* __restrict__ q, int sign) {
-    a += blockIdx.z * bs;
-    ex += (long long)blockIdx.z * eb;
-    out += (long long)blockIdx.z * (eb / TILE) * k16 * (BLOCK / 16);
+struct SplitOperand {
+    const double* a;
+    long long rs, ks, bs;
+    int* ex;
+    uint4* out;
+    int rows, eb, rb, sign;
+};
+__global__ void __launch_bounds__(256) oz_split_fused(const __grid_constant__ SplitOperand s0,
+                                                      const __grid_constant__ SplitOperand s1, int k, int k16,
+                                                      const int* __restrict__ q) {
+    const SplitOperand& S = blockIdx.y ? s1 : s0;
+    const long long rs = S.rs, ks = S.ks;
+    const int rows = S.rows, rb = S.rb, sign = S.sign;
+    const double* __restrict__ a = S.a + blockIdx.z * S.bs;
+    int* __restrict__ ex = S.ex + (long long)blockIdx.z * S.eb;
+    uint4* __restrict__ out = S.out + (long long)blockIdx.z * (S.eb / TILE) * k16 * (BLOCK / 16);
     extern __shared__ double xs[];  // [k][33]
     __shared__ int em[32], sk[FUSED_K];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r0 = blockIdx.x * 32;
+    if (r0 >= rows) return;
     const int kp = k16 * 16;
     if (threadIdx.x < 32) em[lane] = 0;
     for (int c = threadIdx.x; c < kp; c += 256) sk[c] = c < k ? shift_at(q, c, sign) : 0;
@@ -861,8 +875,8 @@ static void set_up() {
     });
 }
 
-void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int k_, cudaStream_t st, bool right,
-                  int batch_, long long bs_, const int* q) {
+void OzMat::lay_out(const double* a, long long rs_, long long ks_, int rows_, int k_, cudaStream_t st, bool right_,
+                    int batch_, long long bs_) {
     set_up();
     rows = rows_;
     k = k_;
@@ -872,28 +886,45 @@ void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int 
     rs = rs_;
     ks = ks_;
     bs = bs_;
+    right = right_;
     block = right && k16 <= HI_CHUNK ? 64 : TILE;
+    const int nb = ceil_div(rows, TILE);
+    d.alloc((size_t)batch * nb * k16 * (BLOCK / 16), st);
+    ex.alloc((size_t)batch * nb * TILE, st);
+}
+
+// whether exponents and digits take one launch
+static bool fused(const OzMat& m) { return m.k <= FUSED_K && (m.rs == 1 || m.ks == 1); }
+static SplitOperand operand(const OzMat& m) {
+    return {m.src, m.rs, m.ks, m.bs, m.ex.get(), m.d.get(), m.rows, ceil_div(m.rows, TILE) * TILE, m.block, m.right ? -1 : 1};
+}
+
+void OzMat::split(const double* a, long long rs_, long long ks_, int rows_, int k_, cudaStream_t st, bool right_,
+                  int batch_, long long bs_, const int* q) {
+    lay_out(a, rs_, ks_, rows_, k_, st, right_, batch_, bs_);
+    split_values(q, st);
+}
+
+void OzMat::split_values(const int* q, cudaStream_t st) {
     const int sign = right ? -1 : 1;
     const int nb = ceil_div(rows, TILE), eb = nb * TILE;
-    d.alloc((size_t)batch * nb * k16 * (BLOCK / 16), st);
-    ex.alloc((size_t)batch * eb, st);
-    if (k <= FUSED_K && (rs == 1 || ks == 1)) {
-        LAUNCH(oz_split_fused, dim3(ceil_div(rows, 32), 1, batch), 256, k16 * 16 * 33 * 8, st, a, rs, ks, rows, k, k16,
-               ex.get(), d.get(), bs, eb, block, q, sign);
+    if (fused(*this)) {
+        const SplitOperand s = operand(*this);
+        LAUNCH(oz_split_fused, dim3(ceil_div(rows, 32), 1, batch), 256, k16 * 16 * 33 * 8, st, s, s, k, k16, q);
         return;
     }
     if (ks == 1) {
-        LAUNCH(oz_exponent_cols, dim3(ceil_div(rows, 8), 1, batch), 256, 0, st, a, rs, rows, k, ex.get(), bs, eb, q,
+        LAUNCH(oz_exponent_cols, dim3(ceil_div(rows, 8), 1, batch), 256, 0, st, src, rs, rows, k, ex.get(), bs, eb, q,
                sign);
     } else {
         ex.zero();
         const int kper = 32;
-        LAUNCH(oz_exponent_rows, dim3(nb, ceil_div(k, kper), batch), TILE, 0, st, a, rs, ks, rows, k, kper, ex.get(), bs,
-               eb, q, sign);
+        LAUNCH(oz_exponent_rows, dim3(nb, ceil_div(k, kper), batch), TILE, 0, st, src, rs, ks, rows, k, kper, ex.get(),
+               bs, eb, q, sign);
     }
     // about four CTAs per SM's worth of k16 steps
     const int gy = std::max(1, std::min(k16, 152 * 8 / (nb * batch)));
-    LAUNCH(oz_split, dim3(nb, gy, batch), dim3(TILE, 2), 0, st, a, rs, ks, rows, k, k16, ex.get(), d.get(), bs,
+    LAUNCH(oz_split, dim3(nb, gy, batch), dim3(TILE, 2), 0, st, src, rs, ks, rows, k, k16, ex.get(), d.get(), bs,
            eb, block, q, sign);
 }
 
@@ -971,8 +1002,15 @@ void oz_product(const double* A, long long ars, long long aks, const double* B, 
     }
     oz_scales(B, brs, bks, N, K, q, st);
     OzMat a, b;
-    a.split(A, ars, aks, M, K, st, false, 1, 0, q);
-    b.split(B, brs, bks, N, K, st, true, 1, 0, q);
+    a.lay_out(A, ars, aks, M, K, st, false);
+    b.lay_out(B, brs, bks, N, K, st, true);
+    if (fused(a) && fused(b)) {
+        LAUNCH(oz_split_fused, dim3(ceil_div(std::max(M, N), 32), 2), 256, a.k16 * 16 * 33 * 8, st, operand(a), operand(b), K,
+               a.k16, q);
+    } else {
+        a.split_values(q, st);
+        b.split_values(q, st);
+    }
     oz_gemm(a, b, alpha, beta, C, ldc, err, st);
 }
 

@@ -35,6 +35,7 @@ struct OzMat {
     DevBuf<uint4> d;
     DevBuf<int> ex;
     int rows = 0, k = 0, k16 = 0, batch = 1, block = 128;
+    bool right = false;
     // the values' source, for rows that hold an infinity or a NaN
     const double* src = nullptr;
     long long rs = 0, ks = 0, bs = 0;
@@ -42,6 +43,10 @@ struct OzMat {
     // (blocks of 64 rows then, while k <= 256); q: scales along k (oz_scales), the same for A and B
     void split(const double* a, long long rs, long long ks, int rows, int k, cudaStream_t st, bool right = false,
                int batch = 1, long long bs = 0, const int* q = nullptr);
+    // its two halves: sizes and buffers, then the digits
+    void lay_out(const double* a, long long rs, long long ks, int rows, int k, cudaStream_t st, bool right,
+                 int batch = 1, long long bs = 0);
+    void split_values(const int* q, cudaStream_t st);
 };
 
 // C (M x N, column-major) = alpha A B + beta C for the digits of A (M rows) and of
