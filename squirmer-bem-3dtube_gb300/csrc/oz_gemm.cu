@@ -154,10 +154,10 @@ __global__ void __launch_bounds__(256) oz_scale_fused(const double* __restrict__
 __global__ void __launch_bounds__(128) oz_scale(const double* __restrict__ b, long long rs, long long ks, int rows, int k,
                                                 const int* __restrict__ ex, int* __restrict__ q) {
     if (ks == 1) {
-        const int c = blockIdx.x * 128 + threadIdx.x, r1 = min(rows, (int)(blockIdx.y + 1) * 32);
+        const int c = blockIdx.y * 128 + threadIdx.x, r1 = min(rows, (int)(blockIdx.x + 1) * 32);
         if (c >= k) return;
         int m = 0;
-        for (int r0 = blockIdx.y * 32; r0 < r1; r0 += LOADS) {
+        for (int r0 = blockIdx.x * 32; r0 < r1; r0 += LOADS) {
             double x[LOADS];
 #pragma unroll
             for (int u = 0; u < LOADS; ++u) x[u] = r0 + u < r1 ? b[(r0 + u) * rs + c] : 0.0;
@@ -983,7 +983,7 @@ void oz_scales(const double* B, long long rs, long long ks, int N, int K, int* q
     DevBuf<int> ex(N, st);
     if (ks == 1) {
         LAUNCH(oz_exponent_cols, ceil_div(N, 8), 256, 0, st, B, rs, N, K, ex.get(), 0, 0, nullptr, 0);
-        LAUNCH(oz_scale, dim3(ceil_div(K, 128), ceil_div(N, 32)), 128, 0, st, B, rs, ks, N, K, ex.get(), q);
+        LAUNCH(oz_scale, dim3(ceil_div(N, 32), ceil_div(K, 128)), 128, 0, st, B, rs, ks, N, K, ex.get(), q);
     } else {
         ex.zero();
         LAUNCH(oz_exponent_rows, dim3(ceil_div(N, TILE), ceil_div(K, 32)), TILE, 0, st, B, rs, ks, N, K, 32, ex.get(), 0,
