@@ -483,7 +483,7 @@ def main():
         if not top:
             return None
         nl, secs, fl, by = st[top]
-        if top == "tc_gemm":
+        if top in ("tc_gemm", "oz_gemm"):
             achieved, peak, unit, bound, src = fl / secs / 1e12, peaks["bf16_tflops"], "TFLOP/s", "tensor", \
                 peaks["source"]
         elif top in ("dgemm", "assemble_near"):
