@@ -1112,8 +1112,8 @@ void panel_pairs(int n, const PanelRec* P, const double* x0, const int* self, do
 // u_j(x0) = sum_p [SL_p,ij f_p,i / (8 pi mu) - DL_p,ij u_p,i / (8 pi)]  (field.hpp:18-34)
 //
 // The lanes of a warp take panels, a warp PPW points (so that a staged panel serves
-// several), or, for few points, the eight warps of a CTA (and the CTAs of a cluster)
-// one point.  Pass 1 applies the 7-point rule to far panels while near ones (d < 3) are
+// several), or, for few points, two, four or the eight warps of a CTA (and the CTAs of a
+// cluster) one point.  Pass 1 applies the 7-point rule to far panels while near ones (d < 3) are
 // collected, in panel order, in shared memory; in pass 2 the warp integrates each near
 // panel, its lanes splitting the rule's points.  Fixed order, hence deterministic.
 //
@@ -1370,10 +1370,14 @@ __device__ void field_near(const FieldJob& job, int p, int rule, const FieldPoin
     u += v;
 }
 
-// PPW points per warp, each warp all panels; or (SHARED) one point per CTA -- per
-// cluster -- whose warps and CTAs share the panels.
-template <class TC, int PPW, bool SHARED>
+// PPW points per warp, each warp all panels (G = 1); or G warps per point, the CTAs of a cluster one
+// point together where G = 8.  They share the panels: the CTAs every cluster-size-th one, so that near
+// panels, which are neighbours, go to all of them; the warps 32 at a time (a warp costs the same
+// with one lane as with all) and then, in turn, the entries of all their near lists.
+template <class TC, int PPW, int G>
 __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job) {
+    constexpr bool SHARED = G > 1, ALL = G == FIELD_WARPS;
+    static_assert(!SHARED || PPW == 1, "shared points have warps of their own");
     constexpr int TP = SHARED ? 256 : 128;  // panels per tile
     constexpr int W = FieldArith<TC>::WORDS;
     extern __shared__ __align__(16) unsigned char field_smem[];
@@ -1386,8 +1390,9 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
     __shared__ int clnear;
     cg::cluster_group cl = cg::this_cluster();
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const int ncl = SHARED ? (int)cl.num_blocks() : 1, rank = SHARED ? (int)cl.block_rank() : 0;
-    const int pt0 = SHARED ? blockIdx.x / ncl : (blockIdx.x * FIELD_WARPS + wl) * PPW;
+    const int ncl = ALL ? (int)cl.num_blocks() : 1, rank = ALL ? (int)cl.block_rank() : 0;
+    const int sub = wl % G;  // of the point's warps
+    const int pt0 = ALL ? blockIdx.x / ncl : (blockIdx.x * FIELD_WARPS + wl) / G * PPW;
     FieldPoint X[PPW];
     FieldArith<TC> F[PPW];
 #pragma unroll
@@ -1402,14 +1407,8 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
     // lane 3 k + c: component c of point k, for the offsets from a tile's origin
     const double xc = lane < 3 * PPW ? job.pts[3LL * min(pt0 + lane / 3, job.npts - 1) + lane % 3] : 0.0;
     int* const list = lists + wl * PPW * FIELD_NEAR_CAP;
-    // SHARED: consecutive panels go to different CTAs and warps, so that the near ones, which are
-    // neighbours, are shared out too (by whole tiles one warp had them all: 200 us for 60
-    // points)
-    auto index = [&](int base, int q) {
-        return SHARED ? base + (q & 31) * (FIELD_WARPS * ncl) + (q >> 5) * ncl + rank : base + q;
-    };
     for (int base = 0; base < job.P; base += ncl * TP) {
-        const int mine = index(base, threadIdx.x);
+        const int mine = base + (int)threadIdx.x * ncl + rank;
         const bool has = (int)threadIdx.x < TP && mine < job.P;
         __syncthreads();
         if (threadIdx.x == 0) tex = twide = 0;
@@ -1422,10 +1421,10 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
         const int ex = tex;
         // the origin of a tile's lengths: a vertex of its first panel (no point, which may be
         // anything, has a say in another's result), or the one point of the CTA
-        const double* const o = SHARED ? job.pts + 3LL * pt0 : job.panels[base].v;
+        const double* const o = ALL ? job.pts + 3LL * pt0 : job.panels[base].v;
         if (has && FieldArith<TC>::stage(tile + threadIdx.x * W, job, mine, o, ex)) twide = 1;
         __syncthreads();
-        const bool wide = !SHARED && twide != 0;
+        const bool wide = !ALL && twide != 0;
         if (sizeof(TC) == 4) {
             float hi, lo;
             split2(xc - o[lane % 3], hi, lo);
@@ -1437,8 +1436,8 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
         }
 #pragma unroll
         for (int k = 0; k < PPW; ++k) F[k].begin();
-        for (int s = SHARED ? wl * 32 : 0; s < (SHARED ? wl * 32 + 32 : min(TP, job.P - base)); s += 32) {
-            const int q = s + lane, p = index(base, q);
+        for (int s = sub * 32; s < TP && base + s * ncl + rank < job.P; s += 32 * G) {
+            const int q = s + lane, p = base + q * ncl + rank;
 #pragma unroll
             for (int k = 0; k < PPW; ++k) {
                 int rule = 0;
@@ -1455,7 +1454,12 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
 #pragma unroll
         for (int k = 0; k < PPW; ++k) F[k].flush(X[k], scale);
     }
-    __syncwarp();
+    if (SHARED) {
+        if (lane == 0) pnear[wl] = X[0].near;
+        __syncthreads();
+    } else {
+        __syncwarp();
+    }
 #pragma unroll
     for (int k = 0; k < PPW; ++k) {
         // the far part: warp sums (fixed butterfly order), component j to lane j
@@ -1464,24 +1468,39 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) X[k].u[j] += __shfl_xor_sync(0xffffffffu, X[k].u[j], d);
         double u = lane == 0 ? X[k].u[0] : lane == 1 ? X[k].u[1] : X[k].u[2];
-        const int nn = min(X[k].near, FIELD_NEAR_CAP);
         double t = 0.0;
-        if (SHARED || pt0 + k < job.npts)
-            for (int n = 0; n < nn; ++n) {
-                const int e = list[k * FIELD_NEAR_CAP + n];
-                field_near<sizeof(TC) == 4>(job, e & 0x0fffffff, e >> 28, X[k], lane, u, t);
+        auto near = [&](int e) { field_near<sizeof(TC) == 4>(job, e & 0x0fffffff, e >> 28, X[k], lane, u, t); };
+        if (SHARED) {
+            for (int w = 0, first = sub; pt0 < job.npts && w < G; ++w) {  // first: of this warp's in list w
+                const int c = min(pnear[wl - sub + w], FIELD_NEAR_CAP);
+                for (; first < c; first += G) near(lists[(wl - sub + w) * FIELD_NEAR_CAP + first]);
+                first -= c;
             }
+        } else if (pt0 + k < job.npts) {
+            const int nn = min(X[k].near, FIELD_NEAR_CAP);
+            for (int n = 0; n < nn; ++n) near(list[k * FIELD_NEAR_CAP + n]);
+        }
         if (sizeof(TC) == 4) u += t + __shfl_down_sync(0xffffffffu, t, 3) + __shfl_down_sync(0xffffffffu, t, 6);
         if (!SHARED && pt0 + k < job.npts) {
             if (lane < 3) job.out[3 * (pt0 + k) + lane] = u;
             if (lane == 0 && X[k].near > FIELD_NEAR_CAP) atomicExch(job.overflow, 1);
         }
-        if (SHARED) {
-            if (lane < 3) part[wl][lane] = u;
-            if (lane == 0) pnear[wl] = X[k].near;
+        if (SHARED && lane < 3) part[wl][lane] = u;
+    }
+    if (SHARED && !ALL) {
+        __syncthreads();
+        if (sub == 0 && lane < 4 && pt0 < job.npts) {
+            double u = 0.0;
+            int n = 0;
+            for (int w = wl; w < wl + G; ++w) {
+                if (lane < 3) u += part[w][lane];
+                else n += pnear[w];
+            }
+            if (lane < 3) job.out[3 * pt0 + lane] = u;
+            else if (n > FIELD_NEAR_CAP) atomicExch(job.overflow, 1);
         }
     }
-    if (SHARED) {
+    if (ALL) {
         __syncthreads();
         if (threadIdx.x < 3) {
             double u = 0.0;
@@ -1518,19 +1537,19 @@ void rsqrt_nr_eval(int n, const double* x, double* y, cudaStream_t st) {
 }
 
 namespace {
-template <class TC, int PPW, bool SHARED>
+template <class TC, int PPW, int G>
 void field_launch(const FieldJob& job, int cluster, cudaStream_t st) {
-    constexpr int TP = SHARED ? 256 : 128;
+    constexpr int TP = G > 1 ? 256 : 128;
     constexpr size_t smem =
         sizeof(TC) * TP * FieldArith<TC>::WORDS + sizeof(int) * FIELD_WARPS * PPW * FIELD_NEAR_CAP;
     static std::once_flag once;
     std::call_once(once, [] {
-        CUDA_CHECK(cudaFuncSetAttribute((const void*)field_kernel<TC, PPW, SHARED>,
+        CUDA_CHECK(cudaFuncSetAttribute((const void*)field_kernel<TC, PPW, G>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     });
     cudaLaunchConfig_t c = {};
     cudaLaunchAttribute at[1];
-    c.gridDim = dim3(SHARED ? (unsigned)job.npts * cluster : (unsigned)ceil_div(job.npts, FIELD_WARPS * PPW));
+    c.gridDim = dim3((unsigned)ceil_div(job.npts, FIELD_WARPS / G * PPW) * cluster);
     c.blockDim = dim3(FIELD_WARPS * 32);
     c.dynamicSmemBytes = smem;
     c.stream = st;
@@ -1539,18 +1558,32 @@ void field_launch(const FieldJob& job, int cluster, cudaStream_t st) {
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     c.attrs = at;
     c.numAttrs = 1;
-    CUDA_CHECK(cudaLaunchKernelEx(&c, field_kernel<TC, PPW, SHARED>, job));
+    CUDA_CHECK(cudaLaunchKernelEx(&c, field_kernel<TC, PPW, G>, job));
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-// Four points per warp once every SM has its 32 points; below that one per warp, and a few
-// points share a CTA or a cluster of four or eight each, which costs staging every panel
-// per point.
+// Four points per warp once every SM has its 32 points, one per warp once it has eight.  Below that
+// fewer points per CTA, with more warps each: staging the panels costs a CTA as much as eight (mixed)
+// points' far panels or one's (FP64), so four or two points share it while every SM has a CTA, and
+// then one point's warps, or the CTAs of a cluster, share its near panels.  The lines follow the
+// whole rounds of the 152 SMs; in FP64, where the near panels weigh more than the staging, two CTAs
+// per point also fill the ends of such rounds (with few panels they have too little to share).
+// Whole calls, us, points in the duct / far away from it (120 of them are the call's own):
+//   1680 panels, 1200 points, mixed: 445 / 334 (a CTA per point: 967 / 818; one warp: 491 / 307)
+//   1680 panels,  300 points, FP64: 535 / 387 (four CTAs per point: 661 / 540; one warp: 1447 / 940)
+//     56 panels,  300 points, FP64: - / 121 (four CTAs per point, 32 panels of a tile to each: 307; a warp
+//                                   per point and nothing staged: 142)
 template <class TC>
 void field_dispatch(const FieldJob& job, cudaStream_t st) {
-    if (job.npts >= 152 * FIELD_WARPS * 4) field_launch<TC, 4, false>(job, 1, st);
-    else if (job.npts >= 152 * FIELD_WARPS) field_launch<TC, 1, false>(job, 1, st);
-    else field_launch<TC, 1, true>(job, job.npts < 152 ? 8 : job.npts < 152 * 2 ? 4 : 1, st);
+    const int n = job.npts;
+    const bool fp64 = sizeof(TC) == 8;
+    if (n >= 152 * FIELD_WARPS * 4) field_launch<TC, 4, 1>(job, 1, st);
+    else if (n >= 152 * FIELD_WARPS) field_launch<TC, 1, 1>(job, 1, st);
+    else if (n <= 38) field_launch<TC, 1, 8>(job, 8, st);
+    else if (n <= 76 || (n <= 114 && job.P >= 1024)) field_launch<TC, 1, 8>(job, 4, st);
+    else if (n <= 152 || (fp64 && job.P >= 64 && (n <= 228 || (n > 304 && n <= 456)))) field_launch<TC, 1, 8>(job, 2, st);
+    else if (n <= 304 || (fp64 && n > 608 && n <= 912)) field_launch<TC, 1, 4>(job, 1, st);
+    else field_launch<TC, 1, 2>(job, 1, st);
 }
 }  // namespace
 
