@@ -18,7 +18,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <map>
 #include <mutex>
 #include <vector>
 
@@ -1083,40 +1082,43 @@ __global__ void __launch_bounds__(TW_THREADS) trsv_wide_kernel(const __grid_cons
 }
 
 namespace {
-// Whether m members of order n go through trsv_wide_kernel: clusters of 16 take most of a GPC
-// each, so up to 8 members; beyond that the narrow clusters fill the GPU.  The GPU has to
-// place such a cluster at all (asked once per size).
+// Whether the GPU holds m members' clusters of 16 at once, an SM to each CTA (it is asked once;
+// seven).  With one more, or with two CTAs on an SM, some wait for the others: eight members of
+// order 3840 took 485 us for two columns, 417 on the narrow clusters.
 bool trsv_wide_fits(int n, int m) {
-    if (m > 8 || trsv_wide_smem(n) > 227 * 1024) return false;
-    static std::mutex mu;
-    static std::map<int, bool> known;
-    static bool usable = true;
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = known.find(n);
-    if (it != known.end()) return it->second;
-    if (known.empty())
-        usable = cudaFuncSetAttribute(trsv_wide_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                 cudaFuncSetAttribute(trsv_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) ==
-                     cudaSuccess;
-    cudaLaunchConfig_t c = {};
-    cudaLaunchAttribute at[1];
-    c.gridDim = dim3(TW_CL);
-    c.blockDim = dim3(TW_THREADS);
-    c.dynamicSmemBytes = trsv_wide_smem(n);
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = TW_CL;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    c.attrs = at;
-    c.numAttrs = 1;
-    int clusters = 0;
-    const bool ok = usable && cudaOccupancyMaxActiveClusters(&clusters, trsv_wide_kernel, &c) == cudaSuccess && clusters > 0;
-    (void)cudaGetLastError();
-    known[n] = ok;
-    return ok;
+    static int clusters = 0;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        if (cudaFuncSetAttribute(trsv_wide_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaFuncSetAttribute(trsv_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess) {
+            cudaLaunchConfig_t c = {};
+            cudaLaunchAttribute at[1];
+            c.gridDim = dim3(TW_CL);
+            c.blockDim = dim3(TW_THREADS);
+            c.dynamicSmemBytes = 227 * 1024;
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = TW_CL;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            c.attrs = at;
+            c.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&clusters, trsv_wide_kernel, &c) != cudaSuccess) clusters = 0;
+        }
+        (void)cudaGetLastError();
+    });
+    return m <= clusters && trsv_wide_smem(n) <= 227 * 1024;
+}
+
+// Whether r columns go through the wide clusters, two at a time, rather than through the narrow
+// ones, two or (eight: they fit) up to eight at once.  us per launch, wide / narrow two / narrow
+// eight: order 256 16 / 14 / 28, 1024 51 / 54 / 128, 3840 238 / 417 / 860.
+bool trsv_wide_pays(int n, int r, bool eight) {
+    if (!eight) return n >= 896;
+    return r <= 4 ? n >= 640 : r <= 6 && n >= 2304;
 }
 
 template <int R>
-void trsv_launch(const std::vector<const MixedLU*>& g, const std::vector<TrsvIO>& io, int c0, int r, cudaStream_t st) {
+void trsv_launch(const std::vector<const MixedLU*>& g, const std::vector<TrsvIO>& io, int c0, int r, bool wide,
+                 cudaStream_t st) {
     const int n = g[0]->n;
     const size_t smem = trsv_smem(n, R);
     static std::once_flag attr;
@@ -1135,7 +1137,7 @@ void trsv_launch(const std::vector<const MixedLU*>& g, const std::vector<TrsvIO>
                       q.out + (long long)c0 * q.ldo, q.ldo, q.n_true};
         }
         const double by = (double)m * ((double)n * n * 4.0 + 2.0 * n * r * 8.0);
-        if (R == 2 && trsv_wide_fits(n, m)) {
+        if (R == 2 && wide) {
             cudaLaunchConfig_t c = {};
             cudaLaunchAttribute at[1];
             c.gridDim = dim3((unsigned)(m * TW_CL));
@@ -1168,13 +1170,13 @@ void trsv_group_io(const std::vector<const MixedLU*>& g, const std::vector<TrsvI
         if (nt < 1 || nt > n || io[k].ldi < nt || io[k].ldo < nt) fail(SQBEM_ERR_ARG, "trsv: bad row count");
     }
     if (trsv_smem(n, 2) > 227 * 1024) fail(SQBEM_ERR_ARG, "trsv: %d unknowns exceed shared memory", n);
-    // eight columns at once, or (few members) two at a time on wide clusters: 3840 unknowns and six
-    // columns took 860 us at once
-    if (r > 2 && trsv_smem(n, 8) <= 227 * 1024 && !trsv_wide_fits(n, (int)g.size())) {
-        trsv_launch<8>(g, io, 0, r, st);
+    const bool eight = r > 2 && trsv_smem(n, 8) <= 227 * 1024;
+    const bool wide = trsv_wide_pays(n, r, eight) && trsv_wide_fits(n, (int)g.size());
+    if (eight && !wide) {
+        trsv_launch<8>(g, io, 0, r, false, st);
         return;
     }
-    for (int c0 = 0; c0 < r; c0 += 2) trsv_launch<2>(g, io, c0, std::min(2, r - c0), st);
+    for (int c0 = 0; c0 < r; c0 += 2) trsv_launch<2>(g, io, c0, std::min(2, r - c0), wide, st);
 }
 
 void trsv_group(const std::vector<const MixedLU*>& g, const std::vector<const double*>& in,
