@@ -1406,6 +1406,21 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
     }
     // lane 3 k + c: component c of point k, for the offsets from a tile's origin
     const double xc = lane < 3 * PPW ? job.pts[3LL * min(pt0 + lane / 3, job.npts - 1) + lane % 3] : 0.0;
+    // the origin of the staged lengths: a vertex of the first panel (no point, which may be
+    // anything, has a say in another's result), or the one point of the CTA
+    const double* o;
+    auto set_origin = [&](const double* v) {
+        o = v;
+        if (sizeof(TC) != 4) return;
+        float hi, lo;
+        split2(xc - o[lane % 3], hi, lo);
+#pragma unroll
+        for (int k = 0; k < PPW; ++k)
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                F[k].offset(c, __shfl_sync(0xffffffffu, hi, 3 * k + c), __shfl_sync(0xffffffffu, lo, 3 * k + c));
+    };
+    set_origin(ALL ? job.pts + 3LL * pt0 : job.panels[0].v);
     int* const list = lists + wl * PPW * FIELD_NEAR_CAP;
     for (int base = 0; base < job.P; base += ncl * TP) {
         const int mine = base + (int)threadIdx.x * ncl + rank;
@@ -1419,20 +1434,17 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
         }
         __syncthreads();
         const int ex = tex;
-        // the origin of a tile's lengths: a vertex of its first panel (no point, which may be
-        // anything, has a say in another's result), or the one point of the CTA
-        const double* const o = ALL ? job.pts + 3LL * pt0 : job.panels[base].v;
         if (has && FieldArith<TC>::stage(tile + threadIdx.x * W, job, mine, o, ex)) twide = 1;
         __syncthreads();
-        const bool wide = !ALL && twide != 0;
-        if (sizeof(TC) == 4) {
-            float hi, lo;
-            split2(xc - o[lane % 3], hi, lo);
-#pragma unroll
-            for (int k = 0; k < PPW; ++k)
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    F[k].offset(c, __shfl_sync(0xffffffffu, hi, 3 * k + c), __shfl_sync(0xffffffffu, lo, 3 * k + c));
+        bool wide = !ALL && twide != 0;
+        if (wide && o != job.panels[base].v) {  // too far from the origin: once more from its own first panel
+            __syncthreads();
+            if (threadIdx.x == 0) twide = 0;
+            set_origin(job.panels[base].v);
+            __syncthreads();
+            if (has && FieldArith<TC>::stage(tile + threadIdx.x * W, job, mine, o, ex)) twide = 1;
+            __syncthreads();
+            wide = twide != 0;
         }
 #pragma unroll
         for (int k = 0; k < PPW; ++k) F[k].begin();
