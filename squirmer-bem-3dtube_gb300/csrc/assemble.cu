@@ -1149,6 +1149,39 @@ struct FieldPoint {
     int near;
 };
 
+// A panel's far share of a point's velocity in mixed precision from the FP64 coordinates and values, for
+// tiles with an infinity or a NaN among f and u, or with panels far apart; nonzero rule: not far.
+// Not inlined: the pair loop, which the instruction cache does not hold, does without its code.
+struct FarShare {
+    int rule;
+    double u[3];
+};
+__device__ __noinline__ FarShare far_share(const PanelRec* P, const double* f, const double* u, double sscale,
+                                           double dscale, double x, double y, double z) {
+    FarShare r;
+    r.rule = rule_of(*P, x, y, z);
+    r.u[0] = r.u[1] = r.u[2] = 0.0;
+    if (r.rule != 0) return r;
+    float e[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) e[k] = (float)(P->v[k] - (k % 3 == 0 ? x : k % 3 == 1 ? y : z));
+    const float mx = (float)P->n[0], my = (float)P->n[1], mz = (float)P->n[2], area = (float)P->area;
+    Acc<float> A;
+    A.zero();
+#pragma unroll 1
+    for (int q = 0; q < 7; ++q) {
+        const float l0 = c_rule7f[q].l0, l1 = c_rule7f[q].l1, l2 = c_rule7f[q].l2, w = c_rule7f[q].w;
+        accum<float, true>(A, l0 * e[0] + l1 * e[3] + l2 * e[6], l0 * e[1] + l1 * e[4] + l2 * e[7],
+                           l0 * e[2] + l1 * e[5] + l2 * e[8], w * area, mx, my, mz);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            r.u[j] += (double)sl_entry(A, i, j) * f[i] * sscale + (double)dl_entry(A, i, j) * u[i] * dscale;
+    return r;
+}
+
 // The panel-independent state of a point and its far sum over the panels of a tile, for both
 // arithmetics: stage() writes one panel's record, pair() returns the rule and adds the
 // panel if it is far, flush() moves the tile's sum to FP64.
@@ -1182,7 +1215,7 @@ struct FieldArith<double> {
     double a[3];
     __device__ void offset(int, double, double) {}
     __device__ void begin() { a[0] = a[1] = a[2] = 0.0; }
-    __device__ int pair(const double* d, const FieldJob& job, int p, const FieldPoint& X, bool, bool) {
+    __device__ int pair(const double* d, const FieldJob& job, int p, const FieldPoint& X) {
         const double bx = d[24] - X.x, by = d[25] - X.y, bz = d[26] - X.z;
         // within 1e-12 of the threshold and below: the exact test
         if (!(bx * bx + by * by + bz * bz > d[27])) {
@@ -1261,15 +1294,13 @@ struct FieldArith<float> {
 #pragma unroll
         for (int k = 0; k < 3; ++k) s[k] = c[k] = 0.f;
     }
-    // wide: the offsets from the FP64 coordinates
-    __device__ int pair(const float* d, const FieldJob& job, int p, FieldPoint& X, bool special, bool wide) {
+    __device__ int pair(const float* d, const FieldJob& job, int p, const FieldPoint& X) {
         const float bx = (d[22] - xh[0]) + (d[25] - xl[0]), by = (d[23] - xh[1]) + (d[26] - xl[1]),
                     bz = (d[24] - xh[2]) + (d[27] - xl[2]);
         const float d2 = bx * bx + by * by + bz * bz;
-        if (wide || !(d2 > d[33])) {
+        if (!(d2 > d[33])) {
             int rule;
-            if (wide) rule = rule_of(job.panels[p], X.x, X.y, X.z);
-            else if (d2 < d[30] && d2 > d[32]) rule = 1;
+            if (d2 < d[30] && d2 > d[32]) rule = 1;
             else if (d2 < d[29] && d2 > d[31]) rule = 2;
             else if (d2 < d[28]) rule = 3;
             else rule = rule_of(job.panels[p], X.x, X.y, X.z);
@@ -1282,10 +1313,6 @@ struct FieldArith<float> {
             two_diff(d[k], xh[k % 3], hi, lo);
             e[k] = __fadd_rn(hi, __fadd_rn(lo, __fsub_rn(d[9 + k], xl[k % 3])));
         }
-        if (wide) {
-#pragma unroll
-            for (int k = 0; k < 9; ++k) e[k] = (float)(job.panels[p].v[k] - (k % 3 == 0 ? X.x : k % 3 == 1 ? X.y : X.z));
-        }
         Acc<float> A;
         A.zero();
         const float mx = d[18], my = d[19], mz = d[20], area = d[21];
@@ -1294,15 +1321,6 @@ struct FieldArith<float> {
             const float l0 = c_rule7f[q].l0, l1 = c_rule7f[q].l1, l2 = c_rule7f[q].l2, w = c_rule7f[q].w;
             accum<float, true>(A, l0 * e[0] + l1 * e[3] + l2 * e[6], l0 * e[1] + l1 * e[4] + l2 * e[7],
                                l0 * e[2] + l1 * e[5] + l2 * e[8], w * area, mx, my, mz);
-        }
-        if (special) {  // an infinity or a NaN among the tile's f and u: plain products
-#pragma unroll
-            for (int j = 0; j < 3; ++j)
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-                    X.u[j] += (double)sl_entry(A, i, j) * job.f[3 * p + i] * job.sscale +
-                              (double)dl_entry(A, i, j) * job.u[3 * p + i] * job.dscale;
-            return 0;
         }
 #pragma unroll
         for (int j = 0; j < 3; ++j)
@@ -1446,20 +1464,33 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
             __syncthreads();
             wide = twide != 0;
         }
+        const bool plain = sizeof(TC) == 4 && (wide || ex == 0x7ff);
 #pragma unroll
         for (int k = 0; k < PPW; ++k) F[k].begin();
-        for (int s = sub * 32; s < TP && base + s * ncl + rank < job.P; s += 32 * G) {
+        auto append = [&](int k, int p, int rule) {
+            const unsigned m = __ballot_sync(0xffffffffu, rule > 0);
+            if (rule > 0) {
+                const int slot = X[k].near + __popc(m & ((1u << lane) - 1));
+                if (slot < FIELD_NEAR_CAP) list[k * FIELD_NEAR_CAP + slot] = p | (rule << 28);
+            }
+            X[k].near += __popc(m);
+        };
+        for (int s = sub * 32; !plain && s < TP && base + s * ncl + rank < job.P; s += 32 * G) {
             const int q = s + lane, p = base + q * ncl + rank;
 #pragma unroll
+            for (int k = 0; k < PPW; ++k) append(k, p, p < job.P ? F[k].pair(tile + q * W, job, p, X[k]) : 0);
+        }
+#pragma unroll 1
+        for (int s = sub * 32; plain && s < TP && base + s * ncl + rank < job.P; s += 32 * G) {
+            const int p = base + (s + lane) * ncl + rank;
+#pragma unroll
             for (int k = 0; k < PPW; ++k) {
-                int rule = 0;
-                if (p < job.P) rule = F[k].pair(tile + q * W, job, p, X[k], ex == 0x7ff, wide);
-                const unsigned m = __ballot_sync(0xffffffffu, rule > 0);
-                if (rule > 0) {
-                    const int slot = X[k].near + __popc(m & ((1u << lane) - 1));
-                    if (slot < FIELD_NEAR_CAP) list[k * FIELD_NEAR_CAP + slot] = p | (rule << 28);
-                }
-                X[k].near += __popc(m);
+                FarShare r = {};
+                if (p < job.P)
+                    r = far_share(job.panels + p, job.f + 3 * p, job.u + 3 * p, job.sscale, job.dscale, X[k].x, X[k].y, X[k].z);
+#pragma unroll
+                for (int j = 0; j < 3; ++j) X[k].u[j] += r.u[j];
+                append(k, p, r.rule);
             }
         }
         const double scale = ex > 0 && ex < 0x7ff ? scalbn(1.0, ex - 1023) : 1.0;
