@@ -1438,7 +1438,7 @@ __global__ void __launch_bounds__(FIELD_WARPS * 32, 2) field_kernel(FieldJob job
             for (int c = 0; c < 3; ++c)
                 F[k].offset(c, __shfl_sync(0xffffffffu, hi, 3 * k + c), __shfl_sync(0xffffffffu, lo, 3 * k + c));
     };
-    set_origin(ALL ? job.pts + 3LL * pt0 : job.panels[0].v);
+    set_origin(ALL ? job.pts + 3LL * pt0 : job.P > 0 ? job.panels[0].v : job.pts);
     int* const list = lists + wl * PPW * FIELD_NEAR_CAP;
     for (int base = 0; base < job.P; base += ncl * TP) {
         const int mine = base + (int)threadIdx.x * ncl + rank;

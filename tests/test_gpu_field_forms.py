@@ -77,3 +77,11 @@ def test_more_near_panels_than_the_list_holds_is_an_error():
     for n in (5, 60, 120, 250, 400, 500, 700, 1000, 1300, 4900):
         with pytest.raises(sqbem.BEMError):
             sqbem.velocity_at(crowd, u, u, 1.0, np.repeat(p, n, 0))
+
+
+@pytest.mark.parametrize("n", [1, 60, 120, 200, 250, 400, 500, 700, 1000, 1300, 4900])
+@pytest.mark.parametrize("precision", [sqbem.FP64, sqbem.MIXED])
+def test_no_panels_no_velocity(n, precision):
+    m = sqbem.Mesh(np.zeros((0, 9)), np.zeros(0, int))
+    got = sqbem.velocity_at(m, np.zeros((0, 3)), np.zeros((0, 3)), 1.0, points(n, False), precision)
+    np.testing.assert_array_equal(got, np.zeros((n, 3)))
